@@ -171,6 +171,55 @@ def test_gemm_simt_rows_do_not_depend_on_the_batch(ops):
     assert torch.equal(full[37:38], one)
 
 
+# (M, N, K): edges of the tiles of 16 to 128 rows and of 128 weight rows, one K block and several chunks of 8, rows that are not whole
+# groups of 8
+F32_SHAPES = [(1, 128, 64), (16, 129, 512), (17, 200, 520), (33, 127, 1100), (64, 256, 1544), (65, 130, 2049), (129, 384, 1023),
+              (200, 72, 640)]
+
+
+@pytest.mark.parametrize("M,N,K", F32_SHAPES)
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
+                                     (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+def test_gemm_f32_in_every_tile_width_and_sharing_of_k(ops, M, N, K, adt, wdt):
+    """Every plan gives the same bits, and sums as exact as float32 allows: a chunk of 512 products is cut off 8 x 4 times a
+    level, 32 x 2^-24 of its size at most, and the chunks add roundings of 2^-24 each."""
+    a, w, res = g((M, K), adt, 15).to(DEV), g((N, K), wdt, 16, 0.05).to(DEV), g((M, N), torch.float32, 17).to(DEV)
+    want = a.double() @ w.double().t() + res.double()
+    bound = 48 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + res.double().abs())
+    chunks = -(-(-(-K // 64)) // 8)
+    first = None
+    for bn in (16, 32, 64, 128):
+        for slices in {1, chunks}:
+            out = res.clone()
+            ops.gemm_simt(a, w, out, out, plan=bn | (slices << 16))
+            assert bool(((out.double() - want).abs() <= bound).all()), (bn, slices)
+            first = out if first is None else first
+            assert torch.equal(out, first), (bn, slices)
+    row = torch.empty(1, N, device=DEV)                      # a row alone, at an address that need not suit wide loads
+    r = M - 1
+    ops.gemm_simt(a[r:], w, row, res[r:].contiguous())
+    assert torch.equal(row, first[r:])
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("slices", [1, 3])
+def test_gemm_f32_infinities_and_overflow(ops, slices):
+    """Infinities, NaN and sums beyond the range come out as a plain sum of products gives them."""
+    a, w = g((20, 1300), torch.float32, 18).to(DEV), g((140, 1300), torch.float32, 19, 0.05).to(DEV)
+    a[3, 7], a[5, 9], a[6, 0], w[100, 1299] = math.inf, math.nan, 3e38, -math.inf
+    w[:, 0] = 1.5
+    want = a.double() @ w.double().t()
+    out = torch.empty(20, 140, device=DEV)
+    ops.gemm_simt(a, w, out, plan=32 | (slices << 16))
+    big = want.abs() > 3.4028235e38                          # beyond float32
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.isposinf(), want.isposinf() | (big & (want > 0)))
+    assert torch.equal(out.isneginf(), want.isneginf() | (big & (want < 0)))
+    fine = torch.isfinite(out)
+    assert float(((out.double() - want)[fine] / want[fine].abs().clamp_min(1)).abs().max()) < 1e-5
+    ops.check_errors()
+
+
 TC_SHAPES = [(1, 128, 64), (8, 6144, 4096), (5, 311, 80), (16, 256, 128), (17, 384, 200), (64, 4096, 1024),
              (100, 1000, 512), (256, 512, 4096), (257, 512, 256), (300, 311, 264), (1024, 768, 512),
              (2048, 4096, 4096), (128, 128, 8), (130, 6144, 4096), (300, 1000, 264), (513, 1256, 72)]
