@@ -511,6 +511,54 @@ def test_flash_attention_bf16(ops, case):
     assert rel_err(out, gen) < 1e-2
 
 
+@pytest.mark.parametrize("nq,nkv,d,new,old,window,keep", [
+    (32, 8, 128, [1, 1, 1], [300, 127, 1100], 0, 0),           # 4 rows a tile
+    (8, 1, 48, [1, 2], [128, 255], 0, 0),                      # 8 and 16 rows, a head of 48
+    (4, 2, 17, [3, 1], [130, 0], 0, 0),                        # a head that is no whole group of 4
+    (8, 2, 256, [1, 4], [500, 63], 0, 0),                      # 2 groups of columns a lane
+    (2, 2, 512, [5, 1], [200, 700], 0, 0),                     # 4 groups, one stage of keys
+    (8, 2, 128, [1, 7], [900, 400], 150, 0),                   # a window: chunks ahead of it are not walked
+    (8, 2, 80, [1, 2], [900, 400], 100, 40),                   # ... and first keys that stay
+])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_float32_attention_does_not_depend_on_how_the_keys_are_shared_out(ops, dt, nq, nkv, d, new, old, window, keep):
+    """One CTA for all chunks of keys, and shares of them joined by the second kernel, give the same bits; so does a token in a
+    step of its own.  A later token's NaN value does not reach the tokens ahead of it."""
+    page = 16
+    entries, tables, cache, qkv = _paged_case(nq, nkv, d, page, new, old, window, dt, seed=75, layers=2)
+    T = sum(new)
+    q = qkv[:, :nq * d].contiguous()
+    cache = cache.clone()
+    n, o = new[-1], old[-1]
+    if n > 1:                                                  # the last request's last token: its value
+        cache[tables[-1][(o + n - 1) // page], 1, 1, :, (o + n - 1) % page] = float("nan")
+    bc = build_step_batch(entries, old, list(range(len(new))), [tables], "cpu")
+    bg = build_step_batch(entries, old, list(range(len(new))), [tables], DEV)
+    args = (bg.block_tables[0], cache.to(DEV), 1, page)
+    outs = []
+    for shares in (1, 2, 5):
+        slots = -(-(max(new) + max(old)) // 128) + 1
+        out = torch.full((T, nq * d), float("nan"), dtype=dt, device=DEV)
+        ops._attention_generic_launch(q.to(DEV), bg, *args, out, nq, nkv, d, d, 1 / math.sqrt(d), window, keep=keep,
+                                      plan=shares | ((slots << 16) if shares > 1 else 0))
+        outs.append(out)
+    assert torch.equal(outs[0].nan_to_num(7.0), outs[1].nan_to_num(7.0)) and torch.equal(outs[0].nan_to_num(7.0), outs[2].nan_to_num(7.0))
+    rows = T if n == 1 else T - 1
+    want = torch.empty(T, nq * d, dtype=dt)
+    if keep == 0:
+        CpuOps().attention(q, bc, bc.block_tables[0], cache.nan_to_num(0.0), 1, page, want, nq, nkv, d, 1 / math.sqrt(d), window)
+        assert torch.isfinite(outs[0][:rows]).all()
+        assert rel_err(outs[0][:rows], want[:rows]) < (3e-6 if dt == torch.float32 else 1e-2)
+    for i in range(len(new) if max(new) > 1 else 0):           # each request's first token in a step of its own
+        e = [type(entries[i])(entries[i].req, list(entries[i].tokens)[:1], (0,))]
+        b1 = build_step_batch(e, [old[i]], [0], [[tables[i]]], DEV)
+        one = torch.empty(1, nq * d, dtype=dt, device=DEV)
+        r = sum(new[:i])
+        ops._attention_generic_launch(q[r:r + 1].to(DEV).contiguous(), b1, b1.block_tables[0], args[1], 1, page, one, nq, nkv, d, d,
+                                      1 / math.sqrt(d), window, keep=keep)
+        assert torch.equal(one[0], outs[0][r])
+
+
 @pytest.mark.parametrize("nq,nkv,d,page,new,old", [(32, 8, 128, 16, [700], [300]), (8, 2, 64, 32, [333, 40], [0, 1000]),
                                                    (8, 8, 128, 8, [129, 2], [65, 3]),
                                                    # CTAs of two tiles whose tiles take turns at the exponentials: an odd

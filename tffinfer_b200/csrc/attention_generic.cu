@@ -1,6 +1,5 @@
-// Causal grouped-query attention over the paged cache for flat token rows: one warp
-// per (token, query head), any head size, any numbers of heads and groups, optional
-// sliding window.  It is the attention of the true 32-bit path and takes every size
+// Causal grouped-query attention over the paged cache for flat token rows in float32 arithmetic: any head size up to 512,
+// any numbers of heads and groups, optional sliding window.  It is the attention of the true 32-bit path and takes every size
 // the faster bfloat16 kernels refuse.
 //
 // For the token at position p of request b and query head h (kv head h / (nq/nkv),
@@ -8,137 +7,406 @@
 //   s[n] = (q . k[n]) * scale for lo <= n <= p, lo = window ? max(0, p-window+1) : 0; with ``keep`` > 0 also for n < keep
 //   s[n] = softcap * tanh(s[n] / softcap)                      when softcap > 0
 //   out  = sum_n softmax(s)[n] * v[n]
-// with the running-maximum ("online") softmax of the reference
-// (paged_flash_attention.cu:696-792) in float32, over key blocks of 32 aligned to
-// absolute positions.  The block boundaries depend on p and the window only, so a
-// token's result does not depend on how the batch was cut or what else is in it.
 // With ``sink`` the softmax has one more term in its denominator, a key that has no value and whose score (neither
 // scaled nor capped) is sink_val[h], or 0 when sink_val is null: weights exp(s[n]) / (exp(sink) + sum exp(s)).  With ``gate`` (float32 [tokens, nq]) the head's output is multiplied by
 // gate[t, h].  Keys have d elements and values dv; both lie in cache slots of dc >= max(d, dv) elements.
+//
+// A CTA takes a tile of packed rows (token, query head of the group) of one request and kv head and walks the keys in
+// blocks of 32, which come to shared memory once for all its rows; a warp has up to 8 rows: for the scores a lane is
+// a key, for the values a lane has 4 (8, 16) columns.  The running-maximum ("online") softmax of the reference
+// (paged_flash_attention.cu:696-792) starts afresh every CHUNK keys, at absolute positions, and the chunks' results are
+// joined in ascending order: a step of few rows behind long contexts shares the chunks out to several CTAs and joins them in
+// a second kernel, with the same operations in the same order.  A token's result so depends neither on how the batch
+// was cut nor on what else is in it.
+//
+// What bounds it: the loads from shared memory (a key's 4 elements by every lane and the rows' 4 by all, for 4 FMAs a row), 12 cycles for
+// 8 of FMAs at 8 rows a warp; for one token behind a context the cache's bytes.  A warp a (token, head) that read the
+// keys from the second-level cache, a lane a key, took 750 us for four prompts of 134 tokens of the 8B shape; this takes 75.
 #include "common.cuh"
 #include "attention_common.h"
 
 namespace {
 
-constexpr int WARPS = 4;
+constexpr int WARPS = 4, BLOCK = 32, CHUNK = 128, PER_CHUNK = CHUNK / BLOCK;
 
+struct GenericParams {
+    const int *q_start, *pos_start, *block_table;
+    int table_width, row_stride, layer, nq, nkv, d, dv, window, sink, keep, splits, slots, stages, vec;
+    float scale, softcap;
+    const float *sink_val, *gate;
+    float *part_o, *part_ml;
+    KvLayout L;
+};
+
+// Joins a chunk's (maximum, sum) to the running ones; what the running and the chunk's outputs are to be multiplied by.
+__device__ __forceinline__ void join(float& m, float& l, float mc, float lc, float& a, float& b) {
+    if (mc == -INFINITY && lc == 0.f) { a = 1.f; b = 0.f; return; }      // no key of the chunk is visible
+    const float mn = fmaxf(m, mc);
+    a = m == -INFINITY ? 0.f : expf(m - mn);
+    b = expf(mc - mn);
+    l = __fmaf_rn(l, a, __fmul_rn(lc, b));
+    m = mn;
+}
+__device__ __forceinline__ float join_value(float o, float a, float oc, float b) { return __fmaf_rn(o, a, __fmul_rn(oc, b)); }
+
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 u = *(const uint2*)p;
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xffff0000u));
+}
+
+// RW rows a warp, ND groups of 128 value columns (4 a lane).
+template <typename T, int RW, int ND>
+__global__ void __launch_bounds__(WARPS * 32)
+attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache, T* __restrict__ out, const GenericParams p) {
+    extern __shared__ float4 smem4[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int G = p.nq / p.nkv, kvh = blockIdx.y, split = blockIdx.z % p.splits, b = blockIdx.z / p.splits;
+    const int k4 = (p.d + 3) / 4, v4 = (p.dv + 3) / 4;        // groups of 4 elements a row
+    const int ks = k4 | 1;                                    // an odd pitch: 8 lanes read 8 rows' groups in all banks
+    const int stage4 = BLOCK * (ks + v4);
+    float4* sq = smem4 + p.stages * stage4;                   // [WARPS * RW][k4]
+    float* sp = (float*)(sq + WARPS * RW * k4) + warp * RW * BLOCK;       // the warp's weights [RW][32]
+    pdl_launch_dependents();
+    pdl_wait();
+    const int q0 = p.q_start[b], rows = (p.q_start[b + 1] - q0) * G, row0 = blockIdx.x * WARPS * RW;
+    if (row0 >= rows) return;
+    const int pos0 = p.pos_start[b];
+    const int* table = p.block_table + (size_t)b * p.table_width;
+    // what the tile's rows see
+    const int first_pos = pos0 + row0 / G, hi = pos0 + (min(row0 + WARPS * RW, rows) - 1) / G;
+    const int lo_tile = p.window > 0 ? max(0, first_pos - p.window + 1) : 0;
+    const KeyWalk walk(p.keep, CHUNK, lo_tile / CHUNK, hi / CHUNK);
+    const int per = (walk.count + p.splits - 1) / p.splits, w0 = split * per, w1 = min(walk.count, w0 + per);
+    if (w0 >= w1) return;
+
+    for (int i = threadIdx.x; i < WARPS * RW * k4; i += WARPS * 32) {
+        const int r = row0 + i / k4, c = (i % k4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < rows) {
+            const T* src = q_in + (size_t)(q0 + r / G) * p.row_stride + (size_t)(kvh * G + r % G) * p.d + c;
+            v.x = to_f32<T>(src[0]);
+            if (c + 1 < p.d) v.y = to_f32<T>(src[1]);
+            if (c + 2 < p.d) v.z = to_f32<T>(src[2]);
+            if (c + 3 < p.d) v.w = to_f32<T>(src[3]);
+        }
+        sq[i] = v;
+    }
+
+    auto live = [&](int n0) { return n0 <= hi && (n0 + BLOCK - 1 >= lo_tile || n0 < p.keep); };
+    // Keys and values n0 .. n0 + 31 to a stage; those that no row of the tile sees are zeros (their slots may hold anything,
+    // and their pages may have been given back).
+    auto fetch = [&](int n0, int stage) {
+        float4* sk = smem4 + stage * stage4;
+        float4* sv = sk + BLOCK * ks;
+        for (int kr = warp; kr < BLOCK; kr += WARPS) {
+            const int n = n0 + kr;
+            const bool ok = n <= hi && (n >= lo_tile || n < p.keep);
+            const T* kp = nullptr;
+            if (ok)
+                kp = cache + (size_t)table[n / p.L.page_size] * p.L.page_stride + (size_t)p.layer * p.L.layer_stride +
+                     (size_t)kvh * p.L.head_stride + (size_t)(n % p.L.page_size) * p.L.head_dim;
+            const T* vp = ok ? kp + p.L.kv_stride : nullptr;
+            auto row = [&](const T* src, int n4, int len, float4* dst) {
+                for (int c = lane; c < n4; c += 32) {
+                    if (!ok) dst[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    else if (p.vec) {                         // rows of whole, aligned groups
+                        if constexpr (sizeof(T) == 4)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                         ::"r"((uint32_t)__cvta_generic_to_shared(dst + c)), "l"(src + c * 4) : "memory");
+                        else dst[c] = load4(src + c * 4);
+                    } else {
+                        float4 v = make_float4(to_f32<T>(src[c * 4]), 0.f, 0.f, 0.f);
+                        if (c * 4 + 1 < len) v.y = to_f32<T>(src[c * 4 + 1]);
+                        if (c * 4 + 2 < len) v.z = to_f32<T>(src[c * 4 + 2]);
+                        if (c * 4 + 3 < len) v.w = to_f32<T>(src[c * 4 + 3]);
+                        dst[c] = v;
+                    }
+                }
+            };
+            row(kp, k4, p.d, sk + kr * ks);
+            row(vp, v4, p.dv, sv + kr * v4);
+        }
+    };
+
+    const int wrow = row0 + warp * RW;                        // the warp's first row
+    int rp[RW], rlo[RW];                                      // positions of the rows, their windows' first keys
+#pragma unroll
+    for (int j = 0; j < RW; ++j) {
+        rp[j] = wrow + j < rows ? pos0 + (wrow + j) / G : -1;
+        rlo[j] = p.window > 0 ? max(0, rp[j] - p.window + 1) : 0;
+    }
+    const float inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
+    float m[RW], l[RW], mc[RW], lc[RW], o[RW][4 * ND], oc[RW][4 * ND];
+#pragma unroll
+    for (int j = 0; j < RW; ++j) {
+        // the sink is a key ahead of all others: its score starts the running maximum and the sum
+        const int h = kvh * G + (wrow + j) % G;
+        m[j] = p.sink ? (p.sink_val ? p.sink_val[h] : 0.f) : -INFINITY;
+        l[j] = p.sink ? 1.f : 0.f;
+        mc[j] = -INFINITY; lc[j] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4 * ND; ++c) { o[j][c] = 0.f; oc[j][c] = 0.f; }
+    }
+
+    const int total = (w1 - w0) * PER_CHUNK;
+    auto block_start = [&](int i) { return walk.block(w0 + i / PER_CHUNK) * CHUNK + (i % PER_CHUNK) * BLOCK; };
+    if (p.stages > 1) {
+        if (live(block_start(0))) fetch(block_start(0), 0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int i = 0; i < total; ++i) {
+        const int n0 = block_start(i), stage = p.stages > 1 ? (i & 1) : 0;
+        if (p.stages > 1) {
+            if (i + 1 < total && live(block_start(i + 1))) fetch(block_start(i + 1), stage ^ 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            if (live(n0)) fetch(n0, 0);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
+        __syncthreads();
+        if (live(n0) && wrow < rows) {
+            const float4* sk = smem4 + stage * stage4 + lane * ks;
+            const float4* sv = smem4 + stage * stage4 + BLOCK * ks;
+            const float4* qr = sq + warp * RW * k4;
+            // ------------------------------------------------ scores: key n0 + lane against the warp's rows
+            float acc[RW][4];
+#pragma unroll
+            for (int j = 0; j < RW; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < k4; ++c) {
+                const float4 k = sk[c];
+#pragma unroll
+                for (int j = 0; j < RW; ++j) {
+                    const float4 q = qr[j * k4 + c];
+                    acc[j][0] = fmaf(q.x, k.x, acc[j][0]);
+                    acc[j][1] = fmaf(q.y, k.y, acc[j][1]);
+                    acc[j][2] = fmaf(q.z, k.z, acc[j][2]);
+                    acc[j][3] = fmaf(q.w, k.w, acc[j][3]);
+                }
+            }
+            const int n = n0 + lane;
+            bool whole = true;                                // every row sees every key of the block
+#pragma unroll
+            for (int j = 0; j < RW; ++j) {
+                float s = ((acc[j][0] + acc[j][1]) + (acc[j][2] + acc[j][3])) * p.scale;
+                if (p.softcap > 0.f) s = p.softcap * tanhf(s * inv_cap);
+                const bool valid = n <= rp[j] && (n >= rlo[j] || n < p.keep);
+                whole = whole && n0 + BLOCK - 1 <= rp[j] && (n0 >= rlo[j] || n0 + BLOCK <= p.keep);
+                s = valid ? s : -INFINITY;
+                const float mn = fmaxf(mc[j], warp_max(s));
+                const float alpha = mc[j] == -INFINITY ? (mn == -INFINITY ? 1.f : 0.f) : expf(mc[j] - mn);
+                const float pr = valid ? expf(s - mn) : 0.f;
+                lc[j] = lc[j] * alpha + warp_sum(pr);
+                mc[j] = mn;
+                if (alpha != 1.f) {
+#pragma unroll
+                    for (int c = 0; c < 4 * ND; ++c) oc[j][c] *= alpha;
+                }
+                sp[j * BLOCK + lane] = pr;
+            }
+            __syncwarp();
+            // ------------------------------------------------ values: the lane's columns of the warp's rows
+#pragma unroll 1
+            for (int c = 0; c < BLOCK; c += 4) {
+                float4 w[RW];
+#pragma unroll
+                for (int j = 0; j < RW; ++j) w[j] = *(const float4*)(sp + j * BLOCK + c);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int key = n0 + c + e;
+                    float4 v[ND];
+#pragma unroll
+                    for (int g = 0; g < ND; ++g) {
+                        const int at = lane + 32 * g;
+                        v[g] = at < v4 ? sv[(c + e) * v4 + at] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                    for (int j = 0; j < RW; ++j) {
+                        // a key that the row does not see adds nothing, whatever its value is
+                        if (!whole && !(key <= rp[j] && (key >= rlo[j] || key < p.keep))) continue;
+                        const float x = e == 0 ? w[j].x : e == 1 ? w[j].y : e == 2 ? w[j].z : w[j].w;
+#pragma unroll
+                        for (int g = 0; g < ND; ++g) {
+                            oc[j][4 * g] = fmaf(x, v[g].x, oc[j][4 * g]);
+                            oc[j][4 * g + 1] = fmaf(x, v[g].y, oc[j][4 * g + 1]);
+                            oc[j][4 * g + 2] = fmaf(x, v[g].z, oc[j][4 * g + 2]);
+                            oc[j][4 * g + 3] = fmaf(x, v[g].w, oc[j][4 * g + 3]);
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (i % PER_CHUNK == PER_CHUNK - 1) {                 // the chunk's end
+            const int slot = w0 + i / PER_CHUNK;
+#pragma unroll
+            for (int j = 0; j < RW; ++j) {
+                if (p.splits > 1) {
+                    if (wrow + j < rows) {
+                        const size_t at = ((size_t)(q0 + (wrow + j) / G) * p.nq + kvh * G + (wrow + j) % G) * p.slots + slot;
+                        if (lane == 0) { p.part_ml[2 * at] = mc[j]; p.part_ml[2 * at + 1] = lc[j]; }
+#pragma unroll
+                        for (int c = 0; c < 4 * ND; ++c) {
+                            const int col = (lane + 32 * (c / 4)) * 4 + c % 4;
+                            if (col < p.dv) p.part_o[at * p.dv + col] = oc[j][c];
+                        }
+                    }
+                } else {
+                    float a, bb;
+                    join(m[j], l[j], mc[j], lc[j], a, bb);
+#pragma unroll
+                    for (int c = 0; c < 4 * ND; ++c) o[j][c] = join_value(o[j][c], a, oc[j][c], bb);
+                }
+                mc[j] = -INFINITY; lc[j] = 0.f;
+#pragma unroll
+                for (int c = 0; c < 4 * ND; ++c) oc[j][c] = 0.f;
+            }
+        }
+        __syncthreads();
+    }
+    if (p.splits > 1) return;
+#pragma unroll
+    for (int j = 0; j < RW; ++j) {
+        if (wrow + j >= rows) continue;
+        const int h = kvh * G + (wrow + j) % G;
+        const size_t t = q0 + (wrow + j) / G;
+        const float inv = (p.gate ? p.gate[t * p.nq + h] : 1.f) / l[j];
+#pragma unroll
+        for (int c = 0; c < 4 * ND; ++c) {
+            const int col = (lane + 32 * (c / 4)) * 4 + c % 4;
+            if (col < p.dv) out[(t * p.nq + h) * p.dv + col] = from_f32<T>(o[j][c] * inv);
+        }
+    }
+}
+
+// Joins the chunks' results in ascending order: one warp per (token, head).  The rows of a request are one tile.
 template <typename T>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_generic_kernel(const T* __restrict__ q_in, int row_stride,
-                         const int* __restrict__ positions, const int* __restrict__ tok_req,
-                         const int* __restrict__ block_table, int table_width,
-                         const T* __restrict__ cache, KvLayout L, int layer,
-                         T* __restrict__ out, int num_tokens, int nq, int nkv, int d, int dv,
-                         float scale, int window, float softcap, int sink, const float* __restrict__ sink_val,
-                         const float* __restrict__ gate, int keep) {
-    extern __shared__ float smem[];            // WARPS * d floats: the warp's query row
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * WARPS + warp;
-    if (item >= (long long)num_tokens * nq) return;
-    const int t = (int)(item / nq), h = (int)(item % nq);
-    const int kvh = h / (nq / nkv);
-    const int p = positions[t];
-    const int b = tok_req[t];
-    const int* table = block_table + (size_t)b * table_width;
-    float* q = smem + warp * d;
-    const T* qrow = q_in + (size_t)t * row_stride + (size_t)h * d;
-    for (int i = lane; i < d; i += 32) q[i] = to_f32<T>(qrow[i]);
-    __syncwarp();
-
-    const int lo = window > 0 ? max(0, p - window + 1) : 0;
-    const int nd = (dv + 31) / 32;             // output dims per lane (<= 16 for dv <= 512)
-    const int dc = L.head_dim;                 // elements of a cache slot
+attention_generic_join_kernel(T* __restrict__ out, const int* __restrict__ tok_req, int num_tokens, const GenericParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
+    if (item >= (long long)num_tokens * p.nq) return;
+    const int t = (int)(item / p.nq), h = (int)(item % p.nq), b = tok_req[t];
+    const int pos0 = p.pos_start[b], q_len = p.q_start[b + 1] - p.q_start[b];
+    const int lo_tile = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
+    const KeyWalk walk(p.keep, CHUNK, lo_tile / CHUNK, (pos0 + q_len - 1) / CHUNK);
+    float m = p.sink ? (p.sink_val ? p.sink_val[h] : 0.f) : -INFINITY, l = p.sink ? 1.f : 0.f;
     float o[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) o[j] = 0.f;
-    // the sink is a key ahead of all others: its score starts the running maximum and the sum
-    float m = sink ? (sink_val ? sink_val[h] : 0.f) : -INFINITY, l = sink ? 1.f : 0.f;
-    const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
-
-    const KeyWalk walk(keep, 32, lo / 32, p / 32);
     for (int w = 0; w < walk.count; ++w) {
-        const int n = walk.block(w) * 32 + lane;
-        const bool valid = n <= p && (n >= lo || n < keep);
-        float s = -INFINITY;
-        const T* vbase = nullptr;
-        if (valid) {
-            const int page = table[n / L.page_size];
-            const T* kbase = cache + (size_t)page * L.page_stride + (size_t)layer * L.layer_stride +
-                             (size_t)kvh * L.head_stride + (size_t)(n % L.page_size) * dc;
-            vbase = kbase + L.kv_stride;
-            float acc = 0.f;
-            for (int i = 0; i < d; ++i) acc = fmaf(q[i], to_f32<T>(kbase[i]), acc);
-            s = acc * scale;
-            if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
-        }
-        const float bm = warp_max(s);          // at least lane with n == max(k0, lo) .. is valid
-        const float m_new = fmaxf(m, bm);
-        const float alpha = (m == -INFINITY) ? 0.f : expf(m - m_new);
-        const float pr = valid ? expf(s - m_new) : 0.f;
-        l = l * alpha + warp_sum(pr);
+        const size_t at = (size_t)item * p.slots + w;
+        float a, bb;
+        join(m, l, p.part_ml[2 * at], p.part_ml[2 * at + 1], a, bb);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) o[j] *= alpha;
-        for (int kk = 0; kk < 32; ++kk) {
-            const float pk = __shfl_sync(0xffffffffu, pr, kk);
-            const unsigned long long vp = __shfl_sync(0xffffffffu, (unsigned long long)vbase, kk);
-            if (vp == 0ull) continue;          // uniform across the warp
-            const T* v = (const T*)vp;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                if (j < nd) {
-                    const int i = j * 32 + lane;
-                    if (i < dv) o[j] = fmaf(pk, to_f32<T>(v[i]), o[j]);
-                }
-            }
+        for (int j = 0; j < 16; ++j) {
+            const int col = j * 32 + lane;
+            if (col < p.dv) o[j] = join_value(o[j], a, p.part_o[at * p.dv + col], bb);
         }
-        m = m_new;
     }
-    const float inv = (gate ? gate[(size_t)t * nq + h] : 1.f) / l;
-    T* orow = out + (size_t)t * nq * dv + (size_t)h * dv;
+    const float inv = (p.gate ? p.gate[(size_t)t * p.nq + h] : 1.f) / l;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-        if (j < nd) {
-            const int i = j * 32 + lane;
-            if (i < dv) orow[i] = from_f32<T>(o[j] * inv);
-        }
+        const int col = j * 32 + lane;
+        if (col < p.dv) out[(size_t)item * p.dv + col] = from_f32<T>(o[j] * inv);
     }
 }
+
+template <typename T, int RW, int ND>
+int launch(const void* q, const void* cache, void* out, GenericParams p, int num_requests, int max_q_len, cudaStream_t s) {
+    auto kern = attention_generic_kernel<T, RW, ND>;
+    const int k4 = (p.d + 3) / 4, v4 = (p.dv + 3) / 4;
+    const size_t stage = (size_t)BLOCK * ((k4 | 1) + v4) * 16;
+    const size_t rest = (size_t)WARPS * RW * k4 * 16 + (size_t)WARPS * RW * BLOCK * 4;
+    p.stages = 2 * stage + rest <= 200 * 1024 ? 2 : 1;
+    const size_t smem = p.stages * stage + rest;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return TFF_ERR_LAUNCH;
+        configured = true;
+    }
+    const long long rows = (long long)max_q_len * (p.nq / p.nkv), z = (long long)num_requests * p.splits;
+    if (smem > 200 * 1024 || z > 65535 || p.nkv > 65535) return TFF_ERR_UNSUPPORTED;
+    return tff_launch_pdl(kern, dim3((unsigned)((rows + WARPS * RW - 1) / (WARPS * RW)), p.nkv, (unsigned)z), dim3(WARPS * 32), smem,
+                          s, (const T*)q, (const T*)cache, (T*)out, p);
+}
+
+template <typename T>
+int dispatch(const void* q, const void* cache, void* out, const GenericParams& p, int num_requests, int max_q_len, cudaStream_t s) {
+    // rows a warp: 4 warps share the keys in shared memory, so as many as the step has, and as the registers hold columns
+    const long long rows = (long long)max_q_len * (p.nq / p.nkv);
+    if (p.dv <= 128) {
+        if (rows <= 4) return launch<T, 1, 1>(q, cache, out, p, num_requests, max_q_len, s);
+        if (rows <= 8) return launch<T, 2, 1>(q, cache, out, p, num_requests, max_q_len, s);
+        if (rows <= 16) return launch<T, 4, 1>(q, cache, out, p, num_requests, max_q_len, s);
+        return launch<T, 8, 1>(q, cache, out, p, num_requests, max_q_len, s);
+    }
+    if (p.dv <= 256) {
+        if (rows <= 4) return launch<T, 1, 2>(q, cache, out, p, num_requests, max_q_len, s);
+        return launch<T, 4, 2>(q, cache, out, p, num_requests, max_q_len, s);
+    }
+    if (rows <= 4) return launch<T, 1, 4>(q, cache, out, p, num_requests, max_q_len, s);
+    return launch<T, 2, 4>(q, cache, out, p, num_requests, max_q_len, s);
+}
+
+// Rows that may be one tile whatever the head size is: what a step's chunks may be shared out for.
+int tile_rows(int dv) { return dv <= 128 ? 32 : dv <= 256 ? 16 : 8; }
 
 }  // namespace
 
-// The general entry: keys of d and values of dv elements in cache slots of dc, score cap, sink, head gates.
-TFF_API int tff_attention_generic_ext(
-    const void* qkv, int is_bf16, int row_stride,
-    const int* positions, const int* tok_req, const int* block_table, int table_width,
-    const void* cache, int cache_layers, int layer, int page_size,
-    void* out, int num_tokens, int nq, int nkv, int d, int dv, int dc, float scale, int window,
-    float softcap, int sink, const float* sink_val, const float* gate, int keep, cudaStream_t stream) {
-    if (num_tokens <= 0) return TFF_OK;
-    if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || d <= 0 || dv <= 0 || dc < d || dc < dv || page_size <= 0 || softcap < 0.f || keep < 0)
-        return TFF_ERR_BAD_ARGUMENT;
-    if (d > 512 || dv > 512) return TFF_ERR_UNSUPPORTED;
-    if (window <= 0) keep = 0;
-    const KvLayout L = make_kv_layout(cache_layers, nkv, page_size, dc);
-    const long long items = (long long)num_tokens * nq;
-    const unsigned blocks = (unsigned)((items + WARPS - 1) / WARPS);
-    const size_t smem = (size_t)WARPS * d * sizeof(float);
-    if (is_bf16)
-        attention_generic_kernel<bf16><<<blocks, WARPS * 32, smem, stream>>>(
-            (const bf16*)qkv, row_stride, positions, tok_req, block_table, table_width,
-            (const bf16*)cache, L, layer, (bf16*)out, num_tokens, nq, nkv, d, dv, scale, window, softcap, sink, sink_val, gate, keep);
-    else
-        attention_generic_kernel<float><<<blocks, WARPS * 32, smem, stream>>>(
-            (const float*)qkv, row_stride, positions, tok_req, block_table, table_width,
-            (const float*)cache, L, layer, (float*)out, num_tokens, nq, nkv, d, dv, scale, window, softcap, sink, sink_val, gate, keep);
-    return tff_launch_status();
+// In how many shares (low 16 bits) the chunks of a step's keys go to different CTAs, and for how many chunks there must be
+// room for a partial result of dv + 2 floats per (token, head) (above).  One share and no room for steps of long
+// portions and for steps with enough requests: two CTAs an SM.  ``max_kv`` bounds the contexts.
+TFF_API int tff_attention_generic_plan(int num_requests, int max_q_len, int max_kv, int nq, int nkv, int dv, int window, int keep,
+                                       int sms) {
+    if (num_requests <= 0 || max_q_len <= 0 || max_kv <= 0 || nkv <= 0 || nq % nkv || sms <= 0) return 1;
+    if ((long long)max_q_len * (nq / nkv) > tile_rows(dv)) return 1;
+    long long slots = (max_kv + CHUNK - 1) / CHUNK;
+    if (window > 0) {
+        const long long seen = ((long long)window + max_q_len + CHUNK - 1) / CHUNK + 1 + (keep > 0 ? (keep + CHUNK - 1) / CHUNK : 0);
+        slots = slots < seen ? slots : seen;
+    }
+    const long long ctas = (long long)num_requests * nkv;
+    long long splits = 2ll * sms / ctas;
+    if (splits > slots) splits = slots;
+    if (splits < 2 || slots > 32767 || num_requests * splits > 65535) return 1;
+    return (int)(splits | (slots << 16));
 }
 
+// Keys of d and values of dv elements in cache slots of dc, score cap, sink, head gates.  ``plan`` as
+// tff_attention_generic_plan gives it; with more than one share ``ws`` holds tokens * nq * slots * (dv + 2) floats.
 TFF_API int tff_attention_generic(
-    const void* qkv, int is_bf16, int row_stride,
-    const int* positions, const int* tok_req, const int* block_table, int table_width,
+    const void* qkv, int is_bf16, int row_stride, const int* tok_req, const int* q_start, const int* pos_start, int num_requests,
+    int max_q_len, const int* block_table, int table_width,
     const void* cache, int cache_layers, int layer, int page_size,
-    void* out, int num_tokens, int nq, int nkv, int d, float scale, int window, cudaStream_t stream) {
-    return tff_attention_generic_ext(qkv, is_bf16, row_stride, positions, tok_req, block_table, table_width, cache,
-                                     cache_layers, layer, page_size, out, num_tokens, nq, nkv, d, d, d, scale, window,
-                                     0.f, 0, nullptr, nullptr, 0, stream);
+    void* out, int num_tokens, int nq, int nkv, int d, int dv, int dc, float scale, int window,
+    float softcap, int sink, const float* sink_val, const float* gate, int keep, int plan, float* ws, cudaStream_t stream) {
+    if (num_tokens <= 0 || num_requests <= 0) return TFF_OK;
+    if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || d <= 0 || dv <= 0 || dc < d || dc < dv || page_size <= 0 || softcap < 0.f || keep < 0 || max_q_len <= 0)
+        return TFF_ERR_BAD_ARGUMENT;
+    if (d > 512 || dv > 512) return TFF_ERR_UNSUPPORTED;
+    GenericParams p = {};
+    p.q_start = q_start; p.pos_start = pos_start; p.block_table = block_table; p.table_width = table_width;
+    p.row_stride = row_stride; p.layer = layer; p.nq = nq; p.nkv = nkv; p.d = d; p.dv = dv;
+    p.window = window > 0 ? window : 0; p.keep = window > 0 ? keep : 0;
+    p.sink = sink; p.sink_val = sink_val; p.gate = gate; p.scale = scale; p.softcap = softcap;
+    p.L = make_kv_layout(cache_layers, nkv, page_size, dc);
+    p.splits = plan & 0xffff; p.slots = plan >> 16;
+    if (p.splits < 1 || (p.splits > 1 && (ws == nullptr || p.slots < 1 || (long long)max_q_len * (nq / nkv) > tile_rows(dv))))
+        return TFF_ERR_BAD_ARGUMENT;
+    if (p.splits > 1) { p.part_ml = ws; p.part_o = ws + (size_t)num_tokens * nq * p.slots * 2; }
+    // 4 elements are read at a time where rows and slots are whole groups at aligned addresses
+    p.vec = d % 4 == 0 && dv % 4 == 0 && dc % 4 == 0 && ((uintptr_t)cache & 15) == 0;
+    int st = is_bf16 ? dispatch<bf16>(qkv, cache, out, p, num_requests, max_q_len, stream)
+                     : dispatch<float>(qkv, cache, out, p, num_requests, max_q_len, stream);
+    if (st == TFF_OK && p.splits > 1) {
+        const unsigned blocks = (unsigned)(((long long)num_tokens * nq + WARPS - 1) / WARPS);
+        st = is_bf16 ? tff_launch_pdl(attention_generic_join_kernel<bf16>, dim3(blocks), dim3(WARPS * 32), (size_t)0, stream, (bf16*)out, tok_req, num_tokens, p)
+                     : tff_launch_pdl(attention_generic_join_kernel<float>, dim3(blocks), dim3(WARPS * 32), (size_t)0, stream, (float*)out, tok_req, num_tokens, p);
+    }
+    return st;
 }

@@ -735,16 +735,8 @@ class CudaKernels:
             self.attention_bf16(q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, scale, window,
                                 extra=(float(softcap), sink, gates, int(keep)))
             return
-        c_ptr, _, c_layers, c_layer = self._cache_args(kv_cache, kv_layer)
-        sink_on, sink_val = self._sink_args(sink, nq)
-        self._check(self.lib.tff_attention_generic_ext(
-            _ptr(q), _c_int(_dt(q)), _c_int(q.shape[1]),
-            _ptr(batch.positions), _ptr(batch.tok_req), _ptr(block_table), _c_int(block_table.shape[1]),
-            c_ptr, _c_int(c_layers), _c_int(c_layer), _c_int(page_size),
-            _ptr(out), _c_int(T), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(dv), _c_int(dc), _c_float(scale),
-            _c_int(window), _c_float(softcap), _c_int(1 if sink_on else 0), _ptr(sink_val), _ptr(gates), _c_int(keep), self._stream()),
-            "attention_generic_ext")
-        self.launches += 1
+        self._attention_generic_launch(q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, dv, scale, window,
+                                       softcap, sink, gates, keep)
 
     def retain(self, h, w_in, freq, batch, state, decay, out, H, d, dv, k_scale: float, eps: float) -> None:
         """The whole of a retention mixer between its input rows and its output projection: one product for q, k, v
@@ -2010,15 +2002,30 @@ class CudaKernels:
 
     def attention_generic(self, q, batch, block_table, kv_cache, kv_layer, page_size, out,
                           nq, nkv, d, scale, window) -> None:
-        T = q.shape[0]
+        self._attention_generic_launch(q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, d, scale, window)
+
+    def _attention_generic_launch(self, q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, dv, scale, window,
+                                  softcap: float = 0.0, sink=False, gates=None, keep: int = 0, plan=None) -> None:
+        """``plan`` as tff_attention_generic_plan gives it (None: its choice): how the keys are shared out changes no result."""
+        T, B = q.shape[0], batch.num_requests
         c_ptr, _, c_layers, c_layer = self._cache_args(kv_cache, kv_layer)
+        sink_on, sink_val = self._sink_args(sink, nq)
+        if plan is None:
+            # a step replayed as a graph is captured once for all contexts that its block tables can hold
+            graph = getattr(batch, "graph_bucket", None) is not None
+            max_kv = block_table.shape[1] * page_size if graph else int(batch.max_kv_len)
+            plan = self.lib.tff_attention_generic_plan(_c_int(B), _c_int(batch.max_q_len), _c_int(max_kv), _c_int(nq), _c_int(nkv),
+                                                       _c_int(dv), _c_int(window), _c_int(keep), _c_int(self.NUM_SMS))
+        splits, slots = plan & 0xffff, plan >> 16
+        ws = torch.empty(T * nq * slots * (dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
         self._check(self.lib.tff_attention_generic(
-            _ptr(q), _c_int(_dt(q)), _c_int(q.shape[1]),
-            _ptr(batch.positions), _ptr(batch.tok_req), _ptr(block_table), _c_int(block_table.shape[1]),
+            _ptr(q), _c_int(_dt(q)), _c_int(q.shape[1]), _ptr(batch.tok_req), _ptr(batch.q_start), _ptr(batch.pos_start),
+            _c_int(B), _c_int(batch.max_q_len), _ptr(block_table), _c_int(block_table.shape[1]),
             c_ptr, _c_int(c_layers), _c_int(c_layer), _c_int(page_size),
-            _ptr(out), _c_int(T), _c_int(nq), _c_int(nkv), _c_int(d), _c_float(scale), _c_int(window),
-            self._stream()), "attention_generic")
-        self.launches += 1
+            _ptr(out), _c_int(T), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(dv), _c_int(kv_cache.shape[-1]), _c_float(scale),
+            _c_int(window), _c_float(softcap), _c_int(1 if sink_on else 0), _ptr(sink_val), _ptr(gates), _c_int(keep),
+            _c_int(plan), _ptr(ws), self._stream()), "attention_generic")
+        self.launches += 2 if splits > 1 else 1
 
     def gemm_swiglu(self, a, w_gate_up, out) -> None:
         """out[T, I] = silu(a @ Wg^T) * (a @ Wu^T), w_gate_up being merge_gate_up(Wg, Wu)."""
