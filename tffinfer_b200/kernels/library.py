@@ -12,8 +12,10 @@ falls back to another implementation.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
+import re
 from typing import Optional
 
 import numpy as np
@@ -21,8 +23,11 @@ import torch
 
 from ..csrc import build as _build
 
-_c_int = ctypes.c_int
-_c_float = ctypes.c_float
+# What a call passes are plain numbers: the functions' argument types are declared when the library is loaded (declare_functions),
+# and ctypes converts.  An object of a ctypes type for every argument, and torch's stream object for every launch, were
+# half of a call's host time.
+_c_int = int
+_c_float = float
 _vp = ctypes.c_void_p
 
 _STATUS = {
@@ -47,7 +52,42 @@ def _dt(t: torch.Tensor) -> int:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return _vp(t.data_ptr()) if t is not None else _vp(0)
+    return t.data_ptr() if t is not None else None
+
+
+_SIGNATURE = re.compile(r"TFF_API\s+(int|long long)\s+(tff_\w+)\s*\(([^)]*)\)")
+
+
+def function_signatures(text: str):
+    """[(name, result type, argument types)] of the entry points declared in a CUDA source."""
+    out = []
+    for result, name, params in _SIGNATURE.findall(re.sub(r"//[^\n]*", "", text)):
+        types = []
+        for param in (p.strip() for p in params.split(",")):
+            if not param or param == "void":
+                continue
+            if "*" in param or "cudaStream_t" in param:
+                types.append(_vp)
+            elif "long long" in param:
+                types.append(ctypes.c_longlong)
+            elif re.match(r"(const\s+)?float\b", param):
+                types.append(ctypes.c_float)
+            elif re.match(r"(const\s+)?int\b", param):
+                types.append(ctypes.c_int)
+            else:
+                raise KernelError(f"{name}: no ctypes type for the parameter '{param}'")
+        out.append((name, ctypes.c_longlong if result == "long long" else ctypes.c_int, types))
+    return out
+
+
+def declare_functions(lib) -> None:
+    """Sets the argument and result types of every entry point that ``lib`` has, as its sources declare them."""
+    for source in _build.sources():
+        with open(os.path.join(_build.CSRC_DIR, source), encoding="utf-8") as f:
+            for name, result, types in function_signatures(f.read()):
+                fn = getattr(lib, name, None)             # a library of some sources lacks the others' functions
+                if fn is not None:
+                    fn.argtypes, fn.restype = types, result
 
 
 def effective_requests(kv_lens) -> float:
@@ -105,6 +145,7 @@ class CudaKernels:
             self.lib = ctypes.CDLL(path)
         except OSError as e:
             raise KernelError(f"cannot load the kernel library {path}: {e}") from None
+        declare_functions(self.lib)
         self.path = path
         self.launches = 0          # number of kernel launches issued through this object
         self._accumulators = {}    # (shape, device) -> float32 buffer kept at zero between uses
@@ -119,7 +160,7 @@ class CudaKernels:
     # ------------------------------------------------------------- plumbing
     @staticmethod
     def _stream():
-        return _vp(torch.cuda.current_stream().cuda_stream)
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
     def _check(self, status: int, what: str) -> None:
         if status != 0:
@@ -142,11 +183,11 @@ class CudaKernels:
         64 KB out of every ``layers`` x 64 KB).  For the second the launcher is given the layer's own
         [pages, 1, ...] block."""
         if kv_cache is None:
-            return _vp(0), 0, 1, kv_layer
+            return None, 0, 1, kv_layer
         if not kv_cache.is_cuda:
             raise KernelError("a tensor given to a CUDA kernel is not on a CUDA device")
         if kv_cache.is_contiguous():
-            return _vp(kv_cache.data_ptr()), kv_cache.shape[0], kv_cache.shape[1], kv_layer
+            return kv_cache.data_ptr(), kv_cache.shape[0], kv_cache.shape[1], kv_layer
         st, block = kv_cache.stride(), 1
         for i in range(kv_cache.dim() - 1, 1, -1):             # the [2, kv heads, page, head] block of a page is dense
             if st[i] != block:
@@ -154,7 +195,7 @@ class CudaKernels:
             block *= kv_cache.shape[i]
         else:
             if st[0] == block and st[1] == block * kv_cache.shape[0]:
-                return (_vp(kv_cache.data_ptr() + kv_layer * st[1] * kv_cache.element_size()),
+                return (kv_cache.data_ptr() + kv_layer * st[1] * kv_cache.element_size(),
                         kv_cache.shape[0], 1, 0)
         raise KernelError("the cache is neither contiguous nor a view of layer-major storage")
 
@@ -180,7 +221,7 @@ class CudaKernels:
         """In place: logits * scale, then softcap * tanh(. / softcap) when softcap > 0."""
         self._need_cuda(logits)
         assert logits.dtype == torch.float32
-        self._check(self.lib.tff_logit_transform(_ptr(logits), ctypes.c_longlong(logits.numel()), _c_float(scale),
+        self._check(self.lib.tff_logit_transform(_ptr(logits), _c_int(logits.numel()), _c_float(scale),
                                                  _c_float(softcap), self._stream()), "logit_transform")
         self.launches += 1
 
@@ -275,15 +316,20 @@ class CudaKernels:
     def prompt_costs(self, M: int, N: int, K: int, added: bool, kinds=(512, 256, 128)):
         """{bn: (estimated us, slices)} of the normal-orientation configurations for a prompt-sized product; the
         last wave's tiles are cut along K only where the result is added to a float32 buffer."""
+        return dict(self._prompt_costs(self.NUM_SMS, self.USE_SM_PAIRS, M, N, K, added, tuple(kinds)))
+
+    @staticmethod
+    @functools.lru_cache(maxsize=4096)
+    def _prompt_costs(num_sms: int, pairs: bool, M: int, N: int, K: int, added: bool, kinds):
         kb = -(-K // 64)
         costs = {}
         for bn in kinds:
-            if bn == 512 and (not self.USE_SM_PAIRS or N <= 128):
+            if bn == 512 and (not pairs or N <= 128):
                 continue
-            c, launch, tm, tn, sms = self.TILE_COST[bn]
-            tiles, slots = -(-M // tm) * -(-N // tn), max(1, self.NUM_SMS // sms)
+            c, launch, tm, tn, sms = CudaKernels.TILE_COST[bn]
+            tiles, slots = -(-M // tm) * -(-N // tn), max(1, num_sms // sms)
             waves, tail = divmod(tiles, slots)
-            slices = self.tail_slices(tiles, kb, slots) if added else 0
+            slices = CudaKernels.tail_slices(tiles, kb, slots) if added else 0
             if tail:
                 waves += (-(-tail * slices // slots) / slices + 0.02 * slices) if slices else 1
             costs[bn] = (waves * kb * c + launch, slices)
@@ -335,7 +381,7 @@ class CudaKernels:
 
     def zero_f32(self, t) -> None:
         assert t.dtype == torch.float32 and t.is_contiguous()
-        self._check(self.lib.tff_zero_f32(_ptr(t), ctypes.c_longlong(t.numel()), self._stream()), "zero_f32")
+        self._check(self.lib.tff_zero_f32(_ptr(t), _c_int(t.numel()), self._stream()), "zero_f32")
         self.launches += 1
 
     def reset_state_slots(self, state, slots, pos_start) -> None:
@@ -344,7 +390,7 @@ class CudaKernels:
         self._need_cuda(state, slots, pos_start)
         assert slots.dtype == pos_start.dtype == torch.int32 and slots.numel() == pos_start.numel()
         slot_bytes = state[0].numel() * state.element_size()
-        self._check(self.lib.tff_reset_state_slots(_ptr(state), ctypes.c_longlong(slot_bytes), _c_int(state.shape[0]),
+        self._check(self.lib.tff_reset_state_slots(_ptr(state), _c_int(slot_bytes), _c_int(state.shape[0]),
                                                    _ptr(slots), _ptr(pos_start), _c_int(slots.numel()),
                                                    self._stream()), "reset_state_slots")
         self.launches += 1
@@ -771,7 +817,6 @@ class CudaKernels:
         T = q.shape[0]
         ws = None
         if chunked:
-            self.lib.tff_retention_workspace.restype = ctypes.c_longlong
             need = int(self.lib.tff_retention_workspace(_c_int(T), _c_int(batch.num_requests), _c_int(H), _c_int(d), _c_int(dv)))
             ws = torch.empty(need, dtype=torch.float32, device=q.device)
         clear = 1 if vg.data_ptr() in self._acc_zero else 0
@@ -823,7 +868,6 @@ class CudaKernels:
         def run(ch: int):
             ws = None
             if ch:
-                self.lib.tff_retention_workspace.restype = ctypes.c_longlong
                 need = int(self.lib.tff_retention_workspace(_c_int(T), _c_int(batch.num_requests), _c_int(H), _c_int(d), _c_int(dv)))
                 ws = torch.empty(need, dtype=torch.float32, device=proj.device)
             return self.lib.tff_retention_raw(
@@ -892,7 +936,6 @@ class CudaKernels:
         def run(ch: int):
             ws = None
             if ch:
-                self.lib.tff_mlstm_workspace.restype = ctypes.c_longlong
                 need = int(self.lib.tff_mlstm_workspace(_c_int(T), _c_int(batch.num_requests), _c_int(H), _c_int(K), _c_int(V)))
                 ws = torch.empty(need, dtype=torch.float32, device=proj.device)
             return self.lib.tff_mlstm(
@@ -957,7 +1000,7 @@ class CudaKernels:
             part_ml = torch.empty(T * nq * splits * 2, dtype=torch.float32, device=q.device)
         self._check(self.lib.tff_attention_tile(
             _ptr(q), _c_int(_dt(q)), _c_int(q.shape[1]), _ptr(batch.q_start), _ptr(batch.pos_start), _ptr(block_table),
-            _c_int(block_table.shape[1]), c_ptr, ctypes.c_longlong(page_stride), _c_int(planes), _c_int(page_size),
+            _c_int(block_table.shape[1]), c_ptr, _c_int(page_stride), _c_int(planes), _c_int(page_size),
             _c_int(slot), _ptr(out), _c_int(out.shape[1]), _c_int(out_off), _c_int(batch.num_requests),
             _c_int(batch.max_q_len), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(dv), _c_float(scale), _c_int(window),
             _c_int(chunk), _ptr(temp), _ptr(r1), _ptr(r2), _c_float(out_scale), _c_int(T), _c_int(splits), _ptr(part_o),
@@ -1021,7 +1064,7 @@ class CudaKernels:
             code = 0                      # a plain product: only a function of one product ("relu2") is applied to it
         act = _c_int(code)
         clip = (_c_float(limit), _c_float(self.CLIPPED_SLOPE))
-        ll = ctypes.c_longlong
+        ll = int
         if self.grouped_on_tensor_cores(a, b, K, lda, a_gs, ldb, b_gs, gated, N) and tile_rows in (
                 0, self.grouped_tile_rows(True), self.grouped_tile_rows(True, True)):
             if not tile_rows:
@@ -1095,7 +1138,7 @@ class CudaKernels:
             assert nw is None or (nw.dtype == torch.float32 and nw.numel() == width)
         if taps > 1:
             assert state is not None and state.dtype == torch.float32 and tuple(state.shape[1:]) == (taps - 1, C)
-        widths = (_c_int * n)(*[int(w) for w, _, _ in segments])
+        widths = (ctypes.c_int * n)(*[int(w) for w, _, _ in segments])
         convs = (_vp * n)(*[cw.data_ptr() if cw is not None else None for _, cw, _ in segments])
         norms = (_vp * n)(*[nw.data_ptr() if nw is not None else None for _, _, nw in segments])
         self._check(self.lib.tff_short_conv_norm(_ptr(proj), _c_int(ld), _ptr(out), _c_int(n), widths, convs, norms,
@@ -1163,7 +1206,7 @@ class CudaKernels:
         W = x.shape[-1]
         assert state.dtype == torch.int32 and x.dtype == torch.float32 and tuple(table.shape) == (buckets + 1, W)
         assert x.shape[0] == batch.num_tokens and (copies == 0 or x.shape[1] == copies)
-        ll = ctypes.c_longlong
+        ll = int
         self._check(self.lib.tff_pair_embed(_ptr(batch.token_ids), _ptr(batch.positions), _ptr(batch.tok_req),
                                             _ptr(batch.q_start), _ptr(batch.slots), _ptr(state), _ptr(table),
                                             _c_int(_dt(table)), _c_int(buckets), ll(mul_prev), ll(mul_cur), _ptr(x),
@@ -1177,7 +1220,7 @@ class CudaKernels:
         self._need_cuda(x, out)
         assert x.numel() == out.numel() and (x.dtype == out.dtype or x.dtype == torch.float32)
         clear = 1 if (x.data_ptr() in self._acc_zero and x.data_ptr() != out.data_ptr()) else 0
-        self._check(self.lib.tff_unary_act(_ptr(x), _c_int(_dt(x)), _ptr(out), _c_int(_dt(out)), ctypes.c_longlong(x.numel()),
+        self._check(self.lib.tff_unary_act(_ptr(x), _c_int(_dt(x)), _ptr(out), _c_int(_dt(out)), _c_int(x.numel()),
                                            _c_int(self.ACTIVATION_CODES[activation]), _c_int(clear), self._stream()), "unary_act")
         if clear:
             self._acc_zero[x.data_ptr()] = True
@@ -1481,7 +1524,6 @@ class CudaKernels:
         clear = 1 if proj.data_ptr() in self._acc_zero else 0
         if batch.max_q_len > self.GRU_CHUNKED_FROM:
             # long portions: chunks of a request side by side (three passes), not one thread walking thousands of tokens
-            self.lib.tff_min_gru_workspace.restype = ctypes.c_longlong
             need = int(self.lib.tff_min_gru_workspace(_c_int(batch.num_requests), _c_int(batch.max_q_len), _c_int(width)))
             ws = torch.empty(need, dtype=torch.float32, device=proj.device)
             self._check(self.lib.tff_min_gru_chunked(
@@ -1526,7 +1568,6 @@ class CudaKernels:
         for t, n in ((dec_bias, H if m == 2 else H * K), (rate_log, H), (skip, H)):
             assert t is None or (t.dtype == torch.float32 and t.numel() == n)
         T = qt.shape[0]
-        self.lib.tff_linear_recurrence_workspace.restype = ctypes.c_longlong
         need = int(self.lib.tff_linear_recurrence_workspace(_c_int(T), _c_int(batch.num_requests), _c_int(batch.max_q_len),
                                                             _c_int(H), _c_int(K), _c_int(V), _c_int(m)))
         factors = torch.empty(need, dtype=torch.float32, device=qt.device)
@@ -1534,8 +1575,8 @@ class CudaKernels:
         self._check(self.lib.tff_linear_recurrence(
             _ptr(qt), _c_int(qt.shape[1]), _c_int(q0), _ptr(kt), _c_int(kt.shape[1]), _c_int(k0), _ptr(vt),
             _c_int(vt.shape[1]), _c_int(vo), _ptr(dt), _c_int(dt.shape[1]), _c_int(d0), _ptr(dec_bias), _ptr(rate_log),
-            _ptr(skip), _c_int(m), _c_float(inv_tau), _c_float(q_scale), _ptr(state), ctypes.c_longlong(state.shape[1]),
-            ctypes.c_longlong(state_off), _ptr(batch.q_start), _ptr(batch.pos_start), _ptr(batch.slots), _ptr(out),
+            _ptr(skip), _c_int(m), _c_float(inv_tau), _c_float(q_scale), _ptr(state), _c_int(state.shape[1]),
+            _c_int(state_off), _ptr(batch.q_start), _ptr(batch.pos_start), _ptr(batch.slots), _ptr(out),
             _c_int(out.shape[1]), _ptr(factors), _c_int(T), _c_int(batch.num_requests), _c_int(batch.max_q_len), _c_int(H),
             _c_int(K), _c_int(V), _c_int(share), self._stream()), "linear_recurrence")
         self.launches += 4 if segmented else 2
@@ -1582,8 +1623,8 @@ class CudaKernels:
         fused = bool(update_state) and batch.max_q_len == 1 and taps > 1
         self._check(self.lib.tff_causal_conv(
             _ptr(proj), _c_int(proj.shape[1]), _c_int(col0), _c_int(channels), _ptr(weight), _ptr(bias), _c_int(taps),
-            _c_int({"none": 0, "silu": 1}[activation]), _ptr(state), ctypes.c_longlong(state.shape[1] if state is not None else 0),
-            ctypes.c_longlong(state_off), _ptr(batch.positions), _ptr(batch.tok_req), _ptr(batch.q_start), _ptr(batch.slots),
+            _c_int({"none": 0, "silu": 1}[activation]), _ptr(state), _c_int(state.shape[1] if state is not None else 0),
+            _c_int(state_off), _ptr(batch.positions), _ptr(batch.tok_req), _ptr(batch.q_start), _ptr(batch.slots),
             _ptr(out), _c_int(T), _c_int(1 if fused else 0), self._stream()), "causal_conv")
         self.launches += 1
         return fused
@@ -1596,7 +1637,7 @@ class CudaKernels:
         self._need_cuda(proj, state)
         self._check(self.lib.tff_causal_conv_state(
             _ptr(proj), _c_int(proj.shape[1]), _c_int(col0), _c_int(channels), _c_int(taps), _ptr(state),
-            ctypes.c_longlong(state.shape[1]), ctypes.c_longlong(state_off), _ptr(batch.q_start), _ptr(batch.slots),
+            _c_int(state.shape[1]), _c_int(state_off), _ptr(batch.q_start), _ptr(batch.slots),
             _c_int(batch.num_requests), self._stream()), "causal_conv_state")
         self.launches += 1
 
@@ -1725,7 +1766,7 @@ class CudaKernels:
             _c_int(rot_dims), _c_int(1 if halves else 0), _c_float(mag), *qh, _ptr(q_norm_w), _ptr(kv_norm_w), _c_float(eps),
             _ptr(freq), _ptr(batch.positions),
             _ptr(batch.tok_req), _ptr(block_table), _c_int(block_table.shape[1]), c_ptr if kv_rank > 0 else _vp(0),
-            ctypes.c_longlong(page_stride), _c_int(page_size), _c_int(kv_cache.shape[-1]), _ptr(cq), _c_int(_dt(act)),
+            _c_int(page_stride), _c_int(page_size), _c_int(kv_cache.shape[-1]), _ptr(cq), _c_int(_dt(act)),
             _ptr(dense_out), _c_int(T), self._stream()), "latent_finish")
         if clear:
             self._acc_zero[proj.data_ptr()] = True
@@ -1993,7 +2034,7 @@ class CudaKernels:
         self._check(self.lib.tff_attention_bf16_paged_ext(
             _ptr(q), _ptr(batch.q_start), _ptr(batch.pos_start), _ptr(req_ids), _ptr(block_table),
             _c_int(block_table.shape[1]),
-            c_ptr, ctypes.c_longlong(c_pages), _c_int(c_layers), _c_int(c_layer),
+            c_ptr, _c_int(c_pages), _c_int(c_layers), _c_int(c_layer),
             _c_int(page_size),
             _ptr(out), _ptr(ws), _c_int(T), _c_int(num_requests), _c_int(max_q_len), _c_int(splits),
             _c_int(nq), _c_int(nkv), _c_int(d), _c_float(scale), _c_int(window), _c_float(softcap),
