@@ -326,7 +326,7 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 
 struct MmaGeom { int dpad, kst, vst; };      // padded key size, elements between key rows and between value rows in shared memory
 
-// RG groups of 16 rows (a tile has 16 * RG rows and 4 * RG warps: steps of one token need one group, portions four);
+// RG groups of 16 rows (a tile has 16 * RG rows and 4 * RG warps: two groups or four);
 // a warp of the value phase owns 16 rows x NT * 8 columns
 template <int NT, int RG>
 __global__ void __launch_bounds__(128 * RG)
@@ -546,6 +546,225 @@ attention_tile_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     }
 }
 
+// Steps of at most 16 packed rows a (request, kv head) -- decoded tokens -- are a stream of the cache: the same phases on
+// blocks of 32 keys, two of them in shared memory, so that a block's copies run behind the block ahead of it, and with the rows
+// of a latent cache (576 elements) still two CTAs an SM.  Where a warp's keys lie is looked up one block ahead of their copies.
+constexpr int FKB = 32, FPST = FKB + 8, FSST = FKB + 4, FSTAGES = 2;
+
+__device__ __forceinline__ void ldsm2(uint32_t (&r)[2], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+
+template <int NT>
+__global__ void __launch_bounds__(128)
+attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, bf16* __restrict__ out, TileArgs a,
+                          MmaGeom gm) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    constexpr int MROWS = 16, MTHREADS = 128, KPW = FKB / 4;       // keys a warp brings, and scores
+    const int d = a.d, dv = a.dv, G = a.nq / a.nkv;
+    const bool dense = a.k_dense != nullptr;
+    const bool own_v = a.v_offset != 0 || dense;
+    const int kst = gm.kst, vst = gm.vst, dpad = gm.dpad;
+    const int stage = FKB * (kst + (own_v ? vst : 0));
+    bf16* Qs = (bf16*)smraw;                                    // [MROWS][kst]
+    bf16* Ks0 = Qs + MROWS * kst;                               // stages of [FKB][kst] (and [FKB][vst])
+    bf16* Pb = Ks0 + FSTAGES * stage;                           // [MROWS][FPST] probabilities
+    float* Ss = (float*)(Pb + MROWS * FPST);                    // [MROWS][FSST] scores
+    float* alpha_s = Ss + MROWS * FSST;                         // [MROWS]
+    float* m_fin = alpha_s + MROWS;                             // [MROWS]
+
+    pdl_launch_dependents();
+    const int b = blockIdx.z, kvh = blockIdx.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int t0 = a.q_start[b], q_len = a.q_start[b + 1] - t0, pos0 = a.pos_start[b];
+    const int split = blockIdx.x;
+    const int n_rows = q_len * G;                               // at most MROWS
+    if (n_rows <= 0) return;
+    const int p_max = pos0 + q_len - 1;
+    auto low = [&](int p) {
+        int lo = 0;
+        if (a.window > 0) lo = max(lo, p - a.window + 1);
+        if (a.chunk > 0) lo = max(lo, (p / a.chunk) * a.chunk);
+        return lo;
+    };
+    const int lo_min = low(pos0);
+    const int* table = a.block_table + (size_t)b * a.table_width;
+    const int kb_first = lo_min / FKB, kb_count = p_max / FKB - kb_first + 1;
+    const int kb_lo = kb_first + (int)((long long)kb_count * split / a.splits);
+    const int kb_hi = kb_first + (int)((long long)kb_count * (split + 1) / a.splits);
+    const int dch = dpad / 8, vch = own_v ? (vst - 8) / 8 : 0;
+
+    // lane l < KPW: where key warp * KPW + l of a block lies (null: no row sees it, or its page has been given back)
+    auto key_at = [&](int block) -> const bf16* {
+        const int n = block * FKB + warp * KPW + lane;
+        if (lane >= KPW || block >= kb_hi || n < lo_min || n > p_max) return nullptr;
+        if (dense) return (const bf16*)a.k_dense + (size_t)(t0 + n - pos0) * a.k_ld + (size_t)kvh * d;
+        const int page = table[n / a.page_size];
+        return page < 0 ? nullptr : cache + (size_t)page * a.page_stride + (size_t)kvh * a.head_stride + (size_t)(n % a.page_size) * a.slot;
+    };
+    auto bring = [&](int block, const bf16* at) {              // the warp's keys of a block, 16 bytes a copy
+        bf16* Ks = Ks0 + (block & 1) * stage;
+#pragma unroll
+        for (int j = 0; j < KPW; ++j) {
+            const bf16* src = (const bf16*)__shfl_sync(0xffffffffu, (unsigned long long)at, j);
+            bf16* dst = Ks + (warp * KPW + j) * kst;
+            for (int c = lane; c < dch; c += 32) {
+                const bool ok = src && c * 8 < d;
+                cp_async_16(sm_addr(dst + c * 8), ok ? (const void*)(src + c * 8) : (const void*)q, ok ? 16 : 0);
+            }
+            if (own_v) {
+                const int n = block * FKB + warp * KPW + j;
+                const bf16* vsrc = dense ? (const bf16*)a.v_dense + (size_t)(t0 + n - pos0) * a.v_ld + (size_t)kvh * dv : src + a.v_offset;
+                bf16* vdst = Ks + FKB * kst + (warp * KPW + j) * vst;
+                for (int c = lane; c < vch; c += 32) {
+                    const bool ok = src && c * 8 < dv;
+                    cp_async_16(sm_addr(vdst + c * 8), ok ? (const void*)(vsrc + c * 8) : (const void*)q, ok ? 16 : 0);
+                }
+            }
+        }
+    };
+    pdl_wait();
+    const bf16* at = key_at(kb_lo);
+    if (kb_lo < kb_hi) bring(kb_lo, at);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    at = key_at(kb_lo + 1);
+
+    for (int idx = tid; idx < MROWS * dch; idx += MTHREADS) {
+        const int rr = idx / dch, c = (idx % dch) * 8;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (rr < n_rows && c < d) v = *(const uint4*)(q + (size_t)(t0 + rr / G) * a.q_ld + (size_t)(kvh * G + rr % G) * d + c);
+        *(uint4*)(Qs + rr * kst + c) = v;
+    }
+    const int fr = lane >> 2, fc = 2 * (lane & 3);              // a thread's place in an accumulator tile: rows fr, fr+8; columns fc, fc+1
+    const int ra = fr, rb = fr + 8;
+    const int pa = ra < n_rows ? pos0 + ra / G : -1, pb = rb < n_rows ? pos0 + rb / G : -1;
+    const int la = pa >= 0 ? low(pa) : 0, lb = pb >= 0 ? low(pb) : 0;
+    const int ha = kvh * G + ra % G, hb = kvh * G + rb % G;
+    const float sa = a.scale * (a.temp ? a.temp[ha] : 1.f), sb = a.scale * (a.temp ? a.temp[hb] : 1.f);
+    const bool biased = a.r1 != nullptr;
+    const float r1a = biased ? a.r1[ha] : 0.f, r2a = biased ? a.r2[ha] : 0.f;
+    const float r1b = biased ? a.r1[hb] : 0.f, r2b = biased ? a.r2[hb] : 0.f;
+    float o[NT][4];
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+    float m_run[4], l_run[4];                                   // softmax phase: warp w owns rows 4w .. 4w+3
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m_run[i] = -INFINITY; l_run[i] = 0.f;
+        if (a.sink && split == 0) { m_run[i] = a.sink[kvh * G + (warp * 4 + i) % G]; l_run[i] = 1.f; }
+    }
+
+    for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (kb + 1 < kb_hi) bring(kb + 1, at);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        at = key_at(kb + 2);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const bf16* Ks = Ks0 + (kb & 1) * stage;
+        const bf16* Vs = own_v ? Ks + FKB * kst : Ks;
+        const int k0 = kb * FKB;
+        {   // S = Q K^T: 16 rows, keys warp*8 .. +8; two sums, so that a product does not wait for the one ahead of it
+            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint32_t qa = sm_addr(Qs + (lane & 15) * kst + (lane >> 4) * 8);
+            const uint32_t ka = sm_addr(Ks + (warp * KPW + (lane & 7)) * kst + (lane >> 3) * 8);
+            int kk = 0;
+#pragma unroll 2
+            for (; kk + 32 <= dpad; kk += 32) {
+                uint32_t a0[4], a1[4], bfr[4];
+                ldsm4(a0, qa + kk * 2);
+                ldsm4(a1, qa + kk * 2 + 32);
+                ldsm4(bfr, ka + kk * 2);
+                mma16816(s0, a0, bfr[0], bfr[1]);
+                mma16816(s1, a1, bfr[2], bfr[3]);
+            }
+            if (kk < dpad) {
+                uint32_t a0[4], bfr[2];
+                ldsm4(a0, qa + kk * 2);
+                ldsm2(bfr, sm_addr(Ks + (warp * KPW + (lane & 7)) * kst + ((lane >> 3) & 1) * 8) + kk * 2);
+                mma16816(s0, a0, bfr[0], bfr[1]);
+            }
+            auto score = [&](float dot, float sc, float r1, float r2, int p, int lo, int n) -> float {
+                if (p < 0 || n > p || n < lo) return -INFINITY;
+                float s = dot * sc;
+                if (a.softcap > 0.f) s = a.softcap * attn_tanh(s / a.softcap);
+                if (biased) s -= r1 * log1pf(r2 * (float)(p - n));
+                return s;
+            };
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = warp * KPW + fc + e;
+                Ss[ra * FSST + c] = score(s0[e] + s1[e], sa, r1a, r2a, pa, la, k0 + c);
+                Ss[rb * FSST + c] = score(s0[2 + e] + s1[2 + e], sb, r1b, r2b, pb, lb, k0 + c);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int rr = warp * 4 + i;
+            const float x = Ss[rr * FSST + lane];
+            const float m_new = fmaxf(m_run[i], warp_max(x));
+            float alpha = 1.f, p0 = 0.f;
+            if (m_new != -INFINITY) {
+                alpha = (m_run[i] == -INFINITY) ? 0.f : expf(m_run[i] - m_new);
+                p0 = expf(x - m_new);
+            }
+            l_run[i] = l_run[i] * alpha + warp_sum(p0);
+            m_run[i] = m_new;
+            Pb[rr * FPST + lane] = __float2bfloat16_rn(p0);
+            if (lane == 0) alpha_s[rr] = alpha;
+        }
+        __syncthreads();
+        {   // O += P V: 16 rows, columns warp*NT*8 .. + NT*8
+            const float al_a = alpha_s[ra], al_b = alpha_s[rb];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) { o[j][0] *= al_a; o[j][1] *= al_a; o[j][2] *= al_b; o[j][3] *= al_b; }
+            const uint32_t pa_addr = sm_addr(Pb + (lane & 15) * FPST + (lane >> 4) * 8);
+            const uint32_t va = sm_addr(Vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + warp * NT * 8 + (lane >> 4) * 8);
+#pragma unroll
+            for (int kk = 0; kk < FKB; kk += 16) {
+                uint32_t af[4];
+                ldsm4(af, pa_addr + kk * 2);
+#pragma unroll
+                for (int j2 = 0; j2 < NT / 2; ++j2) {
+                    uint32_t bfr[4];
+                    ldsm4t(bfr, va + (kk * vst + j2 * 16) * 2);
+                    mma16816(o[2 * j2], af, bfr[0], bfr[1]);
+                    mma16816(o[2 * j2 + 1], af, bfr[2], bfr[3]);
+                }
+            }
+        }
+        __syncthreads();                                        // everyone is done with the stage and the probabilities
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (lane == 0) { alpha_s[warp * 4 + i] = l_run[i]; m_fin[warp * 4 + i] = m_run[i]; }
+    __syncthreads();
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const int r = side ? rb : ra;
+        if (r >= n_rows) continue;
+        const int t = t0 + r / G, h = kvh * G + r % G;
+        const size_t slot = ((size_t)t * a.nq + h) * a.splits + split;
+        const float inv = a.splits == 1 ? a.out_scale / alpha_s[r] : 1.f;
+        bf16* orow = out + (size_t)t * a.out_ld + a.out_off + (size_t)h * dv;
+        float* prow = a.part_o + slot * dv;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = warp * NT * 8 + j * 8 + fc + e;
+                if (c < dv) {
+                    if (a.splits == 1) orow[c] = __float2bfloat16_rn(o[j][side * 2 + e] * inv);
+                    else prow[c] = o[j][side * 2 + e];
+                }
+            }
+        if (a.splits > 1 && warp == 0 && fc == 0) { a.part_ml[2 * slot] = m_fin[r]; a.part_ml[2 * slot + 1] = alpha_s[r]; }
+    }
+}
+
 static bool tile_mma_enabled() {
     static int v = -1;
     if (v < 0) { const char* e = getenv("TFFINFER_TILE_MMA"); v = (e && e[0] == '0') ? 0 : 1; }
@@ -573,22 +792,24 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
     const int rows_most = max_q_len * G;
     const int rg = rows_most <= 16 ? 1 : (rows_most <= 32 ? 2 : 4);
     const int MROWS = 16 * rg;
-    const size_t smem = 2 * ((size_t)(MROWS + MKB) * gm.kst + (own_v ? (size_t)MKB * gm.vst : 0) + (size_t)MROWS * PST) +
+    const size_t smem = rg == 1 ? 2 * ((size_t)16 * gm.kst + (size_t)FSTAGES * FKB * (gm.kst + (own_v ? gm.vst : 0)) + 16 * FPST) +
+                                      4 * ((size_t)16 * FSST + 2 * 16)
+                                : 2 * ((size_t)(MROWS + MKB) * gm.kst + (own_v ? (size_t)MKB * gm.vst : 0) + (size_t)MROWS * PST) +
                         4 * ((size_t)MROWS * SST + 2 * MROWS) + 4 * 2 * MROWS + 2 * 8 * MKB;
     if (smem > 220 * 1024) return TFF_ERR_UNSUPPORTED;
     const int tiles = (rows_most + MROWS - 1) / MROWS;
     dim3 grid(tiles * a.splits, a.nkv, num_requests);
 #define TFF_TMMA(NTV)                                                                                                \
     do {                                                                                                             \
-        if (rg == 1) TFF_TMMA_RG(NTV, 1);                                                                            \
-        if (rg == 2) TFF_TMMA_RG(NTV, 2);                                                                            \
-        TFF_TMMA_RG(NTV, 4);                                                                                         \
+        if (rg == 1) TFF_TMMA_RUN((attention_tile_few_kernel<NTV>), 128);                                            \
+        if (rg == 2) TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 2>), 256);                                         \
+        TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 4>), 512);                                                      \
     } while (0)
-#define TFF_TMMA_RG(NTV, RGV)                                                                                        \
+#define TFF_TMMA_RUN(KERNEL, THREADS_)                                                                               \
     do {                                                                                                             \
         if (smem > 48 * 1024)                                                                                        \
-            cudaFuncSetAttribute(attention_tile_mma_kernel<NTV, RGV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        const int st = tff_launch_pdl(attention_tile_mma_kernel<NTV, RGV>, grid, dim3(128 * RGV), smem, stream, (const bf16*)q, \
+            cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                     \
+        const int st = tff_launch_pdl(KERNEL, grid, dim3(THREADS_), smem, stream, (const bf16*)q,                     \
                                       (const bf16*)cache, (bf16*)out, a, gm);                                        \
         if (st != TFF_OK || a.splits == 1) return st;                                                                \
         const long long rows = (long long)num_tokens * a.nq;                                                         \
@@ -601,7 +822,7 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
     if (nt == 8) TFF_TMMA(8);
     TFF_TMMA(16);
 #undef TFF_TMMA
-#undef TFF_TMMA_RG
+#undef TFF_TMMA_RUN
 }
 
 }  // namespace
