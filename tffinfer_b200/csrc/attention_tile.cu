@@ -20,7 +20,7 @@
 // row's running maximum and sum only ever see its own visible keys, so a row's result does not depend on the tile it
 // is in, on how the prompt was cut or on what else is in the batch.  Keys outside the tile's range are never read
 // (pages behind a window may have been given back).
-#include "common.cuh"
+#include "tcgen05.cuh"
 #include "attention_common.h"
 #include <stdlib.h>
 
@@ -326,7 +326,7 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 
 struct MmaGeom { int dpad, kst, vst; };      // padded key size, elements between key rows and between value rows in shared memory
 
-// RG groups of 16 rows (a tile has 16 * RG rows and 4 * RG warps: two groups or four);
+// RG groups of 16 rows (a tile has 16 * RG rows and 4 * RG warps: portions two or four);
 // a warp of the value phase owns 16 rows x NT * 8 columns
 template <int NT, int RG>
 __global__ void __launch_bounds__(128 * RG)
@@ -546,39 +546,59 @@ attention_tile_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     }
 }
 
-// Steps of at most 16 packed rows a (request, kv head) -- decoded tokens -- are a stream of the cache: the same phases on
-// blocks of 32 keys, two of them in shared memory, so that a block's copies run behind the block ahead of it, and with the rows
-// of a latent cache (576 elements) still two CTAs an SM.  Where a warp's keys lie is looked up one block ahead of their copies.
-constexpr int FKB = 32, FPST = FKB + 8, FSST = FKB + 4, FSTAGES = 2;
+// Steps of at most 16 packed rows a (request, kv head) -- decoded tokens -- are a stream of the cache.  A CTA walks its share of the
+// keys in blocks of 64, two of them in shared memory:
+//   warp 8      producer: a lane a key looks up where it lies and asks for its row (rows, with values of their own) by one
+//               bulk copy into a row padded by 16 bytes (ldmatrix without bank conflicts), a block ahead of the others
+//   warps 0-7   S = Q K^T (8 keys each) to shared memory; softmax (two rows each); O += P V (an eighth of the columns each)
+// What bounds it: with the tiles above (four warps a group of rows, sixteen instructions for every 16 bytes it copied) an SM issued an
+// instruction in a quarter of the cycles and every warp's chain of shared-memory loads and products set the pace.
+constexpr int FKB = 64, FROWS = 16, FWARPS = 8, FTHREADS = (FWARPS + 1) * 32, FPST = FKB + 8, FSST = FKB + 4, FSTAGES = 2;
+constexpr int FKPW = FKB / FWARPS;                                  // keys a warp scores
 
-__device__ __forceinline__ void ldsm2(uint32_t (&r)[2], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+__device__ __forceinline__ void few_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void bulk_row(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
 template <int NT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(FTHREADS)
 attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, bf16* __restrict__ out, TileArgs a,
-                          MmaGeom gm) {
+                          MmaGeom gm, int* error_flag) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    constexpr int MROWS = 16, MTHREADS = 128, KPW = FKB / 4;       // keys a warp brings, and scores
     const int d = a.d, dv = a.dv, G = a.nq / a.nkv;
     const bool dense = a.k_dense != nullptr;
     const bool own_v = a.v_offset != 0 || dense;
     const int kst = gm.kst, vst = gm.vst, dpad = gm.dpad;
     const int stage = FKB * (kst + (own_v ? vst : 0));
-    bf16* Qs = (bf16*)smraw;                                    // [MROWS][kst]
-    bf16* Ks0 = Qs + MROWS * kst;                               // stages of [FKB][kst] (and [FKB][vst])
-    bf16* Pb = Ks0 + FSTAGES * stage;                           // [MROWS][FPST] probabilities
-    float* Ss = (float*)(Pb + MROWS * FPST);                    // [MROWS][FSST] scores
-    float* alpha_s = Ss + MROWS * FSST;                         // [MROWS]
-    float* m_fin = alpha_s + MROWS;                             // [MROWS]
+    bf16* Qs = (bf16*)smraw;                                    // [FROWS][kst]
+    bf16* Ks0 = Qs + FROWS * kst;                               // stages of [FKB][kst] (and [FKB][vst])
+    bf16* Pb = Ks0 + FSTAGES * stage;                           // [FROWS][FPST] probabilities
+    float* Ss = (float*)(Pb + FROWS * FPST);                    // [FROWS][FSST] scores
+    float* alpha_s = Ss + FROWS * FSST;                         // [FROWS]
+    float* m_fin = alpha_s + FROWS;                             // [FROWS]
+    const uint32_t bars = sm_addr(m_fin + FROWS);               // full[FSTAGES], empty[FSTAGES] (8-byte aligned: an even number of words lies ahead)
+    volatile int* abort_flag = (volatile int*)(m_fin + FROWS + 4 * FSTAGES);
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (FSTAGES + s); };
 
-    pdl_launch_dependents();
     const int b = blockIdx.z, kvh = blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < FSTAGES; ++s) { tc5::mbar_init(full_bar(s), 1); tc5::mbar_init(empty_bar(s), FWARPS); }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // columns d .. dpad of the keys are multiplied with zeros of the queries: they must not be NaN
+    if (dpad > d)
+        for (int i = tid; i < FSTAGES * FKB; i += FTHREADS)
+            *(uint4*)(Ks0 + (i / FKB) * stage + (i % FKB) * kst + d) = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    pdl_launch_dependents();
     const int t0 = a.q_start[b], q_len = a.q_start[b + 1] - t0, pos0 = a.pos_start[b];
     const int split = blockIdx.x;
-    const int n_rows = q_len * G;                               // at most MROWS
+    const int n_rows = q_len * G;                               // at most FROWS
     if (n_rows <= 0) return;
     const int p_max = pos0 + q_len - 1;
     auto low = [&](int p) {
@@ -588,48 +608,66 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
         return lo;
     };
     const int lo_min = low(pos0);
-    const int* table = a.block_table + (size_t)b * a.table_width;
     const int kb_first = lo_min / FKB, kb_count = p_max / FKB - kb_first + 1;
     const int kb_lo = kb_first + (int)((long long)kb_count * split / a.splits);
     const int kb_hi = kb_first + (int)((long long)kb_count * (split + 1) / a.splits);
-    const int dch = dpad / 8, vch = own_v ? (vst - 8) / 8 : 0;
 
-    // lane l < KPW: where key warp * KPW + l of a block lies (null: no row sees it, or its page has been given back)
-    auto key_at = [&](int block) -> const bf16* {
-        const int n = block * FKB + warp * KPW + lane;
-        if (lane >= KPW || block >= kb_hi || n < lo_min || n > p_max) return nullptr;
-        if (dense) return (const bf16*)a.k_dense + (size_t)(t0 + n - pos0) * a.k_ld + (size_t)kvh * d;
-        const int page = table[n / a.page_size];
-        return page < 0 ? nullptr : cache + (size_t)page * a.page_stride + (size_t)kvh * a.head_stride + (size_t)(n % a.page_size) * a.slot;
-    };
-    auto bring = [&](int block, const bf16* at) {              // the warp's keys of a block, 16 bytes a copy
-        bf16* Ks = Ks0 + (block & 1) * stage;
+    if (warp == FWARPS) {
+        // ------------------------------------------------------------ producer
+        const int* table = a.block_table + (size_t)b * a.table_width;
+        const uint32_t k_bytes = (uint32_t)d * 2u, v_bytes = own_v ? (uint32_t)dv * 2u : 0u;
+        // what the kernel ahead wrote is the queries and the rows of this step's tokens; the keys of earlier steps are older
+        bool waited = false;
+        if (dense) { pdl_wait(); waited = true; }
+        for (int kb = kb_lo; kb < kb_hi; ++kb) {
+            const int i = kb - kb_lo, s = i % FSTAGES;
+            const uint32_t round = i / FSTAGES;
+            if (!waited && (kb * FKB + FKB > pos0 || round > 0)) { pdl_wait(); waited = true; }
+            const bf16* src[FKB / 32];
+            int valid = 0;
 #pragma unroll
-        for (int j = 0; j < KPW; ++j) {
-            const bf16* src = (const bf16*)__shfl_sync(0xffffffffu, (unsigned long long)at, j);
-            bf16* dst = Ks + (warp * KPW + j) * kst;
-            for (int c = lane; c < dch; c += 32) {
-                const bool ok = src && c * 8 < d;
-                cp_async_16(sm_addr(dst + c * 8), ok ? (const void*)(src + c * 8) : (const void*)q, ok ? 16 : 0);
+            for (int u = 0; u < FKB / 32; ++u) {
+                const int n = kb * FKB + u * 32 + lane;
+                src[u] = nullptr;
+                if (n >= lo_min && n <= p_max) {
+                    if (dense) src[u] = (const bf16*)a.k_dense + (size_t)(t0 + n - pos0) * a.k_ld + (size_t)kvh * d;
+                    else {
+                        const int page = table[n / a.page_size];
+                        if (page >= 0)
+                            src[u] = cache + (size_t)page * a.page_stride + (size_t)kvh * a.head_stride + (size_t)(n % a.page_size) * a.slot;
+                    }
+                }
+                valid += __popc(__ballot_sync(0xffffffffu, src[u] != nullptr));
             }
-            if (own_v) {
-                const int n = block * FKB + warp * KPW + j;
-                const bf16* vsrc = dense ? (const bf16*)a.v_dense + (size_t)(t0 + n - pos0) * a.v_ld + (size_t)kvh * dv : src + a.v_offset;
-                bf16* vdst = Ks + FKB * kst + (warp * KPW + j) * vst;
-                for (int c = lane; c < vch; c += 32) {
-                    const bool ok = src && c * 8 < dv;
-                    cp_async_16(sm_addr(vdst + c * 8), ok ? (const void*)(vsrc + c * 8) : (const void*)q, ok ? 16 : 0);
+            bool ok = true;
+            if (round > 0) {
+                if (lane == 0) ok = tc5::mbar_wait(empty_bar(s), (round - 1) & 1, abort_flag);
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+            }
+            if (!ok) break;
+            if (lane == 0) tc5::mbar_expect_tx(full_bar(s), (uint32_t)valid * (k_bytes + v_bytes));
+            __syncwarp();
+            bf16* Ks = Ks0 + s * stage;
+#pragma unroll
+            for (int u = 0; u < FKB / 32; ++u) {
+                if (!src[u]) continue;
+                const int kr = u * 32 + lane;
+                bulk_row(sm_addr(Ks + kr * kst), src[u], k_bytes, full_bar(s));
+                if (own_v) {
+                    const bf16* v = dense ? (const bf16*)a.v_dense + (size_t)(t0 + kb * FKB + kr - pos0) * a.v_ld + (size_t)kvh * dv
+                                          : src[u] + a.v_offset;
+                    bulk_row(sm_addr(Ks + FKB * kst + kr * vst), v, v_bytes, full_bar(s));
                 }
             }
         }
-    };
-    pdl_wait();
-    const bf16* at = key_at(kb_lo);
-    if (kb_lo < kb_hi) bring(kb_lo, at);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    at = key_at(kb_lo + 1);
+        if (!waited) pdl_wait();
+        return;
+    }
 
-    for (int idx = tid; idx < MROWS * dch; idx += MTHREADS) {
+    // ---------------------------------------------------------------- the others
+    pdl_wait();
+    const int dch = dpad / 8;
+    for (int idx = tid; idx < FROWS * dch; idx += FWARPS * 32) {
         const int rr = idx / dch, c = (idx % dch) * 8;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (rr < n_rows && c < d) v = *(const uint4*)(q + (size_t)(t0 + rr / G) * a.q_ld + (size_t)(kvh * G + rr % G) * d + c);
@@ -649,28 +687,34 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-    float m_run[4], l_run[4];                                   // softmax phase: warp w owns rows 4w .. 4w+3
+    constexpr int RPW = FROWS / FWARPS;                         // softmax: warp w owns rows RPW w ..
+    float m_run[RPW], l_run[RPW];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < RPW; ++i) {
         m_run[i] = -INFINITY; l_run[i] = 0.f;
-        if (a.sink && split == 0) { m_run[i] = a.sink[kvh * G + (warp * 4 + i) % G]; l_run[i] = 1.f; }
+        if (a.sink && split == 0) { m_run[i] = a.sink[kvh * G + (warp * RPW + i) % G]; l_run[i] = lane == 0 ? 1.f : 0.f; }
     }
+    few_barrier();                                              // the queries are there
 
     for (int kb = kb_lo; kb < kb_hi; ++kb) {
-        if (kb + 1 < kb_hi) bring(kb + 1, at);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        at = key_at(kb + 2);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();
-        const bf16* Ks = Ks0 + (kb & 1) * stage;
-        const bf16* Vs = own_v ? Ks + FKB * kst : Ks;
-        const int k0 = kb * FKB;
+        const int i = kb - kb_lo, st = i % FSTAGES, k0 = kb * FKB;
+        if (!tc5::mbar_wait(full_bar(st), (i / FSTAGES) & 1, abort_flag)) *abort_flag = 1;
+        bf16* Ks = Ks0 + st * stage;
+        bf16* Vs = own_v ? Ks + FKB * kst : Ks;
+        const int vs = own_v ? vst : kst;
+        if (k0 < lo_min || k0 + FKB - 1 > p_max) {              // rows that nobody asked for: their values must not be NaN
+            for (int kr = warp; kr < FKB; kr += FWARPS)
+                if (k0 + kr < lo_min || k0 + kr > p_max)
+                    for (int c = lane * 8; c < dv; c += 256) *(uint4*)(Vs + kr * vs + c) = make_uint4(0u, 0u, 0u, 0u);
+            tc5::fence_async_smem();                            // ahead of the bulk copies that come to these rows next
+            few_barrier();
+        }
         {   // S = Q K^T: 16 rows, keys warp*8 .. +8; two sums, so that a product does not wait for the one ahead of it
             float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
             const uint32_t qa = sm_addr(Qs + (lane & 15) * kst + (lane >> 4) * 8);
-            const uint32_t ka = sm_addr(Ks + (warp * KPW + (lane & 7)) * kst + (lane >> 3) * 8);
+            const uint32_t ka = sm_addr(Ks + (warp * FKPW + (lane & 7)) * kst + (lane >> 3) * 8);
             int kk = 0;
-#pragma unroll 2
+#pragma unroll 4
             for (; kk + 32 <= dpad; kk += 32) {
                 uint32_t a0[4], a1[4], bfr[4];
                 ldsm4(a0, qa + kk * 2);
@@ -679,10 +723,10 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
                 mma16816(s0, a0, bfr[0], bfr[1]);
                 mma16816(s1, a1, bfr[2], bfr[3]);
             }
-            if (kk < dpad) {
-                uint32_t a0[4], bfr[2];
+            if (kk < dpad) {                                    // (the matrices of lanes 16-31 are not used)
+                uint32_t a0[4], bfr[4];
                 ldsm4(a0, qa + kk * 2);
-                ldsm2(bfr, sm_addr(Ks + (warp * KPW + (lane & 7)) * kst + ((lane >> 3) & 1) * 8) + kk * 2);
+                ldsm4(bfr, sm_addr(Ks + (warp * FKPW + (lane & 7)) * kst + ((lane >> 3) & 1) * 8) + kk * 2);
                 mma16816(s0, a0, bfr[0], bfr[1]);
             }
             auto score = [&](float dot, float sc, float r1, float r2, int p, int lo, int n) -> float {
@@ -694,34 +738,37 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
             };
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int c = warp * KPW + fc + e;
+                const int c = warp * FKPW + fc + e;
                 Ss[ra * FSST + c] = score(s0[e] + s1[e], sa, r1a, r2a, pa, la, k0 + c);
                 Ss[rb * FSST + c] = score(s0[2 + e] + s1[2 + e], sb, r1b, r2b, pb, lb, k0 + c);
             }
         }
-        __syncthreads();
+        few_barrier();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int rr = warp * 4 + i;
-            const float x = Ss[rr * FSST + lane];
-            const float m_new = fmaxf(m_run[i], warp_max(x));
-            float alpha = 1.f, p0 = 0.f;
+        for (int r = 0; r < RPW; ++r) {
+            const int rr = warp * RPW + r;
+            const float x0 = Ss[rr * FSST + lane], x1 = Ss[rr * FSST + lane + 32];
+            const float m_new = fmaxf(m_run[r], warp_max(fmaxf(x0, x1)));
+            float alpha = 1.f, p0 = 0.f, p1 = 0.f;
             if (m_new != -INFINITY) {
-                alpha = (m_run[i] == -INFINITY) ? 0.f : expf(m_run[i] - m_new);
-                p0 = expf(x - m_new);
+                alpha = (m_run[r] == -INFINITY) ? 0.f : expf(m_run[r] - m_new);
+                p0 = expf(x0 - m_new); p1 = expf(x1 - m_new);
             }
-            l_run[i] = l_run[i] * alpha + warp_sum(p0);
-            m_run[i] = m_new;
+            l_run[r] = l_run[r] * alpha + (p0 + p1);            // a lane's own share; the warp's are added at the end
+            m_run[r] = m_new;
             Pb[rr * FPST + lane] = __float2bfloat16_rn(p0);
+            Pb[rr * FPST + lane + 32] = __float2bfloat16_rn(p1);
             if (lane == 0) alpha_s[rr] = alpha;
         }
-        __syncthreads();
+        few_barrier();
         {   // O += P V: 16 rows, columns warp*NT*8 .. + NT*8
             const float al_a = alpha_s[ra], al_b = alpha_s[rb];
+            if (__any_sync(0xffffffffu, al_a != 1.f || al_b != 1.f)) {
 #pragma unroll
-            for (int j = 0; j < NT; ++j) { o[j][0] *= al_a; o[j][1] *= al_a; o[j][2] *= al_b; o[j][3] *= al_b; }
+                for (int j = 0; j < NT; ++j) { o[j][0] *= al_a; o[j][1] *= al_a; o[j][2] *= al_b; o[j][3] *= al_b; }
+            }
             const uint32_t pa_addr = sm_addr(Pb + (lane & 15) * FPST + (lane >> 4) * 8);
-            const uint32_t va = sm_addr(Vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + warp * NT * 8 + (lane >> 4) * 8);
+            const uint32_t va = sm_addr(Vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vs + warp * NT * 8 + (lane >> 4) * 8);
 #pragma unroll
             for (int kk = 0; kk < FKB; kk += 16) {
                 uint32_t af[4];
@@ -729,19 +776,26 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
 #pragma unroll
                 for (int j2 = 0; j2 < NT / 2; ++j2) {
                     uint32_t bfr[4];
-                    ldsm4t(bfr, va + (kk * vst + j2 * 16) * 2);
+                    ldsm4t(bfr, va + (kk * vs + j2 * 16) * 2);
                     mma16816(o[2 * j2], af, bfr[0], bfr[1]);
                     mma16816(o[2 * j2 + 1], af, bfr[2], bfr[3]);
                 }
             }
         }
-        __syncthreads();                                        // everyone is done with the stage and the probabilities
+        __syncwarp();
+        if (lane == 0) tc5::mbar_arrive(empty_bar(st));         // this warp is done with the stage
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        if (lane == 0) { alpha_s[warp * 4 + i] = l_run[i]; m_fin[warp * 4 + i] = m_run[i]; }
-    __syncthreads();
+    for (int r = 0; r < RPW; ++r) {
+        const float l = warp_sum(l_run[r]);
+        if (lane == 0) { alpha_s[warp * RPW + r] = l; m_fin[warp * RPW + r] = m_run[r]; }
+    }
+    few_barrier();
+    if (*abort_flag) {
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);         // copies in flight land before the CTA leaves
+        if (tid == 0) atomicExch(error_flag, 1);
+        return;
+    }
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
         const int r = side ? rb : ra;
@@ -763,6 +817,29 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
             }
         if (a.splits > 1 && warp == 0 && fc == 0) { a.part_ml[2 * slot] = m_fin[r]; a.part_ml[2 * slot + 1] = alpha_s[r]; }
     }
+}
+
+// Launches it (without the merge of the shares); TFF_ERR_UNSUPPORTED for heads too large for two stages of keys.
+template <int NT>
+int launch_few(const void* q, const void* cache, void* out, const TileArgs& a, int num_requests, cudaStream_t stream) {
+    const bool own_v = a.v_offset != 0 || a.k_dense != nullptr;
+    MmaGeom gm;
+    gm.dpad = (a.d + 15) / 16 * 16;
+    gm.kst = (own_v ? gm.dpad : max(gm.dpad, NT * 64)) + 8;
+    gm.vst = own_v ? NT * 64 + 8 : gm.kst;
+    const size_t smem = 2 * ((size_t)FROWS * gm.kst + (size_t)FSTAGES * FKB * (gm.kst + (own_v ? gm.vst : 0)) + FROWS * FPST) +
+                        4 * ((size_t)FROWS * FSST + 2 * FROWS) + 8 * 2 * FSTAGES + 16;
+    if (smem > 220 * 1024) return TFF_ERR_UNSUPPORTED;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(attention_tile_few_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
+            return TFF_ERR_LAUNCH;
+        configured = true;
+    }
+    int* flag = tff_device_error_flag();
+    if (flag == nullptr) return TFF_ERR_LAUNCH;
+    return tff_launch_pdl(attention_tile_few_kernel<NT>, dim3(a.splits, a.nkv, num_requests), dim3(FTHREADS), smem, stream, (const bf16*)q,
+                          (const bf16*)cache, (bf16*)out, a, gm, flag);
 }
 
 static bool tile_mma_enabled() {
@@ -790,18 +867,26 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
     gm.kst = (own_v ? gm.dpad : max(gm.dpad, nt * 32)) + 8;
     gm.vst = own_v ? nt * 32 + 8 : gm.kst;
     const int rows_most = max_q_len * G;
-    const int rg = rows_most <= 16 ? 1 : (rows_most <= 32 ? 2 : 4);
+    const int rg = rows_most <= 16 ? 1 : (rows_most <= 32 ? 2 : 4);       // (one group: heads too large for the kernel of few rows)
     const int MROWS = 16 * rg;
-    const size_t smem = rg == 1 ? 2 * ((size_t)16 * gm.kst + (size_t)FSTAGES * FKB * (gm.kst + (own_v ? gm.vst : 0)) + 16 * FPST) +
-                                      4 * ((size_t)16 * FSST + 2 * 16)
-                                : 2 * ((size_t)(MROWS + MKB) * gm.kst + (own_v ? (size_t)MKB * gm.vst : 0) + (size_t)MROWS * PST) +
+    if (rows_most <= FROWS) {
+        int st = a.dv <= 128 ? launch_few<2>(q, cache, out, a, num_requests, stream)
+               : a.dv <= 256 ? launch_few<4>(q, cache, out, a, num_requests, stream)
+                             : launch_few<8>(q, cache, out, a, num_requests, stream);
+        if (st == TFF_OK && a.splits > 1)
+            st = tff_launch_pdl(attention_tile_merge_kernel<bf16>, dim3((unsigned)(num_tokens * a.nq)), dim3(MERGE_THREADS), 0, stream,
+                                (const float*)a.part_o, (const float*)a.part_ml, (bf16*)out, a.out_ld, a.out_off, a.nq, a.dv, a.splits,
+                                a.out_scale);
+        if (st != TFF_ERR_UNSUPPORTED) return st;
+    }
+    const size_t smem = 2 * ((size_t)(MROWS + MKB) * gm.kst + (own_v ? (size_t)MKB * gm.vst : 0) + (size_t)MROWS * PST) +
                         4 * ((size_t)MROWS * SST + 2 * MROWS) + 4 * 2 * MROWS + 2 * 8 * MKB;
     if (smem > 220 * 1024) return TFF_ERR_UNSUPPORTED;
     const int tiles = (rows_most + MROWS - 1) / MROWS;
     dim3 grid(tiles * a.splits, a.nkv, num_requests);
 #define TFF_TMMA(NTV)                                                                                                \
     do {                                                                                                             \
-        if (rg == 1) TFF_TMMA_RUN((attention_tile_few_kernel<NTV>), 128);                                            \
+        if (rg == 1) TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 1>), 128);                                         \
         if (rg == 2) TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 2>), 256);                                         \
         TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 4>), 512);                                                      \
     } while (0)

@@ -993,7 +993,13 @@ class CudaKernels:
             planes, slot = kv_cache.shape[2], kv_cache.shape[-1]
             assert kv_cache.dtype == q.dtype and tuple(kv_cache.shape[3:5]) == (nkv, page_size)
             c_ptr, page_stride = self._layer_cache(kv_cache, kv_layer)
-        splits = self.tile_splits(batch, nq, nkv, window, chunk) if num_splits is None else int(num_splits)
+        if num_splits is not None:
+            splits = int(num_splits)
+        elif q.dtype == torch.bfloat16 and batch.max_q_len * (nq // nkv) <= 16 and d % 8 == 0 and dv <= 512:
+            # the kernel of few rows: two stages of 64 keys (and values) in shared memory say how many CTAs an SM has
+            splits = self.few_row_splits(batch, nkv, 1 if d + (dv if planes == 2 else 0) > 384 else 2, window, chunk)
+        else:
+            splits = self.tile_splits(batch, nq, nkv, window, chunk)
         part_o = part_ml = None
         if splits > 1:
             part_o = torch.empty(T * nq * splits * dv, dtype=torch.float32, device=q.device)
@@ -1026,6 +1032,14 @@ class CudaKernels:
             _c_int(batch.num_requests), _c_int(batch.max_q_len), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(dv),
             _c_float(scale), _c_int(window), _c_float(softcap), _ptr(sink), self._stream()), "attention_dense")
         self.launches += 1
+
+    def few_row_splits(self, batch, nkv: int, per_sm: int, window: int = 0, chunk: int = 0) -> int:
+        """In how many shares attention_tile cuts the keys of steps of few rows (at most 32): the count whose rounds of CTAs,
+        ``per_sm`` an SM, take the least time, a CTA's time being its blocks of 64 keys and about two more to start and finish."""
+        items = nkv * batch.num_requests
+        blocks = -(-min([s for s in (window, chunk) if s > 0] + [int(batch.max_kv_len)]) // 64)
+        cost = lambda s: -(-items * s // (per_sm * self.NUM_SMS)) * (-(-blocks // s) + 2)
+        return min(range(1, min(32, max(1, blocks)) + 1), key=lambda s: (cost(s), s))
 
     def tile_splits(self, batch, nq: int, nkv: int, window: int = 0, chunk: int = 0) -> int:
         """In how many shares attention_tile cuts every tile's key range: a power of two such that a step of few rows
