@@ -546,15 +546,16 @@ attention_tile_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     }
 }
 
-// Steps of at most 16 packed rows a (request, kv head) -- decoded tokens -- are a stream of the cache.  A CTA walks its share of the
-// keys in blocks of 64, two of them in shared memory:
+// Steps of at most 32 packed rows a (request, kv head) -- decoded tokens -- are a stream of the cache.  A CTA takes 16 rows and walks
+// its share of the keys in blocks of 32, two of them in shared memory, so that with the rows of a latent cache (576 elements) two
+// CTAs share an SM:
 //   warp 8      producer: a lane a key looks up where it lies and asks for its row (rows, with values of their own) by one
 //               bulk copy into a row padded by 16 bytes (ldmatrix without bank conflicts), a block ahead of the others
-//   warps 0-7   S = Q K^T (8 keys each) to shared memory; softmax (two rows each); O += P V (an eighth of the columns each)
-// What bounds it: with the tiles above (four warps a group of rows, sixteen instructions for every 16 bytes it copied) an SM issued an
-// instruction in a quarter of the cycles and every warp's chain of shared-memory loads and products set the pace.
-constexpr int FKB = 64, FROWS = 16, FWARPS = 8, FTHREADS = (FWARPS + 1) * 32, FPST = FKB + 8, FSST = FKB + 4, FSTAGES = 2;
-constexpr int FKPW = FKB / FWARPS;                                  // keys a warp scores
+//   warps 0-7   S = Q K^T (8 keys and half of the elements each) to shared memory; softmax (two rows each); O += P V (an eighth
+//               of the columns each)
+// What bounds it: the chain of a block (scores, softmax, values, a barrier after each), which the SM's other CTA fills.
+constexpr int FKB = 32, FROWS = 16, FMOST = 32, FWARPS = 8, FTHREADS = (FWARPS + 1) * 32, FPST = FKB + 8, FSST = FKB + 4, FSTAGES = 2;
+constexpr int FKPW = FKB / 4;                                       // keys a warp scores
 
 __device__ __forceinline__ void few_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ void bulk_row(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -563,7 +564,7 @@ __device__ __forceinline__ void bulk_row(uint32_t dst, const void* src, uint32_t
 }
 
 template <int NT>
-__global__ void __launch_bounds__(FTHREADS)
+__global__ void __launch_bounds__(FTHREADS, 2)
 attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, bf16* __restrict__ out, TileArgs a,
                           MmaGeom gm, int* error_flag) {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -575,8 +576,8 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     bf16* Qs = (bf16*)smraw;                                    // [FROWS][kst]
     bf16* Ks0 = Qs + FROWS * kst;                               // stages of [FKB][kst] (and [FKB][vst])
     bf16* Pb = Ks0 + FSTAGES * stage;                           // [FROWS][FPST] probabilities
-    float* Ss = (float*)(Pb + FROWS * FPST);                    // [FROWS][FSST] scores
-    float* alpha_s = Ss + FROWS * FSST;                         // [FROWS]
+    float* Ss = (float*)(Pb + FROWS * FPST);                    // [2][FROWS][FSST] products of each half of the elements
+    float* alpha_s = Ss + 2 * FROWS * FSST;                     // [FROWS]
     float* m_fin = alpha_s + FROWS;                             // [FROWS]
     const uint32_t bars = sm_addr(m_fin + FROWS);               // full[FSTAGES], empty[FSTAGES] (8-byte aligned: an even number of words lies ahead)
     volatile int* abort_flag = (volatile int*)(m_fin + FROWS + 4 * FSTAGES);
@@ -597,17 +598,17 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     __syncthreads();
     pdl_launch_dependents();
     const int t0 = a.q_start[b], q_len = a.q_start[b + 1] - t0, pos0 = a.pos_start[b];
-    const int split = blockIdx.x;
-    const int n_rows = q_len * G;                               // at most FROWS
+    const int split = blockIdx.x % a.splits, r0 = blockIdx.x / a.splits * FROWS;
+    const int n_rows = min(q_len * G - r0, FROWS);
     if (n_rows <= 0) return;
-    const int p_max = pos0 + q_len - 1;
+    const int p_max = pos0 + (r0 + n_rows - 1) / G;
     auto low = [&](int p) {
         int lo = 0;
         if (a.window > 0) lo = max(lo, p - a.window + 1);
         if (a.chunk > 0) lo = max(lo, (p / a.chunk) * a.chunk);
         return lo;
     };
-    const int lo_min = low(pos0);
+    const int lo_min = low(pos0 + r0 / G);
     const int kb_first = lo_min / FKB, kb_count = p_max / FKB - kb_first + 1;
     const int kb_lo = kb_first + (int)((long long)kb_count * split / a.splits);
     const int kb_hi = kb_first + (int)((long long)kb_count * (split + 1) / a.splits);
@@ -670,29 +671,30 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     for (int idx = tid; idx < FROWS * dch; idx += FWARPS * 32) {
         const int rr = idx / dch, c = (idx % dch) * 8;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (rr < n_rows && c < d) v = *(const uint4*)(q + (size_t)(t0 + rr / G) * a.q_ld + (size_t)(kvh * G + rr % G) * d + c);
+        if (rr < n_rows && c < d) v = *(const uint4*)(q + (size_t)(t0 + (r0 + rr) / G) * a.q_ld + (size_t)(kvh * G + (r0 + rr) % G) * d + c);
         *(uint4*)(Qs + rr * kst + c) = v;
     }
     const int fr = lane >> 2, fc = 2 * (lane & 3);              // a thread's place in an accumulator tile: rows fr, fr+8; columns fc, fc+1
     const int ra = fr, rb = fr + 8;
-    const int pa = ra < n_rows ? pos0 + ra / G : -1, pb = rb < n_rows ? pos0 + rb / G : -1;
-    const int la = pa >= 0 ? low(pa) : 0, lb = pb >= 0 ? low(pb) : 0;
-    const int ha = kvh * G + ra % G, hb = kvh * G + rb % G;
-    const float sa = a.scale * (a.temp ? a.temp[ha] : 1.f), sb = a.scale * (a.temp ? a.temp[hb] : 1.f);
-    const bool biased = a.r1 != nullptr;
-    const float r1a = biased ? a.r1[ha] : 0.f, r2a = biased ? a.r2[ha] : 0.f;
-    const float r1b = biased ? a.r1[hb] : 0.f, r2b = biased ? a.r2[hb] : 0.f;
     float o[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
     constexpr int RPW = FROWS / FWARPS;                         // softmax: warp w owns rows RPW w ..
-    float m_run[RPW], l_run[RPW];
+    float m_run[RPW], l_run[RPW], sc[RPW], r1[RPW], r2[RPW];
+    int rp[RPW], rlo[RPW];
+    const bool biased = a.r1 != nullptr;
 #pragma unroll
     for (int i = 0; i < RPW; ++i) {
+        const int r = r0 + warp * RPW + i, h = kvh * G + r % G;
+        rp[i] = warp * RPW + i < n_rows ? pos0 + r / G : -1;
+        rlo[i] = rp[i] >= 0 ? low(rp[i]) : 0;
+        sc[i] = a.scale * (a.temp ? a.temp[h] : 1.f);
+        r1[i] = biased ? a.r1[h] : 0.f;
+        r2[i] = biased ? a.r2[h] : 0.f;
         m_run[i] = -INFINITY; l_run[i] = 0.f;
-        if (a.sink && split == 0) { m_run[i] = a.sink[kvh * G + (warp * RPW + i) % G]; l_run[i] = lane == 0 ? 1.f : 0.f; }
+        if (a.sink && split == 0) { m_run[i] = a.sink[h]; l_run[i] = lane == 0 ? 1.f : 0.f; }
     }
     few_barrier();                                              // the queries are there
 
@@ -709,13 +711,15 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
             tc5::fence_async_smem();                            // ahead of the bulk copies that come to these rows next
             few_barrier();
         }
-        {   // S = Q K^T: 16 rows, keys warp*8 .. +8; two sums, so that a product does not wait for the one ahead of it
+        {   // Q K^T: 16 rows, 8 keys, half of the elements; two sums, so that a product does not wait for the one ahead of it
             float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+            const int kg = warp & 3, half = warp >> 2, n32 = dpad / 32;
             const uint32_t qa = sm_addr(Qs + (lane & 15) * kst + (lane >> 4) * 8);
-            const uint32_t ka = sm_addr(Ks + (warp * FKPW + (lane & 7)) * kst + (lane >> 3) * 8);
-            int kk = 0;
+            const uint32_t ka = sm_addr(Ks + (kg * FKPW + (lane & 7)) * kst + (lane >> 3) * 8);
+            int kk = half ? n32 / 2 * 32 : 0;
+            const int k_end = half ? n32 * 32 : n32 / 2 * 32;
 #pragma unroll 4
-            for (; kk + 32 <= dpad; kk += 32) {
+            for (; kk < k_end; kk += 32) {
                 uint32_t a0[4], a1[4], bfr[4];
                 ldsm4(a0, qa + kk * 2);
                 ldsm4(a1, qa + kk * 2 + 32);
@@ -723,41 +727,35 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
                 mma16816(s0, a0, bfr[0], bfr[1]);
                 mma16816(s1, a1, bfr[2], bfr[3]);
             }
-            if (kk < dpad) {                                    // (the matrices of lanes 16-31 are not used)
+            if (half && kk < dpad) {                            // (the matrices of lanes 16-31 are not used)
                 uint32_t a0[4], bfr[4];
                 ldsm4(a0, qa + kk * 2);
-                ldsm4(bfr, sm_addr(Ks + (warp * FKPW + (lane & 7)) * kst + ((lane >> 3) & 1) * 8) + kk * 2);
+                ldsm4(bfr, sm_addr(Ks + (kg * FKPW + (lane & 7)) * kst + ((lane >> 3) & 1) * 8) + kk * 2);
                 mma16816(s0, a0, bfr[0], bfr[1]);
             }
-            auto score = [&](float dot, float sc, float r1, float r2, int p, int lo, int n) -> float {
-                if (p < 0 || n > p || n < lo) return -INFINITY;
-                float s = dot * sc;
-                if (a.softcap > 0.f) s = a.softcap * attn_tanh(s / a.softcap);
-                if (biased) s -= r1 * log1pf(r2 * (float)(p - n));
-                return s;
-            };
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = warp * FKPW + fc + e;
-                Ss[ra * FSST + c] = score(s0[e] + s1[e], sa, r1a, r2a, pa, la, k0 + c);
-                Ss[rb * FSST + c] = score(s0[2 + e] + s1[2 + e], sb, r1b, r2b, pb, lb, k0 + c);
-            }
+            float* S = Ss + half * FROWS * FSST + kg * FKPW + fc;
+            *(float2*)(S + ra * FSST) = make_float2(s0[0] + s1[0], s0[1] + s1[1]);
+            *(float2*)(S + rb * FSST) = make_float2(s0[2] + s1[2], s0[3] + s1[3]);
         }
         few_barrier();
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-            const int rr = warp * RPW + r;
-            const float x0 = Ss[rr * FSST + lane], x1 = Ss[rr * FSST + lane + 32];
-            const float m_new = fmaxf(m_run[r], warp_max(fmaxf(x0, x1)));
-            float alpha = 1.f, p0 = 0.f, p1 = 0.f;
+            const int rr = warp * RPW + r, n = k0 + lane;
+            float x = -INFINITY;
+            if (n <= rp[r] && n >= rlo[r]) {
+                x = (Ss[rr * FSST + lane] + Ss[(FROWS + rr) * FSST + lane]) * sc[r];
+                if (a.softcap > 0.f) x = a.softcap * attn_tanh(x / a.softcap);
+                if (biased) x -= r1[r] * log1pf(r2[r] * (float)(rp[r] - n));
+            }
+            const float m_new = fmaxf(m_run[r], warp_max(x));
+            float alpha = 1.f, p0 = 0.f;
             if (m_new != -INFINITY) {
                 alpha = (m_run[r] == -INFINITY) ? 0.f : expf(m_run[r] - m_new);
-                p0 = expf(x0 - m_new); p1 = expf(x1 - m_new);
+                p0 = expf(x - m_new);
             }
-            l_run[r] = l_run[r] * alpha + (p0 + p1);            // a lane's own share; the warp's are added at the end
+            l_run[r] = l_run[r] * alpha + p0;                   // a lane's own share; the warp's are added at the end
             m_run[r] = m_new;
             Pb[rr * FPST + lane] = __float2bfloat16_rn(p0);
-            Pb[rr * FPST + lane + 32] = __float2bfloat16_rn(p1);
             if (lane == 0) alpha_s[rr] = alpha;
         }
         few_barrier();
@@ -800,7 +798,7 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     for (int side = 0; side < 2; ++side) {
         const int r = side ? rb : ra;
         if (r >= n_rows) continue;
-        const int t = t0 + r / G, h = kvh * G + r % G;
+        const int t = t0 + (r0 + r) / G, h = kvh * G + (r0 + r) % G;
         const size_t slot = ((size_t)t * a.nq + h) * a.splits + split;
         const float inv = a.splits == 1 ? a.out_scale / alpha_s[r] : 1.f;
         bf16* orow = out + (size_t)t * a.out_ld + a.out_off + (size_t)h * dv;
@@ -821,14 +819,14 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
 
 // Launches it (without the merge of the shares); TFF_ERR_UNSUPPORTED for heads too large for two stages of keys.
 template <int NT>
-int launch_few(const void* q, const void* cache, void* out, const TileArgs& a, int num_requests, cudaStream_t stream) {
+int launch_few(const void* q, const void* cache, void* out, const TileArgs& a, int num_requests, int rows, cudaStream_t stream) {
     const bool own_v = a.v_offset != 0 || a.k_dense != nullptr;
     MmaGeom gm;
     gm.dpad = (a.d + 15) / 16 * 16;
     gm.kst = (own_v ? gm.dpad : max(gm.dpad, NT * 64)) + 8;
     gm.vst = own_v ? NT * 64 + 8 : gm.kst;
     const size_t smem = 2 * ((size_t)FROWS * gm.kst + (size_t)FSTAGES * FKB * (gm.kst + (own_v ? gm.vst : 0)) + FROWS * FPST) +
-                        4 * ((size_t)FROWS * FSST + 2 * FROWS) + 8 * 2 * FSTAGES + 16;
+                        4 * ((size_t)2 * FROWS * FSST + 2 * FROWS) + 8 * 2 * FSTAGES + 16;
     if (smem > 220 * 1024) return TFF_ERR_UNSUPPORTED;
     static bool configured = false;
     if (!configured) {
@@ -838,7 +836,7 @@ int launch_few(const void* q, const void* cache, void* out, const TileArgs& a, i
     }
     int* flag = tff_device_error_flag();
     if (flag == nullptr) return TFF_ERR_LAUNCH;
-    return tff_launch_pdl(attention_tile_few_kernel<NT>, dim3(a.splits, a.nkv, num_requests), dim3(FTHREADS), smem, stream, (const bf16*)q,
+    return tff_launch_pdl(attention_tile_few_kernel<NT>, dim3((rows + FROWS - 1) / FROWS * a.splits, a.nkv, num_requests), dim3(FTHREADS), smem, stream, (const bf16*)q,
                           (const bf16*)cache, (bf16*)out, a, gm, flag);
 }
 
@@ -869,10 +867,10 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
     const int rows_most = max_q_len * G;
     const int rg = rows_most <= 16 ? 1 : (rows_most <= 32 ? 2 : 4);       // (one group: heads too large for the kernel of few rows)
     const int MROWS = 16 * rg;
-    if (rows_most <= FROWS) {
-        int st = a.dv <= 128 ? launch_few<2>(q, cache, out, a, num_requests, stream)
-               : a.dv <= 256 ? launch_few<4>(q, cache, out, a, num_requests, stream)
-                             : launch_few<8>(q, cache, out, a, num_requests, stream);
+    if (rows_most <= FMOST) {
+        int st = a.dv <= 128 ? launch_few<2>(q, cache, out, a, num_requests, rows_most, stream)
+               : a.dv <= 256 ? launch_few<4>(q, cache, out, a, num_requests, rows_most, stream)
+                             : launch_few<8>(q, cache, out, a, num_requests, rows_most, stream);
         if (st == TFF_OK && a.splits > 1)
             st = tff_launch_pdl(attention_tile_merge_kernel<bf16>, dim3((unsigned)(num_tokens * a.nq)), dim3(MERGE_THREADS), 0, stream,
                                 (const float*)a.part_o, (const float*)a.part_ml, (bf16*)out, a.out_ld, a.out_off, a.nq, a.dv, a.splits,

@@ -995,9 +995,8 @@ class CudaKernels:
             c_ptr, page_stride = self._layer_cache(kv_cache, kv_layer)
         if num_splits is not None:
             splits = int(num_splits)
-        elif q.dtype == torch.bfloat16 and batch.max_q_len * (nq // nkv) <= 16 and d % 8 == 0 and dv <= 512:
-            # the kernel of few rows: two stages of 64 keys (and values) in shared memory say how many CTAs an SM has
-            splits = self.few_row_splits(batch, nkv, 1 if d + (dv if planes == 2 else 0) > 384 else 2, window, chunk)
+        elif q.dtype == torch.bfloat16 and batch.max_q_len * (nq // nkv) <= 32 and d % 8 == 0 and dv <= 512:
+            splits = self.few_row_splits(batch, -(-batch.max_q_len * (nq // nkv) // 16) * nkv, window, chunk)
         else:
             splits = self.tile_splits(batch, nq, nkv, window, chunk)
         part_o = part_ml = None
@@ -1033,12 +1032,13 @@ class CudaKernels:
             _c_float(scale), _c_int(window), _c_float(softcap), _ptr(sink), self._stream()), "attention_dense")
         self.launches += 1
 
-    def few_row_splits(self, batch, nkv: int, per_sm: int, window: int = 0, chunk: int = 0) -> int:
-        """In how many shares attention_tile cuts the keys of steps of few rows (at most 32): the count whose rounds of CTAs,
-        ``per_sm`` an SM, take the least time, a CTA's time being its blocks of 64 keys and about two more to start and finish."""
-        items = nkv * batch.num_requests
-        blocks = -(-min([s for s in (window, chunk) if s > 0] + [int(batch.max_kv_len)]) // 64)
-        cost = lambda s: -(-items * s // (per_sm * self.NUM_SMS)) * (-(-blocks // s) + 2)
+    def few_row_splits(self, batch, tiles: int, window: int = 0, chunk: int = 0) -> int:
+        """In how many shares attention_tile cuts the keys of steps of few rows (at most 32), ``tiles`` tiles of 16 rows a request:
+        the count whose rounds of CTAs, two an SM, take the least time, a CTA's time being its blocks of 32 keys and about four
+        more to start and finish."""
+        items = tiles * batch.num_requests
+        blocks = -(-min([s for s in (window, chunk) if s > 0] + [int(batch.max_kv_len)]) // 32)
+        cost = lambda s: -(-items * s // (2 * self.NUM_SMS)) * (-(-blocks // s) + 4)
         return min(range(1, min(32, max(1, blocks)) + 1), key=lambda s: (cost(s), s))
 
     def tile_splits(self, batch, nq: int, nkv: int, window: int = 0, chunk: int = 0) -> int:
