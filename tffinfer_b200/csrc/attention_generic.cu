@@ -31,7 +31,7 @@ constexpr int WARPS = 4, BLOCK = 32, CHUNK = 128, PER_CHUNK = CHUNK / BLOCK;
 
 struct GenericParams {
     const int *q_start, *pos_start, *block_table;
-    int table_width, row_stride, layer, nq, nkv, d, dv, window, sink, keep, splits, slots, stages, vec, q_vec;
+    int table_width, row_stride, layer, nq, nkv, d, dv, window, sink, keep, splits, slots, stages, vec;
     float scale, softcap;
     const float *sink_val, *gate;
     float *part_o, *part_ml;
@@ -49,7 +49,6 @@ __device__ __forceinline__ void join(float& m, float& l, float mc, float lc, flo
 }
 __device__ __forceinline__ float join_value(float o, float a, float oc, float b) { return __fmaf_rn(o, a, __fmul_rn(oc, b)); }
 
-__device__ __forceinline__ float4 load4(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 load4(const bf16* p) {
     const uint2 u = *(const uint2*)p;
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
@@ -81,41 +80,33 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
     const int per = (walk.count + p.splits - 1) / p.splits, w0 = split * per, w1 = min(walk.count, w0 + per);
     if (w0 >= w1) return;
 
-#pragma unroll 4
     for (int i = threadIdx.x; i < WARPS * RW * k4; i += WARPS * 32) {
         const int r = row0 + i / k4, c = (i % k4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < rows) {
             const T* src = q_in + (size_t)(q0 + r / G) * p.row_stride + (size_t)(kvh * G + r % G) * p.d + c;
-            if (p.q_vec) {
-                v = load4(src);
-            } else {
-                v.x = to_f32<T>(src[0]);
-                if (c + 1 < p.d) v.y = to_f32<T>(src[1]);
-                if (c + 2 < p.d) v.z = to_f32<T>(src[2]);
-                if (c + 3 < p.d) v.w = to_f32<T>(src[3]);
-            }
+            v.x = to_f32<T>(src[0]);
+            if (c + 1 < p.d) v.y = to_f32<T>(src[1]);
+            if (c + 2 < p.d) v.z = to_f32<T>(src[2]);
+            if (c + 3 < p.d) v.w = to_f32<T>(src[3]);
         }
         sq[i] = v;
     }
 
     auto live = [&](int n0) { return n0 <= hi && (n0 + BLOCK - 1 >= lo_tile || n0 < p.keep); };
-    // Where key n0 + lane lies: null for keys that no row of the tile sees (their slots may hold anything, and their pages may
-    // have been given back), whose stage rows become zeros.  Looked up a block ahead of the copies.
-    auto locate = [&](int n0) -> const T* {
-        const int n = n0 + lane;
-        if (n > hi || !(n >= lo_tile || n < p.keep)) return nullptr;
-        return cache + (size_t)table[n / p.L.page_size] * p.L.page_stride + (size_t)p.layer * p.L.layer_stride +
-               (size_t)kvh * p.L.head_stride + (size_t)(n % p.L.page_size) * p.L.head_dim;
-    };
-    auto fetch = [&](const T* at, int stage) {
+    // Keys and values n0 .. n0 + 31 to a stage; those that no row of the tile sees are zeros (their slots may hold anything,
+    // and their pages may have been given back).
+    auto fetch = [&](int n0, int stage) {
         float4* sk = smem4 + stage * stage4;
         float4* sv = sk + BLOCK * ks;
-#pragma unroll 2
         for (int kr = warp; kr < BLOCK; kr += WARPS) {
-            const T* kp = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)at, kr);
-            const bool ok = kp != nullptr;
-            const T* vp = kp + p.L.kv_stride;
+            const int n = n0 + kr;
+            const bool ok = n <= hi && (n >= lo_tile || n < p.keep);
+            const T* kp = nullptr;
+            if (ok)
+                kp = cache + (size_t)table[n / p.L.page_size] * p.L.page_stride + (size_t)p.layer * p.L.layer_stride +
+                     (size_t)kvh * p.L.head_stride + (size_t)(n % p.L.page_size) * p.L.head_dim;
+            const T* vp = ok ? kp + p.L.kv_stride : nullptr;
             auto row = [&](const T* src, int n4, int len, float4* dst) {
                 for (int c = lane; c < n4; c += 32) {
                     if (!ok) dst[c] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -160,23 +151,19 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
 
     const int total = (w1 - w0) * PER_CHUNK;
     auto block_start = [&](int i) { return walk.block(w0 + i / PER_CHUNK) * CHUNK + (i % PER_CHUNK) * BLOCK; };
-    const T* at = locate(block_start(0));
     if (p.stages > 1) {
-        if (live(block_start(0))) fetch(at, 0);
+        if (live(block_start(0))) fetch(block_start(0), 0);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (total > 1) at = locate(block_start(1));
     }
     for (int i = 0; i < total; ++i) {
         const int n0 = block_start(i), stage = p.stages > 1 ? (i & 1) : 0;
         if (p.stages > 1) {
-            if (i + 1 < total && live(block_start(i + 1))) fetch(at, stage ^ 1);
+            if (i + 1 < total && live(block_start(i + 1))) fetch(block_start(i + 1), stage ^ 1);
             asm volatile("cp.async.commit_group;" ::: "memory");
-            if (i + 2 < total) at = locate(block_start(i + 2));
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
-            if (live(n0)) fetch(at, 0);
+            if (live(n0)) fetch(n0, 0);
             asm volatile("cp.async.wait_all;" ::: "memory");
-            if (i + 1 < total) at = locate(block_start(i + 1));
         }
         __syncthreads();
         if (live(n0) && wrow < rows) {
@@ -413,7 +400,6 @@ TFF_API int tff_attention_generic(
         return TFF_ERR_BAD_ARGUMENT;
     if (p.splits > 1) { p.part_ml = ws; p.part_o = ws + (size_t)num_tokens * nq * p.slots * 2; }
     // 4 elements are read at a time where rows and slots are whole groups at aligned addresses
-    p.q_vec = d % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)qkv & 15) == 0;
     p.vec = d % 4 == 0 && dv % 4 == 0 && dc % 4 == 0 && ((uintptr_t)cache & 15) == 0;
     int st = is_bf16 ? dispatch<bf16>(qkv, cache, out, p, num_requests, max_q_len, stream)
                      : dispatch<float>(qkv, cache, out, p, num_requests, max_q_len, stream);

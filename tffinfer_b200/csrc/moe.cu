@@ -74,7 +74,7 @@ moe_route_kernel(const TH* __restrict__ h, const TW* __restrict__ w_router, cons
     // A warp takes up to RE outputs side by side (a row's elements are read once for them), a lane eight neighbouring
     // elements a load where the rows allow it (16-byte loads, several in flight), else one.  Either way the order of a dot
     // product's additions is fixed by W alone.  (Index E is the row beside the router's, when there is one.)
-    constexpr int RE = ROUTE_TOK > 1 ? 3 : 1, RW = ROUTE_THREADS / 32, UNROLL = ROUTE_TOK > 1 ? 4 : 16;
+    constexpr int RE = ROUTE_TOK > 1 ? 3 : 1, RW = ROUTE_THREADS / 32, UNROLL = ROUTE_TOK > 1 ? 2 : 8;
     const bool wide = (W & 7) == 0 && (((size_t)w_router | (size_t)row_w) & 15) == 0;
     const int outputs = E + (row_w ? 1 : 0);
     for (int e0 = warp; e0 < outputs; e0 += RW * RE) {
@@ -89,27 +89,29 @@ moe_route_kernel(const TH* __restrict__ h, const TW* __restrict__ w_router, cons
         }
         if (wide) {
 #pragma unroll UNROLL
-            for (int i = lane * 4; i < W; i += 128) {
-                float w4[RE][4];
+            for (int i = lane * 8; i < W; i += 256) {
+                float w8[RE][8];
 #pragma unroll
                 for (int x = 0; x < RE; ++x) {
                     if constexpr (sizeof(TW) == 2) {
-                        const uint2 raw = *reinterpret_cast<const uint2*>(wr[x] + i);
-                        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-                        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-                        w4[x][0] = a.x; w4[x][1] = a.y; w4[x][2] = b.x; w4[x][3] = b.y;
+                        const uint4 raw = *reinterpret_cast<const uint4*>(wr[x] + i);
+                        const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) { const float2 f = __bfloat1622float2(p2[k]); w8[x][2 * k] = f.x; w8[x][2 * k + 1] = f.y; }
                     } else {
-                        const float4 a = *reinterpret_cast<const float4*>(wr[x] + i);
-                        w4[x][0] = a.x; w4[x][1] = a.y; w4[x][2] = a.z; w4[x][3] = a.w;
+                        const float4 a = *reinterpret_cast<const float4*>(wr[x] + i), b = *reinterpret_cast<const float4*>(wr[x] + i + 4);
+                        w8[x][0] = a.x; w8[x][1] = a.y; w8[x][2] = a.z; w8[x][3] = a.w; w8[x][4] = b.x; w8[x][5] = b.y; w8[x][6] = b.z; w8[x][7] = b.w;
                     }
                 }
 #pragma unroll
                 for (int k = 0; k < ROUTE_TOK; ++k) {
-                    const float4 r = *reinterpret_cast<const float4*>(rows + (size_t)k * W + i);
+                    const float* row = rows + (size_t)k * W + i;
+                    const float4 r0 = *reinterpret_cast<const float4*>(row), r1 = *reinterpret_cast<const float4*>(row + 4);
 #pragma unroll
                     for (int x = 0; x < RE; ++x) {
                         float a = acc[x][k];
-                        a = fmaf(r.x, w4[x][0], a); a = fmaf(r.y, w4[x][1], a); a = fmaf(r.z, w4[x][2], a); a = fmaf(r.w, w4[x][3], a);
+                        a = fmaf(r0.x, w8[x][0], a); a = fmaf(r0.y, w8[x][1], a); a = fmaf(r0.z, w8[x][2], a); a = fmaf(r0.w, w8[x][3], a);
+                        a = fmaf(r1.x, w8[x][4], a); a = fmaf(r1.y, w8[x][5], a); a = fmaf(r1.z, w8[x][6], a); a = fmaf(r1.w, w8[x][7], a);
                         acc[x][k] = a;
                     }
                 }
