@@ -1320,7 +1320,7 @@ class CudaKernels:
         # both products run on the same kernel (one tile table): the tensor-core one if both can
         tc = (self.grouped_on_tensor_cores(h, w_gate_up, W, W, 0, W, up_rows * W, "" if plain else layout, ff)
               and self.grouped_on_tensor_cores(h, w_down, ff, ff, 0, ff, W * ff, "", W))
-        if tc and self.GROUPED_TCGEN05 and P >= self.GROUPED_TCGEN05_FROM and W % 4 == 0 and ff % 8 == 0:
+        if tc and self.GROUPED_TCGEN05 and P >= min(self.GROUPED_TCGEN05_FROM, self.GROUPED_TCGEN05_EACH * E + 1) and W % 4 == 0 and ff % 8 == 0:
             # Prompt-sized: the tcgen05 product in its grouped form.  Every expert's rows are padded to whole tiles of 128
             # in the sorted order, both products write in that order, and the sum gathers a token's rows from it.
             rows = -(-(P + E * 127) // 128) * 128
@@ -1360,7 +1360,11 @@ class CudaKernels:
                          identity=(pe[0], pair_weight, h) if pe else None, shared=shared)
 
     GROUPED_TCGEN05 = os.environ.get("TFFINFER_GROUPED_TCGEN05", "1") != "0"
-    GROUPED_TCGEN05_FROM = 1024      # (token, expert) pairs of a step from which the experts run on the tcgen05 product
+    GROUPED_TCGEN05_FROM = 1024      # (token, expert) pairs of a step from which the experts run on the tcgen05 product,
+    # or fewer where an expert has more than these on average: 16 experts of the "2k" sizes (4k) with 160 pairs 178 -> 167 us (521 ->
+    # 505), 192 186 -> 167 (573 -> 507), 400 309 -> 202 (955 -> 569), 838 331 -> 213 (1,054 -> 608); with 128 they are equal (159 and
+    # 161, 499 and 501), with 48 the tiles of few rows are faster (128 and 145, 460 and 479)
+    GROUPED_TCGEN05_EACH = 8
 
     def gemm_tc_grouped(self, a, w, out, groups: int, group_rows: int, K: int, lane_group, gated: bool = False,
                         activation: str = "silu", limit: float = 0.0) -> None:
