@@ -12,26 +12,27 @@
 // gate[t, h].  Keys have d elements and values dv; both lie in cache slots of dc >= max(d, dv) elements.
 //
 // A CTA takes a tile of packed rows (token, query head of the group) of one request and kv head and walks the keys in
-// blocks of 32, which come to shared memory once for all its rows; a warp has up to 8 rows: for the scores a lane is
+// blocks of 32, which come to shared memory once for all its rows; a warp has up to 4 rows: for the scores a lane is
 // a key, for the values a lane has 4 (8, 16) columns.  The running-maximum ("online") softmax of the reference
 // (paged_flash_attention.cu:696-792) starts afresh every CHUNK keys, at absolute positions, and the chunks' results are
 // joined in ascending order: a step of few rows behind long contexts shares the chunks out to several CTAs and joins them in
 // a second kernel, with the same operations in the same order.  A token's result so depends neither on how the batch
 // was cut nor on what else is in it.
 //
-// What bounds it: the loads from shared memory (a key's 4 elements by every lane and the rows' 4 by all, for 4 FMAs a row), 12 cycles for
-// 8 of FMAs at 8 rows a warp; for one token behind a context the cache's bytes.  A warp a (token, head) that read the
-// keys from the second-level cache, a lane a key, took 750 us for four prompts of 134 tokens of the 8B shape; this takes 75.
+// What bounds it: the latency of its chains of shared-memory loads and FMAs (with 8 rows a warp and 8 warps an SM an instruction was
+// issued in a third of the cycles), then those loads; for one token behind a context the chain of its chunk's blocks.  A warp a
+// (token, head) that read the keys from the second-level cache, a lane a key, took 750 us for four prompts of 134 tokens
+// of the 8B shape; this takes 77 (145 with 8 rows a warp).
 #include "common.cuh"
 #include "attention_common.h"
 
 namespace {
 
-constexpr int WARPS = 4, BLOCK = 32, CHUNK = 128, PER_CHUNK = CHUNK / BLOCK;
+constexpr int BLOCK = 32, CHUNK = 64, PER_CHUNK = CHUNK / BLOCK, JOIN_THREADS = 128;
 
 struct GenericParams {
     const int *q_start, *pos_start, *block_table;
-    int table_width, row_stride, layer, nq, nkv, d, dv, window, sink, keep, splits, slots, stages, vec;
+    int table_width, row_stride, layer, nq, nkv, d, dv, window, sink, keep, splits, slots, stages, vec, q_vec;
     float scale, softcap;
     const float *sink_val, *gate;
     float *part_o, *part_ml;
@@ -49,6 +50,7 @@ __device__ __forceinline__ void join(float& m, float& l, float mc, float lc, flo
 }
 __device__ __forceinline__ float join_value(float o, float a, float oc, float b) { return __fmaf_rn(o, a, __fmul_rn(oc, b)); }
 
+__device__ __forceinline__ float4 load4(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 load4(const bf16* p) {
     const uint2 u = *(const uint2*)p;
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
@@ -56,8 +58,8 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 }
 
 // RW rows a warp, ND groups of 128 value columns (4 a lane).
-template <typename T, int RW, int ND>
-__global__ void __launch_bounds__(WARPS * 32)
+template <typename T, int WARPS, int RW, int ND>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1)
 attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache, T* __restrict__ out, const GenericParams p) {
     extern __shared__ float4 smem4[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -80,33 +82,41 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
     const int per = (walk.count + p.splits - 1) / p.splits, w0 = split * per, w1 = min(walk.count, w0 + per);
     if (w0 >= w1) return;
 
+#pragma unroll 4
     for (int i = threadIdx.x; i < WARPS * RW * k4; i += WARPS * 32) {
         const int r = row0 + i / k4, c = (i % k4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < rows) {
             const T* src = q_in + (size_t)(q0 + r / G) * p.row_stride + (size_t)(kvh * G + r % G) * p.d + c;
-            v.x = to_f32<T>(src[0]);
-            if (c + 1 < p.d) v.y = to_f32<T>(src[1]);
-            if (c + 2 < p.d) v.z = to_f32<T>(src[2]);
-            if (c + 3 < p.d) v.w = to_f32<T>(src[3]);
+            if (p.q_vec) {
+                v = load4(src);
+            } else {
+                v.x = to_f32<T>(src[0]);
+                if (c + 1 < p.d) v.y = to_f32<T>(src[1]);
+                if (c + 2 < p.d) v.z = to_f32<T>(src[2]);
+                if (c + 3 < p.d) v.w = to_f32<T>(src[3]);
+            }
         }
         sq[i] = v;
     }
 
     auto live = [&](int n0) { return n0 <= hi && (n0 + BLOCK - 1 >= lo_tile || n0 < p.keep); };
-    // Keys and values n0 .. n0 + 31 to a stage; those that no row of the tile sees are zeros (their slots may hold anything,
-    // and their pages may have been given back).
-    auto fetch = [&](int n0, int stage) {
+    // Where key n0 + lane lies: null for keys that no row of the tile sees (their slots may hold anything, and their pages may
+    // have been given back), whose stage rows become zeros.  Looked up a block ahead of the copies.
+    auto locate = [&](int n0) -> const T* {
+        const int n = n0 + lane;
+        if (n > hi || !(n >= lo_tile || n < p.keep)) return nullptr;
+        return cache + (size_t)table[n / p.L.page_size] * p.L.page_stride + (size_t)p.layer * p.L.layer_stride +
+               (size_t)kvh * p.L.head_stride + (size_t)(n % p.L.page_size) * p.L.head_dim;
+    };
+    auto fetch = [&](const T* at, int stage) {
         float4* sk = smem4 + stage * stage4;
         float4* sv = sk + BLOCK * ks;
+#pragma unroll 2
         for (int kr = warp; kr < BLOCK; kr += WARPS) {
-            const int n = n0 + kr;
-            const bool ok = n <= hi && (n >= lo_tile || n < p.keep);
-            const T* kp = nullptr;
-            if (ok)
-                kp = cache + (size_t)table[n / p.L.page_size] * p.L.page_stride + (size_t)p.layer * p.L.layer_stride +
-                     (size_t)kvh * p.L.head_stride + (size_t)(n % p.L.page_size) * p.L.head_dim;
-            const T* vp = ok ? kp + p.L.kv_stride : nullptr;
+            const T* kp = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)at, kr);
+            const bool ok = kp != nullptr;
+            const T* vp = kp + p.L.kv_stride;
             auto row = [&](const T* src, int n4, int len, float4* dst) {
                 for (int c = lane; c < n4; c += 32) {
                     if (!ok) dst[c] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -151,19 +161,23 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
 
     const int total = (w1 - w0) * PER_CHUNK;
     auto block_start = [&](int i) { return walk.block(w0 + i / PER_CHUNK) * CHUNK + (i % PER_CHUNK) * BLOCK; };
+    const T* at = locate(block_start(0));
     if (p.stages > 1) {
-        if (live(block_start(0))) fetch(block_start(0), 0);
+        if (live(block_start(0))) fetch(at, 0);
         asm volatile("cp.async.commit_group;" ::: "memory");
+        if (total > 1) at = locate(block_start(1));
     }
     for (int i = 0; i < total; ++i) {
         const int n0 = block_start(i), stage = p.stages > 1 ? (i & 1) : 0;
         if (p.stages > 1) {
-            if (i + 1 < total && live(block_start(i + 1))) fetch(block_start(i + 1), stage ^ 1);
+            if (i + 1 < total && live(block_start(i + 1))) fetch(at, stage ^ 1);
             asm volatile("cp.async.commit_group;" ::: "memory");
+            if (i + 2 < total) at = locate(block_start(i + 2));
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
-            if (live(n0)) fetch(n0, 0);
+            if (live(n0)) fetch(at, 0);
             asm volatile("cp.async.wait_all;" ::: "memory");
+            if (i + 1 < total) at = locate(block_start(i + 1));
         }
         __syncthreads();
         if (live(n0) && wrow < rows) {
@@ -207,6 +221,11 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
                 sp[j * BLOCK + lane] = pr;
             }
             __syncwarp();
+            // the keys of the block that a row sees are its first ``to[j]``, those from ``from[j]`` on or among the first ``kept``
+            int to[RW], from[RW];
+#pragma unroll
+            for (int j = 0; j < RW; ++j) { to[j] = rp[j] - n0; from[j] = rlo[j] - n0; }
+            const int kept = p.keep - n0;
             // ------------------------------------------------ values: the lane's columns of the warp's rows
 #pragma unroll 1
             for (int c = 0; c < BLOCK; c += 4) {
@@ -215,7 +234,7 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
                 for (int j = 0; j < RW; ++j) w[j] = *(const float4*)(sp + j * BLOCK + c);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const int key = n0 + c + e;
+                    const int key = c + e;
                     float4 v[ND];
 #pragma unroll
                     for (int g = 0; g < ND; ++g) {
@@ -225,7 +244,7 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
 #pragma unroll
                     for (int j = 0; j < RW; ++j) {
                         // a key that the row does not see adds nothing, whatever its value is
-                        if (!whole && !(key <= rp[j] && (key >= rlo[j] || key < p.keep))) continue;
+                        if (whole || (key <= to[j] && (key >= from[j] || key < kept))) {
                         const float x = e == 0 ? w[j].x : e == 1 ? w[j].y : e == 2 ? w[j].z : w[j].w;
 #pragma unroll
                         for (int g = 0; g < ND; ++g) {
@@ -233,6 +252,7 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
                             oc[j][4 * g + 1] = fmaf(x, v[g].y, oc[j][4 * g + 1]);
                             oc[j][4 * g + 2] = fmaf(x, v[g].z, oc[j][4 * g + 2]);
                             oc[j][4 * g + 3] = fmaf(x, v[g].w, oc[j][4 * g + 3]);
+                        }
                         }
                     }
                 }
@@ -244,7 +264,7 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
 #pragma unroll
             for (int j = 0; j < RW; ++j) {
                 if (p.splits > 1) {
-                    if (wrow + j < rows) {
+                    if (wrow + j < rows && slot < p.slots) {
                         const size_t at = ((size_t)(q0 + (wrow + j) / G) * p.nq + kvh * G + (wrow + j) % G) * p.slots + slot;
                         if (lane == 0) { p.part_ml[2 * at] = mc[j]; p.part_ml[2 * at + 1] = lc[j]; }
 #pragma unroll
@@ -281,44 +301,46 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
     }
 }
 
-// Joins the chunks' results in ascending order: one warp per (token, head).  The rows of a request are one tile.
+// Joins the chunks' results in ascending order: a block per (token, head), a thread a column (of every JOIN_THREADS), eight chunks' loads
+// on their way together.  The rows of a request are one tile.
 template <typename T>
-__global__ void __launch_bounds__(WARPS * 32)
-attention_generic_join_kernel(T* __restrict__ out, const int* __restrict__ tok_req, int num_tokens, const GenericParams p) {
+__global__ void __launch_bounds__(JOIN_THREADS)
+attention_generic_join_kernel(T* __restrict__ out, const int* __restrict__ tok_req, const GenericParams p) {
     pdl_launch_dependents();
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
-    if (item >= (long long)num_tokens * p.nq) return;
-    const int t = (int)(item / p.nq), h = (int)(item % p.nq), b = tok_req[t];
+    const int item = blockIdx.x, t = item / p.nq, h = item % p.nq, b = tok_req[t];
     const int pos0 = p.pos_start[b], q_len = p.q_start[b + 1] - p.q_start[b];
     const int lo_tile = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
     const KeyWalk walk(p.keep, CHUNK, lo_tile / CHUNK, (pos0 + q_len - 1) / CHUNK);
-    float m = p.sink ? (p.sink_val ? p.sink_val[h] : 0.f) : -INFINITY, l = p.sink ? 1.f : 0.f;
-    float o[16];
+    const int count = min(walk.count, p.slots);
+    const float* ml = p.part_ml + (size_t)item * p.slots * 2;
+    for (int col = threadIdx.x; col < p.dv; col += JOIN_THREADS) {
+        const float* po = p.part_o + (size_t)item * p.slots * p.dv + col;
+        float m = p.sink ? (p.sink_val ? p.sink_val[h] : 0.f) : -INFINITY, l = p.sink ? 1.f : 0.f, o = 0.f;
+        for (int w0 = 0; w0 < count; w0 += 8) {
+            float2 x[8];
+            float v[8];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) o[j] = 0.f;
-    for (int w = 0; w < walk.count; ++w) {
-        const size_t at = (size_t)item * p.slots + w;
-        float a, bb;
-        join(m, l, p.part_ml[2 * at], p.part_ml[2 * at + 1], a, bb);
+            for (int u = 0; u < 8; ++u) {
+                if (w0 + u >= count) continue;
+                x[u] = *(const float2*)(ml + 2 * (w0 + u));
+                v[u] = po[(size_t)(w0 + u) * p.dv];
+            }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int col = j * 32 + lane;
-            if (col < p.dv) o[j] = join_value(o[j], a, p.part_o[at * p.dv + col], bb);
+            for (int u = 0; u < 8; ++u) {
+                if (w0 + u >= count) continue;
+                float a, bb;
+                join(m, l, x[u].x, x[u].y, a, bb);
+                o = join_value(o, a, v[u], bb);
+            }
         }
-    }
-    const float inv = (p.gate ? p.gate[(size_t)t * p.nq + h] : 1.f) / l;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const int col = j * 32 + lane;
-        if (col < p.dv) out[(size_t)item * p.dv + col] = from_f32<T>(o[j] * inv);
+        out[(size_t)item * p.dv + col] = from_f32<T>(o * ((p.gate ? p.gate[item] : 1.f) / l));
     }
 }
 
-template <typename T, int RW, int ND>
+template <typename T, int WARPS, int RW, int ND>
 int launch(const void* q, const void* cache, void* out, GenericParams p, int num_requests, int max_q_len, cudaStream_t s) {
-    auto kern = attention_generic_kernel<T, RW, ND>;
+    auto kern = attention_generic_kernel<T, WARPS, RW, ND>;
     const int k4 = (p.d + 3) / 4, v4 = (p.dv + 3) / 4;
     const size_t stage = (size_t)BLOCK * ((k4 | 1) + v4) * 16;
     const size_t rest = (size_t)WARPS * RW * k4 * 16 + (size_t)WARPS * RW * BLOCK * 4;
@@ -337,20 +359,21 @@ int launch(const void* q, const void* cache, void* out, GenericParams p, int num
 
 template <typename T>
 int dispatch(const void* q, const void* cache, void* out, const GenericParams& p, int num_requests, int max_q_len, cudaStream_t s) {
-    // rows a warp: 4 warps share the keys in shared memory, so as many as the step has, and as the registers hold columns
+    // The warps share the keys in shared memory; a warp takes as many rows as the step has and as its registers hold columns.  32 rows
+    // are 8 warps of 4 and not 4 of 8: two shared-memory wavefronts for 4 FMAs instead of 1.5, but twice the warps in flight.
     const long long rows = (long long)max_q_len * (p.nq / p.nkv);
     if (p.dv <= 128) {
-        if (rows <= 4) return launch<T, 1, 1>(q, cache, out, p, num_requests, max_q_len, s);
-        if (rows <= 8) return launch<T, 2, 1>(q, cache, out, p, num_requests, max_q_len, s);
-        if (rows <= 16) return launch<T, 4, 1>(q, cache, out, p, num_requests, max_q_len, s);
-        return launch<T, 8, 1>(q, cache, out, p, num_requests, max_q_len, s);
+        if (rows <= 4) return launch<T, 4, 1, 1>(q, cache, out, p, num_requests, max_q_len, s);
+        if (rows <= 8) return launch<T, 8, 1, 1>(q, cache, out, p, num_requests, max_q_len, s);
+        if (rows <= 16) return launch<T, 8, 2, 1>(q, cache, out, p, num_requests, max_q_len, s);
+        return launch<T, 8, 4, 1>(q, cache, out, p, num_requests, max_q_len, s);
     }
     if (p.dv <= 256) {
-        if (rows <= 4) return launch<T, 1, 2>(q, cache, out, p, num_requests, max_q_len, s);
-        return launch<T, 4, 2>(q, cache, out, p, num_requests, max_q_len, s);
+        if (rows <= 4) return launch<T, 4, 1, 2>(q, cache, out, p, num_requests, max_q_len, s);
+        return launch<T, 8, 2, 2>(q, cache, out, p, num_requests, max_q_len, s);
     }
-    if (rows <= 4) return launch<T, 1, 4>(q, cache, out, p, num_requests, max_q_len, s);
-    return launch<T, 2, 4>(q, cache, out, p, num_requests, max_q_len, s);
+    if (rows <= 4) return launch<T, 4, 1, 4>(q, cache, out, p, num_requests, max_q_len, s);
+    return launch<T, 8, 1, 4>(q, cache, out, p, num_requests, max_q_len, s);
 }
 
 // Rows that may be one tile whatever the head size is: what a step's chunks may be shared out for.
@@ -400,13 +423,14 @@ TFF_API int tff_attention_generic(
         return TFF_ERR_BAD_ARGUMENT;
     if (p.splits > 1) { p.part_ml = ws; p.part_o = ws + (size_t)num_tokens * nq * p.slots * 2; }
     // 4 elements are read at a time where rows and slots are whole groups at aligned addresses
+    p.q_vec = d % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)qkv & 15) == 0;
     p.vec = d % 4 == 0 && dv % 4 == 0 && dc % 4 == 0 && ((uintptr_t)cache & 15) == 0;
     int st = is_bf16 ? dispatch<bf16>(qkv, cache, out, p, num_requests, max_q_len, stream)
                      : dispatch<float>(qkv, cache, out, p, num_requests, max_q_len, stream);
     if (st == TFF_OK && p.splits > 1) {
-        const unsigned blocks = (unsigned)(((long long)num_tokens * nq + WARPS - 1) / WARPS);
-        st = is_bf16 ? tff_launch_pdl(attention_generic_join_kernel<bf16>, dim3(blocks), dim3(WARPS * 32), (size_t)0, stream, (bf16*)out, tok_req, num_tokens, p)
-                     : tff_launch_pdl(attention_generic_join_kernel<float>, dim3(blocks), dim3(WARPS * 32), (size_t)0, stream, (float*)out, tok_req, num_tokens, p);
+        const unsigned blocks = (unsigned)((long long)num_tokens * nq);
+        st = is_bf16 ? tff_launch_pdl(attention_generic_join_kernel<bf16>, dim3(blocks), dim3(JOIN_THREADS), (size_t)0, stream, (bf16*)out, tok_req, p)
+                     : tff_launch_pdl(attention_generic_join_kernel<float>, dim3(blocks), dim3(JOIN_THREADS), (size_t)0, stream, (float*)out, tok_req, p);
     }
     return st;
 }
