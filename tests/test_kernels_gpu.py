@@ -511,6 +511,58 @@ def test_flash_attention_bf16(ops, case):
     assert rel_err(out, gen) < 1e-2
 
 
+@pytest.mark.parametrize("nq,nkv,d,page,new,old,window,splits,extra", [
+    (32, 8, 128, 16, [70, 1, 1], [40, 2500, 9], 0, 4, False),        # shares of the decoded tokens' keys, joined by a third kernel
+    (8, 8, 64, 8, [130, 1, 2, 1], [0, 63, 64, 65], 0, 1, True),      # no grouping, the smaller head
+    (40, 8, 128, 64, [300, 129, 1], [0, 100, 700], 48, 2, True),     # a window, more tiles of portions than one
+    (8, 2, 128, 4, [40, 1], [0, 100], 0, 1, False),                  # pages that the portions' kernel does not take: refused
+])
+@pytest.mark.parametrize("captured", [False, True])
+def test_portions_and_decoded_tokens_in_one_call_equal_two_launches(ops, captured, nq, nkv, d, page, new, old, window, splits, extra):
+    """The two kernels overlap: each call's queries are written by the kernel right ahead of it, and its output read by the
+    one right behind it, several calls in a row.  Every bit equals that of the launches one after the other."""
+    entries, tables, cache, qkv = _paged_case(nq, nkv, d, page, new, old, window, torch.bfloat16, seed=77)
+    T, B = sum(new), len(new)
+    b = build_step_batch(entries, old, list(range(B)), [tables], DEV)
+    short = sum(n * (nq // nkv) <= 16 for n in new)
+    q_short, q_long = int(b.h_sorted_q_lens[short - 1]), int(b.h_sorted_q_lens[-1])
+    assert 0 < short < B and q_short * (nq // nkv) <= 16 < int(b.h_sorted_q_lens[short]) * (nq // nkv)
+    more = (0.0, False, None, 0)
+    if extra:
+        more = (20.0, g((nq,), torch.float32, 78).to(DEV), torch.rand(T, nq, device=DEV), 5 if window else 0)
+    cache = cache.to(DEV)
+    qs = [g((T, nq * d), torch.bfloat16, 80 + i).to(DEV) for i in range(6)]
+    q = torch.zeros_like(qs[0])
+    tail = (nq, nkv, d, 1 / math.sqrt(d), window)
+    head = (b, b.block_tables[0], cache, 1, page)
+    got = [torch.full((T, nq * d), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in qs]
+    out = torch.empty_like(got[0])
+    taken = []
+
+    def calls():
+        for x, r in zip(qs, got):
+            q.copy_(x)
+            taken.append(ops._attention_bf16_mixed(q, *head, out, *tail, splits, short, B, q_short, q_long, more))
+            r.copy_(out)
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            calls()
+        graph.replay()
+    else:
+        calls()
+    torch.cuda.synchronize()
+    assert taken == [page >= 8] * len(qs)
+    for x, r in zip(qs, got):
+        if not taken[0]:
+            continue
+        want = torch.full_like(r, float("nan"))
+        ops._attention_bf16_launch(x, *head, want, *tail, 1, b.req_order[short:], B - short, q_long, more)
+        torch.cuda.synchronize()
+        ops._attention_bf16_launch(x, *head, want, *tail, splits, b.req_order[:short], short, q_short, more)
+        assert torch.isfinite(want).all() and torch.equal(r, want)
+
+
 @pytest.mark.parametrize("nq,nkv,d,new,old,window,keep", [
     (32, 8, 128, [1, 1, 1], [300, 127, 1100], 0, 0),           # 4 rows a tile
     (8, 1, 48, [1, 2], [128, 255], 0, 0),                      # 8 and 16 rows, a head of 48

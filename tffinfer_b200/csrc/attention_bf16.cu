@@ -427,7 +427,7 @@ static int attention_bf16_impl(
     const void* q, const int* q_start, const int* pos_start, const int* req_ids, const int* block_table, int table_width,
     const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
     void* out, void* workspace, int num_tokens, int num_requests, int max_q_len, int num_splits,
-    int nq, int nkv, int d, float scale, int window, AttnExtra extra, cudaStream_t stream) {
+    int nq, int nkv, int d, float scale, int window, AttnExtra extra, cudaStream_t stream, bool beside = false) {
     if (num_tokens <= 0 || num_requests <= 0) return TFF_OK;
     if (extra.softcap < 0.f || extra.keep < 0) return TFF_ERR_BAD_ARGUMENT;
     if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || page_size <= 0 || max_q_len <= 0 || num_splits < 1)
@@ -460,7 +460,7 @@ static int attention_bf16_impl(
     if (keys_mode && cache_pages > 0)      // decode: keys streamed by TMA (attention_decode.cu), when it takes the shape
         st = tff_attention_decode_launch(q, q_start, pos_start, req_ids, block_table, table_width, cache, cache_pages,
                                          cache_layers, layer, page_size, out, p.part_o, p.part_ml, num_requests,
-                                         max_q_len, num_splits, nq, nkv, d, scale, window, extra, stream);
+                                         max_q_len, num_splits, nq, nkv, d, scale, window, extra, stream, beside);
     if (!keys_mode && num_splits == 1 && cache_pages > 0)   // portions: tcgen05 kernel (attention_prefill.cu)
         st = tff_attention_prefill_launch(q, q_start, pos_start, req_ids, block_table, table_width, cache, cache_pages,
                                           cache_layers, layer, page_size, out, num_requests, max_q_len, nq, nkv, d,
@@ -519,6 +519,31 @@ TFF_API int tff_attention_bf16_paged_ext(
     return attention_bf16_impl(q, q_start, pos_start, req_ids, block_table, table_width, cache, cache_pages, cache_layers,
                                layer, page_size, out, workspace, num_tokens, num_requests, max_q_len, num_splits, nq,
                                nkv, d, scale, window, AttnExtra{softcap, sink, gate, sink_val, keep}, stream);
+}
+
+// A step of decoded tokens and portions: the requests of ``req_order`` (their rows, by number of new tokens) from
+// ``num_short`` on are portions on the tcgen05 kernel, those ahead bring few tokens (at most ``max_q_short``) and go to the decode
+// kernel beside it, their keys in ``num_splits`` shares (workspace as above).  TFF_ERR_UNSUPPORTED, with nothing
+// launched, when the tcgen05 kernel does not take the shape.
+TFF_API int tff_attention_bf16_mixed(
+    const void* q, const int* q_start, const int* pos_start, const int* req_order, const int* block_table, int table_width,
+    const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
+    void* out, void* workspace, int num_tokens, int num_short, int num_requests, int max_q_short, int max_q_len, int num_splits,
+    int nq, int nkv, int d, float scale, int window, float softcap, int sink, const float* sink_val, const float* gate, int keep,
+    cudaStream_t stream) {
+    if (num_tokens <= 0 || num_short <= 0 || num_short >= num_requests || !req_order || nq <= 0 || nkv <= 0 || nq % nkv != 0 ||
+        softcap < 0.f || keep < 0 || max_q_short <= 0 || (long long)max_q_short * (nq / nkv) > 16 || num_splits < 1 ||
+        (num_splits > 1 && workspace == nullptr) || page_size <= 0)
+        return TFF_ERR_BAD_ARGUMENT;
+    if (cache_pages <= 0 || num_requests > 65535 || nkv > 65535) return TFF_ERR_UNSUPPORTED;
+    const AttnExtra extra{softcap, sink, gate, sink_val, keep};
+    const int st = tff_attention_prefill_launch(q, q_start, pos_start, req_order + num_short, block_table, table_width, cache, cache_pages,
+                                                cache_layers, layer, page_size, out, num_requests - num_short, max_q_len, nq, nkv, d,
+                                                scale, window, extra, stream, true);
+    if (st != TFF_OK) return st;
+    return attention_bf16_impl(q, q_start, pos_start, req_order, block_table, table_width, cache, cache_pages, cache_layers, layer,
+                               page_size, out, workspace, num_tokens, num_short, max_q_short, num_splits, nq, nkv, d, scale, window,
+                               extra, stream, true);
 }
 
 // ------------------------------------------------------- allocation-free variant

@@ -48,17 +48,21 @@ __device__ __forceinline__ float attn_score_log2(float raw, float scale_log2, fl
 }
 #endif
 
+// Two kernels of one step, the portions' (``companion``) and, next in the stream, the decoded tokens' (``beside``), which write
+// different rows: the first lets the second start once it has itself waited for the kernel ahead of both, so that the
+// second's CTAs run on the SMs that the first leaves free; one CTA of the second waits for the first before it ends.
+
 // Decode kernel (attention_decode.cu): at most 16 packed query rows per (request, kv head),
 // keys streamed by TMA.  Writes ``out`` when num_splits == 1, else the partial results.
 int tff_attention_decode_launch(
     const void* q, const int* q_start, const int* pos_start, const int* req_ids, const int* block_table, int table_width,
     const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
     void* out, float* part_o, float* part_ml, int num_requests, int max_q_len, int num_splits,
-    int nq, int nkv, int d, float scale, int window, AttnExtra extra, cudaStream_t stream);
+    int nq, int nkv, int d, float scale, int window, AttnExtra extra, cudaStream_t stream, bool beside = false);
 
 // Prompt-portion kernel (attention_prefill.cu): 128 packed rows per CTA on tcgen05, keys by TMA.
 int tff_attention_prefill_launch(
     const void* q, const int* q_start, const int* pos_start, const int* req_ids, const int* block_table, int table_width,
     const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
     void* out, int num_requests, int max_q_len, int nq, int nkv, int d, float scale, int window, AttnExtra extra,
-    cudaStream_t stream);
+    cudaStream_t stream, bool companion = false);

@@ -70,6 +70,7 @@ struct DecodeParams {
     int nq, nkv; float scale_log2; int window;
     float scale_over_cap, cap_log2; int sink; const float* gate; const float* sink_val;   // AttnExtra, ready for the kernel
     int keep;
+    int beside;                                  // runs beside the kernel ahead, which wrote nothing that this one reads
     int* error_flag;
 };
 
@@ -142,7 +143,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
         const int j = lane;
         const uint32_t box_bytes = (uint32_t)(2 * D * 2) << p.page_shift;      // K and V of one page
         const int first_new_blk = pos0 / BLOCK_N;                  // key blocks from here on hold slots written just now
-        bool waited = false;
+        bool waited = p.beside != 0;
         for (int w = w_begin; w < w_end; ++w) {
             const int blk = walk.block(w), i = w - w_begin, s = i % NSTAGES;
             const uint32_t round = i / NSTAGES;
@@ -170,14 +171,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
     }
 
     // ---------------------------------------------------------------- compute warps
-    pdl_wait();
+    if (!p.beside) pdl_wait();
     // the query tile: packed rows (token, head of the group), chunks XOR-swizzled by row % 8
     for (int idx = tid; idx < 16 * CH; idx += 128) {
         const int row = idx / CH, chunk = idx % CH;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (row < rows_total)
-            v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + row / G) * p.q_row_stride +
-                                                (size_t)(kvh * G + row % G) * D + chunk * 8);
+            v = __ldcg(reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + row / G) * p.q_row_stride +
+                                                      (size_t)(kvh * G + row % G) * D + chunk * 8));
         *reinterpret_cast<uint4*>(gQ + row * (D * 2) + (((chunk & ~7) | ((chunk ^ row) & 7)) << 4)) = v;
     }
     compute_barrier();
@@ -291,6 +292,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
     if (*abort_flag) {
         for (int i = 0; i < 64; ++i) __nanosleep(1000);    // copies in flight land before the CTA leaves
         if (tid == 0) atomicExch(p.error_flag, 1);
+        if (p.beside && blockIdx.x + blockIdx.y + blockIdx.z == 0) pdl_wait();
         return;
     }
     // ---------------------------------------------- merge the four warps through shared memory
@@ -335,6 +337,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
             }
         }
     }
+    // Whoever waits for this kernel has then waited for the one beside it.  (One CTA does; the others make room.)
+    if (p.beside && blockIdx.x + blockIdx.y + blockIdx.z == 0) pdl_wait();
 }
 
 template <int D>
@@ -358,7 +362,7 @@ int tff_attention_decode_launch(
     const void* q, const int* q_start, const int* pos_start, const int* req_ids, const int* block_table, int table_width,
     const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
     void* out, float* part_o, float* part_ml, int num_requests, int max_q_len, int num_splits,
-    int nq, int nkv, int d, float scale, int window, AttnExtra extra, cudaStream_t stream) {
+    int nq, int nkv, int d, float scale, int window, AttnExtra extra, cudaStream_t stream, bool beside) {
     if (d != 64 && d != 128) return TFF_ERR_UNSUPPORTED;
     if (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64) return TFF_ERR_UNSUPPORTED;
     if ((long long)max_q_len * (nq / nkv) > 16 || cache_pages <= 0) return TFF_ERR_UNSUPPORTED;
@@ -379,6 +383,7 @@ int tff_attention_decode_launch(
     p.cap_log2 = extra.softcap > 0.f ? extra.softcap * 1.4426950408889634f : 0.f;
     p.sink = extra.sink; p.gate = extra.gate; p.sink_val = extra.sink_val;
     p.keep = window > 0 ? extra.keep : 0;
+    p.beside = beside ? 1 : 0;
     p.error_flag = tff_device_error_flag();
     if (p.error_flag == nullptr) return TFF_ERR_LAUNCH;
     return d == 128 ? launch_decode<128>(tm, p, num_requests, stream) : launch_decode<64>(tm, p, num_requests, stream);

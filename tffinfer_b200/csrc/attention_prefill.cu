@@ -166,6 +166,7 @@ __device__ long long ap_dbg[64];
 #endif
 
 struct PrefillParams {
+    int companion;                               // the decoded tokens' kernel follows and runs beside this one
     const bf16* q; int q_row_stride;
     const int* q_start; const int* pos_start; const int* req_ids;
     const int* block_table; int table_width;
@@ -261,8 +262,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_launch_dependents();
-    pdl_wait();
+    if (p.companion) {            // the kernel behind may read what the one ahead of both wrote
+        pdl_wait();
+        pdl_launch_dependents();
+    } else {
+        pdl_launch_dependents();
+        pdl_wait();
+    }
 
     // request geometry (q_start and pos_start come with the step's batch, read after the dependency wait all the same)
     const int b = p.req_ids ? p.req_ids[blockIdx.z] : (int)blockIdx.z;
@@ -690,7 +696,7 @@ int tff_attention_prefill_launch(
     const void* q, const int* q_start, const int* pos_start, const int* req_ids, const int* block_table, int table_width,
     const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
     void* out, int num_requests, int max_q_len, int nq, int nkv, int d, float scale, int window, AttnExtra extra,
-    cudaStream_t stream) {
+    cudaStream_t stream, bool companion) {
     if (d != 64 && d != 128) return TFF_ERR_UNSUPPORTED;
     if (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64) return TFF_ERR_UNSUPPORTED;
     if (cache_pages <= 0 || !(scale > 0.f)) return TFF_ERR_UNSUPPORTED;     // the kernel folds a positive scale into the exponent
@@ -714,6 +720,7 @@ int tff_attention_prefill_launch(
     p.error_flag = tff_device_error_flag();
     if (p.error_flag == nullptr) return TFF_ERR_LAUNCH;
     p.d = p.dv = d; p.k_halves = p.k_head = p.r_col = 0;
+    p.companion = companion ? 1 : 0;
     return d == 128 ? launch_prefill_tiles<128, 128, false>(tm, tm, tm, p, max_q_len, num_requests, stream)
                     : launch_prefill_tiles<64, 64, false>(tm, tm, tm, p, max_q_len, num_requests, stream);
 }

@@ -1989,14 +1989,6 @@ class CudaKernels:
         B = batch.num_requests
         n_short = int(np.searchsorted(sq, 16 // G, side="right")) if (sq is not None and num_splits is None) else 0
         if 0 < n_short < B and batch.req_order is not None:
-            # The two launches write different rows of ``out`` and read what the kernels before them wrote:
-            # they run side by side, the decoded tokens' on a second stream.  The portions' kernel is
-            # launched first; it seldom fills the SMs (a 512-token portion is 80 to 160 CTAs of one an SM),
-            # and the other one, bound by memory, runs on what is left.
-            main = torch.cuda.current_stream()
-            side = None if torch.cuda.is_current_stream_capturing() else self._side_stream(q.device)
-            if side is not None:
-                self._fork.record(main)
             # (One share for the portions here unless their context is long: their few CTAs run beside the decoded
             # tokens' kernel, which has the other SMs; cut into shares they contend with it for all of them.  Measured:
             # the 14B mixed workload, contexts up to 4,096, 3.52-3.61 s with shares against 3.35-3.37 without; a step of
@@ -2004,9 +1996,18 @@ class CudaKernels:
             # 8.1 against 10.6, behind 16,000 keys 8.1 against 15.9.)
             long_kv = int(batch.h_sorted_kv_lens[n_short:].max()) if batch.h_sorted_kv_lens is not None else 0
             shares = self.portion_splits(B - n_short, int(sq[-1]), long_kv, nq, nkv) if long_kv >= self.MIXED_SHARES_FROM else 1
+            splits = self._decode_splits(batch, 0, n_short, int(sq[n_short - 1]), nq, nkv)
+            if shares == 1 and self._attention_bf16_mixed(q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, scale,
+                                                          window, splits, n_short, B, int(sq[n_short - 1]), int(sq[-1]), extra):
+                return
+            # Portions on another kernel: two launches that write different rows of ``out`` and read what the kernels before
+            # them wrote, side by side, the decoded tokens' on a second stream.
+            main = torch.cuda.current_stream()
+            side = None if torch.cuda.is_current_stream_capturing() else self._side_stream(q.device)
+            if side is not None:
+                self._fork.record(main)
             self._attention_bf16_launch(q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, scale,
                                         window, shares, batch.req_order[n_short:], B - n_short, int(sq[-1]), extra)
-            splits = self._decode_splits(batch, 0, n_short, int(sq[n_short - 1]), nq, nkv)
             if side is None:
                 self._attention_bf16_launch(q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d,
                                             scale, window, splits, batch.req_order[:n_short], n_short,
@@ -2029,6 +2030,31 @@ class CudaKernels:
             order = batch.req_order if n_short == B else None
             self._attention_bf16_launch(q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, scale,
                                         window, num_splits, order, B, batch.max_q_len, extra)
+
+    def _attention_bf16_mixed(self, q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, scale, window, splits,
+                              n_short, B, q_short, q_long, extra) -> bool:
+        """Decoded tokens beside portions, one kernel behind the other in the stream, the second one running on the SMs that
+        the portions' leaves free (it seldom fills them: a 512-token portion is 80 to 160 CTAs of one an SM): it does not wait
+        for the first until it ends.  As two launches on two streams, with their events, an attention layer of the 14B sizes
+        with 512 new tokens and 32 decoded ones took 144 us of the host and 142 of the device, now 87 and 139; of the 4B
+        sizes, 469 behind 443 beside 8 behind up to 4,602, 134 and 90.6, now 84 and 83.6.  False, with nothing launched,
+        where the portions' kernel does not take the shape."""
+        T = q.shape[0]
+        c_ptr, c_pages, c_layers, c_layer = self._cache_args(kv_cache, kv_layer)
+        ws = torch.empty(T * nq * splits * (d + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+        softcap, sink, gates, keep = extra
+        sink_on, sink_val = self._sink_args(sink, nq)
+        status = self.lib.tff_attention_bf16_mixed(
+            _ptr(q), _ptr(batch.q_start), _ptr(batch.pos_start), _ptr(batch.req_order), _ptr(block_table), _c_int(block_table.shape[1]),
+            c_ptr, _c_int(c_pages), _c_int(c_layers), _c_int(c_layer), _c_int(page_size), _ptr(out), _ptr(ws), _c_int(T),
+            _c_int(n_short), _c_int(B), _c_int(q_short), _c_int(q_long), _c_int(splits), _c_int(nq), _c_int(nkv), _c_int(d),
+            _c_float(scale), _c_int(window), _c_float(softcap), _c_int(1 if sink_on else 0), _ptr(sink_val), _ptr(gates),
+            _c_int(keep), self._stream())
+        if status == -2:
+            return False
+        self._check(status, "attention_bf16_mixed")
+        self.launches += 3 if splits > 1 else 2
+        return True
 
     def _attention_bf16_launch(self, q, batch, block_table, kv_cache, kv_layer, page_size, out, nq, nkv, d, scale,
                                window, num_splits, req_ids, num_requests, max_q_len, extra=(0.0, False, None, 0)) -> None:
