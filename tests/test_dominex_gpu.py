@@ -280,6 +280,62 @@ def test_routed_experts(ops, dtype, E, top, ff, W, T):
         assert err < (2e-5 if dtype == "float32" else 3e-2), f"{weight_on}: off by {err:.3g}"
 
 
+@pytest.mark.parametrize("tcgen05", [True, False])
+@pytest.mark.parametrize("E,top,T", [(16, 4, 32), (16, 4, 33), (5, 3, 13), (5, 3, 14), (1, 1, 9), (64, 6, 85), (64, 6, 86)])
+def test_routed_experts_where_the_product_changes(ops, monkeypatch, E, top, T, tcgen05):
+    """Steps of 8 pairs an expert and a few more, on both products."""
+    monkeypatch.setattr(type(ops), "GROUPED_TCGEN05", tcgen05)
+    test_routed_experts(ops, "bfloat16", E, top, 64, 136, T)
+
+
+@pytest.mark.parametrize("planes,nq,nkv,d,dv,page,lens,starts,window,chunk,more", [
+    (1, 16, 1, 576, 512, 16, [1, 1, 2], [300, 0, 63], 0, 0, ""),               # rows of a latent cache; 16 and 32 rows
+    (1, 3, 1, 40, 24, 8, [1, 5], [95, 0], 0, 0, "sink"),                       # 15 rows; a key that is no whole 16 elements
+    (1, 32, 1, 288, 256, 32, [1, 1], [31, 32], 20, 0, ""),
+    (2, 6, 2, 24, 40, 16, [1, 3, 2], [200, 29, 64], 33, 0, "bias"),            # values larger than keys
+    (2, 4, 4, 64, 64, 8, [32, 1], [7, 100], 0, 24, "cap sink"),                # 32 rows of one head
+    (2, 8, 1, 256, 256, 8, [4, 1], [31, 500], 0, 0, "bias cap"),
+    (2, 17, 1, 192, 128, 64, [1, 1], [0, 640], 0, 0, "sink"),                  # a second tile of one row
+    (2, 2, 1, 512, 512, 16, [1, 2], [90, 33], 0, 0, ""),                       # too large for two stages of the bulk copies
+])
+@pytest.mark.parametrize("splits", [1, 3, None])
+def test_attention_of_few_rows(ops, splits, planes, nq, nkv, d, dv, page, lens, starts, window, chunk, more):
+    """Steps of at most 32 rows (a request, kv head) in bfloat16 against the same values through the float32 form, which is
+    another kernel.  Two bfloat16 roundings stand between them, of the probabilities (2^-9 of each, and as much of their
+    sum) and of the output: at most 3 x 2^-9 of the largest value."""
+    dev = "cuda"
+    gen = torch.Generator().manual_seed(d + nq)
+    full = fake_batch([n + s for n, s in zip(lens, starts)], [0] * len(lens), dev, page)
+    step = fake_batch(lens, starts, dev, page)
+    step.block_table = full.block_table
+    slot = d if planes == 1 else max(d, dv)
+    cache = torch.full((full.pages + 1, 2, planes, nkv, page, slot), float("nan"))
+    for b, (n, s) in enumerate(zip(lens, starts)):
+        ts = torch.arange(n + s)
+        pg, sl = full.block_table[b].cpu().long()[ts // page], ts % page
+        cache[pg, 1, 0, :, sl, :d] = torch.randn(n + s, nkv, d, generator=gen)
+        if planes == 2:
+            cache[pg, 1, 1, :, sl, :dv] = torch.randn(n + s, nkv, dv, generator=gen)
+    cache = cache.to(dev).bfloat16()
+    q = torch.randn(sum(lens), nq * d, generator=gen).to(dev).bfloat16()
+    kw = dict(window=window, chunk=chunk)
+    vec = lambda: (0.2 + torch.rand(nq, generator=gen)).to(dev)
+    if "bias" in more:
+        kw.update(temp=vec(), r1=vec(), r2=vec())
+    if "cap" in more:
+        kw.update(softcap=3.0)
+    if "sink" in more:
+        kw.update(sink=vec())
+    want = torch.empty(q.shape[0], nq * dv, device=dev)
+    ops.attention_tile(q.float(), step, step.block_table, cache.float(), 1, page, want, nq, nkv, d, dv, d ** -0.5, num_splits=1, **kw)
+    out = torch.full((q.shape[0], nq * dv), float("nan"), device=dev, dtype=torch.bfloat16)
+    ops.attention_tile(q, step, step.block_table, cache, 1, page, out, nq, nkv, d, dv, d ** -0.5, num_splits=splits, **kw)
+    torch.cuda.synchronize()
+    assert torch.isfinite(want).all()
+    err = float((out.float() - want).abs().max())
+    assert err <= 3 * 2.0 ** -9 * float(cache[:, 1, -1].nan_to_num(0.0).abs().max()), err
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("dim,rot,rdims,vd", [(24, 12, 8, 20), (24, 8, 4, 16)])
 def test_latent_attention_far_keys_and_borrowed_cache(ops, dtype, dim, rot, rdims, vd):
