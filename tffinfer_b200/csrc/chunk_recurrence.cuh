@@ -85,26 +85,39 @@ __device__ __forceinline__ float4 load_four(const float* s, int left, bool vec) 
 }
 
 // C rows of ``width`` float32 columns (rows from n on and columns up to wP are zeros) -> bfloat16 rows of ``stride``
-__device__ __forceinline__ void load_rounded(bf16* dst, int stride, const float* __restrict__ src, int ld, int n, int width,
-                                             int wP, int silu) {
-    const int w4 = wP >> 2;
-    const bool vec = ((width | ld) & 3) == 0 && ((uintptr_t)src & 15) == 0;
-    for (int e0 = threadIdx.x; e0 < C * w4; e0 += MT * LOADS) {
-        float4 x[LOADS];                 // a thread's loads are in flight together
+struct Rounded { bf16* dst; int stride; const float* src; int ld, width, wP; };
+
+// N such arrays: a thread's loads of all of them are in flight together (LOADS of 16 bytes of each).
+template <int N>
+__device__ __forceinline__ void load_rounded(const Rounded (&r)[N], int n, int silu) {
+    int most = 0;
 #pragma unroll
-        for (int u = 0; u < LOADS; ++u) {
-            const int e = e0 + u * MT, i = e / w4, c = (e % w4) << 2;
-            x[u] = load_four(src + (size_t)i * ld + c, (i < n && c < width) ? width - c : 0, vec);
+    for (int a = 0; a < N; ++a) most = max(most, C * (r[a].wP >> 2));
+    for (int e0 = threadIdx.x; e0 < most; e0 += MT * LOADS) {
+        float4 x[N][LOADS];
+#pragma unroll
+        for (int a = 0; a < N; ++a) {
+            const int w4 = r[a].wP >> 2;
+            const bool vec = ((r[a].width | r[a].ld) & 3) == 0 && ((uintptr_t)r[a].src & 15) == 0;
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) {
+                const int e = e0 + u * MT, i = e / w4, c = (e % w4) << 2;
+                x[a][u] = load_four(r[a].src + (size_t)i * r[a].ld + c, (i < n && c < r[a].width) ? r[a].width - c : 0, vec);
+            }
         }
 #pragma unroll
-        for (int u = 0; u < LOADS; ++u) {
-            const int e = e0 + u * MT, i = e / w4, c = (e % w4) << 2;
-            if (e >= C * w4) continue;
-            x[u] = ret_in4(x[u], silu);  // (a silu of zero is zero)
-            uint2 v;
-            v.x = pack_bf16(x[u].x, x[u].y);
-            v.y = pack_bf16(x[u].z, x[u].w);
-            *reinterpret_cast<uint2*>(dst + i * stride + c) = v;
+        for (int a = 0; a < N; ++a) {
+            const int w4 = r[a].wP >> 2;
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) {
+                const int e = e0 + u * MT, i = e / w4, c = (e % w4) << 2;
+                if (e >= C * w4) continue;
+                const float4 y = ret_in4(x[a][u], silu);  // (a silu of zero is zero)
+                uint2 v;
+                v.x = pack_bf16(y.x, y.y);
+                v.y = pack_bf16(y.z, y.w);
+                *reinterpret_cast<uint2*>(r[a].dst + i * r[a].stride + c) = v;
+            }
         }
     }
 }
@@ -112,7 +125,8 @@ __device__ __forceinline__ void load_rounded(bf16* dst, int stride, const float*
 // The local part of a chunk of n tokens whose q, k and v are the rows at ``q``, ``k``, ``v`` (leading dimensions behind them):
 //   orow_i = sum_(j<=i) weights.pair(i, j) (q_i . k_j) v_j   (rows o_ld apart),   Uc = sum_j weights.tail(j) k_j v_j^T
 // and, for weights that ask for them (SUMS), weights.row_sum(i, sum_j weights.pair(i, j) (q_i . k_j)).  The rounded k rows
-// stay in shared memory at local_keys().  A chunk's weights are ready in shared memory when this is called.
+// stay in shared memory at local_keys().  What each thread wrote of a chunk's weights to shared memory before it calls this is
+// read behind the first barrier in here.
 static inline size_t local_mma_smem(int d, int dv) {
     return sizeof(bf16) * ((size_t)2 * C * (pad16(d) + 8) + (size_t)C * (pad16(dv) + 8));
 }
@@ -128,9 +142,9 @@ __device__ __forceinline__ void chunk_local_mma(unsigned char* smraw, const floa
     bf16* Ks = local_keys(smraw, d);     // [C][ks]
     bf16* Vs = Ks + C * ks;              // [C][vs]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    load_rounded(Qs, ks, q, q_ld, n, d, dP, silu);
-    load_rounded(Ks, ks, k, k_ld, n, d, dP, silu);
-    load_rounded(Vs, vs, v, v_ld, n, dv, vP, silu);
+    const Rounded qk[2] = {{Qs, ks, q, q_ld, d, dP}, {Ks, ks, k, k_ld, d, dP}}, values[1] = {{Vs, vs, v, v_ld, dv, vP}};
+    load_rounded(qk, n, silu);
+    load_rounded(values, n, silu);       // (with the other two it does not fit in 128 registers)
     __syncthreads();
     {   // a warp: 16 rows of the chunk (all their scores) and half of the value columns
         const int rg = warp & 3, cg = warp >> 2;
@@ -272,21 +286,21 @@ __device__ __forceinline__ void chunk_local_mma(unsigned char* smraw, const floa
 
 // The start state's part, SCOLS value columns from n0 on: orow_i = weights.join(i, (Sc^T q_i), orow_i).  A warp takes eight
 // columns of the state Sc [d, dv] and all rows of the chunk: every element of the state is loaded once, straight into the
-// registers of the product's B operand (three bfloat16 terms), ahead of the queries where d reaches no further than
-// FINISH_ROWS.  Two steps, between which the includer may use the rounded queries in shared memory:
+// registers of the product's B operand (three bfloat16 terms), FINISH_ROWS rows at a time, the first ahead of the queries and
+// the others ahead of the products of those before them.  Two steps, between which the includer may use the rounded queries in shared memory:
 constexpr int FINISH_ROWS = 64, FK = FINISH_ROWS / 16;
-static inline size_t finish_mma_smem(int d) { return sizeof(bf16) * (size_t)C * (pad16(d) + 8); }
+__host__ __device__ inline size_t finish_mma_smem(int d) { return sizeof(bf16) * (size_t)C * (pad16(d) + 8); }
 
-struct FinishRegs { float s[FK][4]; float local[4][4]; };
+struct FinishRegs { float s[FK][4], next[FK][4]; float local[4][4]; };   // next: the FINISH_ROWS rows behind s
 
-__device__ __forceinline__ void finish_load_state(FinishRegs& f, const float* __restrict__ Sc, int d, int dv, int col, int r0) {
+__device__ __forceinline__ void finish_load_state(float (&s)[FK][4], const float* __restrict__ Sc, int d, int dv, int col, int r0) {
     const int kb = 2 * (threadIdx.x & 3);
 #pragma unroll
     for (int kk = 0; kk < FK; ++kk)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int r = r0 + kk * 16 + kb + (e & 1) + (e >> 1) * 8;
-            f.s[kk][e] = (r < d && col < dv) ? __ldcg(Sc + (size_t)r * dv + col) : 0.f;
+            s[kk][e] = (r < d && col < dv) ? __ldcg(Sc + (size_t)r * dv + col) : 0.f;
         }
 }
 
@@ -294,7 +308,7 @@ __device__ __forceinline__ void chunk_finish_load(FinishRegs& f, unsigned char* 
                                                   int n, int d, int dv, int n0, const float* __restrict__ Sc,
                                                   const float* __restrict__ orow, int o_ld) {
     const int dP = pad16(d), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    finish_load_state(f, Sc, d, dv, n0 + warp * 8 + (lane >> 2), 0);
+    finish_load_state(f.s, Sc, d, dv, n0 + warp * 8 + (lane >> 2), 0);
     const int col = n0 + warp * 8 + 2 * (lane & 3);
     const bool two = ((dv | o_ld) & 1) == 0 && ((uintptr_t)orow & 7) == 0;
 #pragma unroll
@@ -308,7 +322,9 @@ __device__ __forceinline__ void chunk_finish_load(FinishRegs& f, unsigned char* 
             else if (i < n) { if (col < dv) x.x = __ldcg(p); if (col + 1 < dv) x.y = __ldcg(p + 1); }
             f.local[rg][2 * hi] = x.x; f.local[rg][2 * hi + 1] = x.y;
         }
-    load_rounded((bf16*)smraw, dP + 8, q, q_ld, n, d, dP, silu);
+    const Rounded rows[1] = {{(bf16*)smraw, dP + 8, q, q_ld, d, dP}};
+    load_rounded(rows, n, silu);
+    finish_load_state(f.next, Sc, d, dv, n0 + warp * 8 + (lane >> 2), FINISH_ROWS);
     __syncthreads();
 }
 
@@ -323,7 +339,13 @@ __device__ __forceinline__ void chunk_finish_mma(FinishRegs& f, const unsigned c
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[rg][e] = 0.f;
     for (int r0 = 0; r0 < dP; r0 += FINISH_ROWS) {
-        if (r0 > 0) finish_load_state(f, Sc, d, dv, n0 + warp * 8 + (lane >> 2), r0);
+        if (r0 > 0) {
+#pragma unroll
+            for (int kk = 0; kk < FK; ++kk)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f.s[kk][e] = f.next[kk][e];
+            if (r0 + FINISH_ROWS < dP) finish_load_state(f.next, Sc, d, dv, n0 + warp * 8 + (lane >> 2), r0 + FINISH_ROWS);
+        }
 #pragma unroll
         for (int kk = 0; kk < FK; ++kk) {
             if (r0 + kk * 16 >= dP) continue;

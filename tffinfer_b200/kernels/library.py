@@ -2036,7 +2036,7 @@ class CudaKernels:
         """Decoded tokens beside portions, one kernel behind the other in the stream, the second one running on the SMs that
         the portions' leaves free (it seldom fills them: a 512-token portion is 80 to 160 CTAs of one an SM): it does not wait
         for the first until it ends.  As two launches on two streams, with their events, an attention layer of the 14B sizes
-        with 512 new tokens and 32 decoded ones took 144 us of the host and 142 of the device, now 87 and 139; of the 4B
+        with 484 new tokens and 28 decoded ones took 144 us of the host and 142 of the device, now 87 and 139; of the 4B
         sizes, 469 behind 443 beside 8 behind up to 4,602, 134 and 90.6, now 84 and 83.6.  False, with nothing launched,
         where the portions' kernel does not take the shape."""
         T = q.shape[0]
