@@ -63,11 +63,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 }
 // x and y as three bfloat16 terms each (a pair a register): 8 + 8 + 8 bits of significand
 __device__ __forceinline__ void split3(float x, float y, uint32_t& t1, uint32_t& t2, uint32_t& t3) {
-    const float x1 = __bfloat162float(__float2bfloat16_rn(x)), y1 = __bfloat162float(__float2bfloat16_rn(y));
-    const float xr = x - x1, yr = y - y1;
-    const float x2 = __bfloat162float(__float2bfloat16_rn(xr)), y2 = __bfloat162float(__float2bfloat16_rn(yr));
-    t1 = pack_bf16(x1, y1);
-    t2 = pack_bf16(x2, y2);
+    t1 = pack_bf16(x, y);                // (one conversion a pair; a term's float32 value is its bits moved up)
+    const float xr = x - __uint_as_float(t1 << 16), yr = y - __uint_as_float(t1 & 0xffff0000u);
+    t2 = pack_bf16(xr, yr);
+    const float x2 = __uint_as_float(t2 << 16), y2 = __uint_as_float(t2 & 0xffff0000u);
     t3 = pack_bf16(xr - x2, yr - y2);
 }
 
@@ -87,39 +86,65 @@ __device__ __forceinline__ float4 load_four(const float* s, int left, bool vec) 
 // C rows of ``width`` float32 columns (rows from n on and columns up to wP are zeros) -> bfloat16 rows of ``stride``
 struct Rounded { bf16* dst; int stride; const float* src; int ld, width, wP; };
 
-// N such arrays: a thread's loads of all of them are in flight together (LOADS of 16 bytes of each).
-template <int N>
-__device__ __forceinline__ void load_rounded(const Rounded (&r)[N], int n, int silu) {
-    int most = 0;
+// N such arrays: a thread's loads of all of them are in flight together (LOADS of 16 bytes of each).  A thread steps from one group
+// of four columns to its next by addition (a division at each, and single conversions in split3: an mlstm layer of 2,048 tokens
+// 180.0 us, now 176.7).  FOURS: every row of every array is whole aligned groups of four.
+template <bool FOURS, int N>
+__device__ __forceinline__ void load_rounded_as(const Rounded (&r)[N], int n, int silu) {
+    int row[N], group[N], rows[N], groups[N];            // the thread's next group, and how far on the one after it lies
+    bool vec[N], more = false;
 #pragma unroll
-    for (int a = 0; a < N; ++a) most = max(most, C * (r[a].wP >> 2));
-    for (int e0 = threadIdx.x; e0 < most; e0 += MT * LOADS) {
+    for (int a = 0; a < N; ++a) {
+        const int w4 = r[a].wP >> 2;
+        row[a] = threadIdx.x / w4; group[a] = threadIdx.x - row[a] * w4;
+        rows[a] = MT / w4; groups[a] = MT - rows[a] * w4;
+        vec[a] = FOURS || (((r[a].width | r[a].ld) & 3) == 0 && ((uintptr_t)r[a].src & 15) == 0);
+        more |= row[a] < C;
+    }
+    auto step = [&](int a, int& i, int& g) {
+        i += rows[a]; g += groups[a];
+        if (g >= (r[a].wP >> 2)) { g -= r[a].wP >> 2; ++i; }
+    };
+    while (more) {
         float4 x[N][LOADS];
 #pragma unroll
         for (int a = 0; a < N; ++a) {
-            const int w4 = r[a].wP >> 2;
-            const bool vec = ((r[a].width | r[a].ld) & 3) == 0 && ((uintptr_t)r[a].src & 15) == 0;
+            int i = row[a], g = group[a];
 #pragma unroll
             for (int u = 0; u < LOADS; ++u) {
-                const int e = e0 + u * MT, i = e / w4, c = (e % w4) << 2;
-                x[a][u] = load_four(r[a].src + (size_t)i * r[a].ld + c, (i < n && c < r[a].width) ? r[a].width - c : 0, vec);
+                const int c = g << 2;
+                const float* at = r[a].src + (size_t)i * r[a].ld + c;
+                const bool in = i < n && c < r[a].width;
+                if (FOURS) x[a][u] = in ? __ldcg(reinterpret_cast<const float4*>(at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                else x[a][u] = load_four(at, in ? r[a].width - c : 0, vec[a]);
+                step(a, i, g);
             }
         }
+        more = false;
 #pragma unroll
         for (int a = 0; a < N; ++a) {
-            const int w4 = r[a].wP >> 2;
 #pragma unroll
             for (int u = 0; u < LOADS; ++u) {
-                const int e = e0 + u * MT, i = e / w4, c = (e % w4) << 2;
-                if (e >= C * w4) continue;
-                const float4 y = ret_in4(x[a][u], silu);  // (a silu of zero is zero)
-                uint2 v;
-                v.x = pack_bf16(y.x, y.y);
-                v.y = pack_bf16(y.z, y.w);
-                *reinterpret_cast<uint2*>(r[a].dst + i * r[a].stride + c) = v;
+                if (row[a] < C) {
+                    const float4 y = ret_in4(x[a][u], silu);  // (a silu of zero is zero)
+                    uint2 v;
+                    v.x = pack_bf16(y.x, y.y);
+                    v.y = pack_bf16(y.z, y.w);
+                    *reinterpret_cast<uint2*>(r[a].dst + row[a] * r[a].stride + (group[a] << 2)) = v;
+                }
+                step(a, row[a], group[a]);
             }
+            more |= row[a] < C;
         }
     }
+}
+template <int N>
+__device__ __forceinline__ void load_rounded(const Rounded (&r)[N], int n, int silu) {
+    bool fours = true;
+#pragma unroll
+    for (int a = 0; a < N; ++a) fours = fours && ((r[a].width | r[a].ld) & 3) == 0 && ((uintptr_t)r[a].src & 15) == 0;
+    if (fours) load_rounded_as<true>(r, n, silu);
+    else load_rounded_as<false>(r, n, silu);
 }
 
 // The local part of a chunk of n tokens whose q, k and v are the rows at ``q``, ``k``, ``v`` (leading dimensions behind them):

@@ -197,7 +197,7 @@ struct LocalWeights {
 
 // What bounds the two kernels of a chunk is a CTA's own chain (loads, products, stores) at two CTAs an SM of up to four waves: the
 // gates' warp works while the others ask for the rows, and the normaliser comes through shared memory.  2,048 tokens, 16
-// heads of 128, the whole layer: 184.1 -> 180.0 us; 3 x 1,123 tokens 306 -> 294.
+// heads of 128, the whole layer: 184.1 -> 176.7 us; 3 x 1,123 tokens 306 -> 294.
 __global__ void __launch_bounds__(MT, 2)
 mlstm_local_kernel(MlstmParams p, int num_requests, Workspace w) {
     extern __shared__ __align__(16) unsigned char smraw[];
