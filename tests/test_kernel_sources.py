@@ -99,3 +99,22 @@ def test_chosen_sources_and_library_names(tmp_path, monkeypatch):
     full = build.library_path()
     assert os.path.basename(full) == build.LIB_NAME and seen[2][1] == build.sources()
     assert build.library_path(files=["latent"]) == full and len(seen) == 3       # the library of all sources serves
+
+
+def _kernel(source, name):
+    """The text of a kernel, from its name to the brace that closes it at the line's start."""
+    with open(os.path.join(build.CSRC_DIR, source), encoding="utf-8") as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    return re.search(r"\n" + name + r"\(.*?\n}\n", text, re.S).group(0)
+
+
+def test_sums_of_few_row_attention_leave_what_the_last_block_reads_alone():
+    """Between the last barrier of a block of keys and the first one behind the loop the warps keep no step: what a warp
+    writes to shared memory behind the loop must not be what another still reads in the block's value phase."""
+    text = _kernel("attention_tile.cu", "attention_tile_few_kernel")
+    loop, behind = text.split("tc5::mbar_arrive(empty_bar(st));")
+    value_phase, hand_over = loop.split("few_barrier();")[-1], behind.split("few_barrier();")[0]
+    read = set(re.findall(r"\b(\w+)\[", value_phase))
+    written = set(re.findall(r"\b(\w+)\[[^\]]*\]\s*=[^=]", hand_over))
+    assert "alpha_s" in read and "m_fin" in written
+    assert not read & written

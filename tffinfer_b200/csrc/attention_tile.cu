@@ -560,7 +560,10 @@ attention_tile_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
 constexpr int FKB = 32, FROWS = 16, FMOST = 32, FWARPS = 8, FTHREADS = (FWARPS + 1) * 32, FPST = FKB + 8, FSST = FKB + 4, FSTAGES = 2;
 constexpr int FKPW = FKB / 4;                                       // keys a warp scores
 
-__device__ __forceinline__ void few_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void few_barrier() {
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    tc5::jitter();
+}
 __device__ __forceinline__ void bulk_row(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -582,8 +585,9 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     float* Ss = (float*)(Pb + FROWS * FPST);                    // [2][FROWS][FSST] products of each half of the elements
     float* alpha_s = Ss + 2 * FROWS * FSST;                     // [FROWS]
     float* m_fin = alpha_s + FROWS;                             // [FROWS]
-    const uint32_t bars = sm_addr(m_fin + FROWS);               // full[FSTAGES], empty[FSTAGES] (8-byte aligned: an even number of words lies ahead)
-    volatile int* abort_flag = (volatile int*)(m_fin + FROWS + 4 * FSTAGES);
+    float* l_fin = m_fin + FROWS;                               // [FROWS]
+    const uint32_t bars = sm_addr(l_fin + FROWS);               // full[FSTAGES], empty[FSTAGES] (8-byte aligned: an even number of words lies ahead)
+    volatile int* abort_flag = (volatile int*)(l_fin + FROWS + 4 * FSTAGES);
     auto full_bar = [&](int s) { return bars + 8u * s; };
     auto empty_bar = [&](int s) { return bars + 8u * (FSTAGES + s); };
 
@@ -786,10 +790,11 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
         __syncwarp();
         if (lane == 0) tc5::mbar_arrive(empty_bar(st));         // this warp is done with the stage
     }
+    // (in arrays of their own: other warps may still be ahead of the last block's values and read alpha_s there)
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
         const float l = warp_sum(l_run[r]);
-        if (lane == 0) { alpha_s[warp * RPW + r] = l; m_fin[warp * RPW + r] = m_run[r]; }
+        if (lane == 0) { l_fin[warp * RPW + r] = l; m_fin[warp * RPW + r] = m_run[r]; }
     }
     few_barrier();
     if (*abort_flag) {
@@ -803,7 +808,7 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
         if (r >= n_rows) continue;
         const int t = t0 + (r0 + r) / G, h = kvh * G + (r0 + r) % G;
         const size_t slot = ((size_t)t * a.nq + h) * a.splits + split;
-        const float inv = a.splits == 1 ? a.out_scale / alpha_s[r] : 1.f;
+        const float inv = a.splits == 1 ? a.out_scale / l_fin[r] : 1.f;
         bf16* orow = out + (size_t)t * a.out_ld + a.out_off + (size_t)h * dv;
         float* prow = a.part_o + slot * dv;
 #pragma unroll
@@ -816,7 +821,7 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
                     else prow[c] = o[j][side * 2 + e];
                 }
             }
-        if (a.splits > 1 && warp == 0 && fc == 0) { a.part_ml[2 * slot] = m_fin[r]; a.part_ml[2 * slot + 1] = alpha_s[r]; }
+        if (a.splits > 1 && warp == 0 && fc == 0) { a.part_ml[2 * slot] = m_fin[r]; a.part_ml[2 * slot + 1] = l_fin[r]; }
     }
 }
 
@@ -829,7 +834,7 @@ int launch_few(const void* q, const void* cache, void* out, const TileArgs& a, i
     gm.kst = (own_v ? gm.dpad : max(gm.dpad, NT * 64)) + 8;
     gm.vst = own_v ? NT * 64 + 8 : gm.kst;
     const size_t smem = 2 * ((size_t)FROWS * gm.kst + (size_t)FSTAGES * FKB * (gm.kst + (own_v ? gm.vst : 0)) + FROWS * FPST) +
-                        4 * ((size_t)2 * FROWS * FSST + 2 * FROWS) + 8 * 2 * FSTAGES + 16;
+                        4 * ((size_t)2 * FROWS * FSST + 3 * FROWS) + 8 * 2 * FSTAGES + 16;
     if (smem > 220 * 1024) return TFF_ERR_UNSUPPORTED;
     static bool configured = false;
     if (!configured) {
