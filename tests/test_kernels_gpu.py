@@ -181,7 +181,7 @@ F32_SHAPES = [(1, 128, 64), (16, 129, 512), (17, 200, 520), (33, 127, 1100), (64
 @pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
                                      (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
 def test_gemm_f32_in_every_tile_width_and_sharing_of_k(ops, M, N, K, adt, wdt):
-    """Every plan gives the same bits, and sums as exact as float32 allows: a chunk of 512 products is cut off 8 x 4 times a
+    """Every plan gives the same bits, and sums as exact as float32 allows: a chunk of 512 products (256 below K = 961) is cut off 8 x 4 times a
     level, 32 x 2^-24 of its size at most, and the chunks add roundings of 2^-24 each."""
     a, w, res = g((M, K), adt, 15).to(DEV), g((N, K), wdt, 16, 0.05).to(DEV), g((M, N), torch.float32, 17).to(DEV)
     want = a.double() @ w.double().t() + res.double()
@@ -200,6 +200,42 @@ def test_gemm_f32_in_every_tile_width_and_sharing_of_k(ops, M, N, K, adt, wdt):
     ops.gemm_simt(a[r:], w, row, res[r:].contiguous())
     assert torch.equal(row, first[r:])
     ops.check_errors()
+
+
+def test_gemm_f32_single_products(ops):
+    """One product an output, of significands whose terms are as large as they get.  The terms left out come to at most
+    2 x 2^-8 x 2^-17 (and 2^-34) of the two powers of two, the sum of the levels is rounded twice (2^-24, and 2^-24 of the 2^-7 that the
+    smaller levels hold at most)."""
+    x = torch.tensor([1 + 2.0 ** -7 - 2.0 ** -23, 1 + 2.0 ** -8 - 2.0 ** -23, 1 + 2.0 ** -8 + 2.0 ** -17, 2 - 2.0 ** -23, 1.5 - 2.0 ** -9 - 2.0 ** -16,
+                      1 + 2.0 ** -8 - 2.0 ** -17 - 2.0 ** -23, 3.4028235e38, 1.0, 1 + 2.0 ** -23, -1 - 2.0 ** -7 + 2.0 ** -23])
+    x = torch.cat([x, g((190,), torch.float32, 20)]).to(DEV)
+    a = torch.zeros(x.numel(), 72, device=DEV)
+    a[torch.arange(x.numel()), torch.arange(x.numel()) % 72] = x
+    y = torch.where(x.abs() > 4, 2.0 ** -100 * torch.sign(x), x)
+    w = y[:, None].expand(-1, 72).contiguous()
+    out = torch.empty(x.numel(), x.numel(), device=DEV)
+    ops.gemm_simt(a, w, out)
+    want = x.double()[:, None] * y.double()[None]
+    bound = (2.0 ** -24 * (1 + 2.0 ** -9) + 2.0 ** -24 * (1 + 2.0 ** -6)) * want.abs()
+    fits = want.abs() <= 3.4028235e38
+    assert torch.equal(out.isinf(), ~fits)
+    assert bool(((out.double() - want).abs() <= bound)[fits].all()), float(((out.double() - want).abs() / want.abs())[fits].max())
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("K", [1, 9, 65, 250, 510, 700, 1020, 1100])
+def test_gemm_f32_is_as_exact_as_a_chain_of_fmas(ops, adt, wdt, K):
+    """The 2-norm of the error beside that of a chain of FMAs (one rounding a product) over the same random operands.  Where they
+    are closest, at one K block, both are a few roundings: 1.15 covers how the norms of 16,384 of them scatter."""
+    a, w = g((64, K), adt, 21).to(DEV), g((256, K), wdt, 22).to(DEV)
+    out, chain = torch.empty(64, 256, device=DEV), torch.zeros(64, 256, device=DEV)
+    ops.gemm_simt(a, w, out)
+    want = a.double() @ w.double().t()
+    for k in range(K):
+        chain = (chain.double() + a[:, k, None].double() * w[None, :, k].double()).float()
+    error, other = float((out.double() - want).norm()), float((chain.double() - want).norm())
+    assert error <= 1.15 * other, (error / float(want.norm()), other / float(want.norm()))
 
 
 @pytest.mark.parametrize("slices", [1, 3])

@@ -2,12 +2,12 @@
 // every operand stored in float32, on the 5th-generation tensor cores.
 // It stands in for the reference's dense fp32 GEMM (src/kernel/cuda/mat_mul.cu:151-660).
 //
-// A float32 number is the sum of three bfloat16 terms x = h + m + l, exactly: each takes the next 8 bits of the
-// significand (cut off, not rounded, so that h never overflows).  Of the nine products of two such sums six are
-// computed, those down to 2^-16 of the largest; the other three are below half a unit in the last place of the product
-// of the two elements.  Products of equal size are summed in accumulators of their own in tensor memory
-// (S0: hh; S1: hm, mh; S2: hl, mm, lh), for CHUNK_BLOCKS blocks of K at a time: the tensor core cuts off where it adds,
-// which drifts over a long sum, so the chunks' sums (S0 + S1) + S2 are added rounded to nearest, in ascending order.
+// A float32 number from 2^-110 on is the sum of three bfloat16 terms x = h + m + l, exactly: each is what is left, rounded to
+// 8 bits, so that |m| <= 2^-8 and |l| <= 2^-17 of x's power of two (below 2^-110 what l loses is at most 2^-134).  Of the nine products
+// of two such sums six are computed, those down to 2^-16 of the largest; the other three (ml, lm, ll) come to at most half a
+// unit in the last place of the product of the two elements, of either sign.  Products of equal size are summed in accumulators
+// of their own in tensor memory (S0: hh; S1: hm, mh; S2: hl, mm, lh), for a chunk of K at a time: the tensor core cuts off where it
+// adds, which drifts over a long sum, so the chunks' sums S0 + (S1 + S2) are added rounded to nearest, in ascending order.
 //
 // Every output element goes through the same sequence of operations whatever M is, which tile it falls in and how the
 // K range was shared out (a product of few rows writes every chunk's sum to a workspace and a second kernel adds
@@ -15,11 +15,12 @@
 // finite is computed once more as a plain sum of products, since a split of an infinity has no meaning.
 //
 // What bounds it.  Few rows: the latency of the memory, since registers hold only the two K blocks (64 KB) on their way while the
-// threads split (4 rows of the 8B shape's gate/up product, 403 MB: 94 us = 4.3 TB/s; down 61 us; as float32 FMAs, one order of
+// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill 140 to 190 bytes (4 rows of the 8B shape's gate/up product, 403 MB: 94 us = 4.3 TB/s; down 61 us; as float32 FMAs, one order of
 // summation a thread, 1.4 ms each).  Asking the L2 for the weights one chunk ahead made it slower (102 us).  Many rows: shared memory, which
 // takes 6 bytes an element from the split and feeds six products, beside the products themselves (512 rows of gate/up 0.71 ms,
-// 145 TFLOP/s; without the products 0.48, without the loads 0.45; FMAs at most 70).  Off 64-bit arithmetic by 5.2e-7
-// (2-norm, K = 4,096 and 12,288); the FMA sum over all of K was by 1.4e-6 and 2.4e-6.
+// 145 TFLOP/s; without the products 0.48, without the loads 0.45; FMAs at most 70).  Off 64-bit arithmetic
+// (2-norm, random operands) by 2.6e-8 at K = 1, 3.1e-8 at 8, 7.0e-8 at 64, 2.3e-7 at 512, 4.8e-7 at 1,024 and 4,096; a chain of FMAs over
+// all of K is by 2.6e-8, 5.4e-8, 1.4e-7, 3.9e-7, 5.7e-7 and 1.1e-6.
 //
 //   warps 1-16   read 8 elements of a row at a time from global memory, one or two K blocks ahead, split them and write
 //                the terms to shared memory as 128-byte-swizzled K-major tiles
@@ -34,7 +35,10 @@ namespace {
 
 using namespace tc5;
 
-constexpr int CHUNK_BLOCKS = 8;                       // K blocks of 64 whose products meet in tensor memory
+// K blocks of 64 whose products meet in tensor memory.  What the tensor core cuts off grows with their number: with 8 an element is
+// off by 4.8e-7 from K = 512 on (2-norm of random operands), a chain of FMAs by 4.0e-7 at 512 and 5.7e-7 at 1,024; with 4 by
+// 2.3e-7 from K = 256 on, the chain by 2.9e-7 at 256.  Short sums so take chunks of 4, long ones half as many drains.
+__host__ __device__ constexpr int chunk_blocks(int kbt) { return kbt < 16 ? 4 : 8; }
 
 template <int BN, int NA, int NW> struct F32Cfg {
     static constexpr int kWPlane = BM * BK * 2, kAPlane = BN * BK * 2;
@@ -107,6 +111,11 @@ __device__ __forceinline__ void st_shared16(uint32_t dst, const uint32_t* v) {
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
 
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {      // rounded to nearest
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
 // The terms of 8 elements, 16 bytes a plane, ``plane`` bytes apart.
 template <typename T>
 __device__ __forceinline__ void split_store(const uint32_t* r, uint32_t dst, uint32_t plane) {
@@ -115,15 +124,12 @@ __device__ __forceinline__ void split_store(const uint32_t* r, uint32_t dst, uin
     } else {
         uint32_t h[4], m[4], l[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t a = r[2 * i], b = r[2 * i + 1];
-            const float ra = __uint_as_float(a) - __uint_as_float(a & 0xffff0000u);       // exact: the lower 16 bits
-            const float rb = __uint_as_float(b) - __uint_as_float(b & 0xffff0000u);
-            const uint32_t ma = __float_as_uint(ra), mb = __float_as_uint(rb);
-            const float la = ra - __uint_as_float(ma & 0xffff0000u), lb = rb - __uint_as_float(mb & 0xffff0000u);
-            h[i] = __byte_perm(a, b, 0x7632);
-            m[i] = __byte_perm(ma, mb, 0x7632);
-            l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+        for (int i = 0; i < 4; ++i) {                // (the differences are exact)
+            const float a = __uint_as_float(r[2 * i]), b = __uint_as_float(r[2 * i + 1]);
+            h[i] = pack2(a, b);
+            const float ra = a - __uint_as_float(h[i] << 16), rb = b - __uint_as_float(h[i] & 0xffff0000u);
+            m[i] = pack2(ra, rb);
+            l[i] = pack2(ra - __uint_as_float(m[i] << 16), rb - __uint_as_float(m[i] & 0xffff0000u));
         }
         st_shared16(dst, h);
         st_shared16(dst + plane, m);
@@ -162,22 +168,22 @@ __device__ __forceinline__ void store_result(void* out, int out_bf16, const floa
 
 // Which part of the product a unit is.  Units of one weight tile and K slice lie together, activation tiles fastest, and go
 // round-robin to the CTAs: those that run together read the same weights.
+struct Share { int slices, blocks, chunk; };      // in how many slices K is cut, K blocks a slice and a chunk
 struct Unit {
-    int n0, m0, slice, kb0, kb1;
-    __device__ Unit(int u, int tiles_m, int slices, int kbt, int bn) {
+    int n0, m0, kb0, kb1;
+    __device__ Unit(int u, int tiles_m, const Share& sh, int kbt, int bn) {
         const int tm = u % tiles_m, v = u / tiles_m;
-        slice = v % slices;
-        n0 = v / slices * BM;
+        n0 = v / sh.slices * BM;
         m0 = tm * bn;
-        kb0 = slices > 1 ? slice * CHUNK_BLOCKS : 0;
-        kb1 = slices > 1 ? min(kb0 + CHUNK_BLOCKS, kbt) : kbt;
+        kb0 = v % sh.slices * sh.blocks;                              // (the launcher has checked that no slice is empty)
+        kb1 = min(kb0 + sh.blocks, kbt);
     }
 };
 
 template <int BN, typename TA, typename TW, bool VEC>
 __global__ void __launch_bounds__(F32Cfg<BN, sizeof(TA) == 4 ? 3 : 1, sizeof(TW) == 4 ? 3 : 1>::kThreads, 1)
 gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, int out_bf16, const float* residual,
-                float* __restrict__ ws, int M, int N, int K, int slices, int* error_flag) {
+                float* __restrict__ ws, int M, int N, int K, const Share sh, int* error_flag) {
     constexpr int NA = sizeof(TA) == 4 ? 3 : 1, NW = sizeof(TW) == 4 ? 3 : 1;
     using Cfg = F32Cfg<BN, NA, NW>;
     constexpr int STAGES = Cfg::kStages, BUFS = Cfg::kBufs;
@@ -195,7 +201,7 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kbt = (K + BK - 1) / BK;
     const int tiles_m = (M + BN - 1) / BN;
-    const int units = (N + BM - 1) / BM * slices * tiles_m;             // the launcher has checked that it fits
+    const int units = (N + BM - 1) / BM * sh.slices * tiles_m;             // the launcher has checked that it fits
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), Cfg::kConv / 32); mbar_init(empty_bar(s), 1); }
@@ -216,13 +222,13 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
             uint32_t n = 0, chunk_no = 0;
             bool ok = true;
             for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
-                const Unit it(u, tiles_m, slices, kbt, BN);
-                for (int c0 = it.kb0; ok && c0 < it.kb1; c0 += CHUNK_BLOCKS, ++chunk_no) {
+                const Unit it(u, tiles_m, sh, kbt, BN);
+                for (int c0 = it.kb0; ok && c0 < it.kb1; c0 += sh.chunk, ++chunk_no) {
                     const uint32_t buf = chunk_no % BUFS, use = chunk_no / BUFS;
                     if (use > 0 && !mbar_wait(tempty_bar(buf), (use - 1) & 1, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t d = tmem_base + buf * Cfg::kBufCols;
-                    const int c1 = min(c0 + CHUNK_BLOCKS, it.kb1);
+                    const int c1 = min(c0 + sh.chunk, it.kb1);
                     for (int kb = c0; kb < c1; ++kb, ++n) {
                         const int s = n % STAGES;
                         if (!mbar_wait(full_bar(s), (n / STAGES) & 1, abort_flag)) { ok = false; break; }
@@ -264,7 +270,7 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
         const uint32_t cell = (uint32_t)row * 128u + (uint32_t)((oct ^ (row & 7)) << 4);
         uint32_t wr[W_ITEMS][WR], ar[A_ITEMS][AR];
         int u = blockIdx.x;
-        Unit it(u, tiles_m, slices, kbt, BN);
+        Unit it(u, tiles_m, sh, kbt, BN);
         int kb = it.kb0;
         const TW* wp;                                                        // this thread's first item of the K block, and how many
         const TA* ap;                                                        // rows and elements of the operands lie from there on
@@ -283,7 +289,7 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
         auto step = [&]() {                                                  // to the next K block of the CTA
             if (++kb >= it.kb1) {
                 u += gridDim.x;
-                if (u < units) { it = Unit(u, tiles_m, slices, kbt, BN); kb = it.kb0; }
+                if (u < units) { it = Unit(u, tiles_m, sh, kbt, BN); kb = it.kb0; }
             }
         };
         for (int g = 0; g < group; ++g) if (u < units) step();
@@ -336,14 +342,14 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
         uint32_t chunk_no = 0;
         bool ok = true;
         for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
-            const Unit it(u, tiles_m, slices, kbt, BN);
+            const Unit it(u, tiles_m, sh, kbt, BN);
             const int n = it.n0 + q * 32 + lane;
-            for (int c0 = it.kb0; c0 < it.kb1; c0 += CHUNK_BLOCKS, ++chunk_no) {
+            for (int c0 = it.kb0; c0 < it.kb1; c0 += sh.chunk, ++chunk_no) {
                 const uint32_t buf = chunk_no % BUFS, use = chunk_no / BUFS;
                 if (!mbar_wait(tfull_bar(buf), use & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t t_addr = t_lane + buf * Cfg::kBufCols;
-                const bool first = c0 == it.kb0, last = c0 + CHUNK_BLOCKS >= it.kb1;
+                const bool first = sh.slices > 1 || c0 == it.kb0, last = sh.slices > 1 || c0 + sh.chunk >= it.kb1;
 #pragma unroll 1
                 for (int j0 = 0; j0 < COLS; j0 += 16) {
                     uint32_t s0[16], s1[16], s2[16], sum[16];
@@ -362,15 +368,15 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         float p = __uint_as_float(s0[j]);
-                        if constexpr (Cfg::kLevels == 3) p = (p + __uint_as_float(s1[j])) + __uint_as_float(s2[j]);
+                        if constexpr (Cfg::kLevels == 3) p += __uint_as_float(s1[j]) + __uint_as_float(s2[j]);
                         sum[j] = __float_as_uint(first ? p : __uint_as_float(sum[j]) + p);
                     }
                     if (!last) {
                         tmem_st16(t_lane + Cfg::kSumCol + j0, sum);
                     } else {
                         const int m1 = it.m0 + first_col + j0;
-                        if (slices > 1) {
-                            float* p = ws + ((size_t)it.slice * M + m1) * N + n;
+                        if (sh.slices > 1) {
+                            float* p = ws + ((size_t)(c0 / sh.chunk) * M + m1) * N + n;
 #pragma unroll
                             for (int j = 0; j < 16; ++j)
                                 if (m1 + j < M && n < N) p[(size_t)j * N] = __uint_as_float(sum[j]);
@@ -421,20 +427,20 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
     }
 }
 
-// out = sum of the slices' partial results, in ascending order (+ residual).
+// out = sum of the chunks' partial results, in ascending order (+ residual).
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(256)
 gemm_f32_sum_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const float* __restrict__ ws, void* out, int out_bf16,
-                    const float* residual, int M, int N, int K, int slices) {
+                    const float* residual, int M, int N, int K, int chunks) {
     pdl_launch_dependents();
     pdl_wait();
     const long long total = (long long)M * N, i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
-    const bool vec = (total & 3) == 0;                       // slices then start 16-byte aligned
+    const bool vec = (total & 3) == 0;                       // chunks then start 16-byte aligned
     const int cnt = i >= total ? 0 : (int)(total - i < 4 ? total - i : 4);
     if (cnt > 0) {
 #pragma unroll 4
-        for (int s = 0; s < slices; ++s) {
+        for (int s = 0; s < chunks; ++s) {
             const float* p = ws + (size_t)s * total + i;
             float t[4] = {0.f, 0.f, 0.f, 0.f};
             if (vec) {
@@ -460,13 +466,17 @@ gemm_f32_sum_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const fl
 
 // ------------------------------------------------------------------- host side
 struct F32Plan { int bn, slices; };
+int chunk_count(int K) {
+    const int kbt = (K + BK - 1) / BK;
+    return (kbt + chunk_blocks(kbt) - 1) / chunk_blocks(kbt);
+}
 
 // Tile width and whether the K range is shared out, from M, N, K and the SM count.  A K block of a tile takes about the
 // clocks below (reading and splitting 128 weight rows and bn activation rows, their products: fitted to 60 times of the products of the
 // 8B shape at 1 to 2,048 rows); tiles run in rounds of one a SM.
 F32Plan f32_plan(int M, int N, int K) {
     const int sms = tff_num_sms() > 0 ? tff_num_sms() : 148;
-    const int kbt = (K + BK - 1) / BK, chunks = (kbt + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;
+    const int kbt = (K + BK - 1) / BK, chunks = chunk_count(K);
     const long long tiles_n = (N + BM - 1) / BM;
     const int bns[4] = {16, 32, 64, 128};
     const double clocks[4] = {1720., 1720., 2300., 3300.};
@@ -479,7 +489,7 @@ F32Plan f32_plan(int M, int N, int K) {
             const int slices = split ? chunks : 1;
             const long long rounds = (tiles * slices + sms - 1) / sms;
             // a round also starts up and drains; the partial results are written and read once more
-            double cost = (double)rounds * (split ? CHUNK_BLOCKS : kbt) * clocks[b] + 3000.;
+            double cost = (double)rounds * (split ? chunk_blocks(kbt) : kbt) * clocks[b] + 3000.;
             if (split) cost += 6000. + 2.0 * slices * (double)M * N * 4. / 2600.;
             if (cost < best_cost) { best_cost = cost; best = {bns[b], slices}; }
         }
@@ -503,12 +513,14 @@ int launch(const void* A, const void* W, void* C, int out_bf16, const float* res
     if (ctas <= 0 || tff_device_error_flag() == nullptr) return TFF_ERR_LAUNCH;
     if (units + ctas >= (1ll << 31)) return TFF_ERR_UNSUPPORTED;
     if (ctas > units) ctas = units;
+    const int chunk = chunk_blocks((K + BK - 1) / BK);
+    const Share sh = {slices, (chunk_count(K) + slices - 1) / slices * chunk, chunk};
     int st = tff_launch_pdl(kern, dim3((unsigned)ctas), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, (const TA*)A,
-                            (const TW*)W, C, out_bf16, residual, ws, M, N, K, slices, tff_device_error_flag());
+                            (const TW*)W, C, out_bf16, residual, ws, M, N, K, sh, tff_device_error_flag());
     if (st == TFF_OK && slices > 1) {
         const long long blocks = ((long long)M * N + 1023) / 1024;
         st = tff_launch_pdl(gemm_f32_sum_kernel<TA, TW>, dim3((unsigned)blocks), dim3(256), (size_t)0, stream, (const TA*)A,
-                            (const TW*)W, (const float*)ws, C, out_bf16, residual, M, N, K, slices);
+                            (const TW*)W, (const float*)ws, C, out_bf16, residual, M, N, K, chunk_count(K));
     }
     return st;
 }
@@ -542,17 +554,20 @@ TFF_API int tff_gemm_f32_plan(int M, int N, int K) {
     return p.bn | (p.slices << 16);
 }
 
+// How many chunks of the K range have a partial result of their own (with more than one slice).
+TFF_API int tff_gemm_f32_chunks(int K) { return K <= 0 ? 1 : chunk_count(K); }
+
 // dtype codes: 0 = float32, 1 = bfloat16.  ``residual`` (float32 [M, N], may alias C
 // when C is float32) is added to the product when it is not null.  ``plan`` as tff_gemm_f32_plan gives it; with more than
-// one slice (then one for every CHUNK_BLOCKS K blocks) ``ws`` holds slices * M * N floats.
+// one slice (each of as many whole chunks, none empty) ``ws`` holds tff_gemm_f32_chunks(K) * M * N floats.
 TFF_API int tff_gemm_f32(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt, const float* residual,
                          float* ws, int M, int N, int K, int plan, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return TFF_OK;
     if (K <= 0 || (a_dt & ~1) || (w_dt & ~1) || (c_dt & ~1)) return TFF_ERR_BAD_ARGUMENT;
     const F32Plan p = {plan & 0xffff, plan >> 16};
-    const int chunks = ((K + BK - 1) / BK + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;
-    if ((p.bn != 16 && p.bn != 32 && p.bn != 64 && p.bn != 128) || (p.slices != 1 && p.slices != chunks) ||
-        (p.slices > 1 && ws == nullptr))
+    const int chunks = chunk_count(K);
+    if ((p.bn != 16 && p.bn != 32 && p.bn != 64 && p.bn != 128) || p.slices < 1 || p.slices > chunks ||
+        (long long)(p.slices - 1) * ((chunks + p.slices - 1) / p.slices) >= chunks || (p.slices > 1 && ws == nullptr))
         return TFF_ERR_BAD_ARGUMENT;
     switch (a_dt * 2 + w_dt) {
         case 0: return dispatch_vec<float, float>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);

@@ -276,7 +276,9 @@ class CudaKernels:
         if plan is None:
             plan = self.lib.tff_gemm_f32_plan(_c_int(M), _c_int(N), _c_int(K))
         slices = plan >> 16
-        ws = torch.empty(slices * M * N, dtype=torch.float32, device=a.device) if slices > 1 else None
+        ws = None
+        if slices > 1:
+            ws = torch.empty(self.lib.tff_gemm_f32_chunks(_c_int(K)) * M * N, dtype=torch.float32, device=a.device)
         self._check(self.lib.tff_gemm_f32(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _ptr(out),
                                           _c_int(_dt(out)), _ptr(residual), _ptr(ws), _c_int(M), _c_int(N), _c_int(K),
                                           _c_int(plan), self._stream()), "gemm_f32")
