@@ -223,7 +223,7 @@ def test_gemm_f32_single_products(ops):
     ops.check_errors()
 
 
-@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("K", [1, 9, 65, 250, 510, 700, 1020, 1100])
 def test_gemm_f32_is_as_exact_as_a_chain_of_fmas(ops, adt, wdt, K):
     """The 2-norm of the error beside that of a chain of FMAs (one rounding a product) over the same random operands.  Where they

@@ -45,7 +45,7 @@ def sources() -> List[str]:
 
 
 # Every model's: embedding, norms, products, sampling, state slots, the host side of TMA.
-CORE = ("elementwise", "gemm_f32", "gemm_tc", "gemm_tc_pair", "sampling", "tma_host")
+CORE = ("elementwise", "gemm_f32", "gemm_simt", "gemm_tc", "gemm_tc_pair", "sampling", "tma_host")
 
 
 def chosen_sources(files: Optional[Iterable[str]]) -> List[str]:

@@ -1,5 +1,5 @@
-// C[M, N] = A[M, K] * W[N, K]^T (+ residual) at float32 precision: the matrix product of the true 32-bit path and of
-// every operand stored in float32, on the 5th-generation tensor cores.
+// C[M, N] = A[M, K] * W[N, K]^T (+ residual) at float32 precision: the matrix product of the true 32-bit path, of
+// an operand at least that is stored in float32, on the 5th-generation tensor cores.
 // It stands in for the reference's dense fp32 GEMM (src/kernel/cuda/mat_mul.cu:151-660).
 //
 // A float32 number from 2^-110 on is the sum of three bfloat16 terms x = h + m + l, exactly: each is what is left, rounded to
@@ -45,7 +45,8 @@ template <int BN, int NA, int NW> struct F32Cfg {
     static constexpr int kStageBytes = NW * kWPlane + NA * kAPlane;
     static constexpr int kFit = (220 * 1024) / kStageBytes;
     static constexpr int kStages = kFit > 4 ? 4 : kFit;
-    static constexpr int kLevels = (NA + NW - 1) > 3 ? 3 : (NA + NW - 1);
+    static constexpr int kLevels = 3;               // one operand at least has three terms
+    static_assert(NA == 3 || NW == 3, "a split operand");
     // tensor memory: one or two buffers of the levels' sums, then the running sum of the chunks
     static constexpr int kBufCols = kLevels * BN;
     static constexpr int kBufs = 2 * kBufCols + BN <= 512 ? 2 : 1;
@@ -354,21 +355,17 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
                 for (int j0 = 0; j0 < COLS; j0 += 16) {
                     uint32_t s0[16], s1[16], s2[16], sum[16];
                     tmem_ld16(t_addr + j0, s0);
-                    if constexpr (Cfg::kLevels == 3) {
-                        tmem_ld16(t_addr + BN + j0, s1);
-                        tmem_ld16(t_addr + 2 * BN + j0, s2);
-                    }
+                    tmem_ld16(t_addr + BN + j0, s1);
+                    tmem_ld16(t_addr + 2 * BN + j0, s2);
                     if (!first) tmem_ld16(t_lane + Cfg::kSumCol + j0, sum);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {                 // nothing below may move ahead of the wait
-                        asm volatile("" : "+r"(s0[j]), "+r"(sum[j]));
-                        if constexpr (Cfg::kLevels == 3) asm volatile("" : "+r"(s1[j]), "+r"(s2[j]));
+                        asm volatile("" : "+r"(s0[j]), "+r"(sum[j]), "+r"(s1[j]), "+r"(s2[j]));
                     }
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        float p = __uint_as_float(s0[j]);
-                        if constexpr (Cfg::kLevels == 3) p += __uint_as_float(s1[j]) + __uint_as_float(s2[j]);
+                        const float p = __uint_as_float(s0[j]) + (__uint_as_float(s1[j]) + __uint_as_float(s2[j]));
                         sum[j] = __float_as_uint(first ? p : __uint_as_float(sum[j]) + p);
                     }
                     if (!last) {
@@ -557,7 +554,7 @@ TFF_API int tff_gemm_f32_plan(int M, int N, int K) {
 // How many chunks of the K range have a partial result of their own (with more than one slice).
 TFF_API int tff_gemm_f32_chunks(int K) { return K <= 0 ? 1 : chunk_count(K); }
 
-// dtype codes: 0 = float32, 1 = bfloat16.  ``residual`` (float32 [M, N], may alias C
+// dtype codes: 0 = float32, 1 = bfloat16 (one operand at most).  ``residual`` (float32 [M, N], may alias C
 // when C is float32) is added to the product when it is not null.  ``plan`` as tff_gemm_f32_plan gives it; with more than
 // one slice (each of as many whole chunks, none empty) ``ws`` holds tff_gemm_f32_chunks(K) * M * N floats.
 TFF_API int tff_gemm_f32(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt, const float* residual,
@@ -573,6 +570,6 @@ TFF_API int tff_gemm_f32(const void* A, int a_dt, const void* W, int w_dt, void*
         case 0: return dispatch_vec<float, float>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);
         case 1: return dispatch_vec<float, bf16>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);
         case 2: return dispatch_vec<bf16, float>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);
-        default: return dispatch_vec<bf16, bf16>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);
     }
+    return TFF_ERR_UNSUPPORTED;                  // two bfloat16 operands: gemm_tc.cu, gemm_simt.cu
 }

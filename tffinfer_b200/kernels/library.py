@@ -269,10 +269,18 @@ class CudaKernels:
             self.gemm_simt(a, w, out, residual)
 
     def gemm_simt(self, a, w, out, residual=None, plan=None) -> None:
-        """The product at float32 precision for any mix of float32 / bfloat16 operands (csrc/gemm_f32.cu): a row of the
-        result does not depend on the other rows.  ``plan`` as tff_gemm_f32_plan gives it (None: its choice)."""
+        """The product at float32 precision for any mix of float32 / bfloat16 operands: a row of the result does not depend on
+        the other rows.  With a float32 operand on the tensor cores (csrc/gemm_f32.cu), ``plan`` as tff_gemm_f32_plan gives it
+        (None: its choice); of two bfloat16 operands as a chain of FMAs (csrc/gemm_simt.cu)."""
         M, K = a.shape
         N = w.shape[0]
+        if out.data_ptr() in self._acc_zero:
+            self._acc_zero[out.data_ptr()] = False     # an accumulator buffer that now holds a product
+        if a.dtype == w.dtype == torch.bfloat16:
+            self._check(self.lib.tff_gemm_simt(_ptr(a), _ptr(w), _ptr(out), _c_int(_dt(out)), _ptr(residual), _c_int(M),
+                                               _c_int(N), _c_int(K), self._stream()), "gemm_simt")
+            self.launches += 1
+            return
         if plan is None:
             plan = self.lib.tff_gemm_f32_plan(_c_int(M), _c_int(N), _c_int(K))
         slices = plan >> 16
@@ -282,8 +290,6 @@ class CudaKernels:
         self._check(self.lib.tff_gemm_f32(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _ptr(out),
                                           _c_int(_dt(out)), _ptr(residual), _ptr(ws), _c_int(M), _c_int(N), _c_int(K),
                                           _c_int(plan), self._stream()), "gemm_f32")
-        if out.data_ptr() in self._acc_zero:
-            self._acc_zero[out.data_ptr()] = False     # an accumulator buffer that now holds a product
         self.launches += 2 if slices > 1 else 1
 
     FOLD_MAX_M = 16           # up to this many rows the norm is folded into the gate/up product (with SwiGLU)
