@@ -52,3 +52,21 @@ def test_parameters_and_their_types(params, want):
 def test_a_type_without_a_counterpart_is_refused():
     with pytest.raises(library.KernelError):
         library.function_signatures("TFF_API int tff_f(double x) {")
+
+
+def test_arguments_are_refused_as_ctypes_refuses_them():
+    """What a call passes goes through makers that take and refuse what ctypes.c_int and ctypes.c_float do."""
+    import numpy as np
+    import torch
+    values = [3, True, -1, 2.5, 2.0, "3", None, np.int64(5), np.float64(1.5), torch.tensor(4), torch.tensor(0.5), [1], 2 ** 31]
+    for maker, kind in ((library._c_int, ctypes.c_int), (library._c_float, ctypes.c_float)):
+        for value in values:
+            try:
+                want = kind(value).value
+            except TypeError:
+                with pytest.raises(TypeError):
+                    maker(value)
+            else:
+                assert kind(maker(value)).value == want, (kind, value)
+    with open(library.__file__, encoding="utf-8") as f:
+        assert " ll = int\n" not in f.read()

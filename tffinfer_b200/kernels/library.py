@@ -14,6 +14,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import math
+import operator
 import os
 import re
 from typing import Optional
@@ -25,9 +26,16 @@ from ..csrc import build as _build
 
 # What a call passes are plain numbers: the functions' argument types are declared when the library is loaded (declare_functions),
 # and ctypes converts.  An object of a ctypes type for every argument, and torch's stream object for every launch, were
-# half of a call's host time.
-_c_int = int
-_c_float = float
+# half of a call's host time.  Each maker refuses what ctypes' own refuses: a whole number is one already, and no text is a number.
+_c_int = operator.index
+
+
+def _c_float(x) -> float:
+    if type(x) is not float:
+        x = ctypes.c_float(x).value
+    return x
+
+
 _vp = ctypes.c_void_p
 
 _STATUS = {
@@ -1086,7 +1094,7 @@ class CudaKernels:
             code = 0                      # a plain product: only a function of one product ("relu2") is applied to it
         act = _c_int(code)
         clip = (_c_float(limit), _c_float(self.CLIPPED_SLOPE))
-        ll = int
+        ll = _c_int
         if self.grouped_on_tensor_cores(a, b, K, lda, a_gs, ldb, b_gs, gated, N) and tile_rows in (
                 0, self.grouped_tile_rows(True), self.grouped_tile_rows(True, True)):
             if not tile_rows:
@@ -1228,7 +1236,7 @@ class CudaKernels:
         W = x.shape[-1]
         assert state.dtype == torch.int32 and x.dtype == torch.float32 and tuple(table.shape) == (buckets + 1, W)
         assert x.shape[0] == batch.num_tokens and (copies == 0 or x.shape[1] == copies)
-        ll = int
+        ll = _c_int
         self._check(self.lib.tff_pair_embed(_ptr(batch.token_ids), _ptr(batch.positions), _ptr(batch.tok_req),
                                             _ptr(batch.q_start), _ptr(batch.slots), _ptr(state), _ptr(table),
                                             _c_int(_dt(table)), _c_int(buckets), ll(mul_prev), ll(mul_cur), _ptr(x),
