@@ -78,6 +78,19 @@ def test_prompt_sized_products_take_the_configuration_with_the_fewest_waves():
     assert plan(2048, 128, 4096, False)[1] in (256, 128)
 
 
+def test_costs_are_those_of_the_library_that_plans():
+    """Plans are kept by size and by what they were made from: another table of costs gives another plan."""
+    def planner(**table):
+        p = CudaKernels.__new__(CudaKernels)
+        p.NUM_SMS, p.USE_SM_PAIRS = 148, True
+        if table:
+            p.TILE_COST = {**CudaKernels.TILE_COST, **{int(bn[1:]): c for bn, c in table.items()}}
+        return p
+    assert planner().prompt_plan(2048, 6144, 4096, False) == (0, 512, 0)
+    assert planner(b512=(9.0, 3.0, 256, 256, 2)).prompt_plan(2048, 6144, 4096, False)[1] == 256
+    assert planner().prompt_plan(2048, 6144, 4096, False) == (0, 512, 0)
+
+
 def test_small_portions_behind_long_contexts_take_key_shares():
     """A portion of up to 256 packed rows (tokens times query heads a key/value head) behind 2,048 or more keys
     is cut along its keys so that every SM gets two CTAs of 64-row tiles; larger portions, short contexts

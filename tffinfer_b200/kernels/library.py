@@ -332,17 +332,17 @@ class CudaKernels:
     def prompt_costs(self, M: int, N: int, K: int, added: bool, kinds=(512, 256, 128)):
         """{bn: (estimated us, slices)} of the normal-orientation configurations for a prompt-sized product; the
         last wave's tiles are cut along K only where the result is added to a float32 buffer."""
-        return dict(self._prompt_costs(self.NUM_SMS, self.USE_SM_PAIRS, M, N, K, added, tuple(kinds)))
+        return dict(self._prompt_costs(self.NUM_SMS, self.USE_SM_PAIRS, M, N, K, added,
+                                       tuple([(bn, *self.TILE_COST[bn]) for bn in kinds])))
 
     @staticmethod
     @functools.lru_cache(maxsize=4096)
     def _prompt_costs(num_sms: int, pairs: bool, M: int, N: int, K: int, added: bool, kinds):
         kb = -(-K // 64)
         costs = {}
-        for bn in kinds:
+        for bn, c, launch, tm, tn, sms in kinds:
             if bn == 512 and (not pairs or N <= 128):
                 continue
-            c, launch, tm, tn, sms = CudaKernels.TILE_COST[bn]
             tiles, slots = -(-M // tm) * -(-N // tn), max(1, num_sms // sms)
             waves, tail = divmod(tiles, slots)
             slices = CudaKernels.tail_slices(tiles, kb, slots) if added else 0
