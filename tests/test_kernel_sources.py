@@ -118,3 +118,29 @@ def test_sums_of_few_row_attention_leave_what_the_last_block_reads_alone():
     written = set(re.findall(r"\b(\w+)\[[^\]]*\]\s*=[^=]", hand_over))
     assert "alpha_s" in read and "m_fin" in written
     assert not read & written
+
+
+# Kernels launched with programmatic dependent launch, and the pointers through which they read what the kernels ahead wrote
+READ_PAST_L1 = [
+    ("gemm_f32.cu", "gemm_f32_kernel", ("A", "W", "residual")),
+    ("gemm_f32.cu", "gemm_f32_sum_kernel", ("A", "W", "ws", "residual", "p")),
+    ("attention_generic.cu", "attention_generic_kernel", ("q_in", "cache", "gate", "src")),
+    ("attention_generic.cu", "attention_generic_join_kernel", ("ml", "po", "gate")),
+    ("attention_tile.cu", "attention_tile_kernel", ("q", "cache", "src")),
+    ("attention_tile.cu", "attention_tile_mma_kernel", ("q", "cache")),
+    ("attention_tile.cu", "attention_tile_few_kernel", ("q", "cache")),
+]
+
+
+@pytest.mark.parametrize("source,kernel,pointers", READ_PAST_L1, ids=lambda x: x if isinstance(x, str) else "")
+def test_what_a_kernel_ahead_wrote_is_read_past_the_first_level_cache(source, kernel, pointers):
+    """None of these pointers is promised to be read-only (which lets the compiler take the read-only path) and none is read
+    by a plain load: an element through a subscript, or a vector through a cast that is dereferenced."""
+    text = _kernel(source, kernel)
+    for name in pointers:
+        assert not re.search(r"\*\s*__restrict__\s+" + name + r"\b", text), name
+        assert not re.search(r"(?<![\w&])(?:p\.)?" + name + r"\[", text), name
+        assert not re.search(r"[^\w)\]]\s*\*\(const \w+\*\)\(?(?:p\.)?" + name + r"\b", text), name
+    with open(os.path.join(build.CSRC_DIR, source), encoding="utf-8") as f:
+        helpers = re.findall(r"(?:load4|load8|plain_dots|store_result)\([^;{]*\{.*?\n}?", f.read(), re.S)
+    assert not any(re.search(r"= \*\(const |\bresidual\[|\br[aw]\[", h) for h in helpers)

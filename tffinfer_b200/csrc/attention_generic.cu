@@ -50,9 +50,10 @@ __device__ __forceinline__ void join(float& m, float& l, float mc, float lc, flo
 }
 __device__ __forceinline__ float join_value(float o, float a, float oc, float b) { return __fmaf_rn(o, a, __fmul_rn(oc, b)); }
 
-__device__ __forceinline__ float4 load4(const float* p) { return *(const float4*)p; }
+// (what the kernels ahead wrote is read past the first-level cache)
+__device__ __forceinline__ float4 load4(const float* p) { return __ldcg((const float4*)p); }
 __device__ __forceinline__ float4 load4(const bf16* p) {
-    const uint2 u = *(const uint2*)p;
+    const uint2 u = __ldcg((const uint2*)p);
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
                        __uint_as_float(u.y & 0xffff0000u));
 }
@@ -60,7 +61,7 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 // RW rows a warp, ND groups of 128 value columns (4 a lane).
 template <typename T, int WARPS, int RW, int ND>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1)
-attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache, T* __restrict__ out, const GenericParams p) {
+attention_generic_kernel(const T* q_in, const T* cache, T* __restrict__ out, const GenericParams p) {
     extern __shared__ float4 smem4[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.nq / p.nkv, kvh = blockIdx.y, split = blockIdx.z % p.splits, b = blockIdx.z / p.splits;
@@ -91,10 +92,10 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
             if (p.q_vec) {
                 v = load4(src);
             } else {
-                v.x = to_f32<T>(src[0]);
-                if (c + 1 < p.d) v.y = to_f32<T>(src[1]);
-                if (c + 2 < p.d) v.z = to_f32<T>(src[2]);
-                if (c + 3 < p.d) v.w = to_f32<T>(src[3]);
+                v.x = ldcg_f32(src);
+                if (c + 1 < p.d) v.y = ldcg_f32(src + 1);
+                if (c + 2 < p.d) v.z = ldcg_f32(src + 2);
+                if (c + 3 < p.d) v.w = ldcg_f32(src + 3);
             }
         }
         sq[i] = v;
@@ -126,10 +127,11 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
                                          ::"r"((uint32_t)__cvta_generic_to_shared(dst + c)), "l"(src + c * 4) : "memory");
                         else dst[c] = load4(src + c * 4);
                     } else {
-                        float4 v = make_float4(to_f32<T>(src[c * 4]), 0.f, 0.f, 0.f);
-                        if (c * 4 + 1 < len) v.y = to_f32<T>(src[c * 4 + 1]);
-                        if (c * 4 + 2 < len) v.z = to_f32<T>(src[c * 4 + 2]);
-                        if (c * 4 + 3 < len) v.w = to_f32<T>(src[c * 4 + 3]);
+                        const T* at = src + c * 4;
+                        float4 v = make_float4(ldcg_f32(at), 0.f, 0.f, 0.f);
+                        if (c * 4 + 1 < len) v.y = ldcg_f32(at + 1);
+                        if (c * 4 + 2 < len) v.z = ldcg_f32(at + 2);
+                        if (c * 4 + 3 < len) v.w = ldcg_f32(at + 3);
                         dst[c] = v;
                     }
                 }
@@ -292,7 +294,7 @@ attention_generic_kernel(const T* __restrict__ q_in, const T* __restrict__ cache
         if (wrow + j >= rows) continue;
         const int h = kvh * G + (wrow + j) % G;
         const size_t t = q0 + (wrow + j) / G;
-        const float inv = (p.gate ? p.gate[t * p.nq + h] : 1.f) / l[j];
+        const float inv = (p.gate ? __ldcg(p.gate + t * p.nq + h) : 1.f) / l[j];
 #pragma unroll
         for (int c = 0; c < 4 * ND; ++c) {
             const int col = (lane + 32 * (c / 4)) * 4 + c % 4;
@@ -323,8 +325,8 @@ attention_generic_join_kernel(T* __restrict__ out, const int* __restrict__ tok_r
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 if (w0 + u >= count) continue;
-                x[u] = *(const float2*)(ml + 2 * (w0 + u));
-                v[u] = po[(size_t)(w0 + u) * p.dv];
+                x[u] = __ldcg((const float2*)(ml + 2 * (w0 + u)));
+                v[u] = __ldcg(po + (size_t)(w0 + u) * p.dv);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -334,7 +336,7 @@ attention_generic_join_kernel(T* __restrict__ out, const int* __restrict__ tok_r
                 o = join_value(o, a, v[u], bb);
             }
         }
-        out[(size_t)item * p.dv + col] = from_f32<T>(o * ((p.gate ? p.gate[item] : 1.f) / l));
+        out[(size_t)item * p.dv + col] = from_f32<T>(o * ((p.gate ? __ldcg(p.gate + item) : 1.f) / l));
     }
 }
 

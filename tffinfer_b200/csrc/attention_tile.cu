@@ -46,7 +46,7 @@ struct TileArgs {
 
 template <typename TQ, typename TC, int NC>
 __global__ void __launch_bounds__(THREADS)
-attention_tile_kernel(const TQ* __restrict__ q, const TC* __restrict__ cache, TQ* __restrict__ out, TileArgs a) {
+attention_tile_kernel(const TQ* q, const TC* cache, TQ* __restrict__ out, TileArgs a) {
     extern __shared__ float sm[];
     const int d = a.d, dv = a.dv, G = a.nq / a.nkv;
     const int kstride = d + 1;                                  // odd: lanes that read one column of 16 keys hit 16 banks
@@ -81,7 +81,7 @@ attention_tile_kernel(const TQ* __restrict__ q, const TC* __restrict__ cache, TQ
     for (int idx = tid; idx < ROWS * d; idx += THREADS) {
         const int rr = idx / d, i = idx % d, r = r0 + rr;
         float v = 0.f;
-        if (r < n_rows) v = to_f32<TQ>(q[(size_t)(t0 + r / G) * a.q_ld + (size_t)(kvh * G + r % G) * d + i]);
+        if (r < n_rows) v = ldcg_f32(q + (size_t)(t0 + r / G) * a.q_ld + (size_t)(kvh * G + r % G) * d + i);
         Qs[idx] = v;
     }
     __syncthreads();
@@ -124,9 +124,9 @@ attention_tile_kernel(const TQ* __restrict__ q, const TC* __restrict__ cache, TQ
                 if (page >= 0)
                     src = cache + (size_t)page * a.page_stride + (size_t)kvh * a.head_stride + (size_t)(n % a.page_size) * a.slot;
             }
-            for (int i = lane; i < d; i += 32) Ks[kk * kstride + i] = src ? to_f32<TC>(src[i]) : 0.f;
+            for (int i = lane; i < d; i += 32) Ks[kk * kstride + i] = src ? ldcg_f32(src + i) : 0.f;
             if (own_v)
-                for (int i = lane; i < dv; i += 32) Vs[kk * dv + i] = src ? to_f32<TC>(src[a.v_offset + i]) : 0.f;
+                for (int i = lane; i < dv; i += 32) Vs[kk * dv + i] = src ? ldcg_f32(src + a.v_offset + i) : 0.f;
         }
         __syncthreads();
         {
@@ -330,7 +330,7 @@ struct MmaGeom { int dpad, kst, vst; };      // padded key size, elements betwee
 // a warp of the value phase owns 16 rows x NT * 8 columns
 template <int NT, int RG>
 __global__ void __launch_bounds__(128 * RG)
-attention_tile_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, bf16* __restrict__ out, TileArgs a,
+attention_tile_mma_kernel(const bf16* q, const bf16* cache, bf16* __restrict__ out, TileArgs a,
                           MmaGeom gm) {
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int MROWS = 16 * RG, MTHREADS = 128 * RG;
@@ -373,7 +373,7 @@ attention_tile_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     for (int idx = tid; idx < MROWS * dch; idx += MTHREADS) {
         const int rr = idx / dch, c = (idx % dch) * 8, r = r0 + rr;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (r < n_rows && c < d) v = *(const uint4*)(q + (size_t)(t0 + r / G) * a.q_ld + (size_t)(kvh * G + r % G) * d + c);
+        if (r < n_rows && c < d) v = __ldcg((const uint4*)(q + (size_t)(t0 + r / G) * a.q_ld + (size_t)(kvh * G + r % G) * d + c));
         *(uint4*)(Qs + rr * kst + c) = v;
     }
     __syncthreads();
@@ -571,7 +571,7 @@ __device__ __forceinline__ void bulk_row(uint32_t dst, const void* src, uint32_t
 
 template <int NT>
 __global__ void __launch_bounds__(FTHREADS, 2)
-attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, bf16* __restrict__ out, TileArgs a,
+attention_tile_few_kernel(const bf16* q, const bf16* cache, bf16* __restrict__ out, TileArgs a,
                           MmaGeom gm, int* error_flag) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int d = a.d, dv = a.dv, G = a.nq / a.nkv;
@@ -678,7 +678,7 @@ attention_tile_few_kernel(const bf16* __restrict__ q, const bf16* __restrict__ c
     for (int idx = tid; idx < FROWS * dch; idx += FWARPS * 32) {
         const int rr = idx / dch, c = (idx % dch) * 8;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (rr < n_rows && c < d) v = *(const uint4*)(q + (size_t)(t0 + (r0 + rr) / G) * a.q_ld + (size_t)(kvh * G + (r0 + rr) % G) * d + c);
+        if (rr < n_rows && c < d) v = __ldcg((const uint4*)(q + (size_t)(t0 + (r0 + rr) / G) * a.q_ld + (size_t)(kvh * G + (r0 + rr) % G) * d + c));
         *(uint4*)(Qs + rr * kst + c) = v;
     }
     const int fr = lane >> 2, fc = 2 * (lane & 3);              // a thread's place in an accumulator tile: rows fr, fr+8; columns fc, fc+1

@@ -53,6 +53,13 @@ template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<bf16>(bf16 v) { return __bfloat162float(v); }
 
+// An element that a kernel ahead of this one wrote, read past the SM's first-level cache: under programmatic dependent launch
+// a block may have found an older line there before that kernel was through.
+__device__ __forceinline__ float ldcg_f32(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ float ldcg_f32(const bf16* p) {
+    return __uint_as_float((unsigned)__ldcg(reinterpret_cast<const unsigned short*>(p)) << 16);
+}
+
 template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }

@@ -70,40 +70,30 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// 8 consecutive elements of a row as float32; elements at or behind ``left`` are zeros (left counts from p).
-// CONST: the weights, which no kernel writes (the read-only path); the activations were written by the kernel ahead.
-template <typename T, bool VEC, bool CONST>
+// 8 consecutive elements of a row as float32; elements at or behind ``left`` are zeros (left counts from p).  Either operand may have
+// been written by the kernel ahead: both are read past the first-level cache.
+template <typename T, bool VEC>
 __device__ __forceinline__ void load8(const T* p, int left, uint32_t* r) {
     if constexpr (VEC) {                             // rows are multiples of 8 elements and aligned: all of the 8 or none
         if (left <= 0) {
 #pragma unroll
             for (int i = 0; i < (sizeof(T) == 4 ? 8 : 4); ++i) r[i] = 0u;
         } else if constexpr (sizeof(T) == 4) {
-            if constexpr (CONST)
-                asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                             : "l"(p));
-            else
-                asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                             : "l"(p) : "memory");
+            asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                         : "l"(p) : "memory");
         } else {
-            if constexpr (CONST)
-                asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p));
-            else
-                asm volatile("ld.global.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
+            asm volatile("ld.global.cg.v4.b32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
         }
-    } else if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = i < left ? __float_as_uint(to_f32<T>(p[i])) : 0u;
     } else {
+        auto one = [&](int i) { return i < left ? __float_as_uint(ldcg_f32(p + i)) : 0u; };
+        if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t lo = 2 * i < left ? (__float_as_uint(to_f32<T>(p[2 * i])) >> 16) : 0u;
-            const uint32_t hi = 2 * i + 1 < left ? (__float_as_uint(to_f32<T>(p[2 * i + 1])) & 0xffff0000u) : 0u;
-            r[i] = lo | hi;
+            for (int i = 0; i < 8; ++i) r[i] = one(i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] = (one(2 * i) >> 16) | one(2 * i + 1);
         }
     }
 }
@@ -148,7 +138,7 @@ __device__ __noinline__ float plain_dots(float v, bool mine, const TA* a, const 
         const TA* ra = (const TA*)__shfl_sync(0xffffffffu, (unsigned long long)a, src);
         const TW* rw = (const TW*)__shfl_sync(0xffffffffu, (unsigned long long)w, src);
         float s = 0.f;
-        for (int k = lane; k < K; k += 32) s = fmaf(to_f32<TA>(ra[k]), to_f32<TW>(rw[k]), s);
+        for (int k = lane; k < K; k += 32) s = fmaf(ldcg_f32(ra + k), ldcg_f32(rw + k), s);
         s = warp_sum(s);
         if (lane == src) v = s;
     }
@@ -162,7 +152,7 @@ __device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
     return __uint_as_float(r);
 }
 __device__ __forceinline__ void store_result(void* out, int out_bf16, const float* residual, size_t at, float v) {
-    if (residual) v = residual[at] + v;
+    if (residual) v = __ldcg(residual + at) + v;
     if (out_bf16) ((bf16*)out)[at] = from_f32<bf16>(v);
     else ((float*)out)[at] = v;
 }
@@ -183,7 +173,7 @@ struct Unit {
 
 template <int BN, typename TA, typename TW, bool VEC>
 __global__ void __launch_bounds__(F32Cfg<BN, sizeof(TA) == 4 ? 3 : 1, sizeof(TW) == 4 ? 3 : 1>::kThreads, 1)
-gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, int out_bf16, const float* residual,
+gemm_f32_kernel(const TA* A, const TW* W, void* out, int out_bf16, const float* residual,
                 float* __restrict__ ws, int M, int N, int K, const Share sh, int* error_flag) {
     constexpr int NA = sizeof(TA) == 4 ? 3 : 1, NW = sizeof(TW) == 4 ? 3 : 1;
     using Cfg = F32Cfg<BN, NA, NW>;
@@ -284,8 +274,8 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
             a_rows = min(M - it.m0, BN) - row;
         };
         const size_t pitch = (size_t)STRIDE * K;
-        auto load_w = [&](int q) { load8<TW, VEC, true>(wp + q * pitch, STRIDE * q < w_rows ? left : 0, wr[q]); };
-        auto load_a = [&](int q) { load8<TA, VEC, false>(ap + q * pitch, STRIDE * q < a_rows ? left : 0, ar[q]); };
+        auto load_w = [&](int q) { load8<TW, VEC>(wp + q * pitch, STRIDE * q < w_rows ? left : 0, wr[q]); };
+        auto load_a = [&](int q) { load8<TA, VEC>(ap + q * pitch, STRIDE * q < a_rows ? left : 0, ar[q]); };
         auto has_a = [&](int q) { return (q + 1) * STRIDE <= BN || row + q * STRIDE < BN; };
         auto step = [&]() {                                                  // to the next K block of the CTA
             if (++kb >= it.kb1) {
@@ -427,7 +417,7 @@ gemm_f32_kernel(const TA* __restrict__ A, const TW* __restrict__ W, void* out, i
 // out = sum of the chunks' partial results, in ascending order (+ residual).
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(256)
-gemm_f32_sum_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const float* __restrict__ ws, void* out, int out_bf16,
+gemm_f32_sum_kernel(const TA* A, const TW* W, const float* ws, void* out, int out_bf16,
                     const float* residual, int M, int N, int K, int chunks) {
     pdl_launch_dependents();
     pdl_wait();
@@ -441,10 +431,10 @@ gemm_f32_sum_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const fl
             const float* p = ws + (size_t)s * total + i;
             float t[4] = {0.f, 0.f, 0.f, 0.f};
             if (vec) {
-                const float4 f = *(const float4*)p;
+                const float4 f = __ldcg((const float4*)p);
                 t[0] = f.x; t[1] = f.y; t[2] = f.z; t[3] = f.w;
             } else {
-                for (int j = 0; j < cnt; ++j) t[j] = p[j];
+                for (int j = 0; j < cnt; ++j) t[j] = __ldcg(p + j);
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = s == 0 ? t[j] : v[j] + t[j];
