@@ -105,7 +105,7 @@ def _kernel(source, name):
     """The text of a kernel, from its name to the brace that closes it at the line's start."""
     with open(os.path.join(build.CSRC_DIR, source), encoding="utf-8") as f:
         text = re.sub(r"//[^\n]*", "", f.read())
-    return re.search(r"\n" + name + r"\(.*?\n}\n", text, re.S).group(0)
+    return re.search(r"\b" + name + r"\(.*?\n}\n", text, re.S).group(0)
 
 
 def test_sums_of_few_row_attention_leave_what_the_last_block_reads_alone():
@@ -126,6 +126,9 @@ READ_PAST_L1 = [
     ("gemm_f32.cu", "gemm_f32_sum_kernel", ("A", "W", "ws", "residual", "p")),
     ("attention_generic.cu", "attention_generic_kernel", ("q_in", "cache", "gate", "src")),
     ("attention_generic.cu", "attention_generic_join_kernel", ("ml", "po", "gate")),
+    ("attention_decode.cu", "attn_decode_kernel", ("q", "gate")),
+    ("attention_prefill.cu", "attn_prefill_tc_kernel", ("gate",)),
+    ("attention_bf16.cu", "attn_combine_kernel", ("gate",)),
     ("attention_tile.cu", "attention_tile_kernel", ("q", "cache", "src")),
     ("attention_tile.cu", "attention_tile_mma_kernel", ("q", "cache")),
     ("attention_tile.cu", "attention_tile_few_kernel", ("q", "cache")),

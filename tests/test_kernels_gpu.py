@@ -555,7 +555,7 @@ def test_flash_attention_bf16(ops, case):
 ])
 @pytest.mark.parametrize("captured", [False, True])
 def test_portions_and_decoded_tokens_in_one_call_equal_two_launches(ops, captured, nq, nkv, d, page, new, old, window, splits, extra):
-    """The two kernels overlap: each call's queries are written by the kernel right ahead of it, and its output read by the
+    """The two kernels overlap: each call's queries (and gates) are written by the kernels right ahead of it, and its output read by the
     one right behind it, several calls in a row.  Every bit equals that of the launches one after the other."""
     entries, tables, cache, qkv = _paged_case(nq, nkv, d, page, new, old, window, torch.bfloat16, seed=77)
     T, B = sum(new), len(new)
@@ -563,9 +563,10 @@ def test_portions_and_decoded_tokens_in_one_call_equal_two_launches(ops, capture
     short = sum(n * (nq // nkv) <= 16 for n in new)
     q_short, q_long = int(b.h_sorted_q_lens[short - 1]), int(b.h_sorted_q_lens[-1])
     assert 0 < short < B and q_short * (nq // nkv) <= 16 < int(b.h_sorted_q_lens[short]) * (nq // nkv)
-    more = (0.0, False, None, 0)
+    more, gates = (0.0, False, None, 0), None
     if extra:
-        more = (20.0, g((nq,), torch.float32, 78).to(DEV), torch.rand(T, nq, device=DEV), 5 if window else 0)
+        gates = [torch.rand(T, nq, device=DEV) for _ in range(6)]
+        more = (20.0, g((nq,), torch.float32, 78).to(DEV), torch.zeros(T, nq, device=DEV), 5 if window else 0)
     cache = cache.to(DEV)
     qs = [g((T, nq * d), torch.bfloat16, 80 + i).to(DEV) for i in range(6)]
     q = torch.zeros_like(qs[0])
@@ -576,7 +577,9 @@ def test_portions_and_decoded_tokens_in_one_call_equal_two_launches(ops, capture
     taken = []
 
     def calls():
-        for x, r in zip(qs, got):
+        for i, (x, r) in enumerate(zip(qs, got)):
+            if gates:
+                more[2].copy_(gates[i])
             q.copy_(x)
             taken.append(ops._attention_bf16_mixed(q, *head, out, *tail, splits, short, B, q_short, q_long, more))
             r.copy_(out)
@@ -589,9 +592,11 @@ def test_portions_and_decoded_tokens_in_one_call_equal_two_launches(ops, capture
         calls()
     torch.cuda.synchronize()
     assert taken == [page >= 8] * len(qs)
-    for x, r in zip(qs, got):
+    for i, (x, r) in enumerate(zip(qs, got)):
         if not taken[0]:
             continue
+        if gates:
+            more[2].copy_(gates[i])
         want = torch.full_like(r, float("nan"))
         ops._attention_bf16_launch(x, *head, want, *tail, 1, b.req_order[short:], B - short, q_long, more)
         torch.cuda.synchronize()

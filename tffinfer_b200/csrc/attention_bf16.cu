@@ -286,7 +286,7 @@ attn_fwd_kernel(const AttnParams p) {
             const size_t grow = (size_t)(q0 + R / G) * p.nq + (kvh * G + R % G);
             if (p.num_splits == 1) {
                 if (p.sink) lsum += exp2f(attn_sink_log2(p.sink_val, kvh * G + R % G) - Ms);   // the sink: a key without a value
-                const float gt = p.gate ? p.gate[grow] : 1.f;
+                const float gt = p.gate ? __ldcg(p.gate + grow) : 1.f;
                 p.out[grow * D + c] = __float2bfloat16_rn(acc * gt / lsum);
             } else {
                 p.part_o[(grow * p.num_splits + split) * D + c] = acc;
@@ -304,7 +304,7 @@ attn_fwd_kernel(const AttnParams p) {
                 l0 += exp2f(attn_sink_log2(p.sink_val, kvh * G + R0 % G) - (m0 == -INFINITY ? 0.f : m0));
                 l1 += exp2f(attn_sink_log2(p.sink_val, kvh * G + R1 % G) - (m1 == -INFINITY ? 0.f : m1));
             }
-            const float i0 = ((p.gate && v0) ? p.gate[g0] : 1.f) / l0, i1 = ((p.gate && v1) ? p.gate[g1] : 1.f) / l1;
+            const float i0 = ((p.gate && v0) ? __ldcg(p.gate + g0) : 1.f) / l0, i1 = ((p.gate && v1) ? __ldcg(p.gate + g1) : 1.f) / l1;
 #pragma unroll
             for (int i = 0; i < D / 8; ++i) {
                 const int c = i * 8 + 2 * (lane & 3);
@@ -363,7 +363,7 @@ __device__ __forceinline__ void combine_row(const float* __restrict__ part_o, co
 template <int D>
 __global__ void attn_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                     bf16* __restrict__ out, int num_splits, const int* __restrict__ q_start,
-                                    const int* __restrict__ req_ids, int nq, int sink, const float* __restrict__ gate,
+                                    const int* __restrict__ req_ids, int nq, int sink, const float* gate,
                                     const float* __restrict__ sink_val) {
     pdl_launch_dependents();          // the next kernel may become resident (it waits before it reads or writes)
     // the step's batch arrays are older than the kernel ahead: they are read before waiting for it
@@ -374,7 +374,7 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o, const floa
     pdl_wait();
     if (t >= q_len) return;
     const size_t row = (size_t)(q0 + t) * nq + h;
-    const float gt = gate ? gate[row] : 1.f;
+    const float gt = gate ? __ldcg(gate + row) : 1.f;
     const float sink_log2 = attn_sink_log2(sink_val, h);
     if (num_splits <= 4) { combine_row<D, 4>(part_o, part_ml, out, num_splits, row, sink, sink_log2, gt); return; }
     if (num_splits <= 8) { combine_row<D, 8>(part_o, part_ml, out, num_splits, row, sink, sink_log2, gt); return; }

@@ -143,7 +143,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
         const int j = lane;
         const uint32_t box_bytes = (uint32_t)(2 * D * 2) << p.page_shift;      // K and V of one page
         const int first_new_blk = pos0 / BLOCK_N;                  // key blocks from here on hold slots written just now
-        bool waited = p.beside != 0;
+        bool waited = p.beside != 0;                               // (see the compute warps' wait)
         for (int w = w_begin; w < w_end; ++w) {
             const int blk = walk.block(w), i = w - w_begin, s = i % NSTAGES;
             const uint32_t round = i / NSTAGES;
@@ -171,6 +171,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
     }
 
     // ---------------------------------------------------------------- compute warps
+    // Beside a portion's kernel there is nothing to wait for here: that kernel lets this one start only after its own wait for
+    // the kernel ahead of both (PrefillParams::companion), which is therefore through.  What it wrote (queries, gates, the
+    // step's cache rows) is read past the first-level cache, since this kernel has not itself waited for it.
     if (!p.beside) pdl_wait();
     // the query tile: packed rows (token, head of the group), chunks XOR-swizzled by row % 8
     for (int idx = tid; idx < 16 * CH; idx += 128) {
@@ -327,7 +330,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
         const size_t grow = (size_t)(q0 + r / G) * p.nq + (kvh * G + r % G);
         if (p.num_splits == 1) {
             if (p.sink) lsum += exp2f(attn_sink_log2(p.sink_val, kvh * G + r % G) - Ms);   // the sink: a key without a value
-            const float gt = p.gate ? p.gate[grow] : 1.f;
+            const float gt = p.gate ? __ldcg(p.gate + grow) : 1.f;
             p.out[grow * D + c] = __float2bfloat16_rn(acc * gt / lsum);
         } else {
             p.part_o[(grow * p.num_splits + split) * D + c] = acc;

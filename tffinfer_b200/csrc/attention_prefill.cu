@@ -616,7 +616,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             tc_fence_after();
             if (p.sink && l > 0.f) l += exp2f(attn_sink_log2(p.sink_val, kvh * G + R % G) - m_used);   // the sink: a key without a value
             float inv = l > 0.f ? 1.f / l : 0.f;
-            if (p.gate && rv) inv *= p.gate[(size_t)(q0 + R / G) * p.nq + (kvh * G + R % G)];
+            if (p.gate && rv) inv *= __ldcg(p.gate + (size_t)(q0 + R / G) * p.nq + (kvh * G + R % G));
             const int dv = DENSE ? p.dv : DV;
             bf16* orow = p.out + ((size_t)(q0 + R / G) * p.nq + (kvh * G + R % G)) * dv;
 #pragma unroll 1
