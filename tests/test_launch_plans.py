@@ -110,3 +110,27 @@ def test_small_portions_behind_long_contexts_take_key_shares():
     assert ps(4, 16, 4016, 32, 8) == 8           # several such portions in a step share the SMs (32 CTAs a share)
     assert CudaKernels.portion_splits(SimpleNamespace(NUM_SMS=74), 1, 64, 4064, 32, 8) == 4
 
+
+
+def test_few_row_attention_plans_a_captured_step_for_every_context_of_its_tables():
+    """A graph taken behind short contexts is the one taken behind long ones, and cuts neither badly; plans are kept."""
+    from types import SimpleNamespace
+    p = CudaKernels.__new__(CudaKernels)
+    p.NUM_SMS = 148
+    step = lambda n, kv, graph: SimpleNamespace(num_requests=n, max_kv_len=kv, graph_bucket=n if graph else None)
+    cost = lambda n, s, blocks: -(-n * s // 296) * (-(-blocks // s) + 4)
+    for n in (1, 2, 8, 16, 32, 64, 96, 256):
+        for table in (640, 4096, 40960):
+            plans = {p.few_row_splits(step(n, kv, True), 1, table) for kv in (1, 100, 600, 4000)}
+            assert len(plans) == 1
+            s, = plans
+            for kv in (table, table // 4, table // 16):
+                own = p.few_row_splits(step(n, kv, False), 1, table)      # the best at this context
+                assert 1 <= own <= 32 and cost(n, s, -(-kv // 32)) <= 1.75 * cost(n, own, -(-kv // 32)), (n, table, kv, s, own)
+    # kernel by kernel a step is planned from its own contexts, never in more shares than there are blocks of 32 keys
+    assert p.few_row_splits(step(32, 4000, False), 1, 40960) == 9 and p.few_row_splits(step(1, 65, False), 1, 40960) == 3
+    assert p.few_row_splits(step(1, 4000, True), 1, 40960, window=64) == 2
+    before = CudaKernels._few_row_splits.cache_info()
+    p.few_row_splits(step(32, 4000, False), 1, 40960)
+    after = CudaKernels._few_row_splits.cache_info()
+    assert (after.hits, after.misses) == (before.hits + 1, before.misses)

@@ -811,16 +811,19 @@ attention_tile_few_kernel(const bf16* q, const bf16* cache, bf16* __restrict__ o
         const float inv = a.splits == 1 ? a.out_scale / l_fin[r] : 1.f;
         bf16* orow = out + (size_t)t * a.out_ld + a.out_off + (size_t)h * dv;
         float* prow = a.part_o + slot * dv;
+        // (a share without a visible key has no weight in the merge, which does not read its sums then)
+        if (a.splits == 1 || m_fin[r] != -INFINITY) {
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
+            for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = warp * NT * 8 + j * 8 + fc + e;
-                if (c < dv) {
-                    if (a.splits == 1) orow[c] = __float2bfloat16_rn(o[j][side * 2 + e] * inv);
-                    else prow[c] = o[j][side * 2 + e];
+                for (int e = 0; e < 2; ++e) {
+                    const int c = warp * NT * 8 + j * 8 + fc + e;
+                    if (c < dv) {
+                        if (a.splits == 1) orow[c] = __float2bfloat16_rn(o[j][side * 2 + e] * inv);
+                        else prow[c] = o[j][side * 2 + e];
+                    }
                 }
-            }
+        }
         if (a.splits > 1 && warp == 0 && fc == 0) { a.part_ml[2 * slot] = m_fin[r]; a.part_ml[2 * slot + 1] = l_fin[r]; }
     }
 }

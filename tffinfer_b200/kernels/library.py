@@ -1012,7 +1012,8 @@ class CudaKernels:
         if num_splits is not None:
             splits = int(num_splits)
         elif q.dtype == torch.bfloat16 and batch.max_q_len * (nq // nkv) <= 32 and d % 8 == 0 and dv <= 512:
-            splits = self.few_row_splits(batch, -(-batch.max_q_len * (nq // nkv) // 16) * nkv, window, chunk)
+            splits = self.few_row_splits(batch, -(-batch.max_q_len * (nq // nkv) // 16) * nkv, block_table.shape[1] * page_size,
+                                         window, chunk)
         else:
             splits = self.tile_splits(batch, nq, nkv, window, chunk)
         part_o = part_ml = None
@@ -1048,14 +1049,26 @@ class CudaKernels:
             _c_float(scale), _c_int(window), _c_float(softcap), _ptr(sink), self._stream()), "attention_dense")
         self.launches += 1
 
-    def few_row_splits(self, batch, tiles: int, window: int = 0, chunk: int = 0) -> int:
+    def few_row_splits(self, batch, tiles: int, table_keys: int, window: int = 0, chunk: int = 0) -> int:
         """In how many shares attention_tile cuts the keys of steps of few rows (at most 32), ``tiles`` tiles of 16 rows a request:
         the count whose rounds of CTAs, two an SM, take the least time, a CTA's time being its blocks of 32 keys and about four
-        more to start and finish."""
-        items = tiles * batch.num_requests
-        blocks = -(-min([s for s in (window, chunk) if s > 0] + [int(batch.max_kv_len)]) // 32)
-        cost = lambda s: -(-items * s // (2 * self.NUM_SMS)) * (-(-blocks // s) + 4)
-        return min(range(1, min(32, max(1, blocks)) + 1), key=lambda s: (cost(s), s))
+        more to start and finish.  A step replayed as a graph is captured once for all contexts that its block tables hold
+        (``table_keys``), whatever they are when it is captured: the count whose time is at worst the least above the best
+        count's, over contexts of all of that, a quarter, a sixteenth and so on."""
+        graph = getattr(batch, "graph_bucket", None) is not None
+        span = min([s for s in (window, chunk) if s > 0] + [int(table_keys if graph else batch.max_kv_len)])
+        return self._few_row_splits(2 * self.NUM_SMS, tiles * batch.num_requests, max(1, -(-span // 32)), graph)
+
+    @staticmethod
+    @functools.lru_cache(maxsize=4096)
+    def _few_row_splits(ctas: int, items: int, blocks: int, graph: bool) -> int:
+        counts = range(1, min(32, blocks) + 1)
+        cost = lambda s, n: -(-items * s // ctas) * (-(-n // s) + 4)
+        contexts = [blocks]
+        while graph and contexts[-1] > 3:
+            contexts.append(contexts[-1] // 4)
+        best = [min(cost(s, n) for s in counts) for n in contexts]
+        return min(counts, key=lambda s: (max(cost(s, n) / b for n, b in zip(contexts, best)), s))
 
     def tile_splits(self, batch, nq: int, nkv: int, window: int = 0, chunk: int = 0) -> int:
         """In how many shares attention_tile cuts every tile's key range: a power of two such that a step of few rows
