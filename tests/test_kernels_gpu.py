@@ -632,12 +632,13 @@ def test_float32_attention_does_not_depend_on_how_the_keys_are_shared_out(ops, d
     # room for every chunk of the longest context, as the library plans it for a device of very many SMs
     slots = ops.lib.tff_attention_generic_plan(len(new), max(new), max(new) + max(old), nq, nkv, d, 0, 0, 1 << 20) >> 16
     assert slots > 1
-    for shares in (1, 2, 5):
+    for shares, room in ((1, 0), (2, slots), (5, slots), (2, 2), (5, 3)):    # (room for fewer than all: the first share takes more)
         out = torch.full((T, nq * d), float("nan"), dtype=dt, device=DEV)
         ops._attention_generic_launch(q.to(DEV), bg, *args, out, nq, nkv, d, d, 1 / math.sqrt(d), window, keep=keep,
-                                      plan=shares | ((slots << 16) if shares > 1 else 0))
+                                      plan=shares | (room << 16))
         outs.append(out)
-    assert torch.equal(outs[0].nan_to_num(7.0), outs[1].nan_to_num(7.0)) and torch.equal(outs[0].nan_to_num(7.0), outs[2].nan_to_num(7.0))
+    for out in outs[1:]:
+        assert torch.equal(outs[0].nan_to_num(7.0), out.nan_to_num(7.0))
     rows = T if n == 1 else T - 1
     want = torch.empty(T, nq * d, dtype=dt)
     if keep == 0:

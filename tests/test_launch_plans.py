@@ -1,5 +1,11 @@
 """Launch decisions taken on the host: how the tensor-core product cuts the tiles of a last, partial wave,
 and how the decode attention shares out the key range."""
+import ctypes
+import os
+
+import pytest
+
+from tffinfer_b200.csrc import build
 from tffinfer_b200.kernels.library import CudaKernels
 
 
@@ -134,3 +140,20 @@ def test_few_row_attention_plans_a_captured_step_for_every_context_of_its_tables
     p.few_row_splits(step(32, 4000, False), 1, 40960)
     after = CudaKernels._few_row_splits.cache_info()
     assert (after.hits, after.misses) == (before.hits + 1, before.misses)
+
+
+def test_partial_results_of_the_float32_attention_have_a_bound():
+    """A step captured for long block tables plans for all of them; what it takes beside the cache stays below 64 MB, and
+    shares that fit are not given up for it."""
+    path = os.path.join(build.CSRC_DIR, "_build", build.LIB_NAME)
+    if not os.path.exists(path):
+        pytest.skip("the kernel library has not been built here")
+    plan = ctypes.CDLL(path).tff_attention_generic_plan
+    for requests in (1, 2, 8, 16, 32, 64):
+        for nq, nkv, dv in ((32, 8, 128), (16, 8, 128), (64, 8, 64), (8, 1, 256), (2, 2, 512)):
+            for keys in (40, 600, 4096, 40960, 1 << 20):
+                both = plan(requests, 1, keys, nq, nkv, dv, 0, 0, 148)
+                shares, slots = both & 0xffff, both >> 16
+                assert requests * nq * slots * (dv + 2) * 4 <= 64 << 20
+                assert shares == max(1, min(296 // (requests * nkv), -(-keys // 64))), (requests, nq, nkv, dv, keys)
+    assert plan(16, 1, 40960, 32, 8, 128, 0, 0, 148) >> 16 == (64 << 20) // (16 * 32 * 130 * 4)

@@ -15,9 +15,9 @@
 // blocks of 32, which come to shared memory once for all its rows; a warp has up to 4 rows: for the scores a lane is
 // a key, for the values a lane has 4 (8, 16) columns.  The running-maximum ("online") softmax of the reference
 // (paged_flash_attention.cu:696-792) starts afresh every CHUNK keys, at absolute positions, and the chunks' results are
-// joined in ascending order: a step of few rows behind long contexts shares the chunks out to several CTAs and joins them in
-// a second kernel, with the same operations in the same order.  A token's result so depends neither on how the batch
-// was cut nor on what else is in it.
+// joined in ascending order: a step of few rows behind long contexts shares the chunks out to several CTAs, of which the first
+// joins its own as it goes and the others leave theirs to a second kernel, with the same operations in the same order.  A token's
+// result so depends neither on how the batch was cut nor on what else is in it.
 //
 // What bounds it: the latency of its chains of shared-memory loads and FMAs (with 8 rows a warp and 8 warps an SM an instruction was
 // issued in a third of the cycles), then those loads; for one token behind a context the chain of its chunk's blocks.  A warp a
@@ -58,6 +58,17 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
                        __uint_as_float(u.y & 0xffff0000u));
 }
 
+// Which of a request's ``count`` chunks a share takes: the first share the first ``first`` of them, whose joined result is partial
+// result 0, the others ``per`` each, every chunk a partial result of its own.  Where there is room for fewer than an even cut takes,
+// the first share takes what is left.
+struct Shares {
+    int first, per;
+    __device__ Shares(int count, int splits, int slots) {
+        first = splits > 1 ? max((count + splits - 1) / splits, count - (slots - 1)) : count;
+        per = splits > 1 ? (count - first + splits - 2) / (splits - 1) : 0;
+    }
+};
+
 // RW rows a warp, ND groups of 128 value columns (4 a lane).
 template <typename T, int WARPS, int RW, int ND>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1)
@@ -80,7 +91,8 @@ attention_generic_kernel(const T* q_in, const T* cache, T* __restrict__ out, con
     const int first_pos = pos0 + row0 / G, hi = pos0 + (min(row0 + WARPS * RW, rows) - 1) / G;
     const int lo_tile = p.window > 0 ? max(0, first_pos - p.window + 1) : 0;
     const KeyWalk walk(p.keep, CHUNK, lo_tile / CHUNK, hi / CHUNK);
-    const int per = (walk.count + p.splits - 1) / p.splits, w0 = split * per, w1 = min(walk.count, w0 + per);
+    const Shares sh(walk.count, p.splits, p.slots);
+    const int w0 = split > 0 ? sh.first + (split - 1) * sh.per : 0, w1 = split > 0 ? min(walk.count, w0 + sh.per) : sh.first;
     if (w0 >= w1) return;
 
 #pragma unroll 4
@@ -160,6 +172,16 @@ attention_generic_kernel(const T* q_in, const T* cache, T* __restrict__ out, con
 #pragma unroll
         for (int c = 0; c < 4 * ND; ++c) { o[j][c] = 0.f; oc[j][c] = 0.f; }
     }
+
+    auto partial = [&](int j, int slot, float mx, float sum, const float (&v)[4 * ND]) {
+        const size_t at = ((size_t)(q0 + (wrow + j) / G) * p.nq + kvh * G + (wrow + j) % G) * p.slots + slot;
+        if (lane == 0) { p.part_ml[2 * at] = mx; p.part_ml[2 * at + 1] = sum; }
+#pragma unroll
+        for (int c = 0; c < 4 * ND; ++c) {
+            const int col = (lane + 32 * (c / 4)) * 4 + c % 4;
+            if (col < p.dv) p.part_o[at * p.dv + col] = v[c];
+        }
+    };
 
     const int total = (w1 - w0) * PER_CHUNK;
     auto block_start = [&](int i) { return walk.block(w0 + i / PER_CHUNK) * CHUNK + (i % PER_CHUNK) * BLOCK; };
@@ -262,19 +284,11 @@ attention_generic_kernel(const T* q_in, const T* cache, T* __restrict__ out, con
             __syncwarp();
         }
         if (i % PER_CHUNK == PER_CHUNK - 1) {                 // the chunk's end
-            const int slot = w0 + i / PER_CHUNK;
+            const int slot = w0 + i / PER_CHUNK - sh.first + 1;
 #pragma unroll
             for (int j = 0; j < RW; ++j) {
-                if (p.splits > 1) {
-                    if (wrow + j < rows && slot < p.slots) {
-                        const size_t at = ((size_t)(q0 + (wrow + j) / G) * p.nq + kvh * G + (wrow + j) % G) * p.slots + slot;
-                        if (lane == 0) { p.part_ml[2 * at] = mc[j]; p.part_ml[2 * at + 1] = lc[j]; }
-#pragma unroll
-                        for (int c = 0; c < 4 * ND; ++c) {
-                            const int col = (lane + 32 * (c / 4)) * 4 + c % 4;
-                            if (col < p.dv) p.part_o[at * p.dv + col] = oc[j][c];
-                        }
-                    }
+                if (split > 0) {
+                    if (wrow + j < rows) partial(j, slot, mc[j], lc[j], oc[j]);
                 } else {
                     float a, bb;
                     join(m[j], l[j], mc[j], lc[j], a, bb);
@@ -288,10 +302,11 @@ attention_generic_kernel(const T* q_in, const T* cache, T* __restrict__ out, con
         }
         __syncthreads();
     }
-    if (p.splits > 1) return;
+    if (split > 0) return;
 #pragma unroll
     for (int j = 0; j < RW; ++j) {
         if (wrow + j >= rows) continue;
+        if (p.splits > 1) { partial(j, 0, m[j], l[j], o[j]); continue; }
         const int h = kvh * G + (wrow + j) % G;
         const size_t t = q0 + (wrow + j) / G;
         const float inv = (p.gate ? __ldcg(p.gate + t * p.nq + h) : 1.f) / l[j];
@@ -303,7 +318,7 @@ attention_generic_kernel(const T* q_in, const T* cache, T* __restrict__ out, con
     }
 }
 
-// Joins the chunks' results in ascending order: a block per (token, head), a thread a column (of every JOIN_THREADS), eight chunks' loads
+// Joins the chunks of the other shares to the first share's result, in ascending order: a block per (token, head), a thread a column (of every JOIN_THREADS), eight chunks' loads
 // on their way together.  The rows of a request are one tile.
 template <typename T>
 __global__ void __launch_bounds__(JOIN_THREADS)
@@ -314,12 +329,12 @@ attention_generic_join_kernel(T* __restrict__ out, const int* __restrict__ tok_r
     const int pos0 = p.pos_start[b], q_len = p.q_start[b + 1] - p.q_start[b];
     const int lo_tile = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
     const KeyWalk walk(p.keep, CHUNK, lo_tile / CHUNK, (pos0 + q_len - 1) / CHUNK);
-    const int count = min(walk.count, p.slots);
+    const int count = walk.count - Shares(walk.count, p.splits, p.slots).first + 1;
     const float* ml = p.part_ml + (size_t)item * p.slots * 2;
     for (int col = threadIdx.x; col < p.dv; col += JOIN_THREADS) {
         const float* po = p.part_o + (size_t)item * p.slots * p.dv + col;
-        float m = p.sink ? (p.sink_val ? p.sink_val[h] : 0.f) : -INFINITY, l = p.sink ? 1.f : 0.f, o = 0.f;
-        for (int w0 = 0; w0 < count; w0 += 8) {
+        float m = __ldcg(ml), l = __ldcg(ml + 1), o = __ldcg(po);
+        for (int w0 = 1; w0 < count; w0 += 8) {
             float2 x[8];
             float v[8];
 #pragma unroll
@@ -383,23 +398,31 @@ int tile_rows(int dv) { return dv <= 128 ? 32 : dv <= 256 ? 16 : 8; }
 
 }  // namespace
 
-// In how many shares (low 16 bits) the chunks of a step's keys go to different CTAs, and for how many chunks there must be
-// room for a partial result of dv + 2 floats per (token, head) (above).  One share and no room for steps of long
+// What the partial results of a step may take at most.  A step captured for block tables of 40,960 tokens would want 85 MB for 16 requests of 32
+// heads of 128, of a memory that the cache's budget leaves to graphs and activations; the first share then takes 389 of the 640 chunks.
+constexpr long long MOST_PARTIALS = 64ll << 20;
+
+// In how many shares (low 16 bits) the chunks of a step's keys go to different CTAs, and for how many partial results of dv + 2
+// floats per (token, head) there must be room (above).  One share and no room for steps of long
 // portions and for steps with enough requests: two CTAs an SM.  ``max_kv`` bounds the contexts.
 TFF_API int tff_attention_generic_plan(int num_requests, int max_q_len, int max_kv, int nq, int nkv, int dv, int window, int keep,
                                        int sms) {
     if (num_requests <= 0 || max_q_len <= 0 || max_kv <= 0 || nkv <= 0 || nq % nkv || sms <= 0) return 1;
     if ((long long)max_q_len * (nq / nkv) > tile_rows(dv)) return 1;
-    long long slots = (max_kv + CHUNK - 1) / CHUNK;
+    long long chunks = (max_kv + CHUNK - 1) / CHUNK;
     if (window > 0) {
         const long long seen = ((long long)window + max_q_len + CHUNK - 1) / CHUNK + 1 + (keep > 0 ? (keep + CHUNK - 1) / CHUNK : 0);
-        slots = slots < seen ? slots : seen;
+        chunks = chunks < seen ? chunks : seen;
     }
     const long long ctas = (long long)num_requests * nkv;
     long long splits = 2ll * sms / ctas;
-    if (splits > slots) splits = slots;
-    if (splits < 2 || slots > 32767 || num_requests * splits > 65535) return 1;
-    return (int)(splits | (slots << 16));
+    if (splits > chunks) splits = chunks;
+    if (splits < 2 || num_requests * splits > 65535) return 1;
+    long long slots = chunks - (chunks + splits - 1) / splits + 1;
+    const long long most = MOST_PARTIALS / ((long long)num_requests * max_q_len * nq * (dv + 2) * 4);
+    if (slots > most) slots = most;
+    if (slots > 32767) slots = 32767;
+    return slots < 2 ? 1 : (int)(splits | (slots << 16));
 }
 
 // Keys of d and values of dv elements in cache slots of dc, score cap, sink, head gates.  ``plan`` as
