@@ -655,6 +655,28 @@ def test_float32_attention_does_not_depend_on_how_the_keys_are_shared_out(ops, d
         assert torch.equal(one[0], outs[0][r])
 
 
+@pytest.mark.parametrize("shares", [1, 3])
+def test_float32_attention_of_scores_of_minus_infinity(ops, shares):
+    """Whole chunks of visible keys whose scores are -infinity (keys with an infinite element) count for nothing, wherever they
+    lie: first, between others, last; a row that sees no other key has no result."""
+    nq, nkv, d, page, keys = 4, 2, 8, 16, 400
+    entries, tables, cache, qkv = _paged_case(nq, nkv, d, page, [1, 1], [keys - 1, 63], 0, torch.float32, seed=76, layers=1)
+    q = qkv[:, :nq * d].abs() + 0.1
+    cache = cache.clone()
+    gone = list(range(70)) + list(range(128, 192)) + list(range(330, 400))
+    for b, ts in ((0, gone), (1, range(64))):
+        for t in ts:
+            cache[tables[b][t // page], 0, 0, :, t % page, 3] = -math.inf
+    batch = build_step_batch(entries, [keys - 1, 63], [0, 1], [tables], DEV)
+    out = torch.empty(2, nq * d, device=DEV)
+    ops._attention_generic_launch(q.to(DEV).contiguous(), batch, batch.block_tables[0], cache.to(DEV), 0, page, out, nq, nkv, d, d, d ** -0.5, 0,
+                                  plan=shares | (7 << 16))
+    kv = torch.stack([cache[tables[0][t // page], 0, :, :, t % page] for t in range(keys)]).double()          # [keys, 2, nkv, d]
+    want = torch.cat([torch.softmax(kv[:, 0, h // 2] @ q[0, h * d:(h + 1) * d].double() * d ** -0.5, 0) @ kv[:, 1, h // 2] for h in range(nq)])
+    assert torch.isfinite(want).all() and rel_err(out[0], want) < 3e-6
+    assert out[1].isnan().all()
+
+
 @pytest.mark.parametrize("nq,nkv,d,page,new,old", [(32, 8, 128, 16, [700], [300]), (8, 2, 64, 32, [333, 40], [0, 1000]),
                                                    (8, 8, 128, 8, [129, 2], [65, 3]),
                                                    # CTAs of two tiles whose tiles take turns at the exponentials: an odd

@@ -235,7 +235,8 @@ attention_generic_kernel(const T* q_in, const T* cache, T* __restrict__ out, con
                 s = valid ? s : -INFINITY;
                 const float mn = fmaxf(mc[j], warp_max(s));
                 const float alpha = mc[j] == -INFINITY ? (mn == -INFINITY ? 1.f : 0.f) : expf(mc[j] - mn);
-                const float pr = valid ? expf(s - mn) : 0.f;
+                // (a score of -infinity has no weight, also in a chunk where no other key is visible)
+                const float pr = valid && s != -INFINITY ? expf(s - mn) : 0.f;
                 lc[j] = lc[j] * alpha + warp_sum(pr);
                 mc[j] = mn;
                 if (alpha != 1.f) {
