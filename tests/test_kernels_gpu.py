@@ -3,6 +3,7 @@ engine's: odd widths, vocabularies that are no power of two, head sizes in steps
 any number of heads and groups, single rows, page edges."""
 import math
 import random
+from types import SimpleNamespace
 
 import numpy as np
 import pytest
@@ -653,6 +654,20 @@ def test_float32_attention_does_not_depend_on_how_the_keys_are_shared_out(ops, d
         ops._attention_generic_launch(q[r:r + 1].to(DEV).contiguous(), b1, b1.block_tables[0], args[1], 1, page, one, nq, nkv, d, d,
                                       1 / math.sqrt(d), window, keep=keep)
         assert torch.equal(one[0], outs[0][r])
+
+
+def test_float32_attention_of_more_requests_than_a_grid_is_deep(ops):
+    """65,537 requests of one token behind two, which share one page: the last two are a launch of their own."""
+    B, d = 65537, 4
+    cache = g((1, 1, 2, 1, 4, d), torch.float32, 83)
+    q = g((B, d), torch.float32, 84)
+    step = SimpleNamespace(num_requests=B, num_tokens=B, max_q_len=1, max_kv_len=3, tok_req=torch.arange(B, dtype=torch.int32, device=DEV),
+                           q_start=torch.arange(B + 1, dtype=torch.int32, device=DEV), pos_start=torch.full((B,), 2, dtype=torch.int32, device=DEV))
+    out = torch.full((B, d), float("nan"), device=DEV)
+    ops.attention_generic(q.to(DEV), step, torch.zeros(B, 1, dtype=torch.int32, device=DEV), cache.to(DEV), 0, 4, out, 1, 1, d, 0.5, 0)
+    k, v = cache[0, 0, 0, 0, :3].double(), cache[0, 0, 1, 0, :3].double()
+    want = torch.softmax(q.double() @ k.t() * 0.5, 1) @ v
+    assert rel_err(out, want) < 3e-6 and rel_err(out[-2:], want[-2:]) < 3e-6
 
 
 @pytest.mark.parametrize("shares", [1, 3])

@@ -369,10 +369,16 @@ int launch(const void* q, const void* cache, void* out, GenericParams p, int num
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return TFF_ERR_LAUNCH;
         configured = true;
     }
-    const long long rows = (long long)max_q_len * (p.nq / p.nkv), z = (long long)num_requests * p.splits;
-    if (smem > 200 * 1024 || z > 65535 || p.nkv > 65535) return TFF_ERR_UNSUPPORTED;
-    return tff_launch_pdl(kern, dim3((unsigned)((rows + WARPS * RW - 1) / (WARPS * RW)), p.nkv, (unsigned)z), dim3(WARPS * 32), smem,
-                          s, (const T*)q, (const T*)cache, (T*)out, p);
+    const long long rows = (long long)max_q_len * (p.nq / p.nkv);
+    if (smem > 200 * 1024 || (p.splits > 1 && (long long)num_requests * p.splits > 65535) || p.nkv > 65535) return TFF_ERR_UNSUPPORTED;
+    int st = TFF_OK;
+    for (int done = 0; done < num_requests && st == TFF_OK; done += 65535) {        // (a grid is 65,535 deep)
+        const int n = num_requests - done < 65535 ? num_requests - done : 65535;
+        st = tff_launch_pdl(kern, dim3((unsigned)((rows + WARPS * RW - 1) / (WARPS * RW)), p.nkv, (unsigned)(n * p.splits)), dim3(WARPS * 32),
+                            smem, s, (const T*)q, (const T*)cache, (T*)out, p);
+        p.q_start += n; p.pos_start += n; p.block_table += (size_t)n * p.table_width;
+    }
+    return st;
 }
 
 template <typename T>
