@@ -296,12 +296,14 @@ def test_routed_experts_where_the_product_changes(ops, monkeypatch, E, top, T, t
     (2, 4, 4, 64, 64, 8, [32, 1], [7, 100], 0, 24, "cap sink"),                # 32 rows of one head
     (2, 8, 1, 256, 256, 8, [4, 1], [31, 500], 0, 0, "bias cap"),
     (2, 17, 1, 192, 128, 64, [1, 1], [0, 640], 0, 0, "sink"),                  # a second tile of one row
-    (2, 2, 1, 512, 512, 16, [1, 2], [90, 33], 0, 0, ""),                       # too large for two stages of the bulk copies
+    (2, 2, 1, 512, 512, 16, [1, 2], [90, 33], 0, 0, ""),
+    (2, 2, 1, 1280, 64, 16, [1, 1], [90, 33], 0, 0, ""),                       # as large as its shared memory holds
+    (1, 4, 1, 1360, 512, 16, [1, 1], [90, 33], 0, 0, ""),
 ])
 @pytest.mark.parametrize("splits", [1, 3, None])
 def test_attention_of_few_rows(ops, splits, planes, nq, nkv, d, dv, page, lens, starts, window, chunk, more):
     """Steps of at most 32 rows (a request, kv head) in bfloat16 against the same values through the float32 form, which is
-    another kernel.  Two bfloat16 roundings stand between them, of the probabilities (2^-9 of each, and as much of their
+    another kernel (or, where the heads are too large for that, through plain sums).  Two bfloat16 roundings stand between them, of the probabilities (2^-9 of each, and as much of their
     sum) and of the output: at most 3 x 2^-9 of the largest value."""
     dev = "cuda"
     gen = torch.Generator().manual_seed(d + nq)
@@ -327,7 +329,14 @@ def test_attention_of_few_rows(ops, splits, planes, nq, nkv, d, dv, page, lens, 
     if "sink" in more:
         kw.update(sink=vec())
     want = torch.empty(q.shape[0], nq * dv, device=dev)
-    ops.attention_tile(q.float(), step, step.block_table, cache.float(), 1, page, want, nq, nkv, d, dv, d ** -0.5, num_splits=1, **kw)
+    if d <= 512 or d == 576:
+        ops.attention_tile(q.float(), step, step.block_table, cache.float(), 1, page, want, nq, nkv, d, dv, d ** -0.5, num_splits=1, **kw)
+    else:
+        for b, s in enumerate(starts):
+            ts = torch.arange(s + 1)
+            rows = cache[full.block_table[b].cpu().long()[ts // page].to(dev), 1, :, 0, (ts % page).to(dev)].double()     # [keys, planes, slot]
+            k, v = rows[:, 0, :d], rows[:, planes - 1, :dv]
+            want[b] = (torch.softmax(q[b].view(nq, d).double() @ k.t() * d ** -0.5, 1) @ v).flatten().float()
     out = torch.full((q.shape[0], nq * dv), float("nan"), device=dev, dtype=torch.bfloat16)
     ops.attention_tile(q, step, step.block_table, cache, 1, page, out, nq, nkv, d, dv, d ** -0.5, num_splits=splits, **kw)
     torch.cuda.synchronize()

@@ -326,9 +326,9 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 
 struct MmaGeom { int dpad, kst, vst; };      // padded key size, elements between key rows and between value rows in shared memory
 
-// RG groups of 16 rows (a tile has 16 * RG rows and 4 * RG warps: portions two or four);
-// a warp of the value phase owns 16 rows x NT * 8 columns
-template <int NT, int RG>
+// RG groups of 16 rows (a tile has 64 rows and 16 warps); a warp of the value phase owns 16 rows x NT * 8 columns
+constexpr int RG = 4;
+template <int NT>
 __global__ void __launch_bounds__(128 * RG)
 attention_tile_mma_kernel(const bf16* q, const bf16* cache, bf16* __restrict__ out, TileArgs a,
                           MmaGeom gm) {
@@ -766,7 +766,7 @@ attention_tile_few_kernel(const bf16* q, const bf16* cache, bf16* __restrict__ o
             if (lane == 0) alpha_s[rr] = alpha;
         }
         few_barrier();
-        {   // O += P V: 16 rows, columns warp*NT*8 .. + NT*8
+        if (warp * NT * 8 < dv) {   // O += P V: 16 rows, columns warp*NT*8 .. + NT*8
             const float al_a = alpha_s[ra], al_b = alpha_s[rb];
             if (__any_sync(0xffffffffu, al_a != 1.f || al_b != 1.f)) {
 #pragma unroll
@@ -828,14 +828,16 @@ attention_tile_few_kernel(const bf16* q, const bf16* cache, bf16* __restrict__ o
     }
 }
 
-// Launches it (without the merge of the shares); TFF_ERR_UNSUPPORTED for heads too large for two stages of keys.
+// Launches it (without the merge of the shares); TFF_ERR_UNSUPPORTED for heads too large for two stages of keys, which are too large
+// for a tile of 64 rows and 64 keys too.
 template <int NT>
 int launch_few(const void* q, const void* cache, void* out, const TileArgs& a, int num_requests, int rows, cudaStream_t stream) {
     const bool own_v = a.v_offset != 0 || a.k_dense != nullptr;
     MmaGeom gm;
     gm.dpad = (a.d + 15) / 16 * 16;
-    gm.kst = (own_v ? gm.dpad : max(gm.dpad, NT * 64)) + 8;
-    gm.vst = own_v ? NT * 64 + 8 : gm.kst;
+    const int columns = (a.dv + NT * 8 - 1) / (NT * 8) * (NT * 8);      // of the warps that have any
+    gm.kst = (own_v ? gm.dpad : max(gm.dpad, columns)) + 8;
+    gm.vst = own_v ? columns + 8 : gm.kst;
     const size_t smem = 2 * ((size_t)FROWS * gm.kst + (size_t)FSTAGES * FKB * (gm.kst + (own_v ? gm.vst : 0)) + FROWS * FPST) +
                         4 * ((size_t)2 * FROWS * FSST + 3 * FROWS) + 8 * 2 * FSTAGES + 16;
     if (smem > 220 * 1024) return TFF_ERR_UNSUPPORTED;
@@ -876,8 +878,7 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
     gm.kst = (own_v ? gm.dpad : max(gm.dpad, nt * 32)) + 8;
     gm.vst = own_v ? nt * 32 + 8 : gm.kst;
     const int rows_most = max_q_len * G;
-    const int rg = rows_most <= 16 ? 1 : (rows_most <= 32 ? 2 : 4);       // (one group: heads too large for the kernel of few rows)
-    const int MROWS = 16 * rg;
+    constexpr int MROWS = 16 * RG;
     if (rows_most <= FMOST) {
         int st = a.dv <= 128 ? launch_few<2>(q, cache, out, a, num_requests, rows_most, stream)
                : a.dv <= 256 ? launch_few<4>(q, cache, out, a, num_requests, rows_most, stream)
@@ -886,7 +887,7 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
             st = tff_launch_pdl(attention_tile_merge_kernel<bf16>, dim3((unsigned)(num_tokens * a.nq)), dim3(MERGE_THREADS), 0, stream,
                                 (const float*)a.part_o, (const float*)a.part_ml, (bf16*)out, a.out_ld, a.out_off, a.nq, a.dv, a.splits,
                                 a.out_scale);
-        if (st != TFF_ERR_UNSUPPORTED) return st;
+        return st;
     }
     const size_t smem = 2 * ((size_t)(MROWS + MKB) * gm.kst + (own_v ? (size_t)MKB * gm.vst : 0) + (size_t)MROWS * PST) +
                         4 * ((size_t)MROWS * SST + 2 * MROWS) + 4 * 2 * MROWS + 2 * 8 * MKB;
@@ -895,15 +896,9 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
     dim3 grid(tiles * a.splits, a.nkv, num_requests);
 #define TFF_TMMA(NTV)                                                                                                \
     do {                                                                                                             \
-        if (rg == 1) TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 1>), 128);                                         \
-        if (rg == 2) TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 2>), 256);                                         \
-        TFF_TMMA_RUN((attention_tile_mma_kernel<NTV, 4>), 512);                                                      \
-    } while (0)
-#define TFF_TMMA_RUN(KERNEL, THREADS_)                                                                               \
-    do {                                                                                                             \
         if (smem > 48 * 1024)                                                                                        \
-            cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                     \
-        const int st = tff_launch_pdl(KERNEL, grid, dim3(THREADS_), smem, stream, (const bf16*)q,                     \
+            cudaFuncSetAttribute(attention_tile_mma_kernel<NTV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        const int st = tff_launch_pdl(attention_tile_mma_kernel<NTV>, grid, dim3(128 * RG), smem, stream, (const bf16*)q, \
                                       (const bf16*)cache, (bf16*)out, a, gm);                                        \
         if (st != TFF_OK || a.splits == 1) return st;                                                                \
         const long long rows = (long long)num_tokens * a.nq;                                                         \
@@ -916,7 +911,6 @@ int launch_tile_mma(const void* q, const void* cache, void* out, const TileArgs&
     if (nt == 8) TFF_TMMA(8);
     TFF_TMMA(16);
 #undef TFF_TMMA
-#undef TFF_TMMA_RUN
 }
 
 }  // namespace
