@@ -122,7 +122,7 @@ def test_sums_of_few_row_attention_leave_what_the_last_block_reads_alone():
 
 # Kernels launched with programmatic dependent launch, and the pointers through which they read what the kernels ahead wrote
 READ_PAST_L1 = [
-    ("gemm_f32.cu", "gemm_f32_kernel", ("A", "W", "residual")),
+    ("gemm_f32.cu", "gemm_f32_kernel", ("A", "residual")),
     ("gemm_f32.cu", "gemm_f32_sum_kernel", ("A", "W", "ws", "residual", "p")),
     ("attention_generic.cu", "attention_generic_kernel", ("q_in", "cache", "gate", "src")),
     ("attention_generic.cu", "attention_generic_join_kernel", ("ml", "po", "gate")),

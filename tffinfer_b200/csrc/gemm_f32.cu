@@ -15,7 +15,7 @@
 // finite is computed once more as a plain sum of products, since a split of an infinity has no meaning.
 //
 // What bounds it.  Few rows: the latency of the memory, since registers hold only the two K blocks (64 KB) on their way while the
-// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill 140 to 190 bytes (4 rows of the 8B shape's gate/up product, 403 MB: 94 us = 4.3 TB/s; down 61 us; as float32 FMAs, one order of
+// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill about 50 bytes (4 rows of the 8B shape's gate/up product, 403 MB: 94 us = 4.3 TB/s; down 61 us; as float32 FMAs, one order of
 // summation a thread, 1.4 ms each).  Asking the L2 for the weights one chunk ahead made it slower (102 us).  Many rows: shared memory, which
 // takes 6 bytes an element from the split and feeds six products, beside the products themselves (512 rows of gate/up 0.71 ms,
 // 145 TFLOP/s; without the products 0.48, without the loads 0.45; FMAs at most 70).  Off 64-bit arithmetic
@@ -70,21 +70,31 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// 8 consecutive elements of a row as float32; elements at or behind ``left`` are zeros (left counts from p).  Either operand may have
-// been written by the kernel ahead: both are read past the first-level cache.
-template <typename T, bool VEC>
+// 8 consecutive elements of a row as float32; elements at or behind ``left`` are zeros (left counts from p).  The activations may have
+// been written by the kernel ahead and are read past the first-level cache.  CONST: the weights, which no kernel of a step writes, on
+// the read-only path, where they take no room in that cache.
+template <typename T, bool VEC, bool CONST>
 __device__ __forceinline__ void load8(const T* p, int left, uint32_t* r) {
     if constexpr (VEC) {                             // rows are multiples of 8 elements and aligned: all of the 8 or none
         if (left <= 0) {
 #pragma unroll
             for (int i = 0; i < (sizeof(T) == 4 ? 8 : 4); ++i) r[i] = 0u;
         } else if constexpr (sizeof(T) == 4) {
-            asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                         : "l"(p) : "memory");
+            if constexpr (CONST)
+                asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                             : "l"(p));
+            else
+                asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                             : "l"(p) : "memory");
         } else {
-            asm volatile("ld.global.cg.v4.b32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
+            if constexpr (CONST)
+                asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p));
+            else
+                asm volatile("ld.global.cg.v4.b32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
         }
     } else {
         auto one = [&](int i) { return i < left ? __float_as_uint(ldcg_f32(p + i)) : 0u; };
@@ -129,7 +139,8 @@ __device__ __forceinline__ void split_store(const uint32_t* r, uint32_t dst, uin
 }
 
 // Elements whose sum of split products is not finite, as plain sums of products: the warp takes the lanes that hold one in
-// turn.  All lanes call it, with the rows of their own element.
+// turn.  All lanes call it, with the rows of their own element.  (Four products' loads together and no more: with a loop that the
+// compiler unrolled as it liked the kernels that call this spilled 200 bytes in place of 50.)
 template <typename TA, typename TW>
 __device__ __noinline__ float plain_dots(float v, bool mine, const TA* a, const TW* w, int K) {
     const int lane = threadIdx.x & 31;
@@ -138,7 +149,15 @@ __device__ __noinline__ float plain_dots(float v, bool mine, const TA* a, const 
         const TA* ra = (const TA*)__shfl_sync(0xffffffffu, (unsigned long long)a, src);
         const TW* rw = (const TW*)__shfl_sync(0xffffffffu, (unsigned long long)w, src);
         float s = 0.f;
-        for (int k = lane; k < K; k += 32) s = fmaf(ldcg_f32(ra + k), ldcg_f32(rw + k), s);
+        int k = lane;
+#pragma unroll 1
+        for (; k + 96 < K; k += 128) {
+            const float a0 = ldcg_f32(ra + k), w0 = ldcg_f32(rw + k), a1 = ldcg_f32(ra + k + 32), w1 = ldcg_f32(rw + k + 32);
+            const float a2 = ldcg_f32(ra + k + 64), w2 = ldcg_f32(rw + k + 64), a3 = ldcg_f32(ra + k + 96), w3 = ldcg_f32(rw + k + 96);
+            s = fmaf(a0, w0, s); s = fmaf(a1, w1, s); s = fmaf(a2, w2, s); s = fmaf(a3, w3, s);
+        }
+#pragma unroll 1
+        for (; k < K; k += 32) s = fmaf(ldcg_f32(ra + k), ldcg_f32(rw + k), s);
         s = warp_sum(s);
         if (lane == src) v = s;
     }
@@ -274,8 +293,8 @@ gemm_f32_kernel(const TA* A, const TW* W, void* out, int out_bf16, const float* 
             a_rows = min(M - it.m0, BN) - row;
         };
         const size_t pitch = (size_t)STRIDE * K;
-        auto load_w = [&](int q) { load8<TW, VEC>(wp + q * pitch, STRIDE * q < w_rows ? left : 0, wr[q]); };
-        auto load_a = [&](int q) { load8<TA, VEC>(ap + q * pitch, STRIDE * q < a_rows ? left : 0, ar[q]); };
+        auto load_w = [&](int q) { load8<TW, VEC, true>(wp + q * pitch, STRIDE * q < w_rows ? left : 0, wr[q]); };
+        auto load_a = [&](int q) { load8<TA, VEC, false>(ap + q * pitch, STRIDE * q < a_rows ? left : 0, ar[q]); };
         auto has_a = [&](int q) { return (q + 1) * STRIDE <= BN || row + q * STRIDE < BN; };
         auto step = [&]() {                                                  // to the next K block of the CTA
             if (++kb >= it.kb1) {
