@@ -15,7 +15,7 @@
 // finite is computed once more as a plain sum of products, since a split of an infinity has no meaning.
 //
 // What bounds it.  Few rows: the latency of the memory, since registers hold only the two K blocks (64 KB) on their way while the
-// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill about 50 bytes (4 rows of the 8B shape's gate/up product, 403 MB: 94 us = 4.3 TB/s; down 61 us; as float32 FMAs, one order of
+// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill 50 to 105 bytes (4 rows of the 8B shape's gate/up product, 403 MB: 94 us = 4.3 TB/s; down 61 us; as float32 FMAs, one order of
 // summation a thread, 1.4 ms each).  Asking the L2 for the weights one chunk ahead made it slower (102 us).  Many rows: shared memory, which
 // takes 6 bytes an element from the split and feeds six products, beside the products themselves (512 rows of gate/up 0.71 ms,
 // 145 TFLOP/s; without the products 0.48, without the loads 0.45; FMAs at most 70).  Off 64-bit arithmetic
@@ -140,7 +140,7 @@ __device__ __forceinline__ void split_store(const uint32_t* r, uint32_t dst, uin
 
 // Elements whose sum of split products is not finite, as plain sums of products: the warp takes the lanes that hold one in
 // turn.  All lanes call it, with the rows of their own element.  (Four products' loads together and no more: with a loop that the
-// compiler unrolled as it liked the kernels that call this spilled 200 bytes in place of 50.)
+// compiler unrolled as it liked the kernels that call this spilled up to 200 bytes in place of 50 to 105.)
 template <typename TA, typename TW>
 __device__ __noinline__ float plain_dots(float v, bool mine, const TA* a, const TW* w, int K) {
     const int lane = threadIdx.x & 31;
