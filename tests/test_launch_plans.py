@@ -157,3 +157,10 @@ def test_partial_results_of_the_float32_attention_have_a_bound():
                 assert requests * nq * slots * (dv + 2) * 4 <= 64 << 20
                 assert shares == max(1, min(296 // (requests * nkv), -(-keys // 64))), (requests, nq, nkv, dv, keys)
     assert plan(16, 1, 40960, 32, 8, 128, 0, 0, 148) >> 16 == (64 << 20) // (16 * 32 * 130 * 4)
+
+
+def test_experts_change_their_product_by_pairs_an_expert():
+    """Above 8 pairs an expert of up to 16, above 12 of more or by a table, never later than at 1,024 pairs."""
+    start = CudaKernels.grouped_tcgen05_from
+    assert (start(4, False), start(16, False), start(17, False), start(64, False), start(128, False)) == (33, 129, 205, 769, 1024)
+    assert (start(4, True), start(16, True), start(64, True), start(128, True)) == (49, 193, 769, 1024)

@@ -1349,7 +1349,7 @@ class CudaKernels:
         # both products run on the same kernel (one tile table): the tensor-core one if both can
         tc = (self.grouped_on_tensor_cores(h, w_gate_up, W, W, 0, W, up_rows * W, "" if plain else layout, ff)
               and self.grouped_on_tensor_cores(h, w_down, ff, ff, 0, ff, W * ff, "", W))
-        if tc and self.GROUPED_TCGEN05 and P >= min(self.GROUPED_TCGEN05_FROM, self.GROUPED_TCGEN05_EACH * E + 1) and W % 4 == 0 and ff % 8 == 0:
+        if tc and self.GROUPED_TCGEN05 and P >= self.grouped_tcgen05_from(E, by_table) and W % 4 == 0 and ff % 8 == 0:
             # Prompt-sized: the tcgen05 product in its grouped form.  Every expert's rows are padded to whole tiles of 128
             # in the sorted order, both products write in that order, and the sum gathers a token's rows from it.
             rows = -(-(P + E * 127) // 128) * 128
@@ -1389,11 +1389,19 @@ class CudaKernels:
                          identity=(pe[0], pair_weight, h) if pe else None, shared=shared)
 
     GROUPED_TCGEN05 = os.environ.get("TFFINFER_GROUPED_TCGEN05", "1") != "0"
-    GROUPED_TCGEN05_FROM = 1024      # (token, expert) pairs of a step from which the experts run on the tcgen05 product,
-    # or fewer where an expert has more than these on average: 16 experts of the "2k" sizes (4k) with 160 pairs 178 -> 167 us (521 ->
-    # 505), 192 186 -> 167 (573 -> 507), 400 309 -> 202 (955 -> 569), 838 331 -> 213 (1,054 -> 608); with 128 they are equal (159 and
-    # 161, 499 and 501), with 48 the tiles of few rows are faster (128 and 145, 460 and 479)
-    GROUPED_TCGEN05_EACH = 8
+    GROUPED_TCGEN05_FROM = 1024      # (token, expert) pairs of a step from which the experts run on the tcgen05 product, or fewer:
+    GROUPED_TCGEN05_EACH = {False: 8, True: 12}      # where an expert has more than these on average, by whether there are many of them
+
+    @classmethod
+    def grouped_tcgen05_from(cls, E: int, by_table: bool) -> int:
+        """From how many pairs of a step E experts run on the tcgen05 product (us, mma.sync and tcgen05).  Above 12 an expert the
+        other one leaves its tiles of few rows: 4 experts of 3,072 x 2,048 with 64 pairs 159 and 70, 16 with 256 263 and 135, 64 of
+        768 x 2,048 with 1,026 268 and 168, 64 of 1,536 x 4,096 with 1,024 875 and 536; chosen by a table 145 and 61, 253 and 127,
+        248 and 151, 843 and 503.  With 9 to 12 an expert that is so for few experts chosen in groups, which have uneven shares: a layer
+        of 16 experts of 3,072 x 2,048 (6,144 x 4,096) and a shared one with 160 pairs 178 and 167 (521 and 505), 192 186 and 167
+        (573 and 507), 128 159 and 161 (499 and 501).  Many experts, or even shares, are faster on tiles of few rows: 64 with 576
+        139 and 166 (456 and 537), chosen by a table 123 and 151 (427 and 509), 16 chosen by a table with 144 122 and 132."""
+        return min(cls.GROUPED_TCGEN05_FROM, cls.GROUPED_TCGEN05_EACH[E > 16 or by_table] * E + 1)
 
     def gemm_tc_grouped(self, a, w, out, groups: int, group_rows: int, K: int, lane_group, gated: bool = False,
                         activation: str = "silu", limit: float = 0.0) -> None:
