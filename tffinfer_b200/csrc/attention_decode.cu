@@ -302,6 +302,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
     float* mO = reinterpret_cast<float*>(gbase);           // [4][16][D] floats: 256 * D bytes <= one stage
     float* mM = reinterpret_cast<float*>(gbase + STAGE_BYTES);
     float* mL = mM + 64;
+    float* mG = mL + 64;                                           // the rows' head gates
+    if (p.gate && p.num_splits == 1 && tid < rows_total) mG[tid] = __ldcg(p.gate + (size_t)(q0 + tid / G) * p.nq + kvh * G + tid % G);
     if ((lane & 3) == 0) {
         mM[warp * 16 + r0] = m0; mM[warp * 16 + r1] = m1;
         mL[warp * 16 + r0] = l0; mL[warp * 16 + r1] = l1;
@@ -330,7 +332,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_cache, const DecodePar
         const size_t grow = (size_t)(q0 + r / G) * p.nq + (kvh * G + r % G);
         if (p.num_splits == 1) {
             if (p.sink) lsum += exp2f(attn_sink_log2(p.sink_val, kvh * G + r % G) - Ms);   // the sink: a key without a value
-            const float gt = p.gate ? __ldcg(p.gate + grow) : 1.f;
+            const float gt = p.gate ? mG[r] : 1.f;
             p.out[grow * D + c] = __float2bfloat16_rn(acc * gt / lsum);
         } else {
             p.part_o[(grow * p.num_splits + split) * D + c] = acc;
