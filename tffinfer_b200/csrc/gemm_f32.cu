@@ -15,8 +15,8 @@
 // finite is computed once more as a plain sum of products, since a split of an infinity has no meaning.
 //
 // What bounds it.  Few rows: the latency of the memory, since registers hold only the two K blocks (64 KB) on their way while the
-// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill 50 to 105 bytes (4 rows of the 8B shape's gate/up product, 403 MB: 94 us = 4.3 TB/s; down 61 us; as float32 FMAs, one order of
-// summation a thread, 1.4 ms each).  Asking the L2 for the weights one chunk ahead made it slower (102 us).  Many rows: shared memory, which
+// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill 50 to 105 bytes (4 rows of the 8B shape's
+// gate/up product, 403 MB: 91 us = 4.4 TB/s; down 58 us; as float32 FMAs, one order of summation a thread, 1.4 ms each).  Asking the L2 for the weights one chunk ahead made it slower (102 us).  Many rows: shared memory, which
 // takes 6 bytes an element from the split and feeds six products, beside the products themselves (512 rows of gate/up 0.71 ms,
 // 145 TFLOP/s; without the products 0.48, without the loads 0.45; FMAs at most 70).  Off 64-bit arithmetic
 // (2-norm, random operands) by 2.6e-8 at K = 1, 3.1e-8 at 8, 7.0e-8 at 64, 2.3e-7 at 512, 4.8e-7 at 1,024 and 4,096; a chain of FMAs over
@@ -444,17 +444,25 @@ gemm_f32_sum_kernel(const TA* A, const TW* W, const float* ws, void* out, int ou
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     const bool vec = (total & 3) == 0;                       // chunks then start 16-byte aligned
     const int cnt = i >= total ? 0 : (int)(total - i < 4 ? total - i : 4);
-    if (cnt > 0) {
-#pragma unroll 4
-        for (int s = 0; s < chunks; ++s) {
-            const float* p = ws + (size_t)s * total + i;
-            float t[4] = {0.f, 0.f, 0.f, 0.f};
-            if (vec) {
-                const float4 f = __ldcg((const float4*)p);
-                t[0] = f.x; t[1] = f.y; t[2] = f.z; t[3] = f.w;
-            } else {
-                for (int j = 0; j < cnt; ++j) t[j] = __ldcg(p + j);
+    if (vec && cnt > 0) {
+        // (eight chunks' loads on their way together: one behind the other, four rows of the 8B shape's down product took 73 us, so 58)
+        for (int s0 = 0; s0 < chunks; s0 += 8) {
+            float4 f[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (s0 + u < chunks) f[u] = __ldcg((const float4*)(ws + (size_t)(s0 + u) * total + i));
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (s0 + u >= chunks) continue;
+                if (s0 + u == 0) { v[0] = f[u].x; v[1] = f[u].y; v[2] = f[u].z; v[3] = f[u].w; }
+                else { v[0] += f[u].x; v[1] += f[u].y; v[2] += f[u].z; v[3] += f[u].w; }
             }
+        }
+    } else {
+        for (int s = 0; s < chunks; ++s) {
+            float t[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t[j] = j < cnt ? __ldcg(ws + (size_t)s * total + i + j) : 0.f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = s == 0 ? t[j] : v[j] + t[j];
         }
