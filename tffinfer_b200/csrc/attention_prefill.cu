@@ -69,8 +69,6 @@ using tc5::tma_load_2d;
 using tc5::fence_async_smem;
 using tc5::tmem_alloc;
 using tc5::tmem_dealloc;
-using tc5::umma_bf16;
-using tc5::umma_commit;
 using tc5::tc_fence_before;
 using tc5::tc_fence_after;
 using tc5::tmem_ld16;
@@ -79,15 +77,18 @@ using tc5::tmem_ld_wait;
 
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_N = 64;
-#ifndef TURN_AFTER
-#define TURN_AFTER 8          // of the 8 chunks of a block's exponentials, after which the other tile may begin its own
-#endif
-constexpr int BARS_PER_TILE = 7;
+constexpr int BARS_PER_TILE = 16;
 constexpr float RESCALE_THRESHOLD = 8.0f;       // in log2 units
 
 // the same for a whole warp: every lane gets the same answer
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+// A box of tff_tensor_map_kv_groups: a page's keys and values of a kv head, from its first group of 8 rows.
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int group) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %3, %4}], [%2];"
+        ::"r"(dst), "l"(tm), "r"(bar), "r"(0), "r"(group) : "memory");
 }
 // 2^x on the special-function unit (float32 in and out; 2^-inf = 0)
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -102,14 +103,30 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// The A operand from tensor memory (lane = row, one 32-bit column = two consecutive K elements), B from shared memory.
-__device__ __forceinline__ void umma_bf16_a_tmem(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
+// The products are issued by a warp whose lanes all go through the loop, one elected lane issuing: addresses and descriptors are
+// then the same in the whole warp for the compiler too.
+__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// The A operand from tensor memory (lane = row, one 32-bit column = two consecutive K elements), B from shared memory.
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void umma_commit_elected(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 
 // Pairs of float32 in a 64-bit register: fma and add on a pair issue as one instruction on sm_100.
@@ -138,14 +155,14 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     return d;
 }
 
-// Shared-memory matrix descriptor, 128-byte swizzle, 8-row groups 1024 bytes apart.  ``lbo_bytes`` is
+// Shared-memory matrix descriptor, 128-byte swizzle, 8-row groups ``sbo_bytes`` apart.  ``lbo_bytes`` is
 // the distance between successive 64-element blocks along the M/N extent of an MN-major operand
 // (not used by K-major operands).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes) {
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
     d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)(sbo_bytes >> 4) << 32;
     d |= (uint64_t)1 << 46;
     d |= (uint64_t)2 << 61;
     return d;
@@ -157,12 +174,12 @@ __host__ __device__ constexpr uint32_t make_idesc(int m, int n, int b_mn_major) 
 }
 
 #ifdef AP_TIMERS
-__device__ long long ap_dbg[64];
-#define AP_T(var) const long long var = clock64()
-#define AP_ACC(slot, a, b) do { if (dbg_on) ap_dbg[slot] += (b) - (a); } while (0)
+__device__ long long ap_dbg[2 * 16 * 160];             // [tile][event][block]
+#define AP_EV(e, j) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (j) < 160 && (warp >= ISSUE_WARP || (lane == 0 && (warp & 3) == 0))) ap_dbg[(x * 16 + (e)) * 160 + (j)] = clock64(); } while (0)
+#define AP_EVL(e, j) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (j) < 160 && lane == 0) ap_dbg[(e) * 160 + (j)] = clock64(); } while (0)
 #else
-#define AP_T(var)
-#define AP_ACC(slot, a, b)
+#define AP_EV(e, j)
+#define AP_EVL(e, j)
 #endif
 
 struct PrefillParams {
@@ -183,11 +200,14 @@ struct PrefillParams {
 
 template <int DK, int DV, int QT>
 struct PrefillCfg {
-    static constexpr int kStageBytes = BLOCK_N * (DK + DV) * 2;     // K then V, each [64-column half][64 keys][128 B]
-    static constexpr int kQExtra = DK > 128 ? (DK - 128) / 64 * BLOCK_M * 128 : 0;     // a tile's query columns beyond 128
-    static constexpr int kStages = DK > 128 ? (QT == 2 ? 3 : 4) : 5;
-    static constexpr int kBars = 2 * kStages + BARS_PER_TILE * QT + 8;
-    static constexpr int kSmem = kStages * kStageBytes + QT * (2 * BLOCK_M * BLOCK_N * 2 + kQExtra) + 8 * kBars + 16 + 1024;
+    static constexpr int kQBytes = BLOCK_M * DK * 2;                // [64-column half][128 rows][128 B]
+    static constexpr int kStageBytes = BLOCK_N * (DK + DV) * 2;     // a block's keys and values
+    static constexpr int kStages = DK > 128 ? (QT == 2 ? 3 : 4) : DK > 64 ? 5 : 8;
+    static constexpr int kExchange = QT * 2 * BLOCK_M * 4;          // a float of every row from either group
+    static constexpr int kBars = 2 * kStages + BARS_PER_TILE * QT;
+    static constexpr int kSmem = QT * kQBytes + kStages * kStageBytes + kExchange + 8 * kBars + 16;
+    static constexpr int kThreads = (8 * QT + 1 + QT) * 32;
+    static constexpr int kTmemCols = QT * 256;
     static_assert(kSmem <= 227 * 1024, "shared memory of the prompt attention kernel");
 };
 
@@ -195,46 +215,40 @@ struct PrefillCfg {
 // DK, DV: elements of a key and of a value (DENSE: rounded up; the query's columns beyond its own are zeros, the output's
 // are not stored).  tm_cache is the cache, or the keys' rows when DENSE; tm_v and tm_r are read by the dense form only.
 template <int DK, int DV, int QT, bool DENSE>
-__global__ void __launch_bounds__(QT == 2 ? 352 : 192, 1)
+__global__ void __launch_bounds__(PrefillCfg<DK, DV, QT>::kThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __grid_constant__ CUtensorMap tm_v,
                        const __grid_constant__ CUtensorMap tm_r, const PrefillParams p) {
     using Cfg = PrefillCfg<DK, DV, QT>;
     static_assert(DENSE || DK == DV, "a slot of the cache holds a key or a value");
-    constexpr int NSTAGES = Cfg::kStages;
     constexpr int KH = DK / 64, VH = DV / 64;                    // 64-column halves of a key and of a value
     constexpr int CH = DV / 8;                                   // 16-byte chunks of a value row
-    constexpr int K_BYTES = BLOCK_N * DK * 2;                    // K of one stage: [half][64 keys][128 B]
-    constexpr int STAGE_BYTES = Cfg::kStageBytes;
-    constexpr int P_BYTES = BLOCK_M * BLOCK_N * 2;               // one tile's probabilities: [128 rows][128 B]
-    constexpr int QT_COLS = DK < 128 ? DK : 128;                 // query elements a row that lie in tensor memory
-    constexpr int TMEM_COLS = 512;
-    constexpr int NBARS = Cfg::kBars;
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t sP = base + NSTAGES * STAGE_BYTES;            // two buffers per tile: [tile][block % 2]
-    const uint32_t sQ = sP + QT * 2 * P_BYTES;                   // the tiles' query columns beyond QT_COLS: [half][128 rows][128 B]
-    const uint32_t bars = sQ + QT * Cfg::kQExtra;
-    uint8_t* gP = gbase + NSTAGES * STAGE_BYTES;
-    uint8_t* gQ = gP + QT * 2 * P_BYTES;
-    // barriers: kv_full[NS], kv_empty[NS]; per tile x: s_full, s_free, p_full[0], pv_done[2], q_ready, p_full[1]
+    constexpr int NSTAGES = Cfg::kStages, STAGE_BYTES = Cfg::kStageBytes;
+    // A stage, in atoms of 8 keys x 64 columns (1 KB).  From the cache, a box a page brings keys and values: [8 keys][K, V][64-column
+    // half].  DENSE: K then V, each [half][8 keys].
+    constexpr int GROUP = DENSE ? 1024 : (KH + VH) * 1024;                // from 8 keys to the next 8
+    constexpr int K_HALF = DENSE ? BLOCK_N * 128 : 1024, V_HALF = K_HALF;  // from a half to the next
+    constexpr int V_AT = DENSE ? KH * K_HALF : KH * 1024;                  // of the stage's first values
+    constexpr int LOAD_WARP = 8 * QT, ISSUE_WARP = LOAD_WARP + 1;              // behind the softmax warps
+    extern __shared__ __align__(1024) uint8_t smem[];            // (the only shared memory of the kernel: it starts 1024-byte aligned)
+    const uint32_t sQ = smem_u32(smem);
+    const uint32_t sKV = sQ + QT * Cfg::kQBytes;
+    constexpr int BARS_AT = QT * Cfg::kQBytes + NSTAGES * STAGE_BYTES + Cfg::kExchange;
+    const uint32_t bars = sQ + BARS_AT;
+    uint8_t* gKV = smem + QT * Cfg::kQBytes;
+    volatile float* exchange = (volatile float*)(gKV + NSTAGES * STAGE_BYTES);       // [tile][group][row]
     auto kv_full = [&](int s) { return bars + 8u * s; };
     auto kv_empty = [&](int s) { return bars + 8u * (NSTAGES + s); };
-    auto s_full = [&](int x) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * x); };
-    auto s_free = [&](int x) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * x + 1); };
-    // P(j) reports to p_full(x, j % 2).  With one barrier a warp that took the short, unmasked path through two
-    // blocks could arrive for block j + 1 before a warp on the masked path had arrived for block j, and PV(j)
-    // went out with that warp's rows of P unwritten; a warp cannot be two blocks ahead (S(j + 2) is issued only
-    // when every warp has read S(j + 1)), so two barriers taken in turn are enough.
-    auto p_full = [&](int x, int b) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * x + 2 + 4 * b); };
-    // PV(j) reports to pv_done(x, j % 2): a waiter is then never more than one completion behind the barrier
-    // it looks at, which a parity wait needs
-    auto pv_done = [&](int x, int b) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * x + 3 + b); };
-    auto q_ready = [&](int x) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * x + 5); };
-    // whose turn it is at the special-function unit: the warps of the two tiles that share a scheduler (the same
-    // lane quarter) take their exponential passes in turn
-    auto turn = [&](int x, int q) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * QT + 4 * x + q); };
-    volatile uint32_t* tmem_slot = (volatile uint32_t*)(gQ + QT * Cfg::kQExtra + 8 * NBARS);
+    auto tile_bar = [&](int x, int i) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * x + i); };
+    // S(j), P(j), PV(j) and the reference of block j report to a barrier of the group that has block j (group j % 2): who waits
+    // for a barrier then waits for every one of its completions in turn, or knows that the one before is in the past, which a
+    // parity wait needs.
+    auto s_full = [&](int x, int g) { return tile_bar(x, g); };
+    auto s_free = [&](int x) { return tile_bar(x, 2); };
+    auto p_full = [&](int x, int g) { return tile_bar(x, 3 + g); };
+    auto pv_done = [&](int x, int g) { return tile_bar(x, 5 + g); };
+    auto q_ready = [&](int x) { return tile_bar(x, 7); };
+    auto ref_bar = [&](int x, int g, int q) { return tile_bar(x, 8 + 4 * g + q); };
+    volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + BARS_AT + 8 * Cfg::kBars);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -248,16 +262,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     if (tid == 0) {
         for (int s = 0; s < NSTAGES; ++s) mbar_init(kv_full(s), 1);
         for (int x = 0; x < QT; ++x) {
-            mbar_init(s_full(x), 1); mbar_init(s_free(x), 4); mbar_init(p_full(x, 0), 4); mbar_init(p_full(x, 1), 4);
-            mbar_init(pv_done(x, 0), 1); mbar_init(pv_done(x, 1), 1); mbar_init(q_ready(x), 4);
+            for (int g = 0; g < 2; ++g) {
+                mbar_init(s_full(x, g), 1); mbar_init(p_full(x, g), 4); mbar_init(pv_done(x, g), 1);
+                for (int q = 0; q < 4; ++q) mbar_init(ref_bar(x, g, q), 1);
+            }
+            mbar_init(s_free(x), 4); mbar_init(q_ready(x), 8);
         }
-        for (int i = 0; i < 8; ++i) mbar_init(turn(i >> 2, i & 3), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_cache) : "memory");
         if (DENSE) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_v) : "memory");
     }
-    if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), TMEM_COLS);
+    if (warp == ISSUE_WARP) tmem_alloc(smem_u32((const void*)tmem_slot), Cfg::kTmemCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -286,203 +302,153 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     const KeyWalk walk(p.keep, BLOCK_N, lo_cta / BLOCK_N, hi / BLOCK_N);
     const int nb = active ? walk.count : 0;
     const int* table = DENSE ? nullptr : p.block_table + (size_t)b * p.table_width;
-    // a stage is free again when the PV products of every tile that has rows have read it
+    // a stage is free again when the products of every tile that has rows have read it
     if (tid == 0) {
         for (int s = 0; s < NSTAGES; ++s) mbar_init(kv_empty(s), (uint32_t)(n_act > 0 ? n_act : 1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int q = 0; q < 4; ++q) mbar_arrive(turn(0, q));      // the first tile begins
     }
     __syncthreads();
 
-    if (warp == 0) {
+    if (warp == LOAD_WARP) {
         // ------------------------------------------------------------ TMA producer
+        // the block table's entries of 32 pages, one a lane, and those of the next 32: a lookup a block would be a read from
+        // global memory on the way to every load
         const int ppb = DENSE ? 0 : BLOCK_N >> p.page_shift;
-        const int nloads = ppb * KH * 2;                          // boxes per stage (<= 32)
-        const int j = lane / (KH * 2), rem = lane % (KH * 2);
-        const int kv = rem / KH, hf = rem % KH;
+        const int table_end = hi >> p.page_shift;
+        int chunk = -1, held = -1, ahead = -1;
+        auto entry = [&](int c) {
+            const int at = c * 32 + lane;
+            return at <= table_end ? table[at] : -1;
+        };
         for (int i = 0; i < nb; ++i) {
             const int s = i % NSTAGES;
             const uint32_t round = i / NSTAGES;
-            bool ok = true;
-            if (round > 0) {
-                if (lane == 0) ok = mbar_wait(kv_empty(s), (round - 1) & 1, abort_flag);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-            }
-            if (!ok) break;
+            if (round > 0 && !mbar_wait_warp(kv_empty(s), (round - 1) & 1, abort_flag)) break;
+            const uint32_t stage = sKV + s * STAGE_BYTES;
+            const int n_first = walk.block(i) * BLOCK_N;
             if constexpr (DENSE) {
                 // key n of the request is row q0 + n; rows beyond the request's are another's or zeros, and masked
                 if (lane == 0) mbar_expect_tx(kv_full(s), (uint32_t)STAGE_BYTES);
                 __syncwarp();
-                const int row = q0 + walk.block(i) * BLOCK_N;
+                const int row = q0 + n_first;
                 if (lane < KH) {
-                    const uint32_t dst = base + s * STAGE_BYTES + lane * (BLOCK_N * 128);
+                    const uint32_t dst = stage + lane * K_HALF;
                     if (lane < p.k_halves) tma_load_2d(dst, &tm_cache, kv_full(s), kvh * p.k_head + lane * 64, row);
                     else tma_load_2d(dst, &tm_r, kv_full(s), p.r_col + (lane - p.k_halves) * 64, row);
                 } else if (lane < KH + VH) {
-                    tma_load_2d(base + s * STAGE_BYTES + K_BYTES + (lane - KH) * (BLOCK_N * 128), &tm_v, kv_full(s),
-                                kvh * p.dv + (lane - KH) * 64, row);
+                    tma_load_2d(stage + V_AT + (lane - KH) * V_HALF, &tm_v, kv_full(s), kvh * p.dv + (lane - KH) * 64, row);
                 }
-                continue;
-            }
-            const int n0 = walk.block(i) * BLOCK_N + (j << p.page_shift);
-            int page = -1;
-            if (lane < nloads && n0 <= hi) page = table[n0 >> p.page_shift];
-            const bool valid = page >= 0;
-            const unsigned mask = __ballot_sync(0xffffffffu, valid);
-            if (lane == 0) mbar_expect_tx(kv_full(s), (uint32_t)__popc(mask) * (uint32_t)(ps * 128));
-            __syncwarp();
-            if (valid) {
-                const long long row = ((((long long)page * p.cache_layers + p.layer) * 2 + kv) * p.nkv + kvh) << p.page_shift;
-                // stage layout: K then V, each [half][64 keys][128 B]
-                const uint32_t dst = base + s * STAGE_BYTES + kv * K_BYTES + hf * (BLOCK_N * 128) +
-                                     (uint32_t)((j << p.page_shift) * 128);
-                tma_load_2d(dst, &tm_cache, kv_full(s), hf * 64, (int)row);
+            } else {
+                const int first = n_first >> p.page_shift;               // (a block's pages lie in one run of 32)
+                if (first >> 5 != chunk) {
+                    held = first >> 5 == chunk + 1 && chunk >= 0 ? ahead : entry(first >> 5);
+                    chunk = first >> 5;
+                    ahead = entry(chunk + 1);
+                }
+                const bool valid = lane >= (first & 31) && lane < (first & 31) + ppb && held >= 0;
+                const unsigned mask = __ballot_sync(0xffffffffu, valid);
+                if (lane == 0) mbar_expect_tx(kv_full(s), (uint32_t)__popc(mask) * (uint32_t)(GROUP << (p.page_shift - 3)));
+                __syncwarp();
+                AP_EVL(13, i);
+                if (valid) {
+                    const long long row = ((((long long)held * p.cache_layers + p.layer) * 2) * p.nkv + kvh) << p.page_shift;
+                    tma_load_5d(stage + (uint32_t)((lane - (first & 31)) * (GROUP << (p.page_shift - 3))), &tm_cache, kv_full(s), (int)(row >> 3));
+                }
             }
         }
-    } else if (warp == 1 || warp == 10) {
+    } else if (warp >= ISSUE_WARP) {
         // -------------------------------------------------------------- MMA issuers, one per tile
-        const int x = warp == 1 ? 0 : 1;
-        if (lane == 0 && x < n_act && nb > 0) {
-            constexpr uint32_t idesc_s = make_idesc(BLOCK_M, BLOCK_N, 0);
-            constexpr uint32_t idesc_pv = make_idesc(BLOCK_M, DV, 1);
-            const uint32_t t_o = tmem_base + x * 128, t_s = tmem_base + 256 + x * 64, t_q = tmem_base + 384 + x * 64;
+        const int x = __shfl_sync(0xffffffffu, warp, 0) - ISSUE_WARP;
+        if (x < n_act && nb > 0) {
+            const uint32_t t_s = tmem_base + x * 256, t_o = t_s + 128;
             // descriptors are built once; a product costs one 64-bit add on each (the low bits of a
             // descriptor are the shared-memory address in units of 16 bytes)
-            const uint64_t kdesc = make_smem_desc(base, 16);                       // + stage * STAGE_BYTES
-            const uint64_t vdesc = make_smem_desc(base + K_BYTES, BLOCK_N * 128);  // + stage * STAGE_BYTES
-            const uint64_t pdesc = make_smem_desc(sP + x * 2 * P_BYTES, 16);      // + (block % 2) * P_BYTES
-            auto issue_s = [&](int jj) {                           // S(jj); K(jj) has landed, the S buffer is free
-                const uint64_t kd = kdesc + (uint64_t)((jj % NSTAGES) * (STAGE_BYTES >> 4));
-#pragma unroll
-                for (int kk = 0; kk < DK / 16; ++kk) {
-                    // Q: 16 elements of a row = 8 columns of tensor memory; K: [half][64 keys][128 B], 32 bytes along a row
-                    const uint32_t koff = ((kk / 4) * (BLOCK_N * 128) + (kk % 4) * 32) >> 4;
-                    if (kk < QT_COLS / 16)
-                        umma_bf16_a_tmem(t_s, t_q + kk * 8, kd + koff, idesc_s, kk > 0 ? 1u : 0u);
-                    else
-                        umma_bf16(t_s, make_smem_desc(sQ + x * Cfg::kQExtra + ((kk * 16 - QT_COLS) / 64) * (BLOCK_M * 128), 16) +
-                                           (uint64_t)((kk % 4) * 2), kd + koff, idesc_s, 1u);
-                }
-                umma_commit(s_full(x));
-            };
-#ifdef AP_TIMERS
-            const bool dbg_on = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
-            const int dslot = x * 8;
-            if (dbg_on) for (int i = 0; i < 8; ++i) ap_dbg[dslot + i] = 0;
-            const long long tm0 = clock64();
-#endif
-            bool ok = mbar_wait(q_ready(x), 0, abort_flag);
-            if (ok) ok = mbar_wait(kv_full(0), 0, abort_flag);
-            if (ok) { tc_fence_after(); issue_s(0); }
-            for (int j = 0; j < nb && ok; ++j) {
-                const int st = j % NSTAGES;
-                AP_T(ta);
-                if (j + 1 < nb) {
-                    // S(j + 1): its keys have landed, and the tile's warps hold S(j) in registers
-                    ok = mbar_wait(kv_full((j + 1) % NSTAGES), (uint32_t)((j + 1) / NSTAGES) & 1, abort_flag);
-                    if (ok) ok = mbar_wait(s_free(x), (uint32_t)j & 1, abort_flag);
+            const uint64_t qdesc = make_smem_desc(sQ + x * Cfg::kQBytes, 16, 1024);
+            const uint64_t kdesc = make_smem_desc(sKV, 16, GROUP);             // + stage * STAGE_BYTES
+            const uint64_t vdesc = make_smem_desc(sKV + V_AT, V_HALF, GROUP);
+            constexpr uint32_t idesc_pv = make_idesc(BLOCK_M, DV, 1);
+            constexpr uint32_t idesc_s = make_idesc(BLOCK_M, BLOCK_N, 0);
+            bool ok = mbar_wait_warp(q_ready(x), 0, abort_flag);
+            // S runs two blocks ahead of PV: a group that has written P(j) finds S(j + 2) finished
+            for (int n = 0; n < nb + 2 && ok; ++n) {
+                if (n < nb) {
+                    AP_EV(0, n);
+                    ok = mbar_wait_warp(kv_full(n % NSTAGES), (uint32_t)(n / NSTAGES) & 1, abort_flag);
+                    AP_EV(15, n);
+                    if (ok && n > 0) ok = mbar_wait_warp(s_free(x), (uint32_t)(n - 1) & 1, abort_flag);   // S(n - 1) is in registers
                     if (!ok) break;
                     tc_fence_after();
-                    AP_T(ta2);
-                    issue_s(j + 1);
-                    AP_T(ta3);
-                    AP_ACC(dslot + 1, ta, ta2); AP_ACC(dslot + 2, ta2, ta3);
-                }
-                AP_T(tb);
-                ok = mbar_wait(p_full(x, j & 1), (uint32_t)(j >> 1) & 1, abort_flag);   // P(j) is in shared memory
-                if (!ok) break;
-                tc_fence_after();
-                AP_T(tc);
-                const uint64_t vd = vdesc + (uint64_t)(st * (STAGE_BYTES >> 4));
+                    AP_EV(1, n);
+                    const uint64_t kd = kdesc + (uint64_t)((n % NSTAGES) * (STAGE_BYTES >> 4));
 #pragma unroll
-                for (int kk = 0; kk < BLOCK_N / 16; ++kk)
-                    umma_bf16(t_o, pdesc + (uint64_t)((j & 1) * (P_BYTES >> 4) + kk * 2), vd + (uint64_t)(kk * 128), idesc_pv,
-                              kk > 0 ? 1u : (j > 0 ? 1u : 0u));
-                umma_commit(pv_done(x, j & 1));                    // O holds block j; that P buffer is free
-                umma_commit(kv_empty(st));                         // this tile has read K and V of the stage
-                AP_T(td);
-                AP_ACC(dslot + 3, tb, tc); AP_ACC(dslot + 4, tc, td);
+                    for (int kk = 0; kk < DK / 16; ++kk) {
+                        const uint64_t qoff = ((kk / 4) * (BLOCK_M * 128) + (kk % 4) * 32) >> 4;
+                        const uint64_t koff = ((kk / 4) * K_HALF + (kk % 4) * 32) >> 4;
+                        umma_ss(t_s, qdesc + qoff, kd + koff, idesc_s, kk > 0 ? 1u : 0u);
+                    }
+                    umma_commit_elected(s_full(x, n & 1));
+                    AP_EV(2, n);
+                }
+                const int j = n - 2;
+                if (j >= 0) {
+                    AP_EV(3, j);
+                    ok = mbar_wait_warp(p_full(x, j & 1), (uint32_t)(j >> 1) & 1, abort_flag);    // P(j) is in tensor memory
+                    if (!ok) break;
+                    tc_fence_after();
+                    AP_EV(4, j);
+                    const uint64_t vd = vdesc + (uint64_t)((j % NSTAGES) * (STAGE_BYTES >> 4));
+#pragma unroll
+                    for (int kk = 0; kk < BLOCK_N / 16; ++kk)
+                        umma_ts(t_o, t_s + 64 + (j & 1) * 32 + kk * 8, vd + (uint64_t)(kk * (2 * GROUP >> 4)), idesc_pv,
+                                         j > 0 || kk > 0 ? 1u : 0u);
+                    umma_commit_elected(pv_done(x, j & 1));                    // O holds block j; that P buffer is free
+                    umma_commit_elected(kv_empty(j % NSTAGES));           // and this tile has read K and V of the stage
+                    AP_EV(5, j);
+                }
             }
-#ifdef AP_TIMERS
-            if (dbg_on) { ap_dbg[dslot + 0] = clock64() - tm0; ap_dbg[dslot + 5] = nb; }
-#endif
         }
-    } else if (warp >= 2 && warp <= 9) {
+    } else {
         // ------------------------------------------------- softmax / rescale / epilogue
-        const int x = (warp - 2) >> 2;                             // query tile of this warp
+        const int x = warp >> 3, g = (warp >> 2) & 1;              // query tile and group of this warp: it has blocks g, g + 2, ...
         const int q = warp & 3;                                    // TMEM lane quarter this warp may touch
         const int r = q * 32 + lane;                               // row of the tile = TMEM lane
-        const int tt = tid - 64 - x * 128;                         // 0..127 within the tile's warps
+        const int tt = tid & 127;                                  // within the group
         const int R = row0 + x * BLOCK_M + r;
         const bool tile_active = x < n_act;
         const bool rv = tile_active && R < rows_total;
         const int pr = pos0 + R / G;
         const int lo_r = p.window > 0 ? max(0, pr - p.window + 1) : 0;
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
-        const uint32_t t_o = t_row + x * 128;
-        const uint32_t t_s = t_row + 256 + x * 64;
-        const uint32_t t_q = t_row + 384 + x * 64;
-        // the query tile: this thread's row, two elements a column, into tensor memory
+        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + x * 256;
+        const uint32_t t_s = t_row, t_p = t_row + 64 + g * 32, t_o = t_row + 128;
+        // the two warps that have a row between them
+        auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + x * 4 + q) : "memory"); };
+        volatile float* mine = exchange + (x * 2 + g) * BLOCK_M + r;
+        volatile float* other = exchange + (x * 2 + (g ^ 1)) * BLOCK_M + r;
+        // the query tile: half of this thread's row into shared memory, K-major rows of 128 bytes, swizzled
         if (tile_active) {
             const bf16* src = p.q + (size_t)(q0 + R / G) * p.q_row_stride + (size_t)(kvh * G + R % G) * (DENSE ? p.d : DK);
+            uint8_t* dst = smem + x * Cfg::kQBytes + r * 128;
 #pragma unroll
-            for (int c16 = 0; c16 < QT_COLS / 32; ++c16) {
-                uint32_t v[16];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                    if (rv && (!DENSE || c16 * 32 + c * 8 < p.d)) u = *reinterpret_cast<const uint4*>(src + c16 * 32 + c * 8);
-                    v[4 * c] = u.x; v[4 * c + 1] = u.y; v[4 * c + 2] = u.z; v[4 * c + 3] = u.w;
-                }
-                tmem_st16(t_q + c16 * 16, v);
+            for (int i = 0; i < DK / 16; ++i) {
+                const int c = g * (DK / 16) + i;
+                uint4 u = make_uint4(0u, 0u, 0u, 0u);
+                if (rv && (!DENSE || c * 8 < p.d)) u = *reinterpret_cast<const uint4*>(src + c * 8);
+                *reinterpret_cast<uint4*>(dst + (c >> 3) * (BLOCK_M * 128) + (((c & 7) ^ (r & 7)) << 4)) = u;
             }
-            if constexpr (DK > QT_COLS) {                          // the columns beyond: K-major rows, swizzled as P is
-#pragma unroll
-                for (int c = 0; c < (DK - QT_COLS) / 8; ++c) {
-                    uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                    if (rv && QT_COLS + c * 8 < p.d) u = *reinterpret_cast<const uint4*>(src + QT_COLS + c * 8);
-                    *reinterpret_cast<uint4*>(gQ + x * Cfg::kQExtra + (c >> 3) * (BLOCK_M * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = u;
-                }
-                fence_async_smem();
-            }
-            tmem_st_wait();
-            tc_fence_before();
+            fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(q_ready(x));
         }
         float m_used = -INFINITY, l = 0.f;
         bool ok = true;
         const int nb_x = tile_active ? nb : 0;
-#ifdef AP_TIMERS
-        const bool dbg_on = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (warp == 2 || warp == 6) && lane == 0;
-        const int dslot = 16 + x * 8;
-        if (dbg_on) for (int i = 0; i < 8; ++i) ap_dbg[dslot + i] = 0;
-        const long long ts0 = clock64();
-#endif
-        for (int j = 0; j < nb_x && ok; ++j) {
-            const int st = j % NSTAGES;
-            const int blk = walk.block(j);
-            if (walk.ragged(j)) {
-                // value rows no query row of the CTA may see (beyond the last key, between the kept ones and the first
-                // window) are cleared, since page slots and unfetched shared memory may hold anything; the warps of both tiles
-                // do it (the same zeros), so that each tile's products wait for its own warps only.
-                ok = mbar_wait_warp(kv_full(st), (j / NSTAGES) & 1, abort_flag);
-                if (!ok) break;
-                uint8_t* gV = gbase + st * STAGE_BYTES + K_BYTES;
-                for (int idx = tt; idx < BLOCK_N * CH; idx += 128) {
-                    const int kr = idx / CH, c = idx % CH;
-                    const int n = blk * BLOCK_N + kr;
-                    if (n > hi || (n < lo_cta && n >= p.keep))
-                        *reinterpret_cast<uint4*>(gV + (c >> 3) * (BLOCK_N * 128) + kr * 128 + (((c & 7) ^ (kr & 7)) << 4)) =
-                            make_uint4(0u, 0u, 0u, 0u);
-                }
-                fence_async_smem();
-            }
-            AP_T(sa);
-            ok = mbar_wait_warp(s_full(x), (uint32_t)j & 1, abort_flag);
+        for (int j = g; j < nb_x && ok; j += 2) {
+            AP_EV(6, j);
+            ok = mbar_wait_warp(s_full(x, g), (uint32_t)(j >> 1) & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            AP_T(sb);
+            AP_EV(7, j);
+            const int n_first = walk.block(j) * BLOCK_N;
             float s[BLOCK_N];
             {
                 uint32_t v[BLOCK_N];                               // the four loads are in flight together
@@ -495,19 +461,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             tc_fence_before();                                     // the scores are in registers: the buffer may
             __syncwarp();                                          // take the next block's
             if (lane == 0) mbar_arrive(s_free(x));
-            AP_T(sc);
+            AP_EV(8, j);
             // Scores stay unscaled in registers; the scale (> 0) is folded into the exponent below.  Key
             // blocks that every row of the warp sees whole need no mask.
             // (four running maxima and, below, four partial sums: chains of 16 dependent operations, not 64)
             float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            const int n_first = blk * BLOCK_N;
-            // (rows beyond the last token have queries of zeros and are not stored: they need no mask either.  While they took
-            // the masked path, on every block, a tile that holds some took 4,850 cycles a block against 2,550: 484 tokens
-            // of 40 heads behind 1,501 cached, beside 28 decoded tokens: the layer 162 -> 144 us.)
-            if (__all_sync(0xffffffffu, !rv || (n_first + BLOCK_N - 1 <= pr && (n_first >= lo_r || n_first + BLOCK_N <= p.keep)))) {
-#pragma unroll
-                for (int i = 0; i < BLOCK_N; i += 2) m4[(i >> 1) & 3] = fmax3(m4[(i >> 1) & 3], s[i], s[i + 1]);
-            } else {
+            // (rows beyond the last token have queries of zeros and are not stored: they need no mask either)
+            if (!__all_sync(0xffffffffu, !rv || (n_first + BLOCK_N - 1 <= pr && (n_first >= lo_r || n_first + BLOCK_N <= p.keep)))) {
                 // in the block's own numbers, which are constants of the unrolled loop
                 const int last = rv ? pr - n_first : -1, low = lo_r - n_first, kept = p.keep - n_first;
                 if (p.window == 0) {
@@ -517,28 +477,58 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
 #pragma unroll
                     for (int i = 0; i < BLOCK_N; ++i) s[i] = i <= last && (i >= low || i < kept) ? s[i] : -INFINITY;
                 }
-#pragma unroll
-                for (int i = 0; i < BLOCK_N; i += 2) m4[(i >> 1) & 3] = fmax3(m4[(i >> 1) & 3], s[i], s[i + 1]);
             }
+#pragma unroll
+            for (int i = 0; i < BLOCK_N; i += 2) m4[(i >> 1) & 3] = fmax3(m4[(i >> 1) & 3], s[i], s[i + 1]);
             const float m_raw = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
             // (a cap is monotonic like the scale: the capped maximum is the cap of the raw one)
             const float m_blk = m_raw == -INFINITY ? -INFINITY
                                                    : attn_score_log2(m_raw, p.scale_log2, p.scale_over_cap, p.cap_log2);
-            // lazy rescale: only when the maximum has grown by more than the threshold (warp-uniform decision)
-            const bool grow = m_blk > m_used + RESCALE_THRESHOLD || (m_used == -INFINITY && m_blk > -INFINITY);
-            // the product of the block before last must have read the P buffer that this block writes
-            AP_T(sd);
-            if (j > 1) {
-                ok = mbar_wait_warp(pv_done(x, j & 1), (uint32_t)((j >> 1) - 1) & 1, abort_flag);
+            AP_EV(9, j);
+            // The reference that the exponentials use goes from block to block, and so from group to group.
+            if (j > 0) {
+                ok = mbar_wait_warp(ref_bar(x, g ^ 1, q), (uint32_t)((j - 1) >> 1) & 1, abort_flag);
                 if (!ok) break;
+                const float m_prev = *other;
+                if (__any_sync(0xffffffffu, m_prev != m_used)) {
+                    if (m_used != m_prev) l = m_used == -INFINITY ? 0.f : l * exp2f(m_used - m_prev);
+                    m_used = m_prev;
+                }
             }
-            AP_T(se);
+            // lazy rescale: only when the maximum has grown by more than the threshold (warp-uniform decision)
+            const float m_old = m_used;
+            const bool grow = m_blk > m_used + RESCALE_THRESHOLD || (m_used == -INFINITY && m_blk > -INFINITY);
+            if (grow) m_used = m_blk;
+            *mine = m_used;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ref_bar(x, g, q));
+            AP_EV(10, j);
+            // the product of the block before last must have read the P buffer that this block writes
+            if (j > 1) {
+                ok = mbar_wait_warp(pv_done(x, g), (uint32_t)((j >> 1) - 1) & 1, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+            }
+            if (walk.ragged(j)) {
+                // value rows no query row of the CTA may see (beyond the last key, between the kept ones and the first
+                // window) are cleared, since page slots and unfetched shared memory may hold anything; the warps of both tiles
+                // do it (the same zeros), so that each tile's products wait for its own warps only.
+                // (S(j) has read the stage's keys: its values have landed with them)
+                uint8_t* rows = gKV + (j % NSTAGES) * STAGE_BYTES + V_AT;
+                for (int idx = tt; idx < BLOCK_N * CH; idx += 128) {
+                    const int kr = idx / CH, c = idx % CH;
+                    const int n = n_first + kr;
+                    if (n > hi || (n < lo_cta && n >= p.keep))
+                        *reinterpret_cast<uint4*>(rows + (c >> 3) * V_HALF + (kr >> 3) * GROUP + (kr & 7) * 128 + (((c & 7) ^ (kr & 7)) << 4)) =
+                            make_uint4(0u, 0u, 0u, 0u);
+                }
+                fence_async_smem();
+            }
             if (__any_sync(0xffffffffu, grow)) {
-                const float m_new = grow ? m_blk : m_used;
-                const float alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - m_new);
+                const float alpha = !grow ? 1.f : m_old == -INFINITY ? 0.f : exp2f(m_old - m_used);
                 if (j > 0) {
                     // O must hold every earlier block before it is rescaled
-                    ok = mbar_wait_warp(pv_done(x, (j - 1) & 1), (uint32_t)((j - 1) >> 1) & 1, abort_flag);
+                    ok = mbar_wait_warp(pv_done(x, g ^ 1), (uint32_t)((j - 1) >> 1) & 1, abort_flag);
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll 1
@@ -547,23 +537,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                         tmem_ld16(t_o + c0, v);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * (grow ? alpha : 1.f));
+                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
                         tmem_st16(t_o + c0, v);
                     }
-                    tmem_st_wait();
-                    tc_fence_before();
                 }
-                if (grow) { l *= alpha; m_used = m_new; }
+                l *= alpha;
             }
             const float ms = m_used == -INFINITY ? 0.f : m_used;
-            if (QT == 2 && n_act == 2) {
-                // the exponentials of a block are bound by the special-function unit (16 a cycle and SM): side by side
-                // the two tiles' passes take twice as long each and leave the unit idle while both tiles do the rest
-                ok = mbar_wait_warp(turn(x, q), (uint32_t)j & 1, abort_flag);
-                if (!ok) break;
-            }
-            AP_T(sf);
-            uint8_t* prow = gP + (x * 2 + (j & 1)) * P_BYTES + r * 128;
+            AP_EV(11, j);
             // scale, subtraction and the row's sum work on pairs of float32 (one instruction a pair)
             uint64_t lsum2[2] = {0ull, 0ull};
             const bool capped = p.cap_log2 > 0.f;
@@ -575,43 +556,48 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                 for (int i = 0; i < BLOCK_N; ++i)                  // a masked score stays masked
                     s[i] = s[i] == -INFINITY ? -INFINITY : attn_tanh(s[i] * p.scale_over_cap);
             }
+            // the probabilities, two a column
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                uint32_t w[4];
+            for (int c = 0; c < 2; ++c) {
+                uint32_t w[16];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < 16; ++i) {
                     float a0, a1;
-                    unpack2(fma2(pack2(s[c * 8 + 2 * i], s[c * 8 + 2 * i + 1]), scale2, negms2), a0, a1);
+                    unpack2(fma2(pack2(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]), scale2, negms2), a0, a1);
                     const float e0 = ex2_approx(a0), e1 = ex2_approx(a1);
                     __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
                     lsum2[i & 1] = add2(lsum2[i & 1], pack2(e0, e1));
                     w[i] = *reinterpret_cast<uint32_t*>(&b2);
                 }
-                *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-                if (c == TURN_AFTER - 1 && QT == 2 && n_act == 2) {
-                    // the other tile's warp of this scheduler may begin its pass (handing over earlier, so that the
-                    // passes overlap in part, was no faster: 3 of 8 chunks 531 us, 6: 525, 8: 522 at 8,192 tokens)
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(turn(x ^ 1, q));
-                }
+                tmem_st16(t_p + c * 16, w);
             }
             {
                 float s0, s1;
                 unpack2(add2(lsum2[0], lsum2[1]), s0, s1);
                 l += s0 + s1;
             }
-            fence_async_smem();
+            tmem_st_wait();
+            tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(p_full(x, j & 1));
-            AP_T(sg);
-            AP_ACC(dslot + 1, sa, sb); AP_ACC(dslot + 2, sb, sc); AP_ACC(dslot + 3, sc, sd); AP_ACC(dslot + 4, sd, se);
-            AP_ACC(dslot + 5, se, sf); AP_ACC(dslot + 6, sf, sg);
+            if (lane == 0) mbar_arrive(p_full(x, g));
+            AP_EV(12, j);
         }
-#ifdef AP_TIMERS
-        if (dbg_on) ap_dbg[dslot + 0] = clock64() - ts0;
-#endif
-        // ---------------------------------------------------------------- epilogue
-        if (ok && nb_x > 0) ok = mbar_wait_warp(pv_done(x, (nb_x - 1) & 1), (uint32_t)((nb_x - 1) >> 1) & 1, abort_flag);
+        // ---------------------------------------------------------------- epilogue: half of the columns a group
+        // the group that does not have the last block takes the last reference; the groups' sums then meet in shared memory
+        const int gl = (nb_x - 1) & 1;                             // the group of the last block
+        if (ok && nb_x > 0 && g != gl) {
+            ok = mbar_wait_warp(ref_bar(x, gl, q), (uint32_t)((nb_x - 1) >> 1) & 1, abort_flag);
+            const float m_last = *other;
+            if (m_used != m_last) l = m_used == -INFINITY ? 0.f : l * exp2f(m_used - m_last);
+            m_used = m_last;
+            // (its own last product first: the other barrier's completion before the one that is waited for is then in the past)
+            if (ok && nb_x > 1) ok = mbar_wait_warp(pv_done(x, g), (uint32_t)((nb_x - 2) >> 1) & 1, abort_flag);
+        }
+        if (ok && nb_x > 0) ok = mbar_wait_warp(pv_done(x, gl), (uint32_t)((nb_x - 1) >> 1) & 1, abort_flag);
+        pair_sync();                                               // both have read the last references
+        *mine = l;
+        pair_sync();
+        l = g == 0 ? l + *other : *other + l;
         if (ok && nb_x > 0) {
             tc_fence_after();
             if (p.sink && l > 0.f) l += exp2f(attn_sink_log2(p.sink_val, kvh * G + R % G) - m_used);   // the sink: a key without a value
@@ -620,7 +606,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             const int dv = DENSE ? p.dv : DV;
             bf16* orow = p.out + ((size_t)(q0 + R / G) * p.nq + (kvh * G + R % G)) * dv;
 #pragma unroll 1
-            for (int c0 = 0; c0 < DV; c0 += 16) {
+            for (int c0 = g * (DV / 2); c0 < (g + 1) * (DV / 2); c0 += 16) {
                 uint32_t v[16];
                 tmem_ld16(t_o + c0, v);
                 tmem_ld_wait();
@@ -645,17 +631,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
         if (tid == 0) atomicExch(p.error_flag, 1);
         __syncthreads();
     }
-    if (warp == 1) {
+    if (warp == ISSUE_WARP) {
         __syncwarp();
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
 }
 
 template <int DK, int DV, int QT, bool DENSE>
 int launch_prefill(const CUtensorMap& tm, const CUtensorMap& tv, const CUtensorMap& tr, const PrefillParams& p, int q_tiles,
                    int B, cudaStream_t stream) {
-    constexpr int NTHREADS = QT == 2 ? 352 : 192;
+    constexpr int NTHREADS = PrefillCfg<DK, DV, QT>::kThreads;
     constexpr int smem = PrefillCfg<DK, DV, QT>::kSmem;
     auto kern = attn_prefill_tc_kernel<DK, DV, QT, DENSE>;
     static bool configured = false;
@@ -686,7 +672,7 @@ int launch_prefill_tiles(const CUtensorMap& tm, const CUtensorMap& tv, const CUt
 
 #ifdef AP_TIMERS
 TFF_API int tff_debug_ap_pair_timers(long long* out) {
-    return cudaMemcpyFromSymbol(out, ap_dbg, sizeof(long long) * 64) == cudaSuccess ? 0 : 1;
+    return cudaMemcpyFromSymbol(out, ap_dbg, sizeof(ap_dbg)) == cudaSuccess ? 0 : 1;
 }
 #endif
 
@@ -704,7 +690,7 @@ int tff_attention_prefill_launch(
     const long long rows = cache_pages * cache_layers * 2 * nkv * page_size;
     if (rows >= (1ll << 31) || num_requests > 65535 || (long long)max_q_len * (nq / nkv) > 65535ll * 256) return TFF_ERR_UNSUPPORTED;
     CUtensorMap tm;
-    if (!tff_tensor_map_2d(cache, rows, d, page_size, 64, 2, &tm)) return TFF_ERR_DRIVER;
+    if (!tff_tensor_map_kv_groups(cache, rows, d, page_size, nkv, &tm)) return TFF_ERR_DRIVER;
     PrefillParams p;
     p.q = (const bf16*)q; p.q_row_stride = nq * d;
     p.q_start = q_start; p.pos_start = pos_start; p.req_ids = req_ids;

@@ -18,6 +18,11 @@ bool tff_tensor_map_2d(const void* ptr, long long rows, long long cols, int box_
 bool tff_tensor_map_kv_page(const void* cache, long long total_rows, int head_dim, int page_size, int kv_heads,
                             CUtensorMap* out);
 
+// The same box (page_size a multiple of 8) in atoms of 8 rows x 64 columns, which the tensor core reads as an operand: shared
+// memory gets [8 rows][K, V][half], 1 KB an atom with 128-byte swizzle.  Coordinates are (0, 0, 0, 0, first K row / 8).
+bool tff_tensor_map_kv_groups(const void* cache, long long total_rows, int head_dim, int page_size, int kv_heads,
+                              CUtensorMap* out);
+
 // Device pointer to the error word (allocated and cleared at first use; nullptr on failure).
 int* tff_device_error_flag();
 
