@@ -726,6 +726,30 @@ def test_prompt_attention_when_the_running_maximum_jumps_late(ops, nq, nkv, d, p
     ops.check_errors()
 
 
+@pytest.mark.parametrize("nq,nkv,d,page,window", [(8, 2, 128, 16, 0), (8, 4, 64, 8, 0), (10, 2, 128, 64, 0), (8, 2, 64, 32, 90), (8, 2, 128, 16, 200)])
+@pytest.mark.parametrize("requests", [1, 40])
+def test_prompt_attention_of_every_number_of_key_blocks(ops, nq, nkv, d, page, window, requests):
+    """Walks of 1 to 14 blocks of 64 keys, by ones: the blocks alternate between two groups of warps, whose references and sums meet at
+    the end, and go round rings of 3 to 8 stages; one tile a CTA (few requests) and two (more tiles than SMs), the second of which may
+    hold no rows."""
+    G = nq // nkv
+    for first in range(0, 14, 1 if requests == 1 else 7):
+        new = [(17 + 5 * i) % (256 // G) + 128 // G if i % 3 else 128 // G + 1 for i in range(requests)]
+        old = [max(0, 64 * ((first + i) % 14) + 70 - n - (i % 5)) for i, n in enumerate(new)]
+        entries, tables, cache, qkv = _paged_case(nq, nkv, d, page, new, old, window, torch.bfloat16, seed=91 + first, layers=1)
+        q = qkv[:, :nq * d].contiguous()
+        T = q.shape[0]
+        bc = build_step_batch(entries, old, list(range(len(new))), [tables], "cpu")
+        bg = build_step_batch(entries, old, list(range(len(new))), [tables], DEV)
+        want = torch.empty(T, nq * d, dtype=torch.bfloat16)
+        CpuOps().attention(q, bc, bc.block_tables[0], cache, 0, page, want, nq, nkv, d, 1 / math.sqrt(d), window)
+        out = torch.full((T, nq * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.attention_bf16(q.to(DEV), bg, bg.block_tables[0], cache.to(DEV), 0, page, out, nq, nkv, d, 1 / math.sqrt(d), window)
+        assert torch.isfinite(out).all()
+        assert rel_err(out, want) < 1e-2, (first, new, old)
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("nq,nkv,new,old", [(40, 8, [300], [0]), (40, 8, [277], [0]), (40, 8, [300], [1500]),
                                             (24, 8, [150, 43], [700, 0]), (32, 8, [301], [900])])
 def test_prompt_attention_with_a_warp_on_the_masked_path_beside_warps_on_the_short_one(ops, nq, nkv, new, old):

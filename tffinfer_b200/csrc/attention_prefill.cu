@@ -3,43 +3,40 @@
 // A CTA takes one or two tiles of 128 packed query rows (row R of a request = token R / G, head
 // kvh*G + R % G) of one (request, kv head) and walks the keys in blocks of 64, once for its tiles.
 // Per tile:
-//   S = Q K^T     tcgen05.mma, M = 128, N = 64, K = head size; Q is the A operand in TENSOR MEMORY
-//                 (written there once by the tile's warps), K the B operand, K-major in
-//                 128-byte-swizzled shared memory; S (float32) in tensor memory, one buffer
-//   softmax       four warps, one thread per row: S row from TMEM (the buffer is given back as soon
-//                 as the row is in registers), causal/window mask by position, running maximum and
-//                 sum in float32, probabilities to shared memory as bfloat16 (K-major, swizzled:
-//                 the A operand of the next product)
-//   O += P V      tcgen05.mma, M = 128, N = head size, K = 64; V is the B operand in
-//                 MN-major form, exactly as TMA lays the pages down; O (float32) stays in
+//   S = Q K^T     tcgen05.mma, M = 128, N = 64, K = head size; both operands K-major in 128-byte-swizzled
+//                 shared memory; S (float32) in tensor memory, one buffer
+//   softmax       two groups of four warps, one thread per row, which take the blocks in turn: S row from
+//                 TMEM (the buffer is given back as soon as the row is in registers), causal/window mask by
+//                 position, running maximum and sum in float32, probabilities to tensor memory as bfloat16
+//                 pairs, a buffer a group
+//   O += P V      tcgen05.mma, M = 128, N = head size, K = 64; P is the A operand in TENSOR MEMORY, V the B
+//                 operand in MN-major form, exactly as TMA lays the pages down; O (float32) stays in
 //                 tensor memory for the whole key walk
 // O is rescaled only when a row's maximum has grown by more than 2^8 since the value the
 // exponentials use (the probabilities then stay below 2^8, harmless in float32/bfloat16), so
-// the read-modify-write of O in tensor memory is rare.
-//   warp 0      TMA producer: one box per (page, 64-column half, K or V) into a ring of stages
-//   warp 1      TMEM allocation (512 columns: O of tile x at 128 x, S at 256 + 64 x, Q at 384 + 64 x);
-//               issues the products of tile 0 (one lane)
-//   warps 2-5   softmax, rescale, epilogue of the first tile (TMEM lane quarter = warp % 4)
-//   warps 6-9   the same for the second tile
-//   warp 10     issues the products of the second tile (one lane)
-// What the schedule rests on (measured on a B200 with probes that only issue products): a
-// 128 x 64 x 16 product with both operands in shared memory occupies the tensor core for 48 cycles
-// (it reads 6 KB at 128 B/cycle), with A in tensor memory for the 32 its arithmetic takes; the PV
-// product takes 64.  Issuing blocks while the product before runs, and a barrier wait by an issuing
-// thread leaves the tensor core idle for 100-175 cycles unless another thread has products queued:
-// so each tile has an issuing thread of its own (two threads keep the tensor core full, measured),
-// and a tile's thread issues S(j + 1) as soon as the softmax warps have read S(j) into registers,
-// PV(j) when they have written P(j).  S(j + 1) is therefore finished long before the softmax of
-// block j is, and one S buffer a tile is enough; the columns that a second buffer took hold Q.
-// P has two buffers a tile, so that the softmax of block j does not wait for PV(j - 1).
-// With the products cheaper the kernel is bound by the exponentials: the special-function unit gives
-// 16 a cycle and SM, a 64-key block of two tiles needs 1,024 cycles of it.  Left alone the two
-// tiles fall into step (both in their exponential pass, each at half speed; then both in the rest of
-// the loop with the unit idle), so the two warps that share a scheduler (the same lane quarter of
-// the two tiles) take their exponential passes in turn, handing over through an mbarrier: one
-// tile's waits, loads and maxima then run under the other tile's exponentials (8,192 tokens:
-// 615 -> 547 us; with scale, subtraction and row sum on pairs of float32, fma.f32x2: 525).
-// A cubic on the FMA pipe for part of the exponentials made it slower at every share tried.
+// the read-modify-write of O in tensor memory is rare.  That reference goes from block to block through shared
+// memory; each group sums its own blocks' probabilities, and the two sums meet at the end.
+//   warps 0-7    softmax, rescale, epilogue of the first tile (TMEM lane quarter = warp % 4)
+//   warps 8-15   the same for the second tile
+//   then         TMA producer: one box a page brings its keys and values (both halves of 64 columns) into a ring of stages;
+//                an issuing warp for each tile, the first of which owns the tensor memory (512 columns: of tile x, S at
+//                256 x, P of the groups at 256 x + 64 and + 96, O at 256 x + 128)
+// What it rests on (cycles counted in the kernel on a B200, two tiles a CTA unless said otherwise):
+//   - A TMA box costs its producer about 110 cycles to issue.  With a box of 2 KB for every page, half, K and V, sixteen a
+//     block, the producer alone took 1,900 cycles a block and bound the kernel whatever the rest did (8,192 tokens of 32/8
+//     heads: 564 us); with one box a page, 496.
+//   - S runs two blocks ahead of PV, so a group that has written P(j) finds S(j + 2) finished; P in tensor memory leaves
+//     PV only V to read from shared memory (62 cycles for 128 x 128 x 16; with P there too 107).
+//   - The issuing warps go through their loops with all lanes, one elected lane issuing four products at a time, and with
+//     the tile's number as a constant: issued from a branch of one lane, a product cost 80 cycles instead of 48.
+//   - Queries and outputs go by whole rows: a thread that took its own row touched 32 lines with every access, 10,000 of
+//     the 20,000 cycles that a CTA spends around its walk (2,048 tokens 52 -> 46 us).
+//   - Masked or capped scores go back through tensor memory, so that the usual block has no second path whose registers
+//     meet the first one's, and a wait is one poll and one vote (1,800 -> 1,590 cycles a block; 8,192 tokens 484 -> 454 us).
+// A block of two tiles then takes 1,590 cycles, of one tile 1,050, for 1,280 (640) of products and 1,024 (512) of exponentials
+// at the 16 a cycle that the special-function unit gives; four softmax warps a scheduler hide each other's waits.  Tried
+// without gain: blocks of 128 keys whose columns two groups share, P over S (tiles fall into step: 772 us at the time against 638);
+// part of the exponentials as a polynomial on the FMA pipe (an eighth -1 %, a quarter and more slower).
 // CTAs are handed out longest walk first over all kv heads.
 // Same contract as the rows mode of attention_bf16.cu, which it replaces when the page size
 // is 8/16/32/64.
@@ -47,14 +44,14 @@
 // cache, for steps whose requests all start at position 0 (a latent attention that has made per-head keys and values of
 // a whole prompt): keys of up to 192 elements, values of up to 128, one box of 64 rows per 64 columns.  A key may lie in
 // two tensors: columns of its own head, and a part that all heads share (the rotated part of a latent attention), which is
-// then read where it is.  Tensor memory has room for 128 elements of a query row of either tile; what goes beyond
-// (columns 128 to 191) lies in shared memory, and its products take A from there.
-//  Every mbarrier wait is bounded; a timeout raises the library's error word.
+// then read where it is.
+// Every mbarrier wait is bounded; a timeout raises the library's error word.
 // Every wait lets the hardware suspend the warp: the waiting warps share their schedulers with the softmax warps
 // of the other tile, and polled they took issue slots from those (5 % of the kernel's time).
 #define TFF_SUSPENDED_WAITS
 #include "tcgen05.cuh"
 #include "attention_common.h"
+#include <type_traits>
 
 namespace {
 
@@ -80,9 +77,23 @@ constexpr int BLOCK_N = 64;
 constexpr int BARS_PER_TILE = 16;
 constexpr float RESCALE_THRESHOLD = 8.0f;       // in log2 units
 
-// the same for a whole warp: every lane gets the same answer
+// A wait of a whole warp: every lane gets the same answer, and the usual case is one poll and one vote.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        tc5::jitter();
+        return true;
+    }
+    const long long t0 = clock64();
+    for (;;) {
+        if (__all_sync(0xffffffffu, tc5::mbar_try_wait_hint(bar, parity, 2000u))) {
+            tc5::jitter();
+            return true;
+        }
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        if (__any_sync(0xffffffffu, clock64() - t0 > tc5::WAIT_LIMIT_CYCLES)) break;
+    }
+    *abort_flag = 1;
+    return false;
 }
 // A box of tff_tensor_map_kv_groups: a page's keys and values of a kv head, from its first group of 8 rows.
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int group) {
@@ -104,23 +115,40 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // The products are issued by a warp whose lanes all go through the loop, one elected lane issuing: addresses and descriptors are
-// then the same in the whole warp for the compiler too.
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// then the same in the whole warp for the compiler too.  Four products at a time, K = 64; the first starts the sum from zero
+// unless ``accumulate``.
+__device__ __forceinline__ void umma4_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "setp.eq.b32 p, 0, 0;\n\t"
+        "add.u64 a, %1, 2;\n\tadd.u64 b, %2, 2;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u64 a, %1, 4;\n\tadd.u64 b, %2, 4;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u64 a, %1, 6;\n\tadd.u64 b, %2, 6;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// The A operand from tensor memory (lane = row, one 32-bit column = two consecutive K elements), B from shared memory.
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// The A operand from tensor memory (lane = row, one 32-bit column = two consecutive K elements), B from shared memory, STEP from
+// 16 of its K to the next.
+template <int STEP>
+__device__ __forceinline__ void umma4_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 b;\n\t.reg .b32 a;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "setp.eq.b32 p, 0, 0;\n\t"
+        "add.u32 a, %1, 8;\n\tadd.u64 b, %2, %5;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, p;\n\t"
+        "add.u32 a, %1, 16;\n\tadd.u64 b, b, %5;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, p;\n\t"
+        "add.u32 a, %1, 24;\n\tadd.u64 b, b, %5;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(STEP) : "memory");
 }
 __device__ __forceinline__ void umma_commit_elected(uint32_t bar) {
     asm volatile(
@@ -173,15 +201,6 @@ __host__ __device__ constexpr uint32_t make_idesc(int m, int n, int b_mn_major) 
            ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-#ifdef AP_TIMERS
-__device__ long long ap_dbg[2 * 16 * 160];             // [tile][event][block]
-#define AP_EV(e, j) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (j) < 160 && (warp >= ISSUE_WARP || (lane == 0 && (warp & 3) == 0))) ap_dbg[(x * 16 + (e)) * 160 + (j)] = clock64(); } while (0)
-#define AP_EVL(e, j) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (j) < 160 && lane == 0) ap_dbg[(e) * 160 + (j)] = clock64(); } while (0)
-#else
-#define AP_EV(e, j)
-#define AP_EVL(e, j)
-#endif
-
 struct PrefillParams {
     int companion;                               // the decoded tokens' kernel follows and runs beside this one
     const bf16* q; int q_row_stride;
@@ -207,7 +226,6 @@ struct PrefillCfg {
     static constexpr int kBars = 2 * kStages + BARS_PER_TILE * QT;
     static constexpr int kSmem = QT * kQBytes + kStages * kStageBytes + kExchange + 8 * kBars + 16;
     static constexpr int kThreads = (8 * QT + 1 + QT) * 32;
-    static constexpr int kTmemCols = QT * 256;
     static_assert(kSmem <= 227 * 1024, "shared memory of the prompt attention kernel");
 };
 
@@ -228,6 +246,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     constexpr int GROUP = DENSE ? 1024 : (KH + VH) * 1024;                // from 8 keys to the next 8
     constexpr int K_HALF = DENSE ? BLOCK_N * 128 : 1024, V_HALF = K_HALF;  // from a half to the next
     constexpr int V_AT = DENSE ? KH * K_HALF : KH * 1024;                  // of the stage's first values
+    constexpr int TMEM_COLS = 512;                               // all of it: the allocation starts at column 0
     constexpr int LOAD_WARP = 8 * QT, ISSUE_WARP = LOAD_WARP + 1;              // behind the softmax warps
     extern __shared__ __align__(1024) uint8_t smem[];            // (the only shared memory of the kernel: it starts 1024-byte aligned)
     const uint32_t sQ = smem_u32(smem);
@@ -273,11 +292,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_cache) : "memory");
         if (DENSE) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_v) : "memory");
     }
-    if (warp == ISSUE_WARP) tmem_alloc(smem_u32((const void*)tmem_slot), Cfg::kTmemCols);
+    if (warp == ISSUE_WARP) tmem_alloc(smem_u32((const void*)tmem_slot), TMEM_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    constexpr uint32_t tmem_base = 0;
     if (p.companion) {            // the kernel behind may read what the one ahead of both wrote
         pdl_wait();
         pdl_launch_dependents();
@@ -324,6 +343,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             const int s = i % NSTAGES;
             const uint32_t round = i / NSTAGES;
             if (round > 0 && !mbar_wait_warp(kv_empty(s), (round - 1) & 1, abort_flag)) break;
+            // the queries are on their way before more than two blocks are asked for: every CTA of a wave starts with both
+            if (i == 2 && !mbar_wait_warp(q_ready(0), 0, abort_flag)) break;
             const uint32_t stage = sKV + s * STAGE_BYTES;
             const int n_first = walk.block(i) * BLOCK_N;
             if constexpr (DENSE) {
@@ -349,7 +370,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                 const unsigned mask = __ballot_sync(0xffffffffu, valid);
                 if (lane == 0) mbar_expect_tx(kv_full(s), (uint32_t)__popc(mask) * (uint32_t)(GROUP << (p.page_shift - 3)));
                 __syncwarp();
-                AP_EVL(13, i);
                 if (valid) {
                     const long long row = ((((long long)held * p.cache_layers + p.layer) * 2) * p.nkv + kvh) << p.page_shift;
                     tma_load_5d(stage + (uint32_t)((lane - (first & 31)) * (GROUP << (p.page_shift - 3))), &tm_cache, kv_full(s), (int)(row >> 3));
@@ -358,8 +378,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
         }
     } else if (warp >= ISSUE_WARP) {
         // -------------------------------------------------------------- MMA issuers, one per tile
-        const int x = __shfl_sync(0xffffffffu, warp, 0) - ISSUE_WARP;
-        if (x < n_act && nb > 0) {
+        auto issue = [&](auto tile) {
+            constexpr int x = decltype(tile)::value;
+            if (x >= n_act || nb == 0) return;
             const uint32_t t_s = tmem_base + x * 256, t_o = t_s + 128;
             // descriptors are built once; a product costs one 64-bit add on each (the low bits of a
             // descriptor are the shared-memory address in units of 16 bytes)
@@ -370,43 +391,37 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             constexpr uint32_t idesc_s = make_idesc(BLOCK_M, BLOCK_N, 0);
             bool ok = mbar_wait_warp(q_ready(x), 0, abort_flag);
             // S runs two blocks ahead of PV: a group that has written P(j) finds S(j + 2) finished
+            uint32_t phase = 0;
+            int st = 0, st_pv = 0;                                 // stages of S(n) and of PV(n - 2)
             for (int n = 0; n < nb + 2 && ok; ++n) {
                 if (n < nb) {
-                    AP_EV(0, n);
-                    ok = mbar_wait_warp(kv_full(n % NSTAGES), (uint32_t)(n / NSTAGES) & 1, abort_flag);
-                    AP_EV(15, n);
+                    ok = mbar_wait_warp(kv_full(st), phase, abort_flag);
                     if (ok && n > 0) ok = mbar_wait_warp(s_free(x), (uint32_t)(n - 1) & 1, abort_flag);   // S(n - 1) is in registers
                     if (!ok) break;
                     tc_fence_after();
-                    AP_EV(1, n);
-                    const uint64_t kd = kdesc + (uint64_t)((n % NSTAGES) * (STAGE_BYTES >> 4));
+                    const uint64_t kd = kdesc + (uint64_t)(st * (STAGE_BYTES >> 4));
 #pragma unroll
-                    for (int kk = 0; kk < DK / 16; ++kk) {
-                        const uint64_t qoff = ((kk / 4) * (BLOCK_M * 128) + (kk % 4) * 32) >> 4;
-                        const uint64_t koff = ((kk / 4) * K_HALF + (kk % 4) * 32) >> 4;
-                        umma_ss(t_s, qdesc + qoff, kd + koff, idesc_s, kk > 0 ? 1u : 0u);
-                    }
+                    for (int h = 0; h < KH; ++h)
+                        umma4_ss(t_s, qdesc + (uint64_t)(h * (BLOCK_M * 128) >> 4), kd + (uint64_t)(h * K_HALF >> 4), idesc_s, h > 0 ? 1u : 0u);
                     umma_commit_elected(s_full(x, n & 1));
-                    AP_EV(2, n);
+                    if (++st == NSTAGES) { st = 0; phase ^= 1; }
                 }
                 const int j = n - 2;
                 if (j >= 0) {
-                    AP_EV(3, j);
                     ok = mbar_wait_warp(p_full(x, j & 1), (uint32_t)(j >> 1) & 1, abort_flag);    // P(j) is in tensor memory
                     if (!ok) break;
                     tc_fence_after();
-                    AP_EV(4, j);
-                    const uint64_t vd = vdesc + (uint64_t)((j % NSTAGES) * (STAGE_BYTES >> 4));
-#pragma unroll
-                    for (int kk = 0; kk < BLOCK_N / 16; ++kk)
-                        umma_ts(t_o, t_s + 64 + (j & 1) * 32 + kk * 8, vd + (uint64_t)(kk * (2 * GROUP >> 4)), idesc_pv,
-                                         j > 0 || kk > 0 ? 1u : 0u);
+                    const uint64_t vd = vdesc + (uint64_t)(st_pv * (STAGE_BYTES >> 4));
+                    umma4_ts<(2 * GROUP >> 4)>(t_o, t_s + 64 + (j & 1) * 32, vd, idesc_pv, j > 0 ? 1u : 0u);
                     umma_commit_elected(pv_done(x, j & 1));                    // O holds block j; that P buffer is free
-                    umma_commit_elected(kv_empty(j % NSTAGES));           // and this tile has read K and V of the stage
-                    AP_EV(5, j);
+                    umma_commit_elected(kv_empty(st_pv));                  // and this tile has read K and V of the stage
+                    if (++st_pv == NSTAGES) st_pv = 0;
                 }
             }
-        }
+        };
+        // (a copy of the loop a tile: with its number known, a product's operands are constants and one register a stage)
+        if (warp == ISSUE_WARP) issue(std::integral_constant<int, 0>());
+        else if constexpr (QT == 2) issue(std::integral_constant<int, 1>());
     } else {
         // ------------------------------------------------- softmax / rescale / epilogue
         const int x = warp >> 3, g = (warp >> 2) & 1;              // query tile and group of this warp: it has blocks g, g + 2, ...
@@ -424,85 +439,94 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
         auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + x * 4 + q) : "memory"); };
         volatile float* mine = exchange + (x * 2 + g) * BLOCK_M + r;
         volatile float* other = exchange + (x * 2 + (g ^ 1)) * BLOCK_M + r;
-        // the query tile: half of this thread's row into shared memory, K-major rows of 128 bytes, swizzled
+        // Rows of 32 go to and from global memory by whole rows: a lane that took its own row would touch 32 lines with every
+        // access (the queries in and the outputs out were 10,000 of a CTA's 20,000 cycles around the key walk).
+        const int tok = R / G, head = kvh * G + R % G;
+        const int rows_left = min(32, rows_total - (R - lane));            // rows of this warp's 32 that exist
+        // the query tile: half of the columns of this warp's rows into shared memory, K-major rows of 128 bytes, swizzled
         if (tile_active) {
-            const bf16* src = p.q + (size_t)(q0 + R / G) * p.q_row_stride + (size_t)(kvh * G + R % G) * (DENSE ? p.d : DK);
-            uint8_t* dst = smem + x * Cfg::kQBytes + r * 128;
+            constexpr int RC = DK / 16;                            // 16-byte chunks of a row that a group has
+            uint4 u[RC];
 #pragma unroll
-            for (int i = 0; i < DK / 16; ++i) {
-                const int c = g * (DK / 16) + i;
-                uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                if (rv && (!DENSE || c * 8 < p.d)) u = *reinterpret_cast<const uint4*>(src + c * 8);
-                *reinterpret_cast<uint4*>(dst + (c >> 3) * (BLOCK_M * 128) + (((c & 7) ^ (r & 7)) << 4)) = u;
+            for (int i = 0; i < RC; ++i) {
+                const int row = (i * 32 + lane) / RC, c = g * RC + (i * 32 + lane) % RC;
+                const int t = __shfl_sync(0xffffffffu, tok, row), h = __shfl_sync(0xffffffffu, head, row);
+                u[i] = make_uint4(0u, 0u, 0u, 0u);
+                if (row < rows_left && (!DENSE || c * 8 < p.d))
+                    u[i] = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + t) * p.q_row_stride + (size_t)h * (DENSE ? p.d : DK) + c * 8);
+            }
+            uint8_t* dst = smem + x * Cfg::kQBytes + q * 32 * 128;
+#pragma unroll
+            for (int i = 0; i < RC; ++i) {
+                const int row = (i * 32 + lane) / RC, c = g * RC + (i * 32 + lane) % RC;
+                *reinterpret_cast<uint4*>(dst + (c >> 3) * (BLOCK_M * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = u[i];
             }
             fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(q_ready(x));
         }
+        const float scale_log2 = p.cap_log2 > 0.f ? p.cap_log2 : p.scale_log2;
         float m_used = -INFINITY, l = 0.f;
         bool ok = true;
         const int nb_x = tile_active ? nb : 0;
         for (int j = g; j < nb_x && ok; j += 2) {
-            AP_EV(6, j);
             ok = mbar_wait_warp(s_full(x, g), (uint32_t)(j >> 1) & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            AP_EV(7, j);
             const int n_first = walk.block(j) * BLOCK_N;
-            float s[BLOCK_N];
-            {
-                uint32_t v[BLOCK_N];                               // the four loads are in flight together
+            // Masked or capped scores are written back over the raw ones, so that the pass below is the same for every block (with the
+            // scores of two paths meeting in registers, 64 moves a block).  Rows beyond the last token have queries of zeros and
+            // are not stored: they need no mask.  With a cap the scores become tanh(s * scale / cap) and the multiplier of the
+            // exponent cap * log2(e).
+            const bool masked = !__all_sync(0xffffffffu, !rv || (n_first + BLOCK_N - 1 <= pr && (n_first >= lo_r || n_first + BLOCK_N <= p.keep)));
+            if (masked || p.cap_log2 > 0.f) {
+                // (in the block's own numbers, which are constants of the unrolled loops)
+                const int last = rv ? pr - n_first : BLOCK_N, low = lo_r - n_first, kept = p.keep - n_first;
+                uint32_t v[BLOCK_N];
 #pragma unroll
                 for (int h = 0; h < BLOCK_N / 16; ++h) tmem_ld16(t_s + h * 16, v + h * 16);
                 tmem_ld_wait();
+                if (p.cap_log2 > 0.f) {
 #pragma unroll
-                for (int i = 0; i < BLOCK_N; ++i) s[i] = __uint_as_float(v[i]);
+                    for (int i = 0; i < BLOCK_N; ++i) v[i] = __float_as_uint(attn_tanh(__uint_as_float(v[i]) * p.scale_over_cap));
+                }
+                if (p.window == 0) {
+#pragma unroll
+                    for (int i = 0; i < BLOCK_N; ++i) v[i] = i <= last ? v[i] : 0xff800000u;                             // -infinity
+                } else if (masked) {
+#pragma unroll
+                    for (int i = 0; i < BLOCK_N; ++i) v[i] = i <= last && (i >= low || i < kept) ? v[i] : 0xff800000u;
+                }
+#pragma unroll
+                for (int h = 0; h < BLOCK_N / 16; ++h) tmem_st16(t_s + h * 16, v + h * 16);
+                tmem_st_wait();
             }
+            uint32_t s[BLOCK_N];
+#pragma unroll
+            for (int h = 0; h < BLOCK_N / 16; ++h) tmem_ld16(t_s + h * 16, s + h * 16);       // the four loads are in flight together
+            tmem_ld_wait();
             tc_fence_before();                                     // the scores are in registers: the buffer may
             __syncwarp();                                          // take the next block's
             if (lane == 0) mbar_arrive(s_free(x));
-            AP_EV(8, j);
-            // Scores stay unscaled in registers; the scale (> 0) is folded into the exponent below.  Key
-            // blocks that every row of the warp sees whole need no mask.
+            // Scores stay unscaled in registers; the scale (> 0) is folded into the exponent below.
             // (four running maxima and, below, four partial sums: chains of 16 dependent operations, not 64)
             float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            // (rows beyond the last token have queries of zeros and are not stored: they need no mask either)
-            if (!__all_sync(0xffffffffu, !rv || (n_first + BLOCK_N - 1 <= pr && (n_first >= lo_r || n_first + BLOCK_N <= p.keep)))) {
-                // in the block's own numbers, which are constants of the unrolled loop
-                const int last = rv ? pr - n_first : -1, low = lo_r - n_first, kept = p.keep - n_first;
-                if (p.window == 0) {
 #pragma unroll
-                    for (int i = 0; i < BLOCK_N; ++i) s[i] = i <= last ? s[i] : -INFINITY;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < BLOCK_N; ++i) s[i] = i <= last && (i >= low || i < kept) ? s[i] : -INFINITY;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < BLOCK_N; i += 2) m4[(i >> 1) & 3] = fmax3(m4[(i >> 1) & 3], s[i], s[i + 1]);
-            const float m_raw = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-            // (a cap is monotonic like the scale: the capped maximum is the cap of the raw one)
-            const float m_blk = m_raw == -INFINITY ? -INFINITY
-                                                   : attn_score_log2(m_raw, p.scale_log2, p.scale_over_cap, p.cap_log2);
-            AP_EV(9, j);
-            // The reference that the exponentials use goes from block to block, and so from group to group.
+            for (int i = 0; i < BLOCK_N; i += 2) m4[(i >> 1) & 3] = fmax3(m4[(i >> 1) & 3], __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+            const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * scale_log2;
+            // The reference that the exponentials use goes from block to block, and so from group to group.  It is moved, and O and the
+            // sums with it, only when the maximum has grown by more than the threshold: a decision of the whole warp.
+            float m_prev = m_used;
             if (j > 0) {
                 ok = mbar_wait_warp(ref_bar(x, g ^ 1, q), (uint32_t)((j - 1) >> 1) & 1, abort_flag);
                 if (!ok) break;
-                const float m_prev = *other;
-                if (__any_sync(0xffffffffu, m_prev != m_used)) {
-                    if (m_used != m_prev) l = m_used == -INFINITY ? 0.f : l * exp2f(m_used - m_prev);
-                    m_used = m_prev;
-                }
+                m_prev = *other;
             }
-            // lazy rescale: only when the maximum has grown by more than the threshold (warp-uniform decision)
-            const float m_old = m_used;
-            const bool grow = m_blk > m_used + RESCALE_THRESHOLD || (m_used == -INFINITY && m_blk > -INFINITY);
-            if (grow) m_used = m_blk;
-            *mine = m_used;
-            __syncwarp();
+            const bool grow = m_blk > m_prev + RESCALE_THRESHOLD || (m_prev == -INFINITY && m_blk > -INFINITY);
+            const float m_new = grow ? m_blk : m_prev;
+            *mine = m_new;
+            const bool moved = __any_sync(0xffffffffu, m_new != m_used);
             if (lane == 0) mbar_arrive(ref_bar(x, g, q));
-            AP_EV(10, j);
             // the product of the block before last must have read the P buffer that this block writes
             if (j > 1) {
                 ok = mbar_wait_warp(pv_done(x, g), (uint32_t)((j >> 1) - 1) & 1, abort_flag);
@@ -524,13 +548,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                 }
                 fence_async_smem();
             }
-            if (__any_sync(0xffffffffu, grow)) {
-                const float alpha = !grow ? 1.f : m_old == -INFINITY ? 0.f : exp2f(m_old - m_used);
-                if (j > 0) {
+            if (moved) {
+                const bool any_grow = __any_sync(0xffffffffu, grow);
+                if (any_grow && j > 0) {
                     // O must hold every earlier block before it is rescaled
                     ok = mbar_wait_warp(pv_done(x, g ^ 1), (uint32_t)((j - 1) >> 1) & 1, abort_flag);
                     if (!ok) break;
                     tc_fence_after();
+                    const float alpha = !grow ? 1.f : m_prev == -INFINITY ? 0.f : exp2f(m_prev - m_new);
 #pragma unroll 1
                     for (int c0 = 0; c0 < DV; c0 += 16) {
                         uint32_t v[16];
@@ -541,21 +566,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                         tmem_st16(t_o + c0, v);
                     }
                 }
-                l *= alpha;
+                if (m_new != m_used) l = m_used == -INFINITY ? 0.f : l * exp2f(m_used - m_new);
+                m_used = m_new;
             }
             const float ms = m_used == -INFINITY ? 0.f : m_used;
-            AP_EV(11, j);
             // scale, subtraction and the row's sum work on pairs of float32 (one instruction a pair)
             uint64_t lsum2[2] = {0ull, 0ull};
-            const bool capped = p.cap_log2 > 0.f;
-            // with a cap, the scores become tanh(s * scale / cap) first and the multiplier of the exponent cap * log2(e)
-            const uint64_t scale2 = capped ? pack2(p.cap_log2, p.cap_log2) : pack2(p.scale_log2, p.scale_log2),
-                           negms2 = pack2(-ms, -ms);
-            if (capped) {
-#pragma unroll
-                for (int i = 0; i < BLOCK_N; ++i)                  // a masked score stays masked
-                    s[i] = s[i] == -INFINITY ? -INFINITY : attn_tanh(s[i] * p.scale_over_cap);
-            }
+            const uint64_t scale2 = pack2(scale_log2, scale_log2), negms2 = pack2(-ms, -ms);
             // the probabilities, two a column
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -563,7 +580,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     float a0, a1;
-                    unpack2(fma2(pack2(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]), scale2, negms2), a0, a1);
+                    unpack2(fma2(pack2(__uint_as_float(s[c * 32 + 2 * i]), __uint_as_float(s[c * 32 + 2 * i + 1])), scale2, negms2), a0, a1);
                     const float e0 = ex2_approx(a0), e1 = ex2_approx(a1);
                     __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
                     lsum2[i & 1] = add2(lsum2[i & 1], pack2(e0, e1));
@@ -580,7 +597,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full(x, g));
-            AP_EV(12, j);
         }
         // ---------------------------------------------------------------- epilogue: half of the columns a group
         // the group that does not have the last block takes the last reference; the groups' sums then meet in shared memory
@@ -600,26 +616,40 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
         l = g == 0 ? l + *other : *other + l;
         if (ok && nb_x > 0) {
             tc_fence_after();
-            if (p.sink && l > 0.f) l += exp2f(attn_sink_log2(p.sink_val, kvh * G + R % G) - m_used);   // the sink: a key without a value
+            if (p.sink && l > 0.f) l += exp2f(attn_sink_log2(p.sink_val, head) - m_used);   // the sink: a key without a value
             float inv = l > 0.f ? 1.f / l : 0.f;
-            if (p.gate && rv) inv *= __ldcg(p.gate + (size_t)(q0 + R / G) * p.nq + (kvh * G + R % G));
-            const int dv = DENSE ? p.dv : DV;
-            bf16* orow = p.out + ((size_t)(q0 + R / G) * p.nq + (kvh * G + R % G)) * dv;
-#pragma unroll 1
-            for (int c0 = g * (DV / 2); c0 < (g + 1) * (DV / 2); c0 += 16) {
-                uint32_t v[16];
-                tmem_ld16(t_o + c0, v);
-                tmem_ld_wait();
-                if (rv) {
-                    uint32_t w[8];
+            if (p.gate && rv) inv *= __ldcg(p.gate + (size_t)(q0 + tok) * p.nq + head);
+            // through shared memory, where the queries lay (every S is finished), 32 rows of half a row's columns a warp
+            constexpr int RC = DV / 16;
+            uint8_t* rows = smem + x * Cfg::kQBytes + (g * 4 + q) * (32 * DV);
+            auto cell = [&](int row, int c) { return rows + row * DV + ((c ^ (RC == 8 ? row & 7 : (row >> 1) & 3)) << 4); };
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(v[2 * i]) * inv, __uint_as_float(v[2 * i + 1]) * inv);
+            for (int half = 0; half < RC / 4; ++half) {
+                uint32_t v[32];
+                tmem_ld16(t_o + g * (DV / 2) + half * 32, v);
+                tmem_ld16(t_o + g * (DV / 2) + half * 32 + 16, v + 16);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(v[8 * c + 2 * i]) * inv, __uint_as_float(v[8 * c + 2 * i + 1]) * inv);
                         w[i] = *reinterpret_cast<uint32_t*>(&b2);
                     }
-                    if (!DENSE || c0 < dv) *reinterpret_cast<uint4*>(orow + c0) = make_uint4(w[0], w[1], w[2], w[3]);
-                    if (!DENSE || c0 + 8 < dv) *reinterpret_cast<uint4*>(orow + c0 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                    *reinterpret_cast<uint4*>(cell(lane, half * 4 + c)) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
+            }
+            __syncwarp();
+            const int dv = DENSE ? p.dv : DV;
+#pragma unroll
+            for (int i = 0; i < RC; ++i) {
+                const int row = (i * 32 + lane) / RC, c = (i * 32 + lane) % RC;
+                const int t = __shfl_sync(0xffffffffu, tok, row), h = __shfl_sync(0xffffffffu, head, row);
+                const int col = (g * RC + c) * 8;
+                if (row < rows_left && (!DENSE || col < dv))
+                    *reinterpret_cast<uint4*>(p.out + ((size_t)(q0 + t) * p.nq + h) * dv + col) =
+                        *reinterpret_cast<const uint4*>(cell(row, c));
             }
         }
     }
@@ -634,7 +664,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     if (warp == ISSUE_WARP) {
         __syncwarp();
         tc_fence_after();
-        tmem_dealloc(tmem_base, Cfg::kTmemCols);
+        tmem_dealloc(tmem_base, TMEM_COLS);
     }
 }
 
@@ -653,11 +683,9 @@ int launch_prefill(const CUtensorMap& tm, const CUtensorMap& tv, const CUtensorM
     return tff_launch_pdl(kern, dim3(p.nkv, q_tiles, B), dim3(NTHREADS), (size_t)smem, stream, tm, tv, tr, p);
 }
 
-// Two query tiles a CTA share one walk over the keys and take turns at the exponentials: a pair of tiles costs
-// 1.08 times what a single tile costs (512 new tokens behind 3,584 cached ones, 32/8 heads: 92 us as 128 CTAs
-// of one tile, 100 us as 64 CTAs of two).  So single tiles only while they all run at once, one an SM; as soon
-// as they would not, pairs (1,536 tokens from scratch: 61 us against 74 as single tiles; 2,816 tokens: 114
-// against 149; 1,536 behind 2,048 cached ones: 123 against 160).
+// Two query tiles a CTA share one walk over the keys: a block takes 1,590 cycles for a pair of tiles, 1,050 for a single one.  So
+// single tiles while they all run at once, one an SM; as soon as they would not, pairs, which get through 1.3 times as many
+// tiles in the same time.
 template <int DK, int DV, bool DENSE>
 int launch_prefill_tiles(const CUtensorMap& tm, const CUtensorMap& tv, const CUtensorMap& tr, const PrefillParams& p,
                          int max_q_len, int B, cudaStream_t stream) {
@@ -669,12 +697,6 @@ int launch_prefill_tiles(const CUtensorMap& tm, const CUtensorMap& tv, const CUt
 }
 
 }  // namespace
-
-#ifdef AP_TIMERS
-TFF_API int tff_debug_ap_pair_timers(long long* out) {
-    return cudaMemcpyFromSymbol(out, ap_dbg, sizeof(ap_dbg)) == cudaSuccess ? 0 : 1;
-}
-#endif
 
 // Prompt-portion attention on tcgen05.  TFF_ERR_UNSUPPORTED when the shape is not one it takes
 // (head size 64/128, page size 8/16/32/64).
