@@ -60,8 +60,9 @@ using tc5::smem_u32;
 using tc5::mbar_init;
 using tc5::mbar_expect_tx;
 using tc5::mbar_arrive;
-using tc5::mbar_try_wait;
-using tc5::mbar_wait;
+using tc5::mbar_wait_warp;
+using tc5::umma4_bf16_elected;
+using tc5::umma_commit_elected;
 using tc5::tma_load_2d;
 using tc5::fence_async_smem;
 using tc5::tmem_alloc;
@@ -77,24 +78,6 @@ constexpr int BLOCK_N = 64;
 constexpr int BARS_PER_TILE = 16;
 constexpr float RESCALE_THRESHOLD = 8.0f;       // in log2 units
 
-// A wait of a whole warp: every lane gets the same answer, and the usual case is one poll and one vote.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
-        tc5::jitter();
-        return true;
-    }
-    const long long t0 = clock64();
-    for (;;) {
-        if (__all_sync(0xffffffffu, tc5::mbar_try_wait_hint(bar, parity, 2000u))) {
-            tc5::jitter();
-            return true;
-        }
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
-        if (__any_sync(0xffffffffu, clock64() - t0 > tc5::WAIT_LIMIT_CYCLES)) break;
-    }
-    *abort_flag = 1;
-    return false;
-}
 // A box of tff_tensor_map_kv_groups: a page's keys and values of a kv head, from its first group of 8 rows.
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int group) {
     asm volatile(
@@ -114,25 +97,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// The products are issued by a warp whose lanes all go through the loop, one elected lane issuing: addresses and descriptors are
-// then the same in the whole warp for the compiler too.  Four products at a time, K = 64; the first starts the sum from zero
-// unless ``accumulate``.
-__device__ __forceinline__ void umma4_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "setp.eq.b32 p, 0, 0;\n\t"
-        "add.u64 a, %1, 2;\n\tadd.u64 b, %2, 2;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
-        "add.u64 a, %1, 4;\n\tadd.u64 b, %2, 4;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
-        "add.u64 a, %1, 6;\n\tadd.u64 b, %2, 6;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The A operand from tensor memory (lane = row, one 32-bit column = two consecutive K elements), B from shared memory, STEP from
+// Four products as umma4_bf16_elected's with the A operand from tensor memory (lane = row, one 32-bit column = two consecutive K elements), B from shared memory, STEP from
 // 16 of its K to the next.
 template <int STEP>
 __device__ __forceinline__ void umma4_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -150,13 +115,6 @@ __device__ __forceinline__ void umma4_ts(uint32_t d_tmem, uint32_t a_tmem, uint6
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(STEP) : "memory");
 }
-__device__ __forceinline__ void umma_commit_elected(uint32_t bar) {
-    asm volatile(
-        "{\n\t.reg .pred e;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
-}
-
 // Pairs of float32 in a 64-bit register: fma and add on a pair issue as one instruction on sm_100.
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t r;
@@ -402,7 +360,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                     const uint64_t kd = kdesc + (uint64_t)(st * (STAGE_BYTES >> 4));
 #pragma unroll
                     for (int h = 0; h < KH; ++h)
-                        umma4_ss(t_s, qdesc + (uint64_t)(h * (BLOCK_M * 128) >> 4), kd + (uint64_t)(h * K_HALF >> 4), idesc_s, h > 0 ? 1u : 0u);
+                        umma4_bf16_elected(t_s, qdesc + (uint64_t)(h * (BLOCK_M * 128) >> 4), kd + (uint64_t)(h * K_HALF >> 4), idesc_s, h > 0 ? 1u : 0u);
                     umma_commit_elected(s_full(x, n & 1));
                     if (++st == NSTAGES) { st = 0; phase ^= 1; }
                 }

@@ -107,6 +107,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
     pdl_launch_dependents();
 
     if (warp == 0) {
+        uint32_t first = 0;
         if (lane == 0) {
             // ------------------------------------------------------ TMA producer
             // The weights do not depend on the kernel before this one: the weight tiles of
@@ -139,6 +140,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
             pdl_wait();
             for (int i = 0; i < pre; ++i)
                 tma_load_2d(base + i * Cfg::kStageBytes + x_off, tm_x, full_bar(i), pre_k[i], pre_xrow[i]);
+            first = pre;
+        }
+        {
+            const uint32_t pre = __shfl_sync(0xffffffffu, first, 0);
             SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
             uint32_t n = 0;
             bool ok = true;
@@ -147,19 +152,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
                 if (grouped) { const int g = lane_group[it.tile % n_lane_tiles]; if (g < 0) continue; goff = g * group_rows; }
                 const int lrow = (it.tile % n_lane_tiles) * BM, crow = (it.tile / n_lane_tiles) * BN + goff;
                 for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
-                    if (n < (uint32_t)pre) continue;                 // already requested above
+                    if (n < pre) continue;                           // already requested above
                     const int s = n % STAGES;
                     const uint32_t round = n / STAGES;
-                    if (!mbar_wait(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
                     const uint32_t a_dst = base + s * Cfg::kStageBytes;
-                    mbar_expect_tx(full_bar(s), Cfg::kStageBytes);
-                    tma_load_2d(a_dst, &tm_lane, full_bar(s), kb * BK, lrow);
-                    tma_load_2d(a_dst + BM * BK * 2, &tm_col, full_bar(s), kb * BK, crow);
+                    mbar_expect_tx_elected(full_bar(s), Cfg::kStageBytes);
+                    tma_load_2d_elected(a_dst, &tm_lane, full_bar(s), kb * BK, lrow);
+                    tma_load_2d_elected(a_dst + BM * BK * 2, &tm_col, full_bar(s), kb * BK, crow);
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             // -------------------------------------------------------- MMA issuer
             constexpr uint32_t idesc = make_idesc(BM, BN);
             SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
@@ -169,26 +174,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
             while (ok && it.next()) {
                 if (grouped && lane_group[it.tile % n_lane_tiles] < 0) continue;
                 const uint32_t acc = seg & 1, use = seg >> 1;
-                if (use > 0 && !mbar_wait(tempty_bar(acc), (use - 1) & 1, abort_flag)) break;   // epilogue has drained it
+                if (use > 0 && !mbar_wait_warp(tempty_bar(acc), (use - 1) & 1, abort_flag)) break;   // epilogue has drained it
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * Cfg::kAccCols;
                 for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
                     const int s = n % STAGES;
                     const uint32_t round = n / STAGES;
-                    if (!mbar_wait(full_bar(s), round & 1, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(s), round & 1, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = base + s * Cfg::kStageBytes;
                     const uint64_t adesc = make_smem_desc(a_addr);
                     const uint64_t bdesc = make_smem_desc(a_addr + BM * BK * 2);
-#pragma unroll
-                    for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-                        // 16 K-elements = 32 bytes = 2 descriptor units further along the swizzled row
-                        umma_bf16(d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc,
-                                  (kb > it.kb0 || kk > 0) ? 1u : 0u);
-                    }
-                    umma_commit(empty_bar(s));          // the stage is free once these MMAs have read it
+                    umma4_bf16_elected(d_tmem, adesc, bdesc, idesc, kb > it.kb0 ? 1u : 0u);
+                    umma_commit_elected(empty_bar(s));          // the stage is free once these MMAs have read it
                 }
-                if (ok) umma_commit(tfull_bar(acc));    // this segment's accumulators are complete
+                if (ok) umma_commit_elected(tfull_bar(acc));    // this segment's accumulators are complete
                 ++seg;
             }
         }

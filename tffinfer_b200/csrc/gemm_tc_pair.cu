@@ -63,7 +63,9 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // a TMA load of one CTA of a pair; ``bar`` is a shared::cluster address and may lie in the other CTA
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int x, int y) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        "{\n\t.reg .pred e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
         ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t cols) {
@@ -73,17 +75,27 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t cols
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-__device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// four products, as umma4_bf16_elected
+__device__ __forceinline__ void umma4_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "setp.eq.b32 p, 0, 0;\n\t"
+        "add.u64 a, %1, 2;\n\tadd.u64 b, %2, 2;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u64 a, %1, 4;\n\tadd.u64 b, %2, 4;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u64 a, %1, 6;\n\tadd.u64 b, %2, 6;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // arrives, once the products issued so far are done, at the barrier at this shared-memory offset in
 // every CTA of the cluster named by ``mask``
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                 "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
                  ::"r"(bar), "h"(mask) : "memory");
 }
 
@@ -135,7 +147,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a,     // activations
     pdl_launch_dependents();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             // ------------------------------------------------------ TMA producer (both CTAs)
             pdl_wait();
             SegIterSlices it(n_tiles, kbt, stream_k, cluster_id, n_clusters);
@@ -147,9 +159,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a,     // activations
                 for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
                     const int s = n % STAGES;
                     const uint32_t round = n / STAGES;
-                    if (round > 0 && !mbar_wait(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
+                    if (round > 0 && !mbar_wait_warp(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
                     const uint32_t first_full = map_to_cta(full_bar(s), 0);
-                    if (rank == 0) mbar_expect_tx(full_bar(s), 2 * P_STAGE_BYTES);     // both CTAs' tiles of the stage
+                    if (rank == 0) mbar_expect_tx_elected(full_bar(s), 2 * P_STAGE_BYTES);     // both CTAs' tiles of the stage
                     const uint32_t a_dst = base + s * P_STAGE_BYTES;
                     tma_load_2d_pair(a_dst, &tm_a, first_full, kb * BK, arow);
                     tma_load_2d_pair(a_dst + BM * BK * 2, &tm_w, first_full, kb * BK, wrow);
@@ -157,7 +169,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a,     // activations
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             // -------------------------------------------------------- MMA issuer (first CTA)
             constexpr uint32_t idesc = make_idesc(2 * BM, PBN);
             SegIterSlices it(n_tiles, kbt, stream_k, cluster_id, n_clusters);
@@ -165,21 +177,18 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a,     // activations
             bool ok = true;
             while (ok && it.next()) {
                 const uint32_t acc = seg & 1, use = seg >> 1;
-                if (use > 0 && !mbar_wait(tempty_bar(acc), (use - 1) & 1, abort_flag)) break;   // both epilogues have drained it
+                if (use > 0 && !mbar_wait_warp(tempty_bar(acc), (use - 1) & 1, abort_flag)) break;   // both epilogues have drained it
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * PBN;
                 for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
                     const int s = n % STAGES;
                     const uint32_t round = n / STAGES;
-                    if (!mbar_wait(full_bar(s), round & 1, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(s), round & 1, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = base + s * P_STAGE_BYTES;
                     const uint64_t adesc = make_smem_desc(a_addr);
                     const uint64_t bdesc = make_smem_desc(a_addr + BM * BK * 2);
-#pragma unroll
-                    for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                        umma_bf16_pair(d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc,
-                                       (kb > it.kb0 || kk > 0) ? 1u : 0u);
+                    umma4_bf16_pair(d_tmem, adesc, bdesc, idesc, kb > it.kb0 ? 1u : 0u);
                     umma_commit_pair(empty_bar(s), 3);       // the stage is free in both CTAs once these products have read it
                 }
                 if (ok) umma_commit_pair(tfull_bar(acc), 3); // this segment's accumulators are complete in both CTAs

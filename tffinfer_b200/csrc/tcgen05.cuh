@@ -150,6 +150,71 @@ static __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
 }
 static __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// The same for a whole warp: every lane gets the same answer, and the usual case is one poll and one vote.
+static __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        jitter();
+        return true;
+    }
+    const long long t0 = clock64();
+    for (;;) {
+#ifdef TFF_SUSPENDED_WAITS
+        const uint32_t done = mbar_try_wait_hint(bar, parity, 2000u);
+#else
+        const uint32_t done = mbar_try_wait(bar, parity);
+#endif
+        if (__all_sync(0xffffffffu, done)) {
+            jitter();
+            return true;
+        }
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        if (__any_sync(0xffffffffu, clock64() - t0 > WAIT_LIMIT_CYCLES)) break;
+    }
+    *abort_flag = 1;
+    return false;
+}
+
+// Loads and products issued by a warp whose lanes all go through the loop, one elected lane issuing.  Addresses and descriptors
+// are then the same in the whole warp for the compiler too; from a branch that one lane takes, each of them is moved to the
+// uniform registers that the instruction wants first, and a product of 128 x 64 x 16 cost 80 cycles to issue instead of the 48 that
+// it runs.
+static __device__ __forceinline__ void mbar_expect_tx_elected(uint32_t bar, uint32_t bytes) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
+}
+static __device__ __forceinline__ void tma_load_2d_elected(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int x, int y) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+        ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+// Four products, K = 64 of a K-major tile with 128-byte swizzle (16 elements of K are 2 descriptor units); the first starts the sum
+// from zero unless ``accumulate``.
+static __device__ __forceinline__ void umma4_bf16_elected(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "setp.eq.b32 p, 0, 0;\n\t"
+        "add.u64 a, %1, 2;\n\tadd.u64 b, %2, 2;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u64 a, %1, 4;\n\tadd.u64 b, %2, 4;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+        "add.u64 a, %1, 6;\n\tadd.u64 b, %2, 6;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+static __device__ __forceinline__ void umma_commit_elected(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128
 // bytes, groups of 8 rows 1024 bytes apart (stride byte offset), descriptor version 1,
 // layout type 2 (SWIZZLE_128B).  Addresses and offsets are in units of 16 bytes.
