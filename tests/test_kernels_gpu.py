@@ -203,6 +203,32 @@ def test_gemm_f32_in_every_tile_width_and_sharing_of_k(ops, M, N, K, adt, wdt):
     ops.check_errors()
 
 
+@pytest.mark.parametrize("M,N,K", [(95, 128, 64), (96, 129, 576), (97, 200, 1544), (193, 130, 2051)])
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+def test_gemm_f32_tiles_of_96_rows(ops, M, N, K, adt, wdt):
+    """The same bits as tiles of 16 rows, which the test above holds to their bound."""
+    a, w, res = g((M, K), adt, 23).to(DEV), g((N, K), wdt, 24, 0.05).to(DEV), g((M, N), torch.float32, 25).to(DEV)
+    kb = -(-K // 64)
+    for slices in {1, -(-kb // (4 if kb < 16 else 8))}:
+        out, few = res.clone(), res.clone()
+        ops.gemm_simt(a, w, out, out, plan=96 | (slices << 16))
+        ops.gemm_simt(a, w, few, few, plan=16 | (1 << 16))
+        assert torch.equal(out, few), slices
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("slices", [1, 3])
+def test_gemm_f32_more_rows_than_have_their_terms_made_at_a_time(ops, slices):
+    """256 MB of terms are 384 rows of K = 116,512: the rows behind them take a pass of their own."""
+    M, N, K = 389, 40, 116512
+    a, w, res = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV), torch.randn(M, N, device=DEV)
+    out, few = res.clone(), res.clone()
+    ops.gemm_simt(a, w, out, out, plan=96 | (slices << 16))
+    ops.gemm_simt(a, w, few, few, plan=16 | (slices << 16))
+    assert torch.equal(out, few)
+    ops.check_errors()
+
+
 def test_gemm_f32_single_products(ops):
     """One product an output, of significands whose terms are as large as they get.  The terms left out come to at most
     2 x 2^-8 x 2^-17 (and 2^-34) of the two powers of two, the sum of the levels is rounded twice (2^-24, and 2^-24 of the 2^-7 that the

@@ -14,20 +14,24 @@
 // them in the same order): its value does not depend on what else is in the batch.  An element whose result is not
 // finite is computed once more as a plain sum of products, since a split of an infinity has no meaning.
 //
-// What bounds it.  Few rows: the latency of the memory, since registers hold only the two K blocks (64 KB) on their way while the
-// threads split, and not all of them: at 72 to 80 registers a thread the float32 forms spill 50 to 105 bytes (4 rows of the 8B shape's
-// gate/up product, 403 MB: 91 us = 4.4 TB/s; down 58 us; as float32 FMAs, one order of summation a thread, 1.4 ms each).  Asking the L2 for the weights one chunk ahead made it slower (102 us).  Many rows: shared memory, which
-// takes 6 bytes an element from the split and feeds six products, beside the products themselves (512 rows of gate/up 0.71 ms,
-// 145 TFLOP/s; without the products 0.48, without the loads 0.45; FMAs at most 70).  Off 64-bit arithmetic
+// What bounds it.  Few rows: 128 weight rows x 64 of K (32 KB) a CTA in 0.6 to 0.7 us where the memory would give them in 0.74: the walk
+// through registers to tensor memory just keeps up (4 rows of the 8B shape's gate/up product, 403 MB: 80 us = 5 TB/s, down 54; with the
+// weights' loads in registers and their terms in shared memory 87 and 58).  Many rows: the six products, 1,152 clocks a K block of 96 rows
+// at their own rate and about 1,900 here, of which some 150 are the issuing warp's wait and the rest the warps that split beside it
+// (536 rows of q/k/v 134 us, of the output projection 107, against 222 and 200 before: both operands' terms then went through shared memory,
+// 96 KB written and 160 KB read a K block of 128 rows, two stages of them).  So the weights' terms are the A operand in
+// TENSOR MEMORY, which costs shared memory nothing, and from 64 rows on the activations' terms are made once, by a kernel of their own
+// (3 us), and come by TMA.  Off 64-bit arithmetic
 // (2-norm, random operands) by 2.6e-8 at K = 1, 3.1e-8 at 8, 7.0e-8 at 64, 2.3e-7 at 512, 4.8e-7 at 1,024 and 4,096; a chain of FMAs over
 // all of K is by 2.6e-8, 5.4e-8, 1.4e-7, 3.9e-7, 5.7e-7 and 1.1e-6.
 //
-//   warps 1-16   read 8 elements of a row at a time from global memory, one or two K blocks ahead, split them and write
-//                the terms to shared memory as 128-byte-swizzled K-major tiles
-//   warp 0       issues the products (M = 128 weight rows on the lanes of tensor memory, BN activation rows as columns; the
+//   warp 0       loads: the weights as they are stored, and the activations' terms, by TMA (ragged rows: the warps below read for themselves)
+//   warp 1       issues the products (M = 128 weight rows on the lanes of tensor memory, BN activation rows as columns; the
 //                terms of the activations lie one behind the other, so one instruction takes a term of the weights
 //                times up to 256 columns of them)
-//   warps 17-20  (17-24 when BN = 128) add the chunks' sums, in tensor memory again, and write the result
+//   next 8 or 16 split the weights: a thread takes 16 of K of a row at a time to the lane of tensor memory that is the row's
+//   next 4       (few rows, ragged rows) split the activations into 128-byte-swizzled K-major tiles
+//   last 4 to 16 add the chunks' sums in registers, 32 columns a warp, and write the result
 #define TFF_SUSPENDED_WAITS
 #include "tcgen05.cuh"
 
@@ -40,61 +44,90 @@ using namespace tc5;
 // 2.3e-7 from K = 256 on, the chain by 2.9e-7 at 256.  Short sums so take chunks of 4, long ones half as many drains.
 __host__ __device__ constexpr int chunk_blocks(int kbt) { return kbt < 16 ? 4 : 8; }
 
-template <int BN, int NA, int NW> struct F32Cfg {
-    static constexpr int kWPlane = BM * BK * 2, kAPlane = BN * BK * 2;
-    static constexpr int kStageBytes = NW * kWPlane + NA * kAPlane;
-    static constexpr int kFit = (220 * 1024) / kStageBytes;
-    static constexpr int kStages = kFit > 4 ? 4 : kFit;
-    static constexpr int kLevels = 3;               // one operand at least has three terms
+template <int BN, int NA, int NW, bool VEC> struct F32Cfg {
     static_assert(NA == 3 || NW == 3, "a split operand");
-    // tensor memory: one or two buffers of the levels' sums, then the running sum of the chunks
-    static constexpr int kBufCols = kLevels * BN;
-    static constexpr int kBufs = 2 * kBufCols + BN <= 512 ? 2 : 1;
-    static constexpr int kSumCol = kBufs * kBufCols;
-    static constexpr int kNeedCols = kSumCol + BN;
-    static constexpr int kTmemCols = kNeedCols <= 32 ? 32 : kNeedCols <= 64 ? 64 : kNeedCols <= 128 ? 128 : kNeedCols <= 256 ? 256 : 512;
-    // 512 threads read and split.  Few activation rows: two groups of 256 take K blocks in turn, so that two blocks are on
-    // their way from memory; many: all 512 share a block, whose registers would not fit 256.
-    static constexpr int kGroups = BN <= 32 ? 2 : 1, kConv = 512 / kGroups;
-    static constexpr int kEpiGroups = BN >= 128 ? 2 : 1;           // groups of 4 epilogue warps; each takes BN / kEpiGroups columns
-    static constexpr int kThreads = 32 + 512 + 128 * kEpiGroups;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
-    static_assert(kStages >= 2 && kNeedCols <= 512, "the configuration does not fit an SM");
+    static constexpr int kRawBytes = BM * BK * (NW == 3 ? 4 : 2);   // a K block of the weights as they are stored
+    static constexpr int kAPlane = BN * BK * 2, kABytes = NA * kAPlane;
+    static constexpr int kAStages = BN <= 32 ? 6 : BN <= 96 ? 3 : 2;
+    // activations that come as their terms, by TMA: bfloat16 ones of whole rows are their own, else tiles of many rows have them made by a kernel ahead
+    // (split in here they were split again for every 128 weight rows, from loads of which only one K block was on its way)
+    static constexpr bool kPlanes = BN >= 64 || (VEC && NA == 1);
+    static constexpr int kRawFit = (220 * 1024 - kAStages * kABytes) / kRawBytes;
+    static constexpr int kRawStages = kRawFit > 6 ? 6 : kRawFit;
+    // tensor memory: buffers of the levels' sums, then a ring of the weights' terms, a slot a K block (half a one when BN = 128) and in
+    // it 16 of K in 8 columns, a term's behind one another.  A wait of the issuing warp costs the tensor core some 150 clocks, so it
+    // waits once a slot.
+    static constexpr int kLevels = 3, kBufCols = kLevels * BN, kBufs = BN <= 32 ? 2 : 1;
+    static constexpr int kSlotsABlock = BN <= 96 ? 1 : 2, kSlotSteps = BK / UMMA_K / kSlotsABlock;
+    static constexpr int kTermCols = 8 * kSlotSteps, kSlotCols = NW * kTermCols, kRingCol = kBufs * kBufCols;
+    static constexpr int kFit = (512 - kRingCol) / kSlotCols, kSlots = kFit > 4 ? 4 : kFit;
+    static constexpr int kNeedCols = kRingCol + kSlots * kSlotCols;
+    static constexpr int kTmemCols = kNeedCols <= 128 ? 128 : kNeedCols <= 256 ? 256 : 512;
+    static constexpr int kAWarps = kPlanes ? 0 : 4;                 // split the activations
+    static constexpr int kCols = BN < 32 ? BN : 32;                 // columns of an epilogue warp
+    static constexpr int kEpiWarps = BN / kCols * 4;
+    // Groups of four warps that split the weights, each a quarter or a half of EVERY K block: a barrier tells a phase from the one
+    // before only, so a group that left K blocks out could take a stage whose load of before is still on its way for its own.
+    static constexpr int kWGroups = 30 - kAWarps - kEpiWarps >= 16 && kSlotsABlock == 1 ? 4 : 2, kGroupSteps = BK / UMMA_K / kWGroups;
+    static constexpr int kWWarps = 4 * kWGroups;
+    static constexpr int kFirstA = 2 + kWWarps, kFirstEpi = kFirstA + kAWarps, kThreads = 32 * (kFirstEpi + kEpiWarps);
+    static constexpr int kSmemBytes = kRawStages * kRawBytes + kAStages * kABytes + 1024 /*alignment slack*/ + 512 /*barriers*/;
+    static_assert(kRawStages >= 2 && kSlots >= 2 && kNeedCols <= 512 && kThreads <= 1024, "the configuration does not fit an SM");
 };
 
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
-        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st1(uint32_t taddr, uint32_t r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%1], {%0};" ::"r"(r), "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+}
+// Two products of 16 of K: A from tensor memory (lane = row, one 32-bit column = two consecutive K elements), B from shared memory.
+__device__ __forceinline__ void umma2_ts(uint32_t d0, uint32_t a0, uint64_t b0, uint32_t idesc0, uint32_t acc0,
+                                         uint32_t d1, uint32_t a1, uint64_t b1, uint32_t idesc1, uint32_t acc1) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %9, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%5], [%6], %7, %8, q;\n\t}"
+        ::"r"(d0), "r"(a0), "l"(b0), "r"(idesc0), "r"(acc0), "r"(d1), "r"(a1), "l"(b1), "r"(idesc1), "r"(acc1) : "memory");
+}
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_2d_elected(const CUtensorMap* tm, int x, int y) {
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                 "@e cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];\n\t}" ::"l"(tm), "r"(x), "r"(y) : "memory");
+}
 
-// 8 consecutive elements of a row as float32; elements at or behind ``left`` are zeros (left counts from p).  The activations may have
-// been written by the kernel ahead and are read past the first-level cache.  CONST: the weights, which no kernel of a step writes, on
-// the read-only path, where they take no room in that cache.
-template <typename T, bool VEC, bool CONST>
+// 8 consecutive elements of a row; elements at or behind ``left`` are zeros (left counts from p).  The activations may have
+// been written by the kernel ahead and are read past the first-level cache.
+template <typename T, bool VEC>
 __device__ __forceinline__ void load8(const T* p, int left, uint32_t* r) {
     if constexpr (VEC) {                             // rows are multiples of 8 elements and aligned: all of the 8 or none
         if (left <= 0) {
 #pragma unroll
             for (int i = 0; i < (sizeof(T) == 4 ? 8 : 4); ++i) r[i] = 0u;
         } else if constexpr (sizeof(T) == 4) {
-            if constexpr (CONST)
-                asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                             : "l"(p));
-            else
-                asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                             : "l"(p) : "memory");
+            asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                         : "l"(p) : "memory");
         } else {
-            if constexpr (CONST)
-                asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p));
-            else
-                asm volatile("ld.global.cg.v4.b32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
+            asm volatile("ld.global.cg.v4.b32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
         }
     } else {
         auto one = [&](int i) { return i < left ? __float_as_uint(ldcg_f32(p + i)) : 0u; };
@@ -117,6 +150,23 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {      // rounded 
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// a and b less the two bfloat16 numbers of t
+__device__ __forceinline__ void less2(uint32_t t, float& a, float& b) {
+    asm("{\n\t.reg .b16 x, y, minus_one;\n\t"
+        "mov.b32 {x, y}, %2;\n\t"
+        "mov.b16 minus_one, 0xBF80;\n\t"
+        "fma.rn.f32.bf16 %0, x, minus_one, %0;\n\t"
+        "fma.rn.f32.bf16 %1, y, minus_one, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(t));
+}
+// The terms of two elements, a and b, each term's two side by side.
+__device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+    h = pack2(a, b);                                 // (the differences are exact)
+    less2(h, a, b);
+    m = pack2(a, b);
+    less2(m, a, b);
+    l = pack2(a, b);
+}
+
 // The terms of 8 elements, 16 bytes a plane, ``plane`` bytes apart.
 template <typename T>
 __device__ __forceinline__ void split_store(const uint32_t* r, uint32_t dst, uint32_t plane) {
@@ -125,13 +175,7 @@ __device__ __forceinline__ void split_store(const uint32_t* r, uint32_t dst, uin
     } else {
         uint32_t h[4], m[4], l[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {                // (the differences are exact)
-            const float a = __uint_as_float(r[2 * i]), b = __uint_as_float(r[2 * i + 1]);
-            h[i] = pack2(a, b);
-            const float ra = a - __uint_as_float(h[i] << 16), rb = b - __uint_as_float(h[i] & 0xffff0000u);
-            m[i] = pack2(ra, rb);
-            l[i] = pack2(ra - __uint_as_float(m[i] << 16), rb - __uint_as_float(m[i] & 0xffff0000u));
-        }
+        for (int i = 0; i < 4; ++i) split2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]), h[i], m[i], l[i]);
         st_shared16(dst, h);
         st_shared16(dst + plane, m);
         st_shared16(dst + 2 * plane, l);
@@ -191,22 +235,29 @@ struct Unit {
 };
 
 template <int BN, typename TA, typename TW, bool VEC>
-__global__ void __launch_bounds__(F32Cfg<BN, sizeof(TA) == 4 ? 3 : 1, sizeof(TW) == 4 ? 3 : 1>::kThreads, 1)
-gemm_f32_kernel(const TA* A, const TW* W, void* out, int out_bf16, const float* residual,
+__global__ void __launch_bounds__(F32Cfg<BN, sizeof(TA) == 4 ? 3 : 1, sizeof(TW) == 4 ? 3 : 1, VEC>::kThreads, 1)
+gemm_f32_kernel(const __grid_constant__ CUtensorMap tm_w,     // weights, boxes of 128 bytes x 128 rows (VEC only)
+                const __grid_constant__ CUtensorMap tm_a,     // the activations' terms, boxes of 64 x BN, one behind the other (kPlanes only)
+                const TA* A, const TW* W, void* out, int out_bf16, const float* residual,
                 float* __restrict__ ws, int M, int N, int K, const Share sh, int* error_flag) {
     constexpr int NA = sizeof(TA) == 4 ? 3 : 1, NW = sizeof(TW) == 4 ? 3 : 1;
-    using Cfg = F32Cfg<BN, NA, NW>;
-    constexpr int STAGES = Cfg::kStages, BUFS = Cfg::kBufs;
+    using Cfg = F32Cfg<BN, NA, NW, VEC>;
+    constexpr int RAW = Cfg::kRawStages, ASTAGES = Cfg::kAStages, SLOTS = Cfg::kSlots, BUFS = Cfg::kBufs;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t bars = base + STAGES * Cfg::kStageBytes;
-    auto full_bar = [&](int s) { return bars + 8u * s; };
-    auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
-    auto tfull_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
-    auto tempty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
-    volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen_base + STAGES * Cfg::kStageBytes + 8 * (2 * STAGES + 4));
+    const uint32_t a_base = base + RAW * Cfg::kRawBytes, bars = a_base + ASTAGES * Cfg::kABytes;
+    auto raw_full = [&](int s) { return bars + 8u * s; };
+    auto raw_empty = [&](int s) { return bars + 8u * (RAW + s); };
+    auto a_full = [&](int s) { return bars + 8u * (2 * RAW + s); };
+    auto a_empty = [&](int s) { return bars + 8u * (2 * RAW + ASTAGES + s); };
+    auto w_full = [&](int s) { return bars + 8u * (2 * (RAW + ASTAGES) + s); };
+    auto w_empty = [&](int s) { return bars + 8u * (2 * (RAW + ASTAGES) + SLOTS + s); };
+    auto tfull_bar = [&](int a) { return bars + 8u * (2 * (RAW + ASTAGES + SLOTS) + a); };
+    auto tempty_bar = [&](int a) { return bars + 8u * (2 * (RAW + ASTAGES + SLOTS) + 2 + a); };
+    volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen_base + (bars - base) + 8 * (2 * (RAW + ASTAGES + SLOTS) + 4));
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    static_assert(8 * (2 * (RAW + ASTAGES + SLOTS) + 4) + 8 <= 512, "room for the barriers");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kbt = (K + BK - 1) / BK;
@@ -214,207 +265,333 @@ gemm_f32_kernel(const TA* A, const TW* W, void* out, int out_bf16, const float* 
     const int units = (N + BM - 1) / BM * sh.slices * tiles_m;             // the launcher has checked that it fits
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), Cfg::kConv / 32); mbar_init(empty_bar(s), 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 4 * Cfg::kEpiGroups); }
+        for (int s = 0; s < RAW; ++s) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), Cfg::kWWarps); }
+        for (int s = 0; s < ASTAGES; ++s) { mbar_init(a_full(s), Cfg::kPlanes ? 1 : Cfg::kAWarps); mbar_init(a_empty(s), 1); }
+        for (int s = 0; s < SLOTS; ++s) { mbar_init(w_full(s), Cfg::kWWarps / Cfg::kSlotsABlock); mbar_init(w_empty(s), 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), Cfg::kEpiWarps); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (VEC) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
+        if (Cfg::kPlanes) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_a) : "memory");
     }
-    if (warp == 0) tmem_alloc(smem_u32((const void*)tmem_slot), Cfg::kTmemCols);
+    if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), Cfg::kTmemCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    const uint32_t ring = tmem_base + Cfg::kRingCol;
     pdl_launch_dependents();
 
     if (warp == 0) {
-        if (lane == 0) {
-            // -------------------------------------------------------- products
-            uint32_t n = 0, chunk_no = 0;
-            bool ok = true;
-            for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
-                const Unit it(u, tiles_m, sh, kbt, BN);
-                for (int c0 = it.kb0; ok && c0 < it.kb1; c0 += sh.chunk, ++chunk_no) {
-                    const uint32_t buf = chunk_no % BUFS, use = chunk_no / BUFS;
-                    if (use > 0 && !mbar_wait(tempty_bar(buf), (use - 1) & 1, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t d = tmem_base + buf * Cfg::kBufCols;
-                    const int c1 = min(c0 + sh.chunk, it.kb1);
-                    for (int kb = c0; kb < c1; ++kb, ++n) {
-                        const int s = n % STAGES;
-                        if (!mbar_wait(full_bar(s), (n / STAGES) & 1, abort_flag)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t w_addr = base + s * Cfg::kStageBytes, a_addr = w_addr + NW * Cfg::kWPlane;
-#pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-                            // term i of the weights times terms 0 .. count-1 of the activations: levels i .. i+count-1
-#pragma unroll
-                            for (int i = 0; i < NW; ++i) {
-                                constexpr int kCols = Cfg::kLevels * BN;
-                                const int cols = (kCols - i * BN) < NA * BN ? (kCols - i * BN) : NA * BN;
-                                const uint64_t wd = make_smem_desc(w_addr + i * Cfg::kWPlane) + (uint64_t)(kk * 2);
-#pragma unroll
-                                for (int c = 0; c < cols; c += 256) {
-                                    const int w = (cols - c) < 256 ? (cols - c) : 256;
-                                    const uint64_t ad = make_smem_desc(a_addr + c * BK * 2) + (uint64_t)(kk * 2);
-                                    // the first product on a level starts it from zero: with three terms of the activations all
-                                    // levels with i = 0, with one term every level with its own i
-                                    const bool fresh = kb == c0 && kk == 0 && (NA == 1 || i == 0);
-                                    umma_bf16(d + (uint32_t)(i * BN + c), wd, ad, make_idesc(BM, w), fresh ? 0u : 1u);
-                                }
-                            }
-                        }
-                        umma_commit(empty_bar(s));
-                    }
-                    if (ok) umma_commit(tfull_bar(buf));
-                }
-            }
-        }
-    } else if (warp <= 16) {
-        // ------------------------------------------------- loads and splits
-        constexpr int CT = Cfg::kConv, GROUPS = Cfg::kGroups, STRIDE = CT / 8;   // rows between a thread's items
-        constexpr int W_ITEMS = BM * 8 / CT;                                 // 8-element items of a K block a thread
-        constexpr int A_ITEMS = (BN * 8 + CT - 1) / CT;
-        constexpr int WR = NW == 3 ? 8 : 4, AR = NA == 3 ? 8 : 4;            // registers an item
-        const int group = (threadIdx.x - 32) / CT, t = (threadIdx.x - 32) % CT;
-        const int row = t >> 3, oct = t & 7;                                 // item q: row + STRIDE * q
-        const uint32_t cell = (uint32_t)row * 128u + (uint32_t)((oct ^ (row & 7)) << 4);
-        uint32_t wr[W_ITEMS][WR], ar[A_ITEMS][AR];
-        int u = blockIdx.x;
-        Unit it(u, tiles_m, sh, kbt, BN);
-        int kb = it.kb0;
-        const TW* wp;                                                        // this thread's first item of the K block, and how many
-        const TA* ap;                                                        // rows and elements of the operands lie from there on
-        int w_rows, a_rows, left;
-        auto aim = [&]() {
-            left = K - (kb * BK + oct * 8);
-            wp = W + ((size_t)(it.n0 + row) * K + (kb * BK + oct * 8));
-            ap = A + ((size_t)(it.m0 + row) * K + (kb * BK + oct * 8));
-            w_rows = N - it.n0 - row;
-            a_rows = min(M - it.m0, BN) - row;
-        };
-        const size_t pitch = (size_t)STRIDE * K;
-        auto load_w = [&](int q) { load8<TW, VEC, true>(wp + q * pitch, STRIDE * q < w_rows ? left : 0, wr[q]); };
-        auto load_a = [&](int q) { load8<TA, VEC, false>(ap + q * pitch, STRIDE * q < a_rows ? left : 0, ar[q]); };
-        auto has_a = [&](int q) { return (q + 1) * STRIDE <= BN || row + q * STRIDE < BN; };
-        auto step = [&]() {                                                  // to the next K block of the CTA
-            if (++kb >= it.kb1) {
-                u += gridDim.x;
-                if (u < units) { it = Unit(u, tiles_m, sh, kbt, BN); kb = it.kb0; }
-            }
-        };
-        for (int g = 0; g < group; ++g) if (u < units) step();
-        if (u < units) {
+        if constexpr (VEC || Cfg::kPlanes) {
+            // ------------------------------------------------- the weights as they are, the activations' terms
+            constexpr int HALF = 128 / (int)sizeof(TW), BOXES = BK / HALF;
+            int u = blockIdx.x, kb = -1;
+            uint32_t n = 0;
             // The L2 may fetch the first weights while the kernel ahead still runs; they are read behind it, since an operand of this
             // path may have been written by whatever came just before.
-            aim();
+            for (int ahead = 0; VEC && ahead < RAW && u < units; ++ahead) {
+                const Unit it(u, tiles_m, sh, kbt, BN);
+                if (kb < 0) kb = it.kb0;
 #pragma unroll
-            for (int q = 0; q < W_ITEMS; ++q)
-                if (STRIDE * q < w_rows && left > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp + q * pitch));
+                for (int b = 0; b < BOXES; ++b) tma_prefetch_2d_elected(&tm_w, kb * BK + b * HALF, it.n0);
+                if (++kb >= it.kb1) { u += gridDim.x; kb = -1; }
+            }
             pdl_wait();
+            bool ok = true;
+            for (u = blockIdx.x; ok && u < units; u += gridDim.x) {
+                const Unit it(u, tiles_m, sh, kbt, BN);
+                for (kb = it.kb0; kb < it.kb1; ++kb, ++n) {
+                    if constexpr (VEC) {
+                        const int s = n % RAW;
+                        const uint32_t round = n / RAW;
+                        if (round > 0 && !mbar_wait_warp(raw_empty(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
+                        mbar_expect_tx_elected(raw_full(s), Cfg::kRawBytes);
 #pragma unroll
-            for (int q = 0; q < W_ITEMS; ++q) load_w(q);
+                        for (int b = 0; b < BOXES; ++b)
+                            tma_load_2d_elected(base + s * Cfg::kRawBytes + b * (BM * 128), &tm_w, raw_full(s), kb * BK + b * HALF, it.n0);
+                    }
+                    if constexpr (Cfg::kPlanes) {
+                        const int t = n % ASTAGES;
+                        const uint32_t a_round = n / ASTAGES;
+                        if (a_round > 0 && !mbar_wait_warp(a_empty(t), (a_round - 1) & 1, abort_flag)) { ok = false; break; }
+                        mbar_expect_tx_elected(a_full(t), Cfg::kABytes);
+                        // (rows of a box behind the last one are the next term's: columns that nobody reads)
 #pragma unroll
-            for (int q = 0; q < A_ITEMS; ++q) load_a(q);
-            for (uint32_t n = group;; n += GROUPS) {
-                const int s = n % STAGES;
-                const uint32_t round = n / STAGES;
-                if (round > 0 && !mbar_wait(empty_bar(s), (round - 1) & 1, abort_flag)) break;
-                const uint32_t w_dst = base + s * Cfg::kStageBytes + cell, a_dst = w_dst + NW * Cfg::kWPlane;
-                // the group's next K block: an item's registers are filled again as soon as they are stored
-#pragma unroll
-                for (int g = 0; g < GROUPS; ++g) if (u < units) step();
-                const bool more = u < units;
-                if (more) aim();
-#pragma unroll
-                for (int q = 0; q < W_ITEMS; ++q) {
-                    split_store<TW>(wr[q], w_dst + q * STRIDE * 128, Cfg::kWPlane);
-                    if (more) load_w(q);
-                }
-#pragma unroll
-                for (int q = 0; q < A_ITEMS; ++q) {
-                    if (has_a(q)) {
-                        split_store<TA>(ar[q], a_dst + q * STRIDE * 128, Cfg::kAPlane);
-                        if (more) load_a(q);
+                        for (int j = 0; j < NA; ++j)
+                            tma_load_2d_elected(a_base + t * Cfg::kABytes + j * Cfg::kAPlane, &tm_a, a_full(t), kb * BK, j * M + it.m0);
                     }
                 }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full_bar(s));
-                if (!more) break;
             }
         }
-    } else {
-        // ------------------------------------------------------------ sums
-        constexpr int COLS = BN / Cfg::kEpiGroups;
-        const int q = warp & 3, first_col = ((warp - 17) >> 2) * COLS;
-        const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16) + first_col;
-        pdl_wait();
-        uint32_t chunk_no = 0;
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ products
+        uint32_t n = 0, chunk_no = 0;
         bool ok = true;
         for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
             const Unit it(u, tiles_m, sh, kbt, BN);
-            const int n = it.n0 + q * 32 + lane;
+            for (int c0 = it.kb0; ok && c0 < it.kb1; c0 += sh.chunk, ++chunk_no) {
+                const uint32_t buf = chunk_no % BUFS, use = chunk_no / BUFS;
+                if (use > 0 && !mbar_wait_warp(tempty_bar(buf), (use - 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t d = tmem_base + buf * Cfg::kBufCols;
+                const int c1 = min(c0 + sh.chunk, it.kb1);
+                for (int kb = c0; ok && kb < c1; ++kb, ++n) {
+                    const int s = n % ASTAGES;
+                    const uint64_t adesc = make_smem_desc(a_base + s * Cfg::kABytes);
+#pragma unroll
+                    for (int part = 0; part < Cfg::kSlotsABlock; ++part) {
+                        const uint32_t slot_no = n * Cfg::kSlotsABlock + part, slot = slot_no % SLOTS;
+                        // (the warps that fill a slot have waited for the activations of its K block)
+                        if (!mbar_wait_warp(w_full(slot), (slot_no / SLOTS) & 1, abort_flag)) { ok = false; break; }
+                        tc_fence_after();
+#pragma unroll
+                        for (int step = 0; step < Cfg::kSlotSteps; ++step) {
+                            const int kk = part * Cfg::kSlotSteps + step;
+                            const uint32_t w0 = ring + slot * Cfg::kSlotCols + step * 8, w1 = w0 + Cfg::kTermCols, w2 = w1 + Cfg::kTermCols;
+                            const uint32_t more = kb > c0 || kk > 0 ? 1u : 0u;       // the first product on a level starts it from zero
+                            // term i of the weights times terms 0 .. of the activations, which lie one behind the other: levels i ..
+                            const uint64_t ad = adesc + (uint64_t)(kk * 2);
+                            if constexpr (NA == 3) {
+                                constexpr int PART = 3 * BN <= 256 ? 3 * BN : 3 * BN / 2;
+                                // the largest come last of a K block, so that the tensor core is busy for longer while the next slot is waited for
+                                if (NW == 3 && kk == 3)
+                                    umma2_ts(d + 2 * BN, w2, ad, make_idesc(BM, BN), 1u, d + BN, w1, ad, make_idesc(BM, 2 * BN), 1u);
+                                if constexpr (PART < 3 * BN)
+                                    umma2_ts(d, w0, ad, make_idesc(BM, PART), more,
+                                             d + PART, w0, ad + (uint64_t)(PART * 128 >> 4), make_idesc(BM, PART), more);
+                                else
+                                    umma_ts(d, w0, ad, make_idesc(BM, PART), more);
+                                if (NW == 3 && kk < 3)
+                                    umma2_ts(d + BN, w1, ad, make_idesc(BM, 2 * BN), 1u, d + 2 * BN, w2, ad, make_idesc(BM, BN), 1u);
+                            } else {
+                                umma_ts(d, w0, ad, make_idesc(BM, BN), more);
+                                umma2_ts(d + BN, w1, ad, make_idesc(BM, BN), more, d + 2 * BN, w2, ad, make_idesc(BM, BN), more);
+                            }
+                        }
+                        umma_commit_elected(w_empty(slot));
+                    }
+                    if (ok) umma_commit_elected(a_empty(s));
+                }
+                if (ok) umma_commit_elected(tfull_bar(buf));
+            }
+        }
+    } else if (warp < Cfg::kFirstA) {
+        // ------------------------------------------------- the weights' terms
+        // A warp holds the 32 rows whose lanes of tensor memory it reaches, a thread one row.
+        constexpr int STEPS = Cfg::kGroupSteps, WR = NW == 3 ? 16 : 8;
+        const int group = (warp - 2) >> 2, row = (warp & 3) * 32 + lane;
+        const uint32_t t_row = ring + ((uint32_t)((warp & 3) * 32) << 16) + (Cfg::kSlotsABlock == 1 ? group * STEPS * 8 : 0);
+        const uint32_t my = (uint32_t)row * 128u, sw = (uint32_t)(row & 7);
+        uint32_t n = 0;                                              // K block of the CTA
+        bool ok = true;
+        if constexpr (!VEC) pdl_wait();
+        for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
+            const Unit it(u, tiles_m, sh, kbt, BN);
+            for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
+                if (VEC && !mbar_wait_warp(raw_full(n % RAW), (n / RAW) & 1, abort_flag)) { ok = false; break; }
+                const uint32_t slot_no = n * Cfg::kSlotsABlock + (Cfg::kSlotsABlock == 1 ? 0 : group), slot = slot_no % SLOTS;
+#pragma unroll
+                for (int step = 0; ok && step < STEPS; ++step) {
+                    const int kk = group * STEPS + step;
+                    uint32_t r[WR], t[NW][8];
+                    const uint32_t src = base + (VEC ? n % RAW : 0u) * Cfg::kRawBytes + my + (NW == 3 ? (uint32_t)(kk >> 1) * (BM * 128) : 0u);
+                    if constexpr (!VEC) {
+                        // the warp's 32 rows, two at a time, into the cells where a load by TMA would put them
+                        const int col = lane & 15, k = kb * BK + kk * UMMA_K + col, r0 = (warp & 3) * 32 + (lane >> 4);
+                        const uint32_t byte = (uint32_t)(NW == 3 ? ((kk & 1) * 16 + col) * 4 : (kk * 16 + col) * 2);
+                        float v[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            v[i] = it.n0 + r0 + 2 * i < N && k < K ? ldcg_f32(W + ((size_t)(it.n0 + r0 + 2 * i) * K + k)) : 0.f;
+                        __syncwarp();                                // (what was there has been read)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const int r = r0 + 2 * i;
+                            const uint32_t at = src - my + (uint32_t)r * 128u + ((((byte >> 4) ^ (uint32_t)(r & 7)) << 4) | (byte & 15u));
+                            if constexpr (NW == 3) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v[i]) : "memory");
+                            else asm volatile("st.shared.b16 [%0], %1;" ::"r"(at), "h"((unsigned short)(__float_as_uint(v[i]) >> 16)) : "memory");
+                        }
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (int c = 0; c < WR / 4; ++c) {
+                        const uint32_t chunk = NW == 3 ? (uint32_t)((kk & 1) * 4 + c) : (uint32_t)(kk * 2 + c);
+                        asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
+                                     : "=r"(r[4 * c]), "=r"(r[4 * c + 1]), "=r"(r[4 * c + 2]), "=r"(r[4 * c + 3])
+                                     : "r"(src + ((chunk ^ sw) << 4)) : "memory");
+                    }
+                    if constexpr (NW == 3) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) split2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]), t[0][i], t[1][i], t[2][i]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) t[0][i] = r[i];
+                    }
+                    if (step == 0) {
+                        const uint32_t use = slot_no / SLOTS;
+                        if (use > 0 && !mbar_wait_warp(w_empty(slot), (use - 1) & 1, abort_flag)) { ok = false; break; }
+                        tc_fence_after();
+                    }
+#pragma unroll
+                    for (int i = 0; i < NW; ++i) tmem_st8(t_row + slot * Cfg::kSlotCols + i * Cfg::kTermCols + step * 8, t[i]);
+                }
+                // the issuing warp then need not wait for the activations too
+                if (!ok || !mbar_wait_warp(a_full(n % ASTAGES), (n / ASTAGES) & 1, abort_flag)) { ok = false; break; }
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(w_full(slot));
+                    if (VEC) mbar_arrive(raw_empty(n % RAW));
+                }
+            }
+        }
+    } else if (warp < Cfg::kFirstEpi) {
+        if constexpr (!Cfg::kPlanes) {
+        // ------------------------------------------------- the activations' terms
+        constexpr int CT = Cfg::kAWarps * 32, STRIDE = CT / 8;               // rows between a thread's items of 8 elements
+        constexpr int ITEMS = (BN * 8 + CT - 1) / CT, AR = NA == 3 ? 8 : 4;  // and registers an item
+        constexpr int DEPTH = BN == 16 ? 4 : BN == 32 ? 2 : 1;               // K blocks on their way from memory
+        const int t = threadIdx.x - 32 * Cfg::kFirstA;
+        const int row = t >> 3, oct = t & 7;                                 // item q: row + STRIDE * q
+        const uint32_t cell = (uint32_t)row * 128u + (uint32_t)((oct ^ (row & 7)) << 4);
+        uint32_t ar[DEPTH][ITEMS][AR];
+        int u = blockIdx.x, kb = 0, kb1 = 0, m0 = 0;                         // of the K block that is read next
+        uint32_t asked = 0;
+        auto begin = [&]() {
+            if (u >= units) return;
+            const Unit it(u, tiles_m, sh, kbt, BN);
+            kb = it.kb0; kb1 = it.kb1; m0 = it.m0;
+        };
+        auto load = [&](int q, uint32_t* r) {
+            const int m = m0 + row + STRIDE * q, k = kb * BK + oct * 8;
+            load8<TA, VEC>(A + ((size_t)m * K + k), m < M && row + STRIDE * q < BN ? K - k : 0, r);
+        };
+        auto step = [&]() {
+            ++asked;
+            if (++kb >= kb1) { u += gridDim.x; begin(); }
+        };
+        begin();
+        pdl_wait();
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+            if (u < units) {
+#pragma unroll
+                for (int q = 0; q < ITEMS; ++q) load(q, ar[d][q]);
+                step();
+            }
+        }
+        bool ok = true;
+        for (uint32_t n = 0; ok && n < asked;) {
+#pragma unroll
+            for (int d = 0; d < DEPTH; ++d, ++n) {
+                if (n >= asked) break;
+                const int s = n % ASTAGES;
+                const uint32_t round = n / ASTAGES;
+                if (round > 0 && !mbar_wait_warp(a_empty(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
+                const uint32_t dst = a_base + s * Cfg::kABytes + cell;
+                // an item's registers are filled again as soon as they are stored
+#pragma unroll
+                for (int q = 0; q < ITEMS; ++q) {
+                    if ((q + 1) * STRIDE <= BN || row + q * STRIDE < BN) split_store<TA>(ar[d][q], dst + q * STRIDE * 128, Cfg::kAPlane);
+                    if (u < units) load(q, ar[d][q]);
+                }
+                if (u < units) step();
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(a_full(s));
+            }
+        }
+        }
+    } else {
+        // ------------------------------------------------------------ sums
+        constexpr int COLS = Cfg::kCols;
+        const int q = warp & 3, first_col = ((warp - Cfg::kFirstEpi) >> 2) * COLS;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16) + first_col;
+        float sum[COLS];
+        uint32_t chunk_no = 0;
+        bool ok = true;
+        pdl_wait();
+        for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
+            const Unit it(u, tiles_m, sh, kbt, BN);
+            const int n = it.n0 + q * 32 + lane, m1 = it.m0 + first_col;
+            const int cols = min(M - m1, COLS);                              // columns that are rows of the result (may be none)
             for (int c0 = it.kb0; c0 < it.kb1; c0 += sh.chunk, ++chunk_no) {
                 const uint32_t buf = chunk_no % BUFS, use = chunk_no / BUFS;
-                if (!mbar_wait(tfull_bar(buf), use & 1, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_warp(tfull_bar(buf), use & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t t_addr = t_lane + buf * Cfg::kBufCols;
                 const bool first = sh.slices > 1 || c0 == it.kb0, last = sh.slices > 1 || c0 + sh.chunk >= it.kb1;
-#pragma unroll 1
-                for (int j0 = 0; j0 < COLS; j0 += 16) {
-                    uint32_t s0[16], s1[16], s2[16], sum[16];
-                    tmem_ld16(t_addr + j0, s0);
-                    tmem_ld16(t_addr + BN + j0, s1);
-                    tmem_ld16(t_addr + 2 * BN + j0, s2);
-                    if (!first) tmem_ld16(t_lane + Cfg::kSumCol + j0, sum);
+#pragma unroll
+                for (int j0 = 0; j0 < COLS; j0 += 8) {
+                    uint32_t s0[8], s1[8], s2[8];
+                    tmem_ld8(t_addr + j0, s0);
+                    tmem_ld8(t_addr + BN + j0, s1);
+                    tmem_ld8(t_addr + 2 * BN + j0, s2);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {                 // nothing below may move ahead of the wait
-                        asm volatile("" : "+r"(s0[j]), "+r"(sum[j]), "+r"(s1[j]), "+r"(s2[j]));
-                    }
+                    for (int j = 0; j < 8; ++j) asm volatile("" : "+r"(s0[j]), "+r"(s1[j]), "+r"(s2[j]));    // nothing below moves ahead of the wait
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
+                    for (int j = 0; j < 8; ++j) {
                         const float p = __uint_as_float(s0[j]) + (__uint_as_float(s1[j]) + __uint_as_float(s2[j]));
-                        sum[j] = __float_as_uint(first ? p : __uint_as_float(sum[j]) + p);
+                        sum[j0 + j] = first ? p : sum[j0 + j] + p;
                     }
-                    if (!last) {
-                        tmem_st16(t_lane + Cfg::kSumCol + j0, sum);
-                    } else {
-                        const int m1 = it.m0 + first_col + j0;
-                        if (sh.slices > 1) {
-                            float* p = ws + ((size_t)(c0 / sh.chunk) * M + m1) * N + n;
+                }
+                if (last && sh.slices == 1) {
+                    bool bad = false;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (m1 + j < M && n < N) p[(size_t)j * N] = __uint_as_float(sum[j]);
-                        } else {
-                            bool bad = false;
+                    for (int j = 0; j < COLS; ++j) bad |= not_finite(sum[j]) && j < cols;
+                    if (__any_sync(0xffffffffu, bad && n < N)) {             // those are written here, from tensor memory
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) bad |= not_finite(__uint_as_float(sum[j])) && m1 + j < M;
-                            if (__any_sync(0xffffffffu, bad && n < N)) {      // those are written here, from tensor memory
-                                tmem_st16(t_lane + Cfg::kSumCol + j0, sum);
-                                tmem_st_wait();
+                        for (int j = 0; j < COLS; ++j) tmem_st1(t_addr + j, __float_as_uint(sum[j]));
+                        tmem_st_wait();
 #pragma unroll 1
-                                for (int j = 0; j < 16 && m1 + j < M; ++j) {
-                                    const float x = tmem_ld1(t_lane + Cfg::kSumCol + j0 + j);
-                                    const bool mine = n < N && not_finite(x);
-                                    const float v = plain_dots<TA, TW>(x, mine, A + (size_t)(m1 + j) * K, W + (size_t)n * K, K);
-                                    if (mine) store_result(out, out_bf16, residual, (size_t)(m1 + j) * N + n, v);
-                                }
-                            }
-                            if (n < N) {
+                        for (int j = 0; j < cols; ++j) {
+                            const float x = tmem_ld1(t_addr + j);
+                            const bool mine = n < N && not_finite(x);
+                            const float v = plain_dots<TA, TW>(x, mine, A + (size_t)(m1 + j) * K, W + (size_t)n * K, K);
+                            if (mine) store_result(out, out_bf16, residual, (size_t)(m1 + j) * N + n, v);
+                        }
+                        __syncwarp();
 #pragma unroll
-                                for (int j = 0; j < 16; ++j)
-                                    if (m1 + j < M && !not_finite(__uint_as_float(sum[j])))
-                                        store_result(out, out_bf16, residual, (size_t)(m1 + j) * N + n, __uint_as_float(sum[j]));
-                            }
+                        for (int j0 = 0; j0 < COLS; j0 += 8) {               // (so that no sum is held in a register over the call)
+                            uint32_t s0[8];
+                            tmem_ld8(t_addr + j0, s0);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) { asm volatile("" : "+r"(s0[j])); sum[j0 + j] = __uint_as_float(s0[j]); }
                         }
                     }
-                    __syncwarp();
                 }
-                if (!last) tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(tempty_bar(buf));
+                if (!last || n >= N) {
+                } else if (sh.slices > 1) {
+                    float* p = ws + ((size_t)(c0 / sh.chunk) * M + m1) * N + n;
+#pragma unroll
+                    for (int j = 0; j < COLS; ++j)
+                        if (j < cols) p[(size_t)j * N] = sum[j];
+                } else {
+                    // eight residuals on their way together (they may lie where the results go)
+#pragma unroll
+                    for (int j0 = 0; j0 < COLS; j0 += 8) {
+                        if (j0 >= cols) break;
+                        const size_t at = (size_t)(m1 + j0) * N + n;
+                        float r[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) r[j] = residual && j0 + j < cols ? __ldcg(residual + at + (size_t)j * N) : 0.f;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (j0 + j >= cols || not_finite(sum[j0 + j])) continue;
+                            const float v = residual ? r[j] + sum[j0 + j] : sum[j0 + j];
+                            if (out_bf16) ((bf16*)out)[at + (size_t)j * N] = from_f32<bf16>(v);
+                            else ((float*)out)[at + (size_t)j * N] = v;
+                        }
+                    }
+                }
+                __syncwarp();
             }
         }
     }
@@ -422,14 +599,39 @@ gemm_f32_kernel(const TA* A, const TW* W, void* out, int out_bf16, const float* 
     tc_fence_before();
     __syncthreads();
     if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);      // products still in flight end before their operands go
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);      // copies and products still in flight end before their memory goes
         if (threadIdx.x == 0) atomicExch(error_flag, 1);
         __syncthreads();
     }
-    if (warp == 0) {
+    if (warp == 1) {
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    }
+}
+
+// The terms of the activations, [3 or 1][M][pitch] bfloat16, pitch = K rounded up to 8 with zeros behind K.
+template <typename TA, bool VEC>
+__global__ void __launch_bounds__(256)
+gemm_f32_terms_kernel(const TA* A, uint4* __restrict__ terms, int M, int K) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int octs = (K + 7) / 8;
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, plane = (long long)M * octs;
+    if (i >= plane) return;
+    const long long row = i / octs;
+    const int k = (int)(i - row * octs) * 8;
+    uint32_t r[8];
+    load8<TA, VEC>(A + row * K + k, K - k, r);
+    if constexpr (sizeof(TA) == 2) {
+        terms[i] = make_uint4(r[0], r[1], r[2], r[3]);
+    } else {
+        uint32_t h[4], m[4], l[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) split2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]), h[j], m[j], l[j]);
+        terms[i] = make_uint4(h[0], h[1], h[2], h[3]);
+        terms[plane + i] = make_uint4(m[0], m[1], m[2], m[3]);
+        terms[2 * plane + i] = make_uint4(l[0], l[1], l[2], l[3]);
     }
 }
 
@@ -486,24 +688,25 @@ int chunk_count(int K) {
 }
 
 // Tile width and whether the K range is shared out, from M, N, K and the SM count.  A K block of a tile takes about the
-// clocks below (reading and splitting 128 weight rows and bn activation rows, their products: fitted to 60 times of the products of the
-// 8B shape at 1 to 2,048 rows); tiles run in rounds of one a SM.
+// clocks below (128 weight rows split, their products with bn activation rows: fitted to 130 times of the products of the 8B shape at 4 to
+// 1,000 rows; the pick was within 8 % of the best of them from K = 4,096 on), with 5,000 for the kernel that makes the activations' terms;
+// tiles run in rounds of one a SM.
 F32Plan f32_plan(int M, int N, int K) {
     const int sms = tff_num_sms() > 0 ? tff_num_sms() : 148;
     const int kbt = (K + BK - 1) / BK, chunks = chunk_count(K);
     const long long tiles_n = (N + BM - 1) / BM;
-    const int bns[4] = {16, 32, 64, 128};
-    const double clocks[4] = {1720., 1720., 2300., 3300.};
+    const int bns[5] = {16, 32, 64, 96, 128};
+    const double clocks[5] = {1350., 1400., 1550., 1900., 2230.};
     F32Plan best = {16, 1};
     double best_cost = 1e30;
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < 5; ++b) {
         if (b > 0 && bns[b - 1] >= M) break;
         const long long tiles = tiles_n * ((M + bns[b] - 1) / bns[b]);
         for (int split = 0; split < (chunks > 1 ? 2 : 1); ++split) {
             const int slices = split ? chunks : 1;
             const long long rounds = (tiles * slices + sms - 1) / sms;
             // a round also starts up and drains; the partial results are written and read once more
-            double cost = (double)rounds * (split ? chunk_blocks(kbt) : kbt) * clocks[b] + 3000.;
+            double cost = (double)rounds * (split ? chunk_blocks(kbt) : kbt) * clocks[b] + 3000. + (bns[b] >= 64 ? 5000. : 0.);
             if (split) cost += 6000. + 2.0 * slices * (double)M * N * 4. / 2600.;
             if (cost < best_cost) { best_cost = cost; best = {bns[b], slices}; }
         }
@@ -511,10 +714,20 @@ F32Plan f32_plan(int M, int N, int K) {
     return best;
 }
 
+// Rows whose terms are made at a time: they take 256 MB at most (or 384 rows).
+int rows_at_a_time(int K) {
+    const long long rows = (256ll << 20) / (6ll * ((K + 7) / 8 * 8)) / 384 * 384;              // whole tiles of every width
+    return rows < 384 ? 384 : rows > (1 << 30) ? (1 << 30) : (int)rows;
+}
+// Floats of the chunks' partial results, in whole lines of 128 bytes.
+long long partial_floats(int M, int N, int K, int slices) {
+    return slices > 1 ? ((long long)chunk_count(K) * M * N + 31) / 32 * 32 : 0;
+}
+
 template <int BN, typename TA, typename TW, bool VEC>
-int launch(const void* A, const void* W, void* C, int out_bf16, const float* residual, float* ws, int M, int N, int K,
+int launch(const TA* A, const TW* W, void* C, int out_bf16, const float* residual, float* ws, int M, int N, int K,
            int slices, cudaStream_t stream) {
-    using Cfg = F32Cfg<BN, sizeof(TA) == 4 ? 3 : 1, sizeof(TW) == 4 ? 3 : 1>;
+    using Cfg = F32Cfg<BN, sizeof(TA) == 4 ? 3 : 1, sizeof(TW) == 4 ? 3 : 1, VEC>;
     auto kern = gemm_f32_kernel<BN, TA, TW, VEC>;
     static bool configured = false;
     if (!configured) {
@@ -527,36 +740,65 @@ int launch(const void* A, const void* W, void* C, int out_bf16, const float* res
     if (ctas <= 0 || tff_device_error_flag() == nullptr) return TFF_ERR_LAUNCH;
     if (units + ctas >= (1ll << 31)) return TFF_ERR_UNSUPPORTED;
     if (ctas > units) ctas = units;
+    CUtensorMap tm_w = {}, tm_a = {};
+    if (VEC && !tff_tensor_map_2d(W, N, K, BM, 128 / (int)sizeof(TW), (int)sizeof(TW), &tm_w)) return TFF_ERR_DRIVER;
+    int st = TFF_OK;
+    if (Cfg::kPlanes) {
+        const void* terms = A;
+        const int pitch = (K + 7) / 8 * 8;
+        if constexpr (sizeof(TA) == 4 || !VEC) {
+            uint4* t = (uint4*)(ws + partial_floats(M, N, K, slices));
+            const long long blocks = ((long long)M * (pitch / 8) + 255) / 256;
+            st = tff_launch_pdl(gemm_f32_terms_kernel<TA, VEC>, dim3((unsigned)blocks), dim3(256), (size_t)0, stream, A, t, M, K);
+            if (st != TFF_OK) return st;
+            terms = t;
+        }
+        if (!tff_tensor_map_2d(terms, (long long)M * (sizeof(TA) == 4 ? 3 : 1), pitch, BN, BK, 2, &tm_a)) return TFF_ERR_DRIVER;
+    }
     const int chunk = chunk_blocks((K + BK - 1) / BK);
     const Share sh = {slices, (chunk_count(K) + slices - 1) / slices * chunk, chunk};
-    int st = tff_launch_pdl(kern, dim3((unsigned)ctas), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, (const TA*)A,
-                            (const TW*)W, C, out_bf16, residual, ws, M, N, K, sh, tff_device_error_flag());
+    st = tff_launch_pdl(kern, dim3((unsigned)ctas), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tm_w, tm_a, A, W, C,
+                        out_bf16, residual, ws, M, N, K, sh, tff_device_error_flag());
     if (st == TFF_OK && slices > 1) {
         const long long blocks = ((long long)M * N + 1023) / 1024;
-        st = tff_launch_pdl(gemm_f32_sum_kernel<TA, TW>, dim3((unsigned)blocks), dim3(256), (size_t)0, stream, (const TA*)A,
-                            (const TW*)W, (const float*)ws, C, out_bf16, residual, M, N, K, chunk_count(K));
+        st = tff_launch_pdl(gemm_f32_sum_kernel<TA, TW>, dim3((unsigned)blocks), dim3(256), (size_t)0, stream, A, W,
+                            (const float*)ws, C, out_bf16, residual, M, N, K, chunk_count(K));
     }
     return st;
 }
 
 template <typename TA, typename TW, bool VEC>
-int dispatch(const F32Plan& p, const void* A, const void* W, void* C, int out_bf16, const float* residual, float* ws, int M,
+int dispatch(const F32Plan& p, const TA* A, const TW* W, void* C, int out_bf16, const float* residual, float* ws, int M,
              int N, int K, cudaStream_t s) {
     switch (p.bn) {
         case 16: return launch<16, TA, TW, VEC>(A, W, C, out_bf16, residual, ws, M, N, K, p.slices, s);
         case 32: return launch<32, TA, TW, VEC>(A, W, C, out_bf16, residual, ws, M, N, K, p.slices, s);
         case 64: return launch<64, TA, TW, VEC>(A, W, C, out_bf16, residual, ws, M, N, K, p.slices, s);
+        case 96: return launch<96, TA, TW, VEC>(A, W, C, out_bf16, residual, ws, M, N, K, p.slices, s);
         default: return launch<128, TA, TW, VEC>(A, W, C, out_bf16, residual, ws, M, N, K, p.slices, s);
     }
 }
 
+bool wants_terms(const F32Plan& p) { return p.bn >= 64; }      // (bfloat16 activations only where their rows do not suit TMA)
+
 template <typename TA, typename TW>
-int dispatch_vec(const F32Plan& p, const void* A, const void* W, void* C, int out_bf16, const float* residual, float* ws,
+int dispatch_vec(const F32Plan& p, const TA* A, const TW* W, void* C, int out_bf16, const float* residual, float* ws,
                  int M, int N, int K, cudaStream_t s) {
     // 8 elements are read at a time: rows must be multiples of 8 elements and start at multiples of 8 elements' bytes
     const bool vec = K % 8 == 0 && ((uintptr_t)A % (8 * sizeof(TA))) == 0 && ((uintptr_t)W % (8 * sizeof(TW))) == 0;
-    return vec ? dispatch<TA, TW, true>(p, A, W, C, out_bf16, residual, ws, M, N, K, s)
-               : dispatch<TA, TW, false>(p, A, W, C, out_bf16, residual, ws, M, N, K, s);
+    // the terms of very many rows are made, and used, for some of them at a time
+    const int part = wants_terms(p) ? rows_at_a_time(K) : M;
+    for (int m = 0; m < M; m += part) {
+        const size_t at = (size_t)m * N;
+        void* c = out_bf16 ? (void*)((bf16*)C + at) : (void*)((float*)C + at);
+        const float* r = residual ? residual + at : nullptr;
+        const TA* a = A + (size_t)m * K;
+        const int rows = M - m < part ? M - m : part;
+        const int st = vec ? dispatch<TA, TW, true>(p, a, W, c, out_bf16, r, ws, rows, N, K, s)
+                           : dispatch<TA, TW, false>(p, a, W, c, out_bf16, r, ws, rows, N, K, s);
+        if (st != TFF_OK || M - m <= part) return st;
+    }
+    return TFF_OK;
 }
 
 }  // namespace
@@ -568,25 +810,31 @@ TFF_API int tff_gemm_f32_plan(int M, int N, int K) {
     return p.bn | (p.slices << 16);
 }
 
-// How many chunks of the K range have a partial result of their own (with more than one slice).
-TFF_API int tff_gemm_f32_chunks(int K) { return K <= 0 ? 1 : chunk_count(K); }
+// Floats of workspace that tff_gemm_f32 wants for a plan: the chunks' partial results where the K range is shared out, the
+// activations' terms (of rows_at_a_time at most) where tiles of many rows read them.
+TFF_API long long tff_gemm_f32_workspace(int M, int N, int K, int a_dt, int plan) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const F32Plan p = {plan & 0xffff, plan >> 16};
+    const int part = wants_terms(p) ? rows_at_a_time(K) : M, rows = M < part ? M : part;
+    return partial_floats(rows, N, K, p.slices) + (wants_terms(p) ? (long long)rows * ((K + 7) / 8 * 4) * (a_dt == 0 ? 3 : 1) : 0);
+}
 
 // dtype codes: 0 = float32, 1 = bfloat16 (one operand at most).  ``residual`` (float32 [M, N], may alias C
-// when C is float32) is added to the product when it is not null.  ``plan`` as tff_gemm_f32_plan gives it; with more than
-// one slice (each of as many whole chunks, none empty) ``ws`` holds tff_gemm_f32_chunks(K) * M * N floats.
+// when C is float32) is added to the product when it is not null.  ``plan`` as tff_gemm_f32_plan gives it (slices of
+// as many whole chunks each, none empty); ``ws`` holds tff_gemm_f32_workspace floats and is 16-byte aligned (null when that is 0).
 TFF_API int tff_gemm_f32(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt, const float* residual,
                          float* ws, int M, int N, int K, int plan, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return TFF_OK;
     if (K <= 0 || (a_dt & ~1) || (w_dt & ~1) || (c_dt & ~1)) return TFF_ERR_BAD_ARGUMENT;
     const F32Plan p = {plan & 0xffff, plan >> 16};
     const int chunks = chunk_count(K);
-    if ((p.bn != 16 && p.bn != 32 && p.bn != 64 && p.bn != 128) || p.slices < 1 || p.slices > chunks ||
-        (long long)(p.slices - 1) * ((chunks + p.slices - 1) / p.slices) >= chunks || (p.slices > 1 && ws == nullptr))
+    if ((p.bn != 16 && p.bn != 32 && p.bn != 64 && p.bn != 96 && p.bn != 128) || p.slices < 1 || p.slices > chunks ||
+        (long long)(p.slices - 1) * ((chunks + p.slices - 1) / p.slices) >= chunks || (tff_gemm_f32_workspace(M, N, K, a_dt, plan) > 0 && (ws == nullptr || (uintptr_t)ws % 16 != 0)))
         return TFF_ERR_BAD_ARGUMENT;
     switch (a_dt * 2 + w_dt) {
-        case 0: return dispatch_vec<float, float>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);
-        case 1: return dispatch_vec<float, bf16>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);
-        case 2: return dispatch_vec<bf16, float>(p, A, W, C, c_dt, residual, ws, M, N, K, stream);
+        case 0: return dispatch_vec<float, float>(p, (const float*)A, (const float*)W, C, c_dt, residual, ws, M, N, K, stream);
+        case 1: return dispatch_vec<float, bf16>(p, (const float*)A, (const bf16*)W, C, c_dt, residual, ws, M, N, K, stream);
+        case 2: return dispatch_vec<bf16, float>(p, (const bf16*)A, (const float*)W, C, c_dt, residual, ws, M, N, K, stream);
     }
     return TFF_ERR_UNSUPPORTED;                  // two bfloat16 operands: gemm_tc.cu, gemm_simt.cu
 }

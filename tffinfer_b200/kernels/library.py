@@ -291,14 +291,13 @@ class CudaKernels:
             return
         if plan is None:
             plan = self.lib.tff_gemm_f32_plan(_c_int(M), _c_int(N), _c_int(K))
-        slices = plan >> 16
-        ws = None
-        if slices > 1:
-            ws = torch.empty(self.lib.tff_gemm_f32_chunks(_c_int(K)) * M * N, dtype=torch.float32, device=a.device)
+        floats = self.lib.tff_gemm_f32_workspace(_c_int(M), _c_int(N), _c_int(K), _c_int(_dt(a)), _c_int(plan))
+        ws = torch.empty(floats, dtype=torch.float32, device=a.device) if floats > 0 else None
         self._check(self.lib.tff_gemm_f32(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _ptr(out),
                                           _c_int(_dt(out)), _ptr(residual), _ptr(ws), _c_int(M), _c_int(N), _c_int(K),
                                           _c_int(plan), self._stream()), "gemm_f32")
-        self.launches += 2 if slices > 1 else 1
+        terms = plan & 0xffff >= 64 and (a.dtype == torch.float32 or K % 8 != 0)      # made by a kernel of their own
+        self.launches += 1 + (plan >> 16 > 1) + terms
 
     FOLD_MAX_M = 16           # up to this many rows the norm is folded into the gate/up product (with SwiGLU)
     CLUSTER_MAX_M = 16        # up to this many rows the gate/up product applies SwiGLU itself (clusters share a tile's K range)
