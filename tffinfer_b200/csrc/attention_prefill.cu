@@ -181,7 +181,12 @@ struct PrefillCfg {
     static constexpr int kStageBytes = BLOCK_N * (DK + DV) * 2;     // a block's keys and values
     static constexpr int kStages = DK > 128 ? (QT == 2 ? 3 : 4) : DK > 64 ? 5 : 8;
     static constexpr int kExchange = QT * 2 * BLOCK_M * 4;          // a float of every row from either group
-    static constexpr int kBars = 2 * kStages + BARS_PER_TILE * QT;
+    // Keys of more than 128 elements leave room for three stages, which S two blocks ahead of PV would hold all: their keys are then
+    // given back when S has read them and their values when PV has, each with barriers of its own (2,355 tokens of 32 heads
+    // of 192: 88 us a layer's attention, 108 with one barrier for both).
+    static constexpr bool kApart = DK > 128;
+    static constexpr int kRingBars = (kApart ? 4 : 2) * kStages;
+    static constexpr int kBars = kRingBars + BARS_PER_TILE * QT;
     static constexpr int kSmem = QT * kQBytes + kStages * kStageBytes + kExchange + 8 * kBars + 16;
     static constexpr int kThreads = (8 * QT + 1 + QT) * 32;
     static_assert(kSmem <= 227 * 1024, "shared memory of the prompt attention kernel");
@@ -215,7 +220,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     volatile float* exchange = (volatile float*)(gKV + NSTAGES * STAGE_BYTES);       // [tile][group][row]
     auto kv_full = [&](int s) { return bars + 8u * s; };
     auto kv_empty = [&](int s) { return bars + 8u * (NSTAGES + s); };
-    auto tile_bar = [&](int x, int i) { return bars + 8u * (2 * NSTAGES + BARS_PER_TILE * x + i); };
+    constexpr bool APART = Cfg::kApart;                          // (kv_full and kv_empty are then the keys' alone)
+    auto v_full = [&](int s) { return bars + 8u * ((APART ? 2 * NSTAGES : 0) + s); };
+    auto v_empty = [&](int s) { return bars + 8u * ((APART ? 3 : 1) * NSTAGES + s); };
+    auto tile_bar = [&](int x, int i) { return bars + 8u * (Cfg::kRingBars + BARS_PER_TILE * x + i); };
     // S(j), P(j), PV(j) and the reference of block j report to a barrier of the group that has block j (group j % 2): who waits
     // for a barrier then waits for every one of its completions in turn, or knows that the one before is in the past, which a
     // parity wait needs.
@@ -237,7 +245,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     const int ps = DENSE ? 0 : 1 << p.page_shift;
 
     if (tid == 0) {
-        for (int s = 0; s < NSTAGES; ++s) mbar_init(kv_full(s), 1);
+        for (int s = 0; s < NSTAGES; ++s) { mbar_init(kv_full(s), 1); if (APART) mbar_init(v_full(s), 1); }
         for (int x = 0; x < QT; ++x) {
             for (int g = 0; g < 2; ++g) {
                 mbar_init(s_full(x, g), 1); mbar_init(p_full(x, g), 4); mbar_init(pv_done(x, g), 1);
@@ -281,7 +289,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     const int* table = DENSE ? nullptr : p.block_table + (size_t)b * p.table_width;
     // a stage is free again when the products of every tile that has rows have read it
     if (tid == 0) {
-        for (int s = 0; s < NSTAGES; ++s) mbar_init(kv_empty(s), (uint32_t)(n_act > 0 ? n_act : 1));
+        for (int s = 0; s < NSTAGES; ++s) {
+            mbar_init(kv_empty(s), (uint32_t)(n_act > 0 ? n_act : 1));
+            if (APART) mbar_init(v_empty(s), (uint32_t)(n_act > 0 ? n_act : 1));
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -307,16 +318,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             const int n_first = walk.block(i) * BLOCK_N;
             if constexpr (DENSE) {
                 // key n of the request is row q0 + n; rows beyond the request's are another's or zeros, and masked
-                if (lane == 0) mbar_expect_tx(kv_full(s), (uint32_t)STAGE_BYTES);
+                if (lane == 0) mbar_expect_tx(kv_full(s), (uint32_t)(APART ? KH * K_HALF : STAGE_BYTES));
                 __syncwarp();
                 const int row = q0 + n_first;
                 if (lane < KH) {
                     const uint32_t dst = stage + lane * K_HALF;
                     if (lane < p.k_halves) tma_load_2d(dst, &tm_cache, kv_full(s), kvh * p.k_head + lane * 64, row);
                     else tma_load_2d(dst, &tm_r, kv_full(s), p.r_col + (lane - p.k_halves) * 64, row);
-                } else if (lane < KH + VH) {
-                    tma_load_2d(stage + V_AT + (lane - KH) * V_HALF, &tm_v, kv_full(s), kvh * p.dv + (lane - KH) * 64, row);
                 }
+                if constexpr (APART) {
+                    if (round > 0 && !mbar_wait_warp(v_empty(s), (round - 1) & 1, abort_flag)) break;
+                    if (lane == 0) mbar_expect_tx(v_full(s), (uint32_t)(VH * V_HALF));
+                    __syncwarp();
+                }
+                if (lane >= KH && lane < KH + VH)
+                    tma_load_2d(stage + V_AT + (lane - KH) * V_HALF, &tm_v, v_full(s), kvh * p.dv + (lane - KH) * 64, row);
             } else {
                 const int first = n_first >> p.page_shift;               // (a block's pages lie in one run of 32)
                 if (first >> 5 != chunk) {
@@ -349,7 +365,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             constexpr uint32_t idesc_s = make_idesc(BLOCK_M, BLOCK_N, 0);
             bool ok = mbar_wait_warp(q_ready(x), 0, abort_flag);
             // S runs two blocks ahead of PV: a group that has written P(j) finds S(j + 2) finished
-            uint32_t phase = 0;
+            uint32_t phase = 0, phase_pv = 0;
             int st = 0, st_pv = 0;                                 // stages of S(n) and of PV(n - 2)
             for (int n = 0; n < nb + 2 && ok; ++n) {
                 if (n < nb) {
@@ -362,18 +378,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                     for (int h = 0; h < KH; ++h)
                         umma4_bf16_elected(t_s, qdesc + (uint64_t)(h * (BLOCK_M * 128) >> 4), kd + (uint64_t)(h * K_HALF >> 4), idesc_s, h > 0 ? 1u : 0u);
                     umma_commit_elected(s_full(x, n & 1));
+                    if constexpr (APART) umma_commit_elected(kv_empty(st));    // this tile has read the keys
                     if (++st == NSTAGES) { st = 0; phase ^= 1; }
                 }
                 const int j = n - 2;
                 if (j >= 0) {
                     ok = mbar_wait_warp(p_full(x, j & 1), (uint32_t)(j >> 1) & 1, abort_flag);    // P(j) is in tensor memory
+                    if constexpr (APART) { if (ok) ok = mbar_wait_warp(v_full(st_pv), phase_pv, abort_flag); }
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t vd = vdesc + (uint64_t)(st_pv * (STAGE_BYTES >> 4));
                     umma4_ts<(2 * GROUP >> 4)>(t_o, t_s + 64 + (j & 1) * 32, vd, idesc_pv, j > 0 ? 1u : 0u);
                     umma_commit_elected(pv_done(x, j & 1));                    // O holds block j; that P buffer is free
-                    umma_commit_elected(kv_empty(st_pv));                  // and this tile has read K and V of the stage
-                    if (++st_pv == NSTAGES) st_pv = 0;
+                    umma_commit_elected(v_empty(st_pv));                   // and this tile has read the stage's values (and keys)
+                    if (++st_pv == NSTAGES) { st_pv = 0; phase_pv ^= 1; }
                 }
             }
         };
@@ -495,7 +513,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                 // value rows no query row of the CTA may see (beyond the last key, between the kept ones and the first
                 // window) are cleared, since page slots and unfetched shared memory may hold anything; the warps of both tiles
                 // do it (the same zeros), so that each tile's products wait for its own warps only.
-                // (S(j) has read the stage's keys: its values have landed with them)
+                // (S(j) has read the stage's keys: its values have landed with them, or are waited for)
+                if constexpr (APART) {
+                    ok = mbar_wait_warp(v_full(j % NSTAGES), (uint32_t)(j / NSTAGES) & 1, abort_flag);
+                    if (!ok) break;
+                }
                 uint8_t* rows = gKV + (j % NSTAGES) * STAGE_BYTES + V_AT;
                 for (int idx = tt; idx < BLOCK_N * CH; idx += 128) {
                     const int kr = idx / CH, c = idx % CH;
