@@ -465,6 +465,24 @@ def test_grouped_product_on_tensor_cores(ops, M, N, K, G):
         assert torch.isnan(c[:, G * N:]).all()
 
 
+@pytest.mark.parametrize("N,K", [(128, 64), (200, 1032)])
+def test_grouped_product_of_few_rows_at_the_edges_of_its_tiles(ops, N, K):
+    """A row's bits do not depend on how many rows its group has: tiles of few rows (up to 32) and of 128."""
+    g = torch.Generator().manual_seed(8)
+    G = 3
+    a = torch.randn(40, G * K, generator=g).to(torch.bfloat16).cuda()
+    b = torch.randn(G, N, K, generator=g).to(torch.bfloat16).cuda()
+    first = None
+    for M in (40, 33, 32, 31, 17, 16, 1):
+        c = torch.full((M + 1, G * N), float("nan")).cuda()
+        ops.gemm_grouped(a, b, c, G, M, N, K, G * K, K, K, N * K, G * N, N)
+        assert torch.isnan(c[M]).all()
+        first = c if first is None else first
+        assert torch.equal(c[:M], first[:M]), M
+    want = torch.cat([a[:, i * K:(i + 1) * K].double() @ b[i].double().T for i in range(G)], dim=1)
+    assert float((first[:40].double() - want).abs().max() / want.abs().max()) < 1e-5
+
+
 # ------------------------------------------------------------------------------ generation through the engine
 @pytest.mark.parametrize("dtype,name", [("float32", "a"), ("float32", "b"), ("bfloat16", "a")])
 def test_greedy_generation_through_the_engine(dtype, name):

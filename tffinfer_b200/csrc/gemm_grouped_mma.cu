@@ -1,14 +1,17 @@
 // The grouped product of gemm_grouped.cu for bfloat16 operands on the tensor cores (mma.sync m16n8k16, float32
 // accumulation): C_g[m, n] = sum_k A_g[m, k] * B_g[n, k], uniform or ragged groups, optional row map, as there.
-// Tiles of 128 x 128 x 64, eight warps of 32 x 64, operands through a three-stage cp.async ring into padded shared
-// memory (rows of 144 bytes: the eight rows of an ldmatrix fall into different banks), fragments by ldmatrix.
+// Tiles of 128 x 128 x 64, eight warps of 32 x 64, operands through a three-stage cp.async ring into shared memory, fragments by
+// ldmatrix.
 // Gated form: B_g holds the gate and up rows of a group alternating in blocks of 64 ([g0..g63 | u0..u63 | g64.. ], the
 // layout of the tcgen05 products), a tile of 128 rows of B being one such pair of blocks; a warp then takes 32 gate
 // rows and the 32 up rows of the same outputs, so that a thread finds act(gate) and up of an output element four
 // accumulator tiles apart; C_g[m, f] = act(gate_f) * up_f has half as many columns as B_g has rows.
-// Steps of few rows a group (decoded tokens: a token or two an expert, a token or eight a head) take tiles of 16 rows
-// instead: the eight warps lie side by side along B's rows, so that a tile multiplies 16 rows and not 128 of which most
+// Steps of few rows a group (decoded tokens: a token or two an expert, a token or eight a head) take tiles of 32 rows
+// instead: the eight warps lie side by side along B's rows, so that a tile multiplies 32 rows and not 128 of which most
 // are not there, and the ring is deeper (five stages, two CTAs an SM), since such a product is a pass of the weights.
+// What bounds such a step is the weights' stream: 64 tokens on 16 experts of 3,072 x 2,048 take 71 us for the gate and up rows (403 MB, 5.7
+// TB/s) and 37 for the down rows, 87 and 50 when tiles held 16 rows (an expert with 17 rows was read twice, and the tiles of the
+// uneven experts made a fourth round of CTAs) and the second-level cache fetched less than 256 bytes of a row at a time.
 // Needs K, lda, ldb and the group strides to be multiples of 8 elements and 16-byte aligned bases (the launcher
 // refuses anything else and the caller takes the FMA kernel).  A row's result does not depend on the tile it is in:
 // every output element adds its products in the same order of k.
@@ -16,17 +19,24 @@
 
 namespace {
 
-constexpr int MBN = 128, MBK = 64, LDS = MBK + 8, THREADS = 256;
+constexpr int MBN = 128, MBK = 64, THREADS = 256;
 constexpr int CHUNKS = MBK / 8;                          // 16-byte pieces of a tile row
-constexpr int BIG_ROWS = 128, SMALL_ROWS = 16;           // rows of a tile
+constexpr int BIG_ROWS = 128, SMALL_ROWS = 32;           // rows of a tile
 template <int BM> struct RingCfg {
     static constexpr int kStages = BM == SMALL_ROWS ? 5 : 3;
-    static constexpr int kSmem = kStages * (BM + MBN) * LDS * 2;
+    static constexpr int kSmem = kStages * (BM + MBN) * MBK * 2;
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Where 8 elements of a tile's row lie: rows of 128 bytes, their 16-byte pieces exchanged by the row's number modulo 8, so that the eight
+// rows of an ldmatrix fall into different banks.
+__device__ __forceinline__ int cell(int row, int k) { return row * MBK + (((k >> 3) ^ (row & 7)) << 3); }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// (the second-level cache fetches 256 bytes of a row at a time: two K blocks)
+__device__ __forceinline__ void cp_async16_ahead(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -62,11 +72,11 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_g
                         float limit, float slope) {
     constexpr int STAGES = RingCfg<MBM>::kStages;
     constexpr bool SMALL = MBM == SMALL_ROWS;
-    constexpr int MI = SMALL ? 1 : 2, NJ = SMALL ? 1 : 4;     // a warp's 16-row pieces of A and of B
+    constexpr int MI = 2, NJ = SMALL ? 1 : 4;     // a warp's 16-row pieces of A and of B
     constexpr int A_LOADS = (MBM * CHUNKS + THREADS - 1) / THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    bf16* As = (bf16*)smem_raw;                               // [STAGES][MBM][LDS]
-    bf16* Bs = As + STAGES * MBM * LDS;                       // [STAGES][MBN][LDS]
+    bf16* As = (bf16*)smem_raw;                               // [STAGES][MBM][MBK]
+    bf16* Bs = As + STAGES * MBM * MBK;                       // [STAGES][MBN][MBK]
     pdl_launch_dependents();
     pdl_wait();
     int g, m0, m_end;
@@ -78,7 +88,7 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_g
     }
     const int n0 = blockIdx.x * MBN;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = SMALL ? 0 : warp >> 1, wn = SMALL ? warp : warp & 1;      // 4 x 2 warps of 32 x 64, or 8 of 16 x 16
+    const int wm = SMALL ? 0 : warp >> 1, wn = SMALL ? warp : warp & 1;      // 4 x 2 warps of 32 x 64, or 8 of 32 x 16
     const bf16* Ag = A + (size_t)g * a_gs;
     const bf16* Bg = B + (size_t)g * b_gs;
     const int kt = (K + MBK - 1) / MBK;
@@ -96,14 +106,14 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_g
             const int c = tid + i * THREADS, r = c / CHUNKS, kc = (c % CHUNKS) * 8;
             if (SMALL && r >= MBM) break;
             const bool oka = k0 + kc < K && (m0 + r < m_end);
-            cp_async16(smem_addr(As + ((size_t)s * MBM + r) * LDS + kc),
+            cp_async16(smem_addr(As + (size_t)s * MBM * MBK + cell(r, kc)),
                        oka ? (const void*)(Ag + a_off[i] + k0 + kc) : (const void*)Ag, oka ? 16 : 0);
         }
 #pragma unroll
         for (int i = 0; i < MBN * CHUNKS / THREADS; ++i) {
             const int c = tid + i * THREADS, r = c / CHUNKS, kc = (c % CHUNKS) * 8;
             const bool okb = k0 + kc < K && (n0 + r < N);
-            cp_async16(smem_addr(Bs + ((size_t)s * MBN + r) * LDS + kc),
+            cp_async16_ahead(smem_addr(Bs + (size_t)s * MBN * MBK + cell(r, kc)),
                        okb ? (const void*)(Bg + (size_t)(n0 + r) * ldb + k0 + kc) : (const void*)Bg, okb ? 16 : 0);
         }
     };
@@ -127,21 +137,21 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_g
         const int nk = kb + STAGES - 1;
         if (nk < kt) load_stage(nk % STAGES, nk * MBK);
         cp_commit();
-        const bf16* as = As + (size_t)(kb % STAGES) * MBM * LDS;
-        const bf16* bs = Bs + (size_t)(kb % STAGES) * MBN * LDS;
+        const bf16* as = As + (size_t)(kb % STAGES) * MBM * MBK;
+        const bf16* bs = Bs + (size_t)(kb % STAGES) * MBN * MBK;
 #pragma unroll
         for (int kk = 0; kk < MBK; kk += 16) {
             uint32_t a[MI][4], b[NJ][4];
 #pragma unroll
             for (int mi = 0; mi < MI; ++mi)
-                ldsm4(a[mi], smem_addr(as + (size_t)(wm * 32 + mi * 16 + (lane & 15)) * LDS + kk + (lane >> 4) * 8));
+                ldsm4(a[mi], smem_addr(as + cell(wm * 32 + mi * 16 + (lane & 15), kk + (lane >> 4) * 8)));
 #pragma unroll
             for (int nj = 0; nj < NJ; ++nj) {
                 // rows of B this warp's 16-row slice nj covers: plain 64 in a row; gated 32 gate rows, then their 32 up
-                // rows (tiles of 16 rows: 16 in a row, or 8 gate rows and their 8 up rows)
+                // rows (tiles of few rows: 16 in a row, or 8 gate rows and their 8 up rows)
                 const int brow = SMALL ? (GATED ? wn * 8 + (lane >> 4) * 56 : wn * 16)
                                        : GATED ? ((nj >> 1) * 64 + wn * 32 + (nj & 1) * 16) : (wn * 64 + nj * 16);
-                ldsm4(b[nj], smem_addr(bs + (size_t)(brow + (lane & 7) + (lane >> 4) * 8) * LDS + kk + ((lane >> 3) & 1) * 8));
+                ldsm4(b[nj], smem_addr(bs + cell(brow + (lane & 7) + (lane >> 4) * 8, kk + ((lane >> 3) & 1) * 8)));
             }
 #pragma unroll
             for (int mi = 0; mi < MI; ++mi)

@@ -205,7 +205,7 @@ moe_route_kernel(const TH* __restrict__ h, const TW* __restrict__ w_router, cons
         if (lane == 0) {
             // an identity expert (index >= num_real) has no rows among the experts' products: -1
             pair_expert[(size_t)t * top + k] = (arg == 0x7fffffff || arg >= num_real) ? -1 : arg;
-            pair_weight[(size_t)t * top + k] = wgt;
+            gbest[k] = wgt;                           // (the groups are through with it)
             if (arg != 0x7fffffff) {
                 if (arg < num_real) atomicAdd(&counts[arg], 1);
                 choice[arg] = -INFINITY;              // taken
@@ -214,18 +214,15 @@ moe_route_kernel(const TH* __restrict__ h, const TW* __restrict__ w_router, cons
         total += wgt;
         __syncwarp();
     }
+    float* pw = pair_weight + (size_t)t * top;
     if (softmax_scores == 2) {                 // the scores are the logits themselves: softmax over the chosen ones only
-        if (lane == 0) {
-            float* pw = pair_weight + (size_t)t * top;
-            float m = -INFINITY, sum = 0.f;
-            for (int k = 0; k < top; ++k) m = fmaxf(m, pw[k]);
-            for (int k = 0; k < top; ++k) { pw[k] = expf(pw[k] - m); sum += pw[k]; }
-            for (int k = 0; k < top; ++k) pw[k] /= sum;
-        }
+        float m = -INFINITY, sum = 0.f;
+        for (int k = 0; k < top; ++k) m = fmaxf(m, gbest[k]);
+        for (int k = 0; k < top; ++k) sum += expf(gbest[k] - m);
+        for (int k = lane; k < top; k += 32) pw[k] = expf(gbest[k] - m) / sum;
         return;
     }
-    if (renormalize && lane == 0)
-        for (int k = 0; k < top; ++k) pair_weight[(size_t)t * top + k] /= total + 1e-20f;   // (all chosen scores may be zero)
+    for (int k = lane; k < top; k += 32) pw[k] = renormalize ? gbest[k] / (total + 1e-20f) : gbest[k];   // (all chosen scores may be zero)
 }
 
 // pad_rows > 0: every expert's rows start at a multiple of pad_rows (= tile_rows): the sorted order then consists of
