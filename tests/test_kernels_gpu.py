@@ -283,6 +283,19 @@ def test_gemm_f32_infinities_and_overflow(ops, slices):
     ops.check_errors()
 
 
+@pytest.mark.parametrize("M,N,K,pitch", [(128, 128, 64, 64), (129, 264, 72, 200), (700, 2048, 512, 576), (3000, 520, 8, 16)])
+def test_gemm_tc_of_rows_with_a_pitch(ops, M, N, K, pitch):
+    """The same bits as the product of the rows laid close together; what lies between the rows is not read."""
+    a, w = torch.full((M, pitch), float("nan"), dtype=torch.bfloat16, device=DEV), g((N, K), torch.bfloat16, 27, 0.05).to(DEV)
+    a[:, :K] = g((M, K), torch.bfloat16, 26).to(DEV)
+    out, want = torch.empty(M, N, dtype=torch.bfloat16, device=DEV), torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    assert ops.gemm_tc_rows(a, K, w, out)
+    ops.gemm_tc(a[:, :K].contiguous(), w, want, plan=ops.prompt_plan(M, N, K, False))
+    assert torch.equal(out, want)
+    assert not ops.gemm_tc_rows(a[:, 1:], K - 8, w[:, :K - 8], out)
+    ops.check_errors()
+
+
 TC_SHAPES = [(1, 128, 64), (8, 6144, 4096), (5, 311, 80), (16, 256, 128), (17, 384, 200), (64, 4096, 1024),
              (100, 1000, 512), (256, 512, 4096), (257, 512, 256), (300, 311, 264), (1024, 768, 512),
              (2048, 4096, 4096), (128, 128, 8), (130, 6144, 4096), (300, 1000, 264), (513, 1256, 72)]

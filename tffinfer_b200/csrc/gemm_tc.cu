@@ -446,6 +446,23 @@ TFF_API int tff_gemm_tc_act(const void* A, const void* W, void* out, int M, int 
     return launch_tc<128, false, EPI_RELU2, bf16, true>(tl, tc, to, out, M, N, K, N, 0, stream);
 }
 
+// out[M, N] = A W^T as bfloat16 for rows of A that lie lda elements apart (a multiple of 8, at least K).  Normal orientation;
+// TFF_ERR_UNSUPPORTED for shapes it does not take.
+TFF_API int tff_gemm_tc_rows(const void* A, long long lda, const void* W, void* out, int M, int N, int K, int bn, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return TFF_OK;
+    if (K <= 0 || lda < K) return TFF_ERR_BAD_ARGUMENT;
+    if (K % 8 != 0 || lda % 8 != 0 || N % 8 != 0 || (bn != 128 && bn != 256 && bn != 512)) return TFF_ERR_UNSUPPORTED;
+    if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)out & 15)) return TFF_ERR_UNSUPPORTED;
+    if (tff_device_error_flag() == nullptr) return TFF_ERR_LAUNCH;
+    CUtensorMap tl, tc, to;
+    if (!tff_tensor_map_2d(A, M, K, BM, BK, 2, &tl, lda)) return TFF_ERR_DRIVER;
+    if (!tff_tensor_map_2d(W, N, K, bn == 512 ? 128 : bn, BK, 2, &tc)) return TFF_ERR_DRIVER;
+    if (!tff_tensor_map_2d(out, M, N, 32, 64, 2, &to)) return TFF_ERR_DRIVER;
+    if (bn == 512) return tff_gemm_tc_pair_launch(tl, tc, to, EPI_STORE, 1, M, N, K, 0, stream);
+    if (bn == 256) return launch_tc<256, false, EPI_STORE, bf16, true>(tl, tc, to, out, M, N, K, N, 0, stream);
+    return launch_tc<128, false, EPI_STORE, bf16, true>(tl, tc, to, out, M, N, K, N, 0, stream);
+}
+
 // Grouped products on the same kernel: the rows of A ([rows, K], rows a multiple of 128) are tiles of 128 rows that
 // each belong to one group (lane_group[tile] on the device; -1: the tile is not used), W is [groups * group_rows, K],
 // and tile t is multiplied with its group's rows of W:  out[rows, group_rows] = A W_g^T (act 2, not gated: the square of

@@ -23,15 +23,17 @@ EncodeTiledFn get_encode_fn() {
 }
 
 struct MapKey {
-    const void* ptr; long long rows; long long cols; int box_rows; int box_cols; int elt;
+    const void* ptr; long long rows; long long cols; int box_rows; int box_cols; int elt; long long pitch;
     bool operator==(const MapKey& o) const {
-        return ptr == o.ptr && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols && elt == o.elt;
+        return ptr == o.ptr && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols && elt == o.elt &&
+               pitch == o.pitch;
     }
 };
 struct MapKeyHash {
     size_t operator()(const MapKey& k) const {
         size_t h = (size_t)k.ptr;
         h ^= (size_t)k.rows * 0x9E3779B97F4A7C15ull; h ^= (size_t)k.cols * 0xC2B2AE3D27D4EB4Full;
+        h ^= (size_t)k.pitch * 0x165667B19E3779F9ull;
         h ^= ((size_t)k.box_rows << 48) ^ ((size_t)k.box_cols << 40) ^ ((size_t)k.elt << 36);
         return h;
     }
@@ -44,9 +46,9 @@ std::mutex g_mu;
 }  // namespace
 
 bool tff_tensor_map_2d(const void* ptr, long long rows, long long cols, int box_rows, int box_cols, int elt,
-                       CUtensorMap* out) {
+                       CUtensorMap* out, long long pitch) {
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-    const MapKey key{ptr, rows, cols, box_rows, box_cols, elt};
+    const MapKey key{ptr, rows, cols, box_rows, box_cols, elt, pitch};
     {
         std::lock_guard<std::mutex> g(g_mu);
         auto it = cache.find(key);
@@ -55,7 +57,7 @@ bool tff_tensor_map_2d(const void* ptr, long long rows, long long cols, int box_
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)cols * elt};
+    const cuuint64_t strides[1] = {(cuuint64_t)(pitch ? pitch : cols) * elt};
     const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     CUtensorMap m;
@@ -76,7 +78,7 @@ bool tff_tensor_map_2d(const void* ptr, long long rows, long long cols, int box_
 bool tff_tensor_map_kv_page(const void* cache, long long total_rows, int head_dim, int page_size, int kv_heads,
                             CUtensorMap* out) {
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache_maps;
-    const MapKey key{cache, total_rows, head_dim, page_size, kv_heads, -4};
+    const MapKey key{cache, total_rows, head_dim, page_size, kv_heads, -4, 0};
     {
         std::lock_guard<std::mutex> g(g_mu);
         auto it = cache_maps.find(key);
@@ -106,7 +108,7 @@ bool tff_tensor_map_kv_page(const void* cache, long long total_rows, int head_di
 bool tff_tensor_map_kv_groups(const void* cache, long long total_rows, int head_dim, int page_size, int kv_heads,
                               CUtensorMap* out) {
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache_maps;
-    const MapKey key{cache, total_rows, head_dim, page_size, kv_heads, -5};
+    const MapKey key{cache, total_rows, head_dim, page_size, kv_heads, -5, 0};
     {
         std::lock_guard<std::mutex> g(g_mu);
         auto it = cache_maps.find(key);

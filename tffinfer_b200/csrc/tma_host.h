@@ -7,9 +7,9 @@
 
 // Tensor map of a row-major matrix [rows, cols] of 2-byte (bfloat16) or 4-byte (float32)
 // elements: boxes of box_cols x box_rows, 128-byte swizzle (box_cols * elt must be 128), zero fill
-// outside the matrix.  Maps are cached by their arguments.  False if the driver refuses.
+// outside the matrix.  ``pitch``: elements between rows (0: cols).  Maps are cached by their arguments.  False if the driver refuses.
 bool tff_tensor_map_2d(const void* ptr, long long rows, long long cols, int box_rows, int box_cols, int elt,
-                       CUtensorMap* out);
+                       CUtensorMap* out, long long pitch = 0);
 
 // Tensor map over a paged cache [pages, layers, 2 (K,V), kv_heads, page_size, head_dim] of bfloat16 whose
 // box is one (page, layer, kv head): 64 columns x (head_dim / 64) halves x page_size rows x {K, V}, with

@@ -394,6 +394,22 @@ class CudaKernels:
                                          self._stream()), "gemm_tc")
         self.launches += 1
 
+    def gemm_tc_rows(self, a, K: int, w, out) -> bool:
+        """out = a[:, :K] @ w^T, bfloat16, where the tcgen05 product takes it (aligned bfloat16 operands, K and the rows of
+        ``a`` and ``out`` multiples of 8 elements); False, and nothing done, elsewhere.  Per-head keys and values of a step's latents
+        are one such product each, since their heads lie side by side (2,355 rows, 32 heads of 128, K = 512: 15 us a product, 51 as a product a
+        head on mma.sync)."""
+        M, N = a.shape[0], w.shape[0]
+        if not (a.dtype == w.dtype == out.dtype == torch.bfloat16 and w.dim() == 2 and out.shape[1] == N and w.shape[1] == K
+                and K % 8 == 0 and N % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) == 1 and w.is_contiguous()
+                and out.is_contiguous() and all(t.data_ptr() % 16 == 0 for t in (a, w, out))):
+            return False
+        bn = self.prompt_plan(M, N, K, False)[1]
+        self._check(self.lib.tff_gemm_tc_rows(_ptr(a), _c_int(a.stride(0)), _ptr(w), _ptr(out), _c_int(M), _c_int(N), _c_int(K),
+                                              _c_int(bn), self._stream()), "gemm_tc_rows")
+        self.launches += 1
+        return True
+
     def zero_f32(self, t) -> None:
         assert t.dtype == torch.float32 and t.is_contiguous()
         self._check(self.lib.tff_zero_f32(_ptr(t), _c_int(t.numel()), self._stream()), "zero_f32")
@@ -1393,7 +1409,8 @@ class CudaKernels:
 
     @classmethod
     def grouped_tcgen05_from(cls, E: int, by_table: bool) -> int:
-        """From how many pairs of a step E experts run on the tcgen05 product (us, mma.sync and tcgen05).  Above 12 an expert the
+        """From how many pairs of a step E experts run on the tcgen05 product (us, mma.sync and tcgen05; the former on tiles of 16
+        rows, which have 32 since and are a tenth faster at 8 pairs an expert).  Above 12 an expert the
         other one leaves its tiles of few rows: 4 experts of 3,072 x 2,048 with 64 pairs 159 and 70, 16 with 256 263 and 135, 64 of
         768 x 2,048 with 1,026 268 and 168, 64 of 1,536 x 4,096 with 1,024 875 and 536; chosen by a table 145 and 61, 253 and 127,
         248 and 151, 843 and 503.  With 9 to 12 an expert that is so for few experts chosen in groups, which have uneven shares: a layer
@@ -1765,16 +1782,18 @@ class CudaKernels:
             apart = dense_tc and dim % 64 == 0 and 0 < rot_dim <= 64
             k_head = dim if apart else dim + rot_dim
             keys = torch.empty((T, heads * k_head), dtype=dt, device=dev)
-            self.gemm_grouped(rows, w_uk, keys, heads, T, dim, kv_rank, slot, 0, kv_rank, dim * kv_rank,
-                              heads * k_head, k_head)
+            if k_head != dim or not self.gemm_tc_rows(rows, kv_rank, w_uk, keys):
+                self.gemm_grouped(rows, w_uk, keys, heads, T, dim, kv_rank, slot, 0, kv_rank, dim * kv_rank,
+                                  heads * k_head, k_head)
             if not apart:
                 self._check(self.lib.tff_latent_spread(_ptr(rows), _c_int(kv_rank), _c_int(rot_dim), _ptr(keys), _c_int(dim),
                                                        _c_int(heads), _c_int(_dt(keys)), _c_int(T), self._stream()),
                             "latent_spread")
                 self.launches += 1
             values = torch.empty((T, heads * vdim), dtype=dt, device=dev)
-            self.gemm_grouped(rows, w_uv, values, heads, T, vdim, kv_rank, slot, 0, kv_rank, vdim * kv_rank,
-                              heads * vdim, vdim)
+            if not self.gemm_tc_rows(rows, kv_rank, w_uv, values):
+                self.gemm_grouped(rows, w_uv, values, heads, T, vdim, kv_rank, slot, 0, kv_rank, vdim * kv_rank,
+                                  heads * vdim, vdim)
             if dense_tc:
                 self.attention_dense(q, batch, keys, k_head, rows if apart else None, kv_rank, values, out, heads, heads,
                                      dim + rot_dim, vdim, scale, window=window, sink=sink)
