@@ -147,3 +147,13 @@ def test_what_a_kernel_ahead_wrote_is_read_past_the_first_level_cache(source, ke
     with open(os.path.join(build.CSRC_DIR, source), encoding="utf-8") as f:
         helpers = re.findall(r"(?:load4|load8|plain_dots|store_result)\([^;{]*\{.*?\n}?", f.read(), re.S)
     assert not any(re.search(r"= \*\(const |\bresidual\[|\br[aw]\[", h) for h in helpers)
+
+
+@pytest.mark.parametrize("source", [s for s in build.sources() if s != "selftest.cu"])
+def test_a_lane_arrives_for_its_warp_behind_a_warp_barrier(source):
+    """One lane's arrival releases what the whole warp wrote and gives back what it read: only __syncwarp (no vote, no shuffle)
+    orders the other lanes' accesses before it."""
+    with open(os.path.join(build.CSRC_DIR, source), encoding="utf-8") as f:
+        text = re.sub(r"\s+", " ", re.sub(r"//[^\n]*", "", f.read()))
+    for before in re.findall(r"(\S+) if \(lane == 0\) \{? ?(?:tc5::)?mbar_arrive", text):
+        assert before == "__syncwarp();", before

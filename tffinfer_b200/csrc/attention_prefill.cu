@@ -502,6 +502,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             const float m_new = grow ? m_blk : m_prev;
             *mine = m_new;
             const bool moved = __any_sync(0xffffffffu, m_new != m_used);
+            __syncwarp();                                          // (a vote orders no memory: every lane's reference, then the arrival)
             if (lane == 0) mbar_arrive(ref_bar(x, g, q));
             // the product of the block before last must have read the P buffer that this block writes
             if (j > 1) {
