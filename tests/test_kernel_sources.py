@@ -157,3 +157,12 @@ def test_a_lane_arrives_for_its_warp_behind_a_warp_barrier(source):
         text = re.sub(r"\s+", " ", re.sub(r"//[^\n]*", "", f.read()))
     for before in re.findall(r"(\S+) if \(lane == 0\) \{? ?(?:tc5::)?mbar_arrive", text):
         assert before == "__syncwarp();", before
+
+
+def test_every_lane_of_a_warp_that_loads_has_waited_for_the_kernel_ahead():
+    """The producer of the products goes on with all its lanes behind a part that lane 0 takes alone: a wait in that part holds for
+    lane 0 only, and the lanes behind it read the table of groups and issue loads."""
+    text = _kernel("gemm_tc.cu", "gemm_tc_kernel")
+    alone, together = text[text.index("if (warp == 0)"):text.index("else if (warp == 1)")].split("__shfl_sync(")
+    assert "tma_load_2d_elected(" in together and "lane_group" in together
+    assert "pdl_wait();" in together[:together.index("SegIter")]

@@ -144,6 +144,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
         }
         {
             const uint32_t pre = __shfl_sync(0xffffffffu, first, 0);
+            pdl_wait();                              // every lane reads the table below, and any may be the one elected to load
             SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
             uint32_t n = 0;
             bool ok = true;
