@@ -129,6 +129,7 @@ READ_PAST_L1 = [
     ("attention_decode.cu", "attn_decode_kernel", ("q", "gate")),
     ("attention_prefill.cu", "attn_prefill_tc_kernel", ("gate",)),
     ("attention_bf16.cu", "attn_combine_kernel", ("gate",)),
+    ("gemm_tc.cu", "gemm_tc_kernel", ("lane_group",)),
     ("attention_tile.cu", "attention_tile_kernel", ("q", "cache", "src")),
     ("attention_tile.cu", "attention_tile_mma_kernel", ("q", "cache")),
     ("attention_tile.cu", "attention_tile_few_kernel", ("q", "cache")),

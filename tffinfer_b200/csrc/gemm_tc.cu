@@ -62,10 +62,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
                const __grid_constant__ CUtensorMap tm_col,    // operand whose rows land on TMEM columns (box 64 x BN)
                const __grid_constant__ CUtensorMap tm_out,    // output, boxes of 128 bytes x 32 rows (TMA_OUT only)
                TC* __restrict__ out, int rows_lane, int rows_col, int K, int ldo, int stream_k, int* error_flag,
-               const int* __restrict__ lane_group, int group_rows, GateConstants gc) {
+               const int* lane_group, int group_rows, GateConstants gc) {
     // lane_group (normal orientation only; null: one product): the 128-row tile t of the lane operand belongs to group
     // lane_group[t] and is multiplied with rows [g * group_rows, (g + 1) * group_rows) of the column operand; a tile of
-    // group -1 is skipped by all three roles.  The table is written by a kernel ahead: read it behind pdl_wait.
+    // group -1 is skipped by all three roles.  The table is written by a kernel ahead: it is read behind pdl_wait, past the first-level cache
+    // (roles that found different groups there would wait for one another).
     const bool grouped = lane_group != nullptr;
     using Cfg = TileCfg<BN, TMA_OUT, SWAP>;
     using SegIter = typename std::conditional<SWAP, SegIterShares, SegIterSlices>::type;
@@ -124,7 +125,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
                 SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
                 while (pre < STAGES && it.next()) {
                     int goff = 0;
-                    if (grouped) { const int g = lane_group[it.tile % n_lane_tiles]; if (g < 0) continue; goff = g * group_rows; }
+                    if (grouped) { const int g = __ldcg(lane_group + it.tile % n_lane_tiles); if (g < 0) continue; goff = g * group_rows; }
                     const int lrow = (it.tile % n_lane_tiles) * BM, crow = (it.tile / n_lane_tiles) * BN + goff;
                     for (int kb = it.kb0; kb < it.kb1 && pre < STAGES; ++kb, ++pre) {
                         pre_k[pre] = kb * BK;
@@ -150,7 +151,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
             bool ok = true;
             while (ok && it.next()) {
                 int goff = 0;
-                if (grouped) { const int g = lane_group[it.tile % n_lane_tiles]; if (g < 0) continue; goff = g * group_rows; }
+                if (grouped) { const int g = __ldcg(lane_group + it.tile % n_lane_tiles); if (g < 0) continue; goff = g * group_rows; }
                 const int lrow = (it.tile % n_lane_tiles) * BM, crow = (it.tile / n_lane_tiles) * BN + goff;
                 for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
                     if (n < pre) continue;                           // already requested above
@@ -173,7 +174,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
             bool ok = true;
             if (grouped) pdl_wait();
             while (ok && it.next()) {
-                if (grouped && lane_group[it.tile % n_lane_tiles] < 0) continue;
+                if (grouped && __ldcg(lane_group + it.tile % n_lane_tiles) < 0) continue;
                 const uint32_t acc = seg & 1, use = seg >> 1;
                 if (use > 0 && !mbar_wait_warp(tempty_bar(acc), (use - 1) & 1, abort_flag)) break;   // epilogue has drained it
                 tc_fence_after();
@@ -200,7 +201,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
         SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
         uint32_t seg = 0, chunk_no = 0;
         while (it.next()) {
-            if (grouped && lane_group[it.tile % n_lane_tiles] < 0) continue;
+            if (grouped && __ldcg(lane_group + it.tile % n_lane_tiles) < 0) continue;
             const uint32_t acc = seg & 1, use = seg >> 1;
             if (!mbar_wait(tfull_bar(acc), use & 1, abort_flag)) break;
             tc_fence_after();
