@@ -127,7 +127,7 @@ READ_PAST_L1 = [
     ("attention_generic.cu", "attention_generic_kernel", ("q_in", "cache", "gate", "src")),
     ("attention_generic.cu", "attention_generic_join_kernel", ("ml", "po", "gate")),
     ("attention_decode.cu", "attn_decode_kernel", ("q", "gate")),
-    ("attention_prefill.cu", "attn_prefill_tc_kernel", ("gate",)),
+    ("attention_prefill.cu", "attn_prefill_tc_kernel", ("q", "gate")),
     ("attention_bf16.cu", "attn_combine_kernel", ("gate",)),
     ("gemm_tc.cu", "gemm_tc_kernel", ("lane_group",)),
     ("attention_tile.cu", "attention_tile_kernel", ("q", "cache", "src")),
@@ -144,7 +144,7 @@ def test_what_a_kernel_ahead_wrote_is_read_past_the_first_level_cache(source, ke
     for name in pointers:
         assert not re.search(r"\*\s*__restrict__\s+" + name + r"\b", text), name
         assert not re.search(r"(?<![\w&])(?:p\.)?" + name + r"\[", text), name
-        assert not re.search(r"[^\w)\]]\s*\*\(const \w+\*\)\(?(?:p\.)?" + name + r"\b", text), name
+        assert not re.search(r"[^\w)\]]\s*\*(?:\(const \w+\*\)|reinterpret_cast<const \w+\*>)\(?(?:p\.)?" + name + r"\b", text), name
     with open(os.path.join(build.CSRC_DIR, source), encoding="utf-8") as f:
         helpers = re.findall(r"(?:load4|load8|plain_dots|store_result)\([^;{]*\{.*?\n}?", f.read(), re.S)
     assert not any(re.search(r"= \*\(const |\bresidual\[|\br[aw]\[", h) for h in helpers)

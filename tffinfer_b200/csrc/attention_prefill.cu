@@ -429,7 +429,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
                 const int t = __shfl_sync(0xffffffffu, tok, row), h = __shfl_sync(0xffffffffu, head, row);
                 u[i] = make_uint4(0u, 0u, 0u, 0u);
                 if (row < rows_left && (!DENSE || c * 8 < p.d))
-                    u[i] = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + t) * p.q_row_stride + (size_t)h * (DENSE ? p.d : DK) + c * 8);
+                    u[i] = __ldcg(reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + t) * p.q_row_stride + (size_t)h * (DENSE ? p.d : DK) + c * 8));
             }
             uint8_t* dst = smem + x * Cfg::kQBytes + q * 32 * 128;
 #pragma unroll
