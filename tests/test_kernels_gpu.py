@@ -292,7 +292,23 @@ def test_gemm_tc_of_rows_with_a_pitch(ops, M, N, K, pitch):
     assert ops.gemm_tc_rows(a, K, w, out)
     ops.gemm_tc(a[:, :K].contiguous(), w, want, plan=ops.prompt_plan(M, N, K, False))
     assert torch.equal(out, want)
-    assert not ops.gemm_tc_rows(a[:, 1:], K - 8, w[:, :K - 8], out)
+    ops.check_errors()
+
+
+def test_gemm_tc_of_rows_refuses_what_a_load_by_tma_cannot_take(ops):
+    """One condition at a time (a refusal leaves the result alone); the last call is the one that all of them spoil."""
+    M, N, K = 130, 128, 64
+    a, w = g((M, 80), torch.bfloat16, 28).to(DEV), g((N, 72), torch.bfloat16, 29).to(DEV)
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    close, odd = w[:, :K].contiguous(), g((M, 76), torch.bfloat16, 30).to(DEV)
+    assert not ops.gemm_tc_rows(a[:, 1:], K, close, out)                                  # rows that start off 16 bytes
+    assert not ops.gemm_tc_rows(odd, K, close, out)                                       # rows 76 elements apart
+    assert not ops.gemm_tc_rows(a, K, w[:, :K], out)                                      # weights that are not contiguous
+    assert not ops.gemm_tc_rows(a, 60, w[:, :60].contiguous(), out)                       # K no multiple of 8
+    assert not ops.gemm_tc_rows(a, K, close[:124], out[:, :124].contiguous())             # nor N
+    assert not ops.gemm_tc_rows(a.float(), K, close, out) and not ops.gemm_tc_rows(a, K, close, out.float())
+    assert torch.isnan(out).all()
+    assert ops.gemm_tc_rows(a[:, 8:], K, close, out) and torch.isfinite(out).all()
     ops.check_errors()
 
 
@@ -769,8 +785,8 @@ def test_prompt_attention_when_the_running_maximum_jumps_late(ops, nq, nkv, d, p
 @pytest.mark.parametrize("requests", [1, 40])
 def test_prompt_attention_of_every_number_of_key_blocks(ops, nq, nkv, d, page, window, requests):
     """Walks of 1 to 14 blocks of 64 keys, by ones: the blocks alternate between two groups of warps, whose references and sums meet at
-    the end, and go round rings of 3 to 8 stages; one tile a CTA (few requests) and two (more tiles than SMs), the second of which may
-    hold no rows."""
+    the end, and go round rings of 5 and 8 stages; one tile a CTA (few requests) and two (more tiles than SMs), the second of which may
+    hold no rows.  (The rings of 3 and 4 stages are those of keys of 192, below.)"""
     G = nq // nkv
     for first in range(0, 14, 1 if requests == 1 else 7):
         new = [(17 + 5 * i) % (256 // G) + 128 // G if i % 3 else 128 // G + 1 for i in range(requests)]
@@ -786,6 +802,41 @@ def test_prompt_attention_of_every_number_of_key_blocks(ops, nq, nkv, d, page, w
         ops.attention_bf16(q.to(DEV), bg, bg.block_tables[0], cache.to(DEV), 0, page, out, nq, nkv, d, 1 / math.sqrt(d), window)
         assert torch.isfinite(out).all()
         assert rel_err(out, want) < 1e-2, (first, new, old)
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("d,dv,rest", [(192, 128, 64), (192, 128, 0), (136, 72, 8)])
+@pytest.mark.parametrize("window", [0, 90, 200])
+@pytest.mark.parametrize("requests", [1, 24])
+def test_prompt_attention_over_plain_rows_of_every_number_of_key_blocks(ops, d, dv, rest, window, requests):
+    """Keys of more than 128 elements, whose stages give keys and values back apart: walks of 1 to 11 blocks, by ones, round rings of 4
+    stages (one tile a CTA) and of 3 (two, where the tiles are more than the SMs; the second may hold no rows)."""
+    H, kh = 4, d - rest
+    for first in range(11 if requests == 1 else 2):
+        lens = [64 * ((first + i) % 11) + 1 + (37 * (first + i)) % 64 for i in range(requests)]
+        T = sum(lens)
+        q, k, v = (g((T, H * n), torch.bfloat16, 31 + first + n).to(DEV) for n in (d, kh, dv))
+        r = g((T, 16 + rest), torch.bfloat16, 32).to(DEV) if rest else None
+        starts = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device=DEV)
+        step = SimpleNamespace(q_start=starts, pos_start=torch.zeros(requests, dtype=torch.int32, device=DEV),
+                               num_requests=requests, max_q_len=max(lens))
+        out = torch.full((T, H * dv), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.attention_dense(q, step, k, kh, r, 16, v, out, H, H, d, dv, d ** -0.5, window=window)
+        assert torch.isfinite(out).all()
+        t0 = 0
+        for n in lens:
+            rows = slice(t0, t0 + n)
+            t0 += n
+            qn, kn, vn = (x[rows].double().reshape(n, H, -1).transpose(0, 1) for x in (q, k, v))
+            if rest:
+                kn = torch.cat([kn, r[rows, 16:].double().expand(H, n, rest)], dim=2)
+            back = torch.arange(n, device=DEV)[:, None] - torch.arange(n, device=DEV)[None]
+            seen = (back >= 0) & (back < window) if window else back >= 0
+            want = (qn @ kn.transpose(1, 2) * d ** -0.5).masked_fill(~seen, -math.inf).softmax(-1) @ vn
+            got = out[rows].double().reshape(n, H, dv).transpose(0, 1)
+            # the probabilities and the result, rounded to 8 bits: 2^-9 of each at most, and about 2^-9 in the 2-norm of all
+            assert float((got - want).norm() / want.norm()) < 2 ** -8, (first, n)
+            assert float((got - want).abs().max() / want.abs().max()) < 2 ** -7, (first, n)
     ops.check_errors()
 
 
