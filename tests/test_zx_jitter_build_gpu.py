@@ -18,8 +18,8 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SELECT = ("prompt_attention or flash_attention or gemm_tc or qkv_projection or norm_gate_up or gate_up_product "
           "or gemm_swiglu or attention_at_long_context or far_key or window_edge or attention_of_few_rows or gemm_f32 "
-          "or portions_and_decoded_tokens")
-FILES = ("test_kernels_gpu.py", "test_dominex_gpu.py")
+          "or portions_and_decoded_tokens or attention_over_plain_rows")
+FILES = ("test_kernels_gpu.py", "test_dominex_gpu.py", "test_kadodra_gpu.py")
 
 
 def test_kernel_tests_pass_with_disturbed_timing(tmp_path):
