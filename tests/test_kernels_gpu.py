@@ -229,6 +229,25 @@ def test_gemm_f32_more_rows_than_have_their_terms_made_at_a_time(ops, slices):
     ops.check_errors()
 
 
+def test_gemm_f32_makes_no_terms_of_bfloat16_rows_that_are_read_as_they_are(ops):
+    """No workspace, and one pass however many the rows; from a base off 16 bytes the terms are made as before."""
+    M, N, K = 389, 40, 116512
+    buf, w = torch.randn(M * K + 8, device=DEV).to(torch.bfloat16), torch.randn(N, K, device=DEV)
+    out, few, odd = (torch.empty(M, N, device=DEV) for _ in range(3))
+    a, shifted = buf[:M * K].view(M, K), buf[1:M * K + 1].view(M, K)
+    ops.gemm_simt(a, w, few, plan=16 | (1 << 16))
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    ops.gemm_simt(a, w, out, plan=96 | (1 << 16))
+    assert torch.cuda.max_memory_allocated() == held
+    assert torch.equal(out, few)
+    ops.gemm_simt(shifted, w, odd, plan=96 | (1 << 16))
+    assert torch.cuda.max_memory_allocated() > held
+    ops.gemm_simt(shifted, w, few, plan=16 | (1 << 16))
+    assert torch.equal(odd, few)
+    ops.check_errors()
+
+
 def test_gemm_f32_single_products(ops):
     """One product an output, of significands whose terms are as large as they get.  The terms left out come to at most
     2 x 2^-8 x 2^-17 (and 2^-34) of the two powers of two, the sum of the levels is rounded twice (2^-24, and 2^-24 of the 2^-7 that the

@@ -779,23 +779,33 @@ int dispatch(const F32Plan& p, const TA* A, const TW* W, void* C, int out_bf16, 
     }
 }
 
-bool wants_terms(const F32Plan& p) { return p.bn >= 64; }      // (bfloat16 activations only where their rows do not suit TMA)
+// What the operands of a call decide: whether their rows can be read 8 elements at a time and by TMA (rows of a multiple of 8 elements
+// that start at multiples of 8 elements' bytes), whether the activations' terms are made in the workspace (not of bfloat16 rows that TMA
+// takes as they are), and how many rows a pass has (the terms of very many rows are made, and used, for some of them at a time).
+struct Passes { bool vec, terms; int part; };
+Passes passes_of(const F32Plan& p, const void* A, int a_dt, const void* W, int w_dt, int M, int K) {
+    Passes c;
+    c.vec = K % 8 == 0 && (uintptr_t)A % (a_dt == 0 ? 32 : 16) == 0 && (uintptr_t)W % (w_dt == 0 ? 32 : 16) == 0;
+    c.terms = p.bn >= 64 && (a_dt == 0 || !c.vec);
+    c.part = c.terms && rows_at_a_time(K) < M ? rows_at_a_time(K) : M;
+    return c;
+}
+long long workspace_floats(const F32Plan& p, const Passes& c, int a_dt, int N, int K) {
+    return partial_floats(c.part, N, K, p.slices) + (c.terms ? (long long)c.part * ((K + 7) / 8 * 4) * (a_dt == 0 ? 3 : 1) : 0);
+}
 
 template <typename TA, typename TW>
-int dispatch_vec(const F32Plan& p, const TA* A, const TW* W, void* C, int out_bf16, const float* residual, float* ws,
+int dispatch_vec(const F32Plan& p, const Passes& c, const TA* A, const TW* W, void* C, int out_bf16, const float* residual, float* ws,
                  int M, int N, int K, cudaStream_t s) {
-    // 8 elements are read at a time: rows must be multiples of 8 elements and start at multiples of 8 elements' bytes
-    const bool vec = K % 8 == 0 && ((uintptr_t)A % (8 * sizeof(TA))) == 0 && ((uintptr_t)W % (8 * sizeof(TW))) == 0;
-    // the terms of very many rows are made, and used, for some of them at a time
-    const int part = wants_terms(p) ? rows_at_a_time(K) : M;
+    const int part = c.part;
     for (int m = 0; m < M; m += part) {
         const size_t at = (size_t)m * N;
-        void* c = out_bf16 ? (void*)((bf16*)C + at) : (void*)((float*)C + at);
+        void* out = out_bf16 ? (void*)((bf16*)C + at) : (void*)((float*)C + at);
         const float* r = residual ? residual + at : nullptr;
         const TA* a = A + (size_t)m * K;
         const int rows = M - m < part ? M - m : part;
-        const int st = vec ? dispatch<TA, TW, true>(p, a, W, c, out_bf16, r, ws, rows, N, K, s)
-                           : dispatch<TA, TW, false>(p, a, W, c, out_bf16, r, ws, rows, N, K, s);
+        const int st = c.vec ? dispatch<TA, TW, true>(p, a, W, out, out_bf16, r, ws, rows, N, K, s)
+                             : dispatch<TA, TW, false>(p, a, W, out, out_bf16, r, ws, rows, N, K, s);
         if (st != TFF_OK || M - m <= part) return st;
     }
     return TFF_OK;
@@ -811,12 +821,11 @@ TFF_API int tff_gemm_f32_plan(int M, int N, int K) {
 }
 
 // Floats of workspace that tff_gemm_f32 wants for a plan: the chunks' partial results where the K range is shared out, the
-// activations' terms (of rows_at_a_time at most) where tiles of many rows read them.
-TFF_API long long tff_gemm_f32_workspace(int M, int N, int K, int a_dt, int plan) {
+// activations' terms (of rows_at_a_time at most) where tiles of many rows read them and the activations are not their own terms.
+TFF_API long long tff_gemm_f32_workspace(const void* A, int a_dt, const void* W, int w_dt, int M, int N, int K, int plan) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     const F32Plan p = {plan & 0xffff, plan >> 16};
-    const int part = wants_terms(p) ? rows_at_a_time(K) : M, rows = M < part ? M : part;
-    return partial_floats(rows, N, K, p.slices) + (wants_terms(p) ? (long long)rows * ((K + 7) / 8 * 4) * (a_dt == 0 ? 3 : 1) : 0);
+    return workspace_floats(p, passes_of(p, A, a_dt, W, w_dt, M, K), a_dt, N, K);
 }
 
 // dtype codes: 0 = float32, 1 = bfloat16 (one operand at most).  ``residual`` (float32 [M, N], may alias C
@@ -829,12 +838,14 @@ TFF_API int tff_gemm_f32(const void* A, int a_dt, const void* W, int w_dt, void*
     const F32Plan p = {plan & 0xffff, plan >> 16};
     const int chunks = chunk_count(K);
     if ((p.bn != 16 && p.bn != 32 && p.bn != 64 && p.bn != 96 && p.bn != 128) || p.slices < 1 || p.slices > chunks ||
-        (long long)(p.slices - 1) * ((chunks + p.slices - 1) / p.slices) >= chunks || (tff_gemm_f32_workspace(M, N, K, a_dt, plan) > 0 && (ws == nullptr || (uintptr_t)ws % 16 != 0)))
+        (long long)(p.slices - 1) * ((chunks + p.slices - 1) / p.slices) >= chunks)
         return TFF_ERR_BAD_ARGUMENT;
+    const Passes c = passes_of(p, A, a_dt, W, w_dt, M, K);
+    if (workspace_floats(p, c, a_dt, N, K) > 0 && (ws == nullptr || (uintptr_t)ws % 16 != 0)) return TFF_ERR_BAD_ARGUMENT;
     switch (a_dt * 2 + w_dt) {
-        case 0: return dispatch_vec<float, float>(p, (const float*)A, (const float*)W, C, c_dt, residual, ws, M, N, K, stream);
-        case 1: return dispatch_vec<float, bf16>(p, (const float*)A, (const bf16*)W, C, c_dt, residual, ws, M, N, K, stream);
-        case 2: return dispatch_vec<bf16, float>(p, (const bf16*)A, (const float*)W, C, c_dt, residual, ws, M, N, K, stream);
+        case 0: return dispatch_vec<float, float>(p, c, (const float*)A, (const float*)W, C, c_dt, residual, ws, M, N, K, stream);
+        case 1: return dispatch_vec<float, bf16>(p, c, (const float*)A, (const bf16*)W, C, c_dt, residual, ws, M, N, K, stream);
+        case 2: return dispatch_vec<bf16, float>(p, c, (const bf16*)A, (const float*)W, C, c_dt, residual, ws, M, N, K, stream);
     }
     return TFF_ERR_UNSUPPORTED;                  // two bfloat16 operands: gemm_tc.cu, gemm_simt.cu
 }

@@ -291,7 +291,8 @@ class CudaKernels:
             return
         if plan is None:
             plan = self.lib.tff_gemm_f32_plan(_c_int(M), _c_int(N), _c_int(K))
-        floats = self.lib.tff_gemm_f32_workspace(_c_int(M), _c_int(N), _c_int(K), _c_int(_dt(a)), _c_int(plan))
+        floats = self.lib.tff_gemm_f32_workspace(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _c_int(M), _c_int(N),
+                                                 _c_int(K), _c_int(plan))
         ws = torch.empty(floats, dtype=torch.float32, device=a.device) if floats > 0 else None
         self._check(self.lib.tff_gemm_f32(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _ptr(out),
                                           _c_int(_dt(out)), _ptr(residual), _ptr(ws), _c_int(M), _c_int(N), _c_int(K),
