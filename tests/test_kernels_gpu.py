@@ -248,6 +248,22 @@ def test_gemm_f32_makes_no_terms_of_bfloat16_rows_that_are_read_as_they_are(ops)
     ops.check_errors()
 
 
+@pytest.mark.parametrize("slices", [1, 3])
+def test_gemm_f32_counts_its_launches(ops, slices):
+    """Product, terms and sum of chunks once a pass: 389 rows of K = 116,512 take two passes where terms are made."""
+    M, N, K = 389, 8, 116512
+    buf, w, out = torch.randn(M * K + 8, device=DEV).to(torch.bfloat16), torch.randn(N, K, device=DEV), torch.empty(M, N, device=DEV)
+
+    def launches(a, w, bn):
+        before = ops.launches
+        ops.gemm_simt(a, w, out[:a.shape[0]], plan=bn | (slices << 16))
+        return ops.launches - before
+    a, more = buf[:M * K].view(M, K), int(slices > 1)
+    assert launches(a, w, 96) == launches(a, w, 16) == 1 + more
+    assert launches(buf[1:M * K + 1].view(M, K), w, 96) == launches(a.float(), w, 96) == 2 * (2 + more)
+    assert launches(a[:384].float(), w, 96) == 2 + more and launches(a[:384].float(), w, 16) == 1 + more
+
+
 def test_gemm_f32_single_products(ops):
     """One product an output, of significands whose terms are as large as they get.  The terms left out come to at most
     2 x 2^-8 x 2^-17 (and 2^-34) of the two powers of two, the sum of the levels is rounded twice (2^-24, and 2^-24 of the 2^-7 that the

@@ -820,17 +820,20 @@ TFF_API int tff_gemm_f32_plan(int M, int N, int K) {
     return p.bn | (p.slices << 16);
 }
 
-// Floats of workspace that tff_gemm_f32 wants for a plan: the chunks' partial results where the K range is shared out, the
-// activations' terms (of rows_at_a_time at most) where tiles of many rows read them and the activations are not their own terms.
-TFF_API long long tff_gemm_f32_workspace(const void* A, int a_dt, const void* W, int w_dt, int M, int N, int K, int plan) {
+// What tff_gemm_f32 takes for these operands and this plan, as launches << 48 | floats of workspace: the chunks' partial results where
+// the K range is shared out, the activations' terms (of rows_at_a_time at most) where tiles of many rows read them and the
+// activations are not their own terms; a kernel each for the product, the terms and the sum of the chunks, in every pass.
+TFF_API long long tff_gemm_f32_needs(const void* A, int a_dt, const void* W, int w_dt, int M, int N, int K, int plan) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     const F32Plan p = {plan & 0xffff, plan >> 16};
-    return workspace_floats(p, passes_of(p, A, a_dt, W, w_dt, M, K), a_dt, N, K);
+    const Passes c = passes_of(p, A, a_dt, W, w_dt, M, K);
+    const long long launches = ((M + (long long)c.part - 1) / c.part) * (1 + (c.terms ? 1 : 0) + (p.slices > 1 ? 1 : 0));
+    return launches << 48 | workspace_floats(p, c, a_dt, N, K);
 }
 
 // dtype codes: 0 = float32, 1 = bfloat16 (one operand at most).  ``residual`` (float32 [M, N], may alias C
 // when C is float32) is added to the product when it is not null.  ``plan`` as tff_gemm_f32_plan gives it (slices of
-// as many whole chunks each, none empty); ``ws`` holds tff_gemm_f32_workspace floats and is 16-byte aligned (null when that is 0).
+// as many whole chunks each, none empty); ``ws`` holds the floats of tff_gemm_f32_needs and is 16-byte aligned (null when there are none).
 TFF_API int tff_gemm_f32(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt, const float* residual,
                          float* ws, int M, int N, int K, int plan, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return TFF_OK;

@@ -291,14 +291,14 @@ class CudaKernels:
             return
         if plan is None:
             plan = self.lib.tff_gemm_f32_plan(_c_int(M), _c_int(N), _c_int(K))
-        floats = self.lib.tff_gemm_f32_workspace(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _c_int(M), _c_int(N),
-                                                 _c_int(K), _c_int(plan))
+        needs = self.lib.tff_gemm_f32_needs(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _c_int(M), _c_int(N), _c_int(K),
+                                            _c_int(plan))
+        floats = needs & ((1 << 48) - 1)
         ws = torch.empty(floats, dtype=torch.float32, device=a.device) if floats > 0 else None
         self._check(self.lib.tff_gemm_f32(_ptr(a), _c_int(_dt(a)), _ptr(w), _c_int(_dt(w)), _ptr(out),
                                           _c_int(_dt(out)), _ptr(residual), _ptr(ws), _c_int(M), _c_int(N), _c_int(K),
                                           _c_int(plan), self._stream()), "gemm_f32")
-        terms = plan & 0xffff >= 64 and (a.dtype == torch.float32 or K % 8 != 0)      # made by a kernel of their own
-        self.launches += 1 + (plan >> 16 > 1) + terms
+        self.launches += needs >> 48
 
     FOLD_MAX_M = 16           # up to this many rows the norm is folded into the gate/up product (with SwiGLU)
     CLUSTER_MAX_M = 16        # up to this many rows the gate/up product applies SwiGLU itself (clusters share a tile's K range)
