@@ -282,9 +282,9 @@ def test_routed_experts(ops, dtype, E, top, ff, W, T):
 
 @pytest.mark.parametrize("tcgen05", [True, False])
 @pytest.mark.parametrize("E,top,T", [(16, 4, 32), (16, 4, 33), (5, 3, 13), (5, 3, 14), (1, 1, 9), (64, 6, 85), (64, 6, 86), (17, 4, 51), (17, 4, 52),
-                                        (64, 6, 128), (64, 6, 129)])
+                                        (64, 6, 128), (64, 6, 129), (8, 4, 16), (8, 4, 17), (9, 3, 72), (9, 3, 73), (64, 6, 256), (64, 6, 257)])
 def test_routed_experts_where_the_product_changes(ops, monkeypatch, E, top, T, tcgen05):
-    """Steps of 8 and of 12 pairs an expert and a few more, on both products."""
+    """Steps of 8, 12 and 24 pairs an expert and a few more, on both products."""
     monkeypatch.setattr(type(ops), "GROUPED_TCGEN05", tcgen05)
     test_routed_experts(ops, "bfloat16", E, top, 64, 136, T)
 

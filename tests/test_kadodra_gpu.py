@@ -461,7 +461,7 @@ def test_attention_over_plain_rows_of_whole_prompts(ops, H, G, D, V, rest, windo
 @pytest.mark.parametrize("E,top,ff,W,T,limit", [(5, 1, 24, 40, 70, 0.4), (7, 3, 64, 128, 130, 0.8), (3, 3, 10, 52, 9, 0.2),
                                                 (1, 1, 16, 64, 3, 1.0), (16, 2, 64, 128, 600, 0.5), (70, 4, 128, 64, 700, 0.6)])
 def test_experts_chosen_by_a_table(ops, dtype, E, top, ff, W, T, limit):
-    """Every kernel of the routed products (FMA, mma.sync, tcgen05 from 1,024 pairs) behind the table, with gates and ups
+    """Every kernel of the routed products (FMA, mma.sync, tcgen05 from 24 pairs an expert) behind the table, with gates and ups
     beyond the limit on both sides, token ids that repeat (one expert gets most rows) and experts nobody chooses."""
     from tffinfer_b200.parts.moe import RoutedExperts
     dev, dt = "cuda", getattr(torch, dtype)

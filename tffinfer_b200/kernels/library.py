@@ -1365,7 +1365,7 @@ class CudaKernels:
         # both products run on the same kernel (one tile table): the tensor-core one if both can
         tc = (self.grouped_on_tensor_cores(h, w_gate_up, W, W, 0, W, up_rows * W, "" if plain else layout, ff)
               and self.grouped_on_tensor_cores(h, w_down, ff, ff, 0, ff, W * ff, "", W))
-        if tc and self.GROUPED_TCGEN05 and P >= self.grouped_tcgen05_from(E, by_table) and W % 4 == 0 and ff % 8 == 0:
+        if tc and self.GROUPED_TCGEN05 and P >= self.grouped_tcgen05_from(E) and W % 4 == 0 and ff % 8 == 0:
             # Prompt-sized: the tcgen05 product in its grouped form.  Every expert's rows are padded to whole tiles of 128
             # in the sorted order, both products write in that order, and the sum gathers a token's rows from it.
             rows = -(-(P + E * 127) // 128) * 128
@@ -1386,7 +1386,10 @@ class CudaKernels:
                              identity=(pe[0], pair_weight, h) if pe else None, shared=shared)
             return
         a_rows = None
-        tile_rows = self.grouped_tile_rows(tc, P <= 12 * E)      # few pairs an expert on average: tiles of few rows
+        # few pairs an expert on average: tiles of few rows.  The products of a layer that the tcgen05 kernel does not take, tiles of 32
+        # and of 128 rows: 16 experts of 3,072 x 2,048 with 64 pairs each 240 and 270 us, with 80 282 and 274; 64 of 768 x 2,048 271 and 292, 323
+        # and 301.
+        tile_rows = self.grouped_tile_rows(tc, P <= 64 * E)
         if by_table:             # the product reads the tokens' rows where they are
             pair_weight, row_map, tiles, a_rows = self.moe_table(router, T, top, E, tile_rows)
             x, pe = h, []
@@ -1405,20 +1408,20 @@ class CudaKernels:
                          identity=(pe[0], pair_weight, h) if pe else None, shared=shared)
 
     GROUPED_TCGEN05 = os.environ.get("TFFINFER_GROUPED_TCGEN05", "1") != "0"
-    GROUPED_TCGEN05_FROM = 1024      # (token, expert) pairs of a step from which the experts run on the tcgen05 product, or fewer:
-    GROUPED_TCGEN05_EACH = {False: 8, True: 12}      # where an expert has more than these on average, by whether there are many of them
+    GROUPED_TCGEN05_EACH = {False: 8, True: 24}      # most pairs an expert has on average on mma.sync, by whether there are more than 8
 
     @classmethod
-    def grouped_tcgen05_from(cls, E: int, by_table: bool) -> int:
-        """From how many pairs of a step E experts run on the tcgen05 product (us, mma.sync and tcgen05; the former on tiles of 16
-        rows, which have 32 since and are a tenth faster at 8 pairs an expert).  Above 12 an expert the
-        other one leaves its tiles of few rows: 4 experts of 3,072 x 2,048 with 64 pairs 159 and 70, 16 with 256 263 and 135, 64 of
-        768 x 2,048 with 1,026 268 and 168, 64 of 1,536 x 4,096 with 1,024 875 and 536; chosen by a table 145 and 61, 253 and 127,
-        248 and 151, 843 and 503.  With 9 to 12 an expert that is so for few experts chosen in groups, which have uneven shares: a layer
-        of 16 experts of 3,072 x 2,048 (6,144 x 4,096) and a shared one with 160 pairs 178 and 167 (521 and 505), 192 186 and 167
-        (573 and 507), 128 159 and 161 (499 and 501).  Many experts, or even shares, are faster on tiles of few rows: 64 with 576
-        139 and 166 (456 and 537), chosen by a table 123 and 151 (427 and 509), 16 chosen by a table with 144 122 and 132."""
-        return min(cls.GROUPED_TCGEN05_FROM, cls.GROUPED_TCGEN05_EACH[E > 16 or by_table] * E + 1)
+    def grouped_tcgen05_from(cls, E: int) -> int:
+        """From how many pairs of a step E experts run on the tcgen05 product (us a layer, mma.sync on tiles of 32 rows and tcgen05).  Tiles
+        of 32 rows read an expert's weights once up to about 32 pairs, twice from there on.  More than 8 experts: 16 of 3,072 x 2,048
+        with 8 pairs each 120 and 133, 24 125 and 160, 32 163 and 161, 40 201 and 160; of 1,024 x 2,048 56 and 66, 62 and 83, 86 and 85, 92 and 89;
+        64 of 768 x 2,048 129 and 165, 150 and 172, 178 and 176, 217 and 186; 64 of 1,536 x 4,096 416 and 531, 448 and 546, 546 and 567, 675 and 566;
+        chosen by a table 64 of 768 x 2,048 115 and 149, 126 and 151, 150 and 154, 188 and 158.  Chosen in groups, which have uneven shares,
+        16 of 3,072 x 2,048 beside a shared one (6,144 x 4,096) with 10 144 and 156 (476 and 491), 20 186 and 191 (490 and 557), 24 193 and 193
+        (571 and 560), 32 203 and 197 (642 and 550).  Few experts have too few tiles of 128 weight rows to fill the SMs twice: 4 of
+        3,072 x 2,048 with 8 and 24 pairs each 74 and 61, 73 and 63 (6,144 x 4,096 165 and 170, 164 and 168), 8 of them 94 and 82, 95 and 100 (215 and
+        256, 218 and 273), from 10 experts on 94 and 105, 96 and 105."""
+        return cls.GROUPED_TCGEN05_EACH[E > 8] * E + 1
 
     def gemm_tc_grouped(self, a, w, out, groups: int, group_rows: int, K: int, lane_group, gated: bool = False,
                         activation: str = "silu", limit: float = 0.0) -> None:
