@@ -192,7 +192,7 @@ struct PrefillCfg {
     static_assert(kSmem <= 227 * 1024, "shared memory of the prompt attention kernel");
 };
 
-// QT: query tiles per CTA.  Two when that still gives every SM a CTA, one otherwise.
+// QT: query tiles per CTA.  One while single tiles all run at once, two as soon as they are more than the SMs (launch_prefill_tiles).
 // DK, DV: elements of a key and of a value (DENSE: rounded up; the query's columns beyond its own are zeros, the output's
 // are not stored).  tm_cache is the cache, or the keys' rows when DENSE; tm_v and tm_r are read by the dense form only.
 template <int DK, int DV, int QT, bool DENSE>
@@ -242,7 +242,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     const int kvh = blockIdx.x;
     const int pair = (int)gridDim.y - 1 - (int)blockIdx.y;
     const int G = p.nq / p.nkv;
-    const int ps = DENSE ? 0 : 1 << p.page_shift;
 
     if (tid == 0) {
         for (int s = 0; s < NSTAGES; ++s) { mbar_init(kv_full(s), 1); if (APART) mbar_init(v_full(s), 1); }

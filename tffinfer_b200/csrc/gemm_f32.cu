@@ -14,9 +14,10 @@
 // them in the same order): its value does not depend on what else is in the batch.  An element whose result is not
 // finite is computed once more as a plain sum of products, since a split of an infinity has no meaning.
 //
-// What bounds it.  Few rows: 128 weight rows x 64 of K (32 KB) a CTA in 0.6 to 0.7 us where the memory would give them in 0.74: the walk
-// through registers to tensor memory just keeps up (4 rows of the 8B shape's gate/up product, 403 MB: 80 us = 5 TB/s, down 54; with the
-// weights' loads in registers and their terms in shared memory 87 and 58).  Many rows: the six products, 1,152 clocks a K block of 96 rows
+// What bounds it.  Few rows: 128 weight rows x 64 of K (32 KB) take a CTA 0.87 us where the memory would give them in 0.74, so the walk
+// through registers to tensor memory does not quite keep up, and some 5 us go to the start, the last units and the sum of the
+// chunks (4 rows, weights beyond the L2: 12,288 x 2,048 in 23 us, the 8B shape's gate/up product, 403 MB, in 77 = 5.2 TB/s, its down product in
+// 55; with the weights' loads in registers and their terms in shared memory 87 and 58).  Many rows: the six products, 1,152 clocks a K block of 96 rows
 // at their own rate and about 1,900 here, of which some 150 are the issuing warp's wait and the rest the warps that split beside it
 // (536 rows of q/k/v 134 us, of the output projection 107, against 222 and 200 before: both operands' terms then went through shared memory,
 // 96 KB written and 160 KB read a K block of 128 rows, two stages of them).  So the weights' terms are the A operand in
@@ -689,8 +690,10 @@ int chunk_count(int K) {
 
 // Tile width and whether the K range is shared out, from M, N, K and the SM count.  A K block of a tile takes about the
 // clocks below (128 weight rows split, their products with bn activation rows: fitted to 130 times of the products of the 8B shape at 4 to
-// 1,000 rows; the pick was within 8 % of the best of them from K = 4,096 on), with 5,000 for the kernel that makes the activations' terms;
-// tiles run in rounds of one a SM.
+// 1,000 rows), with 5,000 for the kernel that makes the activations' terms; tiles run in rounds of one a SM.  Over the four products of a
+// layer at 17 row counts from 1 to 1,000 the pick takes longer than the best of all plans by nothing to 0.5 % at widths of 2,560 and
+// 4,096, by 0.6 % on average and 10 % at most at 2,048 (65 rows of 12,288 x 2,048), by 0.8 % and 12 % at 1,024 (65 to 100 rows of
+// 4,096 x 1,024).
 F32Plan f32_plan(int M, int N, int K) {
     const int sms = tff_num_sms() > 0 ? tff_num_sms() : 148;
     const int kbt = (K + BK - 1) / BK, chunks = chunk_count(K);

@@ -201,7 +201,7 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_g
 
 // A and B bfloat16.  gated != 0: B's N rows are gate and up rows alternating in blocks of 64 and C has N / 2 columns.
 // c_dt 0 = float32, 1 = bfloat16.  ``a_rows`` (ragged form; null: A is in the sorted order), ``act``, ``limit`` and ``slope``
-// as for tff_gemm_grouped.  tile_rows: 128, or 16 for steps of few rows a group.  The ragged form's tiles must have been planned with it.
+// as for tff_gemm_grouped.  tile_rows: 128, or 32 for steps of few rows a group.  The ragged form's tiles must have been planned with it.
 TFF_API int tff_gemm_grouped_mma(
     const void* A, long long lda, long long a_gs, const void* B, long long ldb, long long b_gs,
     void* C, int c_dt, long long ldc, long long c_gs,

@@ -143,56 +143,52 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_lane,   // operand whose r
                 tma_load_2d(base + i * Cfg::kStageBytes + x_off, tm_x, full_bar(i), pre_k[i], pre_xrow[i]);
             first = pre;
         }
-        {
-            const uint32_t pre = __shfl_sync(0xffffffffu, first, 0);
-            pdl_wait();                              // every lane reads the table below, and any may be the one elected to load
-            SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
-            uint32_t n = 0;
-            bool ok = true;
-            while (ok && it.next()) {
-                int goff = 0;
-                if (grouped) { const int g = __ldcg(lane_group + it.tile % n_lane_tiles); if (g < 0) continue; goff = g * group_rows; }
-                const int lrow = (it.tile % n_lane_tiles) * BM, crow = (it.tile / n_lane_tiles) * BN + goff;
-                for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
-                    if (n < pre) continue;                           // already requested above
-                    const int s = n % STAGES;
-                    const uint32_t round = n / STAGES;
-                    if (!mbar_wait_warp(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
-                    const uint32_t a_dst = base + s * Cfg::kStageBytes;
-                    mbar_expect_tx_elected(full_bar(s), Cfg::kStageBytes);
-                    tma_load_2d_elected(a_dst, &tm_lane, full_bar(s), kb * BK, lrow);
-                    tma_load_2d_elected(a_dst + BM * BK * 2, &tm_col, full_bar(s), kb * BK, crow);
-                }
+        const uint32_t pre = __shfl_sync(0xffffffffu, first, 0);
+        pdl_wait();                              // every lane reads the table below, and any may be the one elected to load
+        SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
+        uint32_t n = 0;
+        bool ok = true;
+        while (ok && it.next()) {
+            int goff = 0;
+            if (grouped) { const int g = __ldcg(lane_group + it.tile % n_lane_tiles); if (g < 0) continue; goff = g * group_rows; }
+            const int lrow = (it.tile % n_lane_tiles) * BM, crow = (it.tile / n_lane_tiles) * BN + goff;
+            for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
+                if (n < pre) continue;                           // already requested above
+                const int s = n % STAGES;
+                const uint32_t round = n / STAGES;
+                if (!mbar_wait_warp(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
+                const uint32_t a_dst = base + s * Cfg::kStageBytes;
+                mbar_expect_tx_elected(full_bar(s), Cfg::kStageBytes);
+                tma_load_2d_elected(a_dst, &tm_lane, full_bar(s), kb * BK, lrow);
+                tma_load_2d_elected(a_dst + BM * BK * 2, &tm_col, full_bar(s), kb * BK, crow);
             }
         }
     } else if (warp == 1) {
-        {
-            // -------------------------------------------------------- MMA issuer
-            constexpr uint32_t idesc = make_idesc(BM, BN);
-            SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
-            uint32_t n = 0, seg = 0;
-            bool ok = true;
-            if (grouped) pdl_wait();
-            while (ok && it.next()) {
-                if (grouped && __ldcg(lane_group + it.tile % n_lane_tiles) < 0) continue;
-                const uint32_t acc = seg & 1, use = seg >> 1;
-                if (use > 0 && !mbar_wait_warp(tempty_bar(acc), (use - 1) & 1, abort_flag)) break;   // epilogue has drained it
+        // -------------------------------------------------------- MMA issuer
+        constexpr uint32_t idesc = make_idesc(BM, BN);
+        SegIter it(n_tiles, kbt, stream_k, blockIdx.x, gridDim.x);
+        uint32_t n = 0, seg = 0;
+        bool ok = true;
+        if (grouped) pdl_wait();
+        while (ok && it.next()) {
+            if (grouped && __ldcg(lane_group + it.tile % n_lane_tiles) < 0) continue;
+            const uint32_t acc = seg & 1, use = seg >> 1;
+            if (use > 0 && !mbar_wait_warp(tempty_bar(acc), (use - 1) & 1, abort_flag)) break;   // epilogue has drained it
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + acc * Cfg::kAccCols;
+            for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
+                const int s = n % STAGES;
+                const uint32_t round = n / STAGES;
+                if (!mbar_wait_warp(full_bar(s), round & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * Cfg::kAccCols;
-                for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
-                    const int s = n % STAGES;
-                    const uint32_t round = n / STAGES;
-                    if (!mbar_wait_warp(full_bar(s), round & 1, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a_addr = base + s * Cfg::kStageBytes;
-                    const uint64_t adesc = make_smem_desc(a_addr);
-                    const uint64_t bdesc = make_smem_desc(a_addr + BM * BK * 2);
-                    umma4_bf16_elected(d_tmem, adesc, bdesc, idesc, kb > it.kb0 ? 1u : 0u);
-                    umma_commit_elected(empty_bar(s));          // the stage is free once these MMAs have read it
-                }
-                if (ok) umma_commit_elected(tfull_bar(acc));    // this segment's accumulators are complete
-                ++seg;
+                const uint32_t a_addr = base + s * Cfg::kStageBytes;
+                const uint64_t adesc = make_smem_desc(a_addr);
+                const uint64_t bdesc = make_smem_desc(a_addr + BM * BK * 2);
+                umma4_bf16_elected(d_tmem, adesc, bdesc, idesc, kb > it.kb0 ? 1u : 0u);
+                umma_commit_elected(empty_bar(s));          // the stage is free once these MMAs have read it
             }
+            if (ok) umma_commit_elected(tfull_bar(acc));    // this segment's accumulators are complete
+            ++seg;
         }
     } else {
         // ------------------------------------------------------------ epilogue

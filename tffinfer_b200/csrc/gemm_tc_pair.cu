@@ -147,25 +147,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a,     // activations
     pdl_launch_dependents();
 
     if (warp == 0) {
-        {
-            // ------------------------------------------------------ TMA producer (both CTAs)
-            pdl_wait();
-            SegIterSlices it(n_tiles, kbt, stream_k, cluster_id, n_clusters);
-            uint32_t n = 0;
-            bool ok = true;
-            while (ok && it.next()) {
-                const int arow = ((it.tile % n_m_pairs) * 2 + (int)rank) * BM;
-                const int wrow = (it.tile / n_m_pairs) * PBN + (int)rank * HALF_N;
-                for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
-                    const int s = n % STAGES;
-                    const uint32_t round = n / STAGES;
-                    if (round > 0 && !mbar_wait_warp(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
-                    const uint32_t first_full = map_to_cta(full_bar(s), 0);
-                    if (rank == 0) mbar_expect_tx_elected(full_bar(s), 2 * P_STAGE_BYTES);     // both CTAs' tiles of the stage
-                    const uint32_t a_dst = base + s * P_STAGE_BYTES;
-                    tma_load_2d_pair(a_dst, &tm_a, first_full, kb * BK, arow);
-                    tma_load_2d_pair(a_dst + BM * BK * 2, &tm_w, first_full, kb * BK, wrow);
-                }
+        // ------------------------------------------------------ TMA producer (both CTAs)
+        pdl_wait();
+        SegIterSlices it(n_tiles, kbt, stream_k, cluster_id, n_clusters);
+        uint32_t n = 0;
+        bool ok = true;
+        while (ok && it.next()) {
+            const int arow = ((it.tile % n_m_pairs) * 2 + (int)rank) * BM;
+            const int wrow = (it.tile / n_m_pairs) * PBN + (int)rank * HALF_N;
+            for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
+                const int s = n % STAGES;
+                const uint32_t round = n / STAGES;
+                if (round > 0 && !mbar_wait_warp(empty_bar(s), (round - 1) & 1, abort_flag)) { ok = false; break; }
+                const uint32_t first_full = map_to_cta(full_bar(s), 0);
+                if (rank == 0) mbar_expect_tx_elected(full_bar(s), 2 * P_STAGE_BYTES);     // both CTAs' tiles of the stage
+                const uint32_t a_dst = base + s * P_STAGE_BYTES;
+                tma_load_2d_pair(a_dst, &tm_a, first_full, kb * BK, arow);
+                tma_load_2d_pair(a_dst + BM * BK * 2, &tm_w, first_full, kb * BK, wrow);
             }
         }
     } else if (warp == 1) {

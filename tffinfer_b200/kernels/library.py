@@ -1737,7 +1737,8 @@ class CudaKernels:
         A step of whole prompts (every request starts at position 0, bfloat16, aligned sizes) takes the other form: the
         step's latents are also kept in plain rows (``shared``, a dict that lives for the step, hands them to the layers
         that read this layer's cache), per-head keys [W_uk c | r] and values W_uv c of the step's tokens are made by
-        grouped products (``w_uk`` [heads*dim, kv_rank]), and attention runs with keys of dim + rot_dim and values of
+        one product each on the tensor cores (gemm_tc_rows; ``w_uk`` [heads*dim, kv_rank]; grouped products a head where that
+        does not take them or the rotated part lies in the keys' rows), and attention runs with keys of dim + rot_dim and values of
         vdim elements: a fifth of the absorbed form's arithmetic at the sizes of a large model.  The cache is written
         either way."""
         if isinstance(h, DeferredNorm):
