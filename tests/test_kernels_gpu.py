@@ -840,15 +840,40 @@ def test_prompt_attention_of_every_number_of_key_blocks(ops, nq, nkv, d, page, w
     ops.check_errors()
 
 
+@pytest.mark.parametrize("nq,nkv,d,page,lens,old,window", [
+    (4, 2, 128, 16, [17] * 11 + [600] + [18] * 8, 0, 0),                       # one tile a CTA, the requests' CTAs one behind the other
+    (4, 2, 64, 8, [700] + [17 + i % 9 for i in range(31)], 37, 0),             # 32 requests and, below, 33: a whole scan and one more
+    (10, 2, 128, 64, [17 + i % 9 for i in range(32)] + [400], 0, 90),
+    (8, 4, 128, 16, [18] * 127 + [900] + [19] * 2, 0, 0),                      # more than 128: a second turn; two tiles a CTA
+    (8, 4, 64, 32, [300] + [25] * 139 + [280, 1, 41], 70, 100),                # long ones at both ends, beside a decoded token
+    (16, 8, 128, 16, [33] * 64, 0, 0),                                         # no request has two tiles
+])
+def test_prompt_attention_of_requests_of_uneven_length(ops, nq, nkv, d, page, lens, old, window):
+    """Grids that hold the requests' CTAs one behind the other and not a row of the longest one's number for each."""
+    starts = [old + i % 3 if old else 0 for i in range(len(lens))]
+    entries, tables, cache, qkv = _paged_case(nq, nkv, d, page, lens, starts, window, torch.bfloat16, seed=71, layers=1)
+    q = qkv[:, :nq * d].contiguous()
+    bc = build_step_batch(entries, starts, list(range(len(lens))), [tables], "cpu")
+    bg = build_step_batch(entries, starts, list(range(len(lens))), [tables], DEV)
+    want, out = torch.empty(q.shape[0], nq * d, dtype=torch.bfloat16), torch.full(q.shape, float("nan"), dtype=torch.bfloat16, device=DEV)
+    CpuOps().attention(q, bc, bc.block_tables[0], cache, 0, page, want, nq, nkv, d, 1 / math.sqrt(d), window)
+    ops.attention_bf16(q.to(DEV), bg, bg.block_tables[0], cache.to(DEV), 0, page, out, nq, nkv, d, 1 / math.sqrt(d), window)
+    assert torch.isfinite(out).all()
+    assert rel_err(out, want) < 1e-2
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("d,dv,rest", [(192, 128, 64), (192, 128, 0), (136, 72, 8)])
 @pytest.mark.parametrize("window", [0, 90, 200])
-@pytest.mark.parametrize("requests", [1, 24])
+@pytest.mark.parametrize("requests", [1, 24, 41])
 def test_prompt_attention_over_plain_rows_of_every_number_of_key_blocks(ops, d, dv, rest, window, requests):
     """Keys of more than 128 elements, whose stages give keys and values back apart: walks of 1 to 11 blocks, by ones, round rings of 4
-    stages (one tile a CTA) and of 3 (two, where the tiles are more than the SMs; the second may hold no rows)."""
+    stages (one tile a CTA) and of 3 (two, where the tiles are more than the SMs; the second may hold no rows); 41: one long among short."""
     H, kh = 4, d - rest
     for first in range(11 if requests == 1 else 2):
         lens = [64 * ((first + i) % 11) + 1 + (37 * (first + i)) % 64 for i in range(requests)]
+        if requests == 41:
+            lens = [650 if i == 17 else 9 + (i + first) % 30 for i in range(requests)]
         T = sum(lens)
         q, k, v = (g((T, H * n), torch.bfloat16, 31 + first + n).to(DEV) for n in (d, kh, dv))
         r = g((T, 16 + rest), torch.bfloat16, 32).to(DEV) if rest else None

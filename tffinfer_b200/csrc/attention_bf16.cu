@@ -463,7 +463,7 @@ static int attention_bf16_impl(
                                          max_q_len, num_splits, nq, nkv, d, scale, window, extra, stream, beside);
     if (!keys_mode && num_splits == 1 && cache_pages > 0)   // portions: tcgen05 kernel (attention_prefill.cu)
         st = tff_attention_prefill_launch(q, q_start, pos_start, req_ids, block_table, table_width, cache, cache_pages,
-                                          cache_layers, layer, page_size, out, num_requests, max_q_len, nq, nkv, d,
+                                          cache_layers, layer, page_size, out, num_tokens, num_requests, max_q_len, nq, nkv, d,
                                           scale, window, extra, stream);
     if (st == TFF_ERR_UNSUPPORTED) {
         if (d == 128) st = keys_mode ? launch_attn<128, true>(p, q_tiles, num_requests, stream)
@@ -538,7 +538,7 @@ TFF_API int tff_attention_bf16_mixed(
     if (cache_pages <= 0 || num_requests > 65535 || nkv > 65535) return TFF_ERR_UNSUPPORTED;
     const AttnExtra extra{softcap, sink, gate, sink_val, keep};
     const int st = tff_attention_prefill_launch(q, q_start, pos_start, req_order + num_short, block_table, table_width, cache, cache_pages,
-                                                cache_layers, layer, page_size, out, num_requests - num_short, max_q_len, nq, nkv, d,
+                                                cache_layers, layer, page_size, out, num_tokens, num_requests - num_short, max_q_len, nq, nkv, d,
                                                 scale, window, extra, stream, true);
     if (st != TFF_OK) return st;
     return attention_bf16_impl(q, q_start, pos_start, req_order, block_table, table_width, cache, cache_pages, cache_layers, layer,

@@ -64,5 +64,5 @@ int tff_attention_decode_launch(
 int tff_attention_prefill_launch(
     const void* q, const int* q_start, const int* pos_start, const int* req_ids, const int* block_table, int table_width,
     const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
-    void* out, int num_requests, int max_q_len, int nq, int nkv, int d, float scale, int window, AttnExtra extra,
+    void* out, int num_tokens, int num_requests, int max_q_len, int nq, int nkv, int d, float scale, int window, AttnExtra extra,
     cudaStream_t stream, bool companion = false);

@@ -161,6 +161,7 @@ __host__ __device__ constexpr uint32_t make_idesc(int m, int n, int b_mn_major) 
 
 struct PrefillParams {
     int companion;                               // the decoded tokens' kernel follows and runs beside this one
+    int requests;                                // FLAT: whose CTAs lie one behind the other in the grid
     const bf16* q; int q_row_stride;
     const int* q_start; const int* pos_start; const int* req_ids;
     const int* block_table; int table_width;
@@ -195,7 +196,8 @@ struct PrefillCfg {
 // QT: query tiles per CTA.  One while single tiles all run at once, two as soon as they are more than the SMs (launch_prefill_tiles).
 // DK, DV: elements of a key and of a value (DENSE: rounded up; the query's columns beyond its own are zeros, the output's
 // are not stored).  tm_cache is the cache, or the keys' rows when DENSE; tm_v and tm_r are read by the dense form only.
-template <int DK, int DV, int QT, bool DENSE>
+// FLAT: the requests' CTAs lie one behind the other in the grid's y (launch_prefill), else z is the request.
+template <int DK, int DV, int QT, bool DENSE, bool FLAT>
 __global__ void __launch_bounds__(PrefillCfg<DK, DV, QT>::kThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __grid_constant__ CUtensorMap tm_v,
                        const __grid_constant__ CUtensorMap tm_r, const PrefillParams p) {
@@ -240,7 +242,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     // CTAs are handed out in the order x, y, z: all kv heads of the last rows (which see the most keys)
     // first, the shortest walks last, so that the SMs finish together
     const int kvh = blockIdx.x;
-    const int pair = (int)gridDim.y - 1 - (int)blockIdx.y;
     const int G = p.nq / p.nkv;
 
     if (tid == 0) {
@@ -271,7 +272,42 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     }
 
     // request geometry (q_start and pos_start come with the step's batch, read after the dependency wait all the same)
-    const int b = p.req_ids ? p.req_ids[blockIdx.z] : (int)blockIdx.z;
+    int at = blockIdx.z, pair = (int)gridDim.y - 1 - (int)blockIdx.y;      // request and CTA of it
+    if constexpr (FLAT) {
+        // every warp looks for the CTA's request by itself: the tiles of 128 requests a turn, 32 in a scan
+        int left = blockIdx.y;
+        at = -1;
+        for (int r0 = 0; r0 < p.requests && at < 0; r0 += 128) {
+            int n[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int r = r0 + u * 32 + lane;
+                n[u] = 0;
+                if (r < p.requests) {
+                    const int* start = p.q_start + (p.req_ids ? p.req_ids[r] : r);
+                    n[u] = ((start[1] - start[0]) * G + QT * BLOCK_M - 1) / (QT * BLOCK_M);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                int sum = n[u];
+#pragma unroll
+                for (int o = 1; o < 32; o *= 2) {
+                    const int before = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += before;
+                }
+                const unsigned behind = __ballot_sync(0xffffffffu, left < sum);
+                if (behind && at < 0) {
+                    const int src = __ffs(behind) - 1;
+                    at = r0 + u * 32 + src;
+                    pair = __shfl_sync(0xffffffffu, sum, src) - 1 - left;  // the request's last rows first, as in a grid row of its own
+                }
+                left -= __shfl_sync(0xffffffffu, sum, 31);
+            }
+        }
+        if (at < 0) { at = 0; pair = 1 << 20; }                    // the grid holds a CTA a request more than there may be tiles: no rows
+    }
+    const int b = p.req_ids ? p.req_ids[at] : at;
     const int q0 = p.q_start[b];
     const int q_len = p.q_start[b + 1] - q0;
     const int rows_total = q_len * G;
@@ -648,32 +684,48 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     }
 }
 
-template <int DK, int DV, int QT, bool DENSE>
-int launch_prefill(const CUtensorMap& tm, const CUtensorMap& tv, const CUtensorMap& tr, const PrefillParams& p, int q_tiles,
-                   int B, cudaStream_t stream) {
+template <int DK, int DV, int QT, bool DENSE, bool FLAT>
+int launch_prefill(const CUtensorMap& tm, const CUtensorMap& tv, const CUtensorMap& tr, const PrefillParams& p, const dim3 grid,
+                   cudaStream_t stream) {
     constexpr int NTHREADS = PrefillCfg<DK, DV, QT>::kThreads;
     constexpr int smem = PrefillCfg<DK, DV, QT>::kSmem;
-    auto kern = attn_prefill_tc_kernel<DK, DV, QT, DENSE>;
+    auto kern = attn_prefill_tc_kernel<DK, DV, QT, DENSE, FLAT>;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return TFF_ERR_LAUNCH;
         configured = true;
     }
-    return tff_launch_pdl(kern, dim3(p.nkv, q_tiles, B), dim3(NTHREADS), (size_t)smem, stream, tm, tv, tr, p);
+    return tff_launch_pdl(kern, grid, dim3(NTHREADS), (size_t)smem, stream, tm, tv, tr, p);
+}
+
+// The grid has a row of CTAs for every request, as many as the longest one has, or, where the step's tokens need less than three quarters
+// of those, the requests' CTAs one behind the other.  A CTA without rows takes an SM for 2.6 us, one that looks for its request half a
+// microsecond more: 200 prompts of 18 tokens and one of 1,000 (32/8 heads) 447 us with a row each, 127 so, 64 prompts of which one has
+// 4,096 tokens and the others 20 615 and 168.
+template <int DK, int DV, int QT, bool DENSE>
+int launch_prefill_grid(const CUtensorMap& tm, const CUtensorMap& tv, const CUtensorMap& tr, PrefillParams p, int tiles, int num_tokens,
+                        int B, cudaStream_t stream) {
+    const int rows = (tiles + QT - 1) / QT;
+    const long long most = (long long)num_tokens * (p.nq / p.nkv) / (QT * BLOCK_M) + B;     // every request may have a CTA that is not full
+    p.requests = B;
+    if (most * 4 <= (long long)rows * B * 3 && most <= 65535)
+        return launch_prefill<DK, DV, QT, DENSE, true>(tm, tv, tr, p, dim3(p.nkv, (unsigned)most, 1), stream);
+    return launch_prefill<DK, DV, QT, DENSE, false>(tm, tv, tr, p, dim3(p.nkv, rows, B), stream);
 }
 
 // Two query tiles a CTA share one walk over the keys: a block takes 1,590 cycles for a pair of tiles, 1,050 for a single one.  So
 // single tiles while they all run at once, one an SM; as soon as they would not, pairs, which get through 1.3 times as many
-// tiles in the same time.
+// tiles in the same time.  Where no request has more than one tile a pair would have one too, and twice the warps to start.
 template <int DK, int DV, bool DENSE>
 int launch_prefill_tiles(const CUtensorMap& tm, const CUtensorMap& tv, const CUtensorMap& tr, const PrefillParams& p,
-                         int max_q_len, int B, cudaStream_t stream) {
+                         int max_q_len, int num_tokens, int B, cudaStream_t stream) {
     const int tiles = (max_q_len * (p.nq / p.nkv) + BLOCK_M - 1) / BLOCK_M;
     const long long sms = tff_num_sms() > 0 ? tff_num_sms() : 1;
-    if ((long long)tiles * p.nkv * B > sms)
-        return launch_prefill<DK, DV, 2, DENSE>(tm, tv, tr, p, (tiles + 1) / 2, B, stream);
-    return launch_prefill<DK, DV, 1, DENSE>(tm, tv, tr, p, tiles, B, stream);
+    const long long most = (long long)num_tokens * (p.nq / p.nkv) / BLOCK_M + B, all = (long long)tiles * B;
+    if (tiles > 1 && (most < all ? most : all) * p.nkv > sms)
+        return launch_prefill_grid<DK, DV, 2, DENSE>(tm, tv, tr, p, tiles, num_tokens, B, stream);
+    return launch_prefill_grid<DK, DV, 1, DENSE>(tm, tv, tr, p, tiles, num_tokens, B, stream);
 }
 
 }  // namespace
@@ -683,7 +735,7 @@ int launch_prefill_tiles(const CUtensorMap& tm, const CUtensorMap& tv, const CUt
 int tff_attention_prefill_launch(
     const void* q, const int* q_start, const int* pos_start, const int* req_ids, const int* block_table, int table_width,
     const void* cache, long long cache_pages, int cache_layers, int layer, int page_size,
-    void* out, int num_requests, int max_q_len, int nq, int nkv, int d, float scale, int window, AttnExtra extra,
+    void* out, int num_tokens, int num_requests, int max_q_len, int nq, int nkv, int d, float scale, int window, AttnExtra extra,
     cudaStream_t stream, bool companion) {
     if (d != 64 && d != 128) return TFF_ERR_UNSUPPORTED;
     if (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64) return TFF_ERR_UNSUPPORTED;
@@ -709,8 +761,8 @@ int tff_attention_prefill_launch(
     if (p.error_flag == nullptr) return TFF_ERR_LAUNCH;
     p.d = p.dv = d; p.k_halves = p.k_head = p.r_col = 0;
     p.companion = companion ? 1 : 0;
-    return d == 128 ? launch_prefill_tiles<128, 128, false>(tm, tm, tm, p, max_q_len, num_requests, stream)
-                    : launch_prefill_tiles<64, 64, false>(tm, tm, tm, p, max_q_len, num_requests, stream);
+    return d == 128 ? launch_prefill_tiles<128, 128, false>(tm, tm, tm, p, max_q_len, num_tokens, num_requests, stream)
+                    : launch_prefill_tiles<64, 64, false>(tm, tm, tm, p, max_q_len, num_tokens, num_requests, stream);
 }
 
 // The dense form: every request of the step starts at position 0, and the keys and values of its tokens are the rows
@@ -750,8 +802,8 @@ TFF_API int tff_attention_dense(const void* q, const int* q_start, const int* po
     if (p.error_flag == nullptr) return TFF_ERR_LAUNCH;
     if (d > 128) {
         p.k_halves = shared ? k_head / 64 : 3;
-        return launch_prefill_tiles<192, 128, true>(tk, tv, tr, p, max_q_len, num_requests, stream);
+        return launch_prefill_tiles<192, 128, true>(tk, tv, tr, p, max_q_len, num_tokens, num_requests, stream);
     }
     p.k_halves = shared ? k_head / 64 : 2;
-    return launch_prefill_tiles<128, 128, true>(tk, tv, tr, p, max_q_len, num_requests, stream);
+    return launch_prefill_tiles<128, 128, true>(tk, tv, tr, p, max_q_len, num_tokens, num_requests, stream);
 }
