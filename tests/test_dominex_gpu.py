@@ -483,6 +483,14 @@ def test_grouped_product_of_few_rows_at_the_edges_of_its_tiles(ops, N, K):
     assert float((first[:40].double() - want).abs().max() / want.abs().max()) < 1e-5
 
 
+@pytest.mark.parametrize("few", [1, 2])
+@pytest.mark.parametrize("N,K", [(128, 64), (200, 1032)])
+def test_grouped_product_on_either_of_its_tiles_of_few_rows(ops, monkeypatch, N, K, few):
+    """Tiles of 32 and of 16 rows, whichever the size of the weights would choose."""
+    monkeypatch.setattr(type(ops), "grouped_few_rows", staticmethod(lambda M, weights: few if M <= 32 else 0))
+    test_grouped_product_of_few_rows_at_the_edges_of_its_tiles(ops, N, K)
+
+
 # ------------------------------------------------------------------------------ generation through the engine
 @pytest.mark.parametrize("dtype,name", [("float32", "a"), ("float32", "b"), ("bfloat16", "a")])
 def test_greedy_generation_through_the_engine(dtype, name):

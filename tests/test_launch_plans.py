@@ -163,3 +163,9 @@ def test_experts_change_their_product_by_pairs_an_expert():
     """Above 8 pairs an expert of up to 8, above 24 of more, whatever the number of pairs and whoever chose them."""
     start = CudaKernels.grouped_tcgen05_from
     assert [start(E) for E in (1, 4, 8, 9, 16, 17, 64, 128)] == [9, 33, 65, 217, 385, 409, 1537, 3073]
+
+
+def test_grouped_products_take_the_smallest_tiles_that_hold_a_group():
+    few = CudaKernels.grouped_few_rows
+    assert [few(M, 1 << 23) for M in (1, 16, 17, 32, 33)] == [2, 2, 1, 1, 0]
+    assert [few(M, 1 << 22) for M in (1, 16, 17, 32, 33)] == [2, 2, 2, 2, 0]

@@ -11,7 +11,8 @@
 // are not there, and the ring is deeper (five stages, two CTAs an SM), since such a product is a pass of the weights.
 // What bounds such a step is the weights' stream: 64 tokens on 16 experts of 3,072 x 2,048 take 71 us for the gate and up rows (403 MB, 5.7
 // TB/s) and 37 for the down rows, 87 and 50 when tiles held 16 rows (an expert with 17 rows was read twice, and the tiles of the
-// uneven experts made a fourth round of CTAs) and the second-level cache fetched less than 256 bytes of a row at a time.
+// uneven experts made a fourth round of CTAs) and the second-level cache fetched less than 256 bytes of a row at a time.  Groups of at
+// most 16 rows, and of 32 whose weights are few, take tiles of 16: half the products and fragments shorten a K block.
 // Needs K, lda, ldb and the group strides to be multiples of 8 elements and 16-byte aligned bases (the launcher
 // refuses anything else and the caller takes the FMA kernel).  A row's result does not depend on the tile it is in:
 // every output element adds its products in the same order of k.
@@ -21,9 +22,9 @@ namespace {
 
 constexpr int MBN = 128, MBK = 64, THREADS = 256;
 constexpr int CHUNKS = MBK / 8;                          // 16-byte pieces of a tile row
-constexpr int BIG_ROWS = 128, SMALL_ROWS = 32;           // rows of a tile
+constexpr int BIG_ROWS = 128, SMALL_ROWS = 32, LEAST_ROWS = 16;           // rows of a tile
 template <int BM> struct RingCfg {
-    static constexpr int kStages = BM == SMALL_ROWS ? 5 : 3;
+    static constexpr int kStages = BM == BIG_ROWS ? 3 : 5;
     static constexpr int kSmem = kStages * (BM + MBN) * MBK * 2;
 };
 
@@ -71,8 +72,8 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_g
                         const int* __restrict__ row_map, const int* __restrict__ a_rows, int M, int N, int K, int act,
                         float limit, float slope) {
     constexpr int STAGES = RingCfg<MBM>::kStages;
-    constexpr bool SMALL = MBM == SMALL_ROWS;
-    constexpr int MI = 2, NJ = SMALL ? 1 : 4;     // a warp's 16-row pieces of A and of B
+    constexpr bool SMALL = MBM != BIG_ROWS;
+    constexpr int MI = MBM == LEAST_ROWS ? 1 : 2, NJ = SMALL ? 1 : 4;     // a warp's 16-row pieces of A and of B
     constexpr int A_LOADS = (MBM * CHUNKS + THREADS - 1) / THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* As = (bf16*)smem_raw;                               // [STAGES][MBM][MBK]
@@ -201,14 +202,14 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_g
 
 // A and B bfloat16.  gated != 0: B's N rows are gate and up rows alternating in blocks of 64 and C has N / 2 columns.
 // c_dt 0 = float32, 1 = bfloat16.  ``a_rows`` (ragged form; null: A is in the sorted order), ``act``, ``limit`` and ``slope``
-// as for tff_gemm_grouped.  tile_rows: 128, or 32 for steps of few rows a group.  The ragged form's tiles must have been planned with it.
+// as for tff_gemm_grouped.  tile_rows: 128, or 32 or 16 for steps of few rows a group.  The ragged form's tiles must have been planned with it.
 TFF_API int tff_gemm_grouped_mma(
     const void* A, long long lda, long long a_gs, const void* B, long long ldb, long long b_gs,
     void* C, int c_dt, long long ldc, long long c_gs,
     const int* tile_group, const int* tile_row0, const int* tile_row_end, const int* num_tiles, int max_tiles,
     const int* row_map, const int* a_rows, int groups, int M, int N, int K, int gated, int act, float limit, float slope,
     int tile_rows, cudaStream_t stream) {
-    if (N <= 0 || K <= 0 || !A || !B || !C || (tile_rows != BIG_ROWS && tile_rows != SMALL_ROWS)) return TFF_ERR_BAD_ARGUMENT;
+    if (N <= 0 || K <= 0 || !A || !B || !C || (tile_rows != BIG_ROWS && tile_rows != SMALL_ROWS && tile_rows != LEAST_ROWS)) return TFF_ERR_BAD_ARGUMENT;
     if ((K & 7) || (lda & 7) || (ldb & 7) || (a_gs & 7) || (b_gs & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) ||
         (gated && (N & 127)))
         return TFF_ERR_UNSUPPORTED;
@@ -225,6 +226,7 @@ TFF_API int tff_gemm_grouped_mma(
     if (grid.y > 65535) return TFF_ERR_UNSUPPORTED;
 #define TFF_GM(TCc, G)                                                                                              \
     do {                                                                                                            \
+        if (tile_rows == LEAST_ROWS) TFF_GM_ROWS(TCc, G, LEAST_ROWS);                                               \
         if (tile_rows == SMALL_ROWS) TFF_GM_ROWS(TCc, G, SMALL_ROWS);                                               \
         TFF_GM_ROWS(TCc, G, BIG_ROWS);                                                                              \
     } while (0)
@@ -245,4 +247,5 @@ TFF_API int tff_gemm_grouped_mma(
     return TFF_ERR_BAD_ARGUMENT;
 }
 
-TFF_API int tff_gemm_grouped_mma_tile_rows(int few_rows) { return few_rows ? SMALL_ROWS : BIG_ROWS; }
+// Rows of a tile for groups of few rows (0: no; 1: yes; 2: of 16 at most).
+TFF_API int tff_gemm_grouped_mma_tile_rows(int few_rows) { return few_rows == 2 ? LEAST_ROWS : few_rows ? SMALL_ROWS : BIG_ROWS; }

@@ -1124,10 +1124,10 @@ class CudaKernels:
         act = _c_int(code)
         clip = (_c_float(limit), _c_float(self.CLIPPED_SLOPE))
         ll = _c_int
-        if self.grouped_on_tensor_cores(a, b, K, lda, a_gs, ldb, b_gs, gated, N) and tile_rows in (
-                0, self.grouped_tile_rows(True), self.grouped_tile_rows(True, True)):
+        if self.grouped_on_tensor_cores(a, b, K, lda, a_gs, ldb, b_gs, gated, N) and (
+                tile_rows == 0 or tile_rows in self._grouped_mma_rows):
             if not tile_rows:
-                tile_rows = self.grouped_tile_rows(True, M <= self.GROUPED_FEW_ROWS)
+                tile_rows = self._grouped_mma_rows[self.grouped_few_rows(M, groups * N * K)]
             status = self.lib.tff_gemm_grouped_mma(
                 _ptr(a), ll(lda), ll(a_gs), _ptr(b), ll(ldb), ll(b_gs), _ptr(c), _c_int(_dt(c)), ll(ldc), ll(c_gs),
                 _ptr(tg), _ptr(tr0), _ptr(tre), _ptr(nt), _c_int(max_tiles), _ptr(row_map), _ptr(a_rows), _c_int(groups), _c_int(M),
@@ -1154,14 +1154,24 @@ class CudaKernels:
                 and all(v % 8 == 0 for v in (K, lda, a_gs, ldb, b_gs)) and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0
                 and (not gated or (gated == "interleaved" and N % self.GATE_UP_BLOCK == 0)))
 
-    GROUPED_FEW_ROWS = 32    # up to this many rows a group the tensor-core kernel takes tiles of few rows
+    @staticmethod
+    def grouped_few_rows(M: int, weights: int) -> int:
+        """Which tiles of the tensor-core kernel groups of at most M rows take, whose weights are so many elements in all: 0 = 128
+        rows, 1 = 32, 2 = 16.  Of 16 where that is all there are, and for few weights, which come from the second-level cache, up to 32 rows:
+        half the products a K block (us, tiles of 16 and of 32: 32 groups of 128 x 512 at 4 rows 4.5 and 4.8, at 32 rows 5.2 and 5.8; 8 of 1,024 x
+        1,024, 17 MB, at 4 rows 7.6 and 8.0, at 24 rows 11.6 and 8.8)."""
+        if M <= 16 or (M <= 32 and weights <= 1 << 22):
+            return 2
+        return int(M <= 32)
 
-    def grouped_tile_rows(self, tensor_cores: bool, few: bool = False) -> int:
+    @functools.cached_property
+    def _grouped_mma_rows(self):
+        return [int(self.lib.tff_gemm_grouped_mma_tile_rows(_c_int(few))) for few in (0, 1, 2)]
+
+    def grouped_tile_rows(self, tensor_cores: bool, few: int = 0) -> int:
         """Rows of a tile of the grouped products: of the FMA kernel, or of the tensor-core kernel, which has tiles for
-        prompt-sized groups and for groups of ``few`` rows."""
-        if not tensor_cores:
-            return int(self.lib.tff_gemm_grouped_tile_rows())
-        return int(self.lib.tff_gemm_grouped_mma_tile_rows(_c_int(1 if few else 0)))
+        prompt-sized groups and for groups of ``few`` rows (grouped_few_rows)."""
+        return self._grouped_mma_rows[few] if tensor_cores else int(self.lib.tff_gemm_grouped_tile_rows())
 
     GATE_UP_BLOCK = 64       # rows of a block of the "interleaved" gate/up layout (gate_up_block above: the same)
 
@@ -1386,10 +1396,11 @@ class CudaKernels:
                              identity=(pe[0], pair_weight, h) if pe else None, shared=shared)
             return
         a_rows = None
-        # few pairs an expert on average: tiles of few rows.  The products of a layer that the tcgen05 kernel does not take, tiles of 32
+        # An expert has no more rows than the step has tokens; few pairs an expert on average: tiles of few rows (a layer of 2 tokens on
+        # 16 experts of 3,072 x 2,048: 83 us on tiles of 16, 89 on tiles of 32).  The products of a layer that the tcgen05 kernel does not take, tiles of 32
         # and of 128 rows: 16 experts of 3,072 x 2,048 with 64 pairs each 240 and 270 us, with 80 282 and 274; 64 of 768 x 2,048 271 and 292, 323
         # and 301.
-        tile_rows = self.grouped_tile_rows(tc, P <= 64 * E)
+        tile_rows = self.grouped_tile_rows(tc, 2 if T <= 16 else int(P <= 64 * E))
         if by_table:             # the product reads the tokens' rows where they are
             pair_weight, row_map, tiles, a_rows = self.moe_table(router, T, top, E, tile_rows)
             x, pe = h, []
