@@ -1158,8 +1158,8 @@ class CudaKernels:
     def grouped_few_rows(M: int, weights: int) -> int:
         """Which tiles of the tensor-core kernel groups of at most M rows take, whose weights are so many elements in all: 0 = 128
         rows, 1 = 32, 2 = 16.  Of 16 where that is all there are, and for few weights, which come from the second-level cache, up to 32 rows:
-        half the products a K block (us, tiles of 16 and of 32: 32 groups of 128 x 512 at 4 rows 4.5 and 4.8, at 32 rows 5.2 and 5.8; 8 of 1,024 x
-        1,024, 17 MB, at 4 rows 7.6 and 8.0, at 24 rows 11.6 and 8.8)."""
+        half the products a K block (us, tiles of 16 and of 32: 32 groups of 128 x 512 at 4 rows 4.3 and 4.8, at 32 rows 4.8 and 5.8; 8 of 1,024 x
+        1,024, 17 MB, at 4 rows 6.7 and 8.0, at 24 rows 11.6 and 8.8)."""
         if M <= 16 or (M <= 32 and weights <= 1 << 22):
             return 2
         return int(M <= 32)
@@ -1396,10 +1396,10 @@ class CudaKernels:
                              identity=(pe[0], pair_weight, h) if pe else None, shared=shared)
             return
         a_rows = None
-        # An expert has no more rows than the step has tokens; few pairs an expert on average: tiles of few rows (a layer of 2 tokens on
-        # 16 experts of 3,072 x 2,048: 83 us on tiles of 16, 89 on tiles of 32).  The products of a layer that the tcgen05 kernel does not take, tiles of 32
-        # and of 128 rows: 16 experts of 3,072 x 2,048 with 64 pairs each 240 and 270 us, with 80 282 and 274; 64 of 768 x 2,048 271 and 292, 323
-        # and 301.
+        # An expert has no more rows than the step has tokens: up to 16, tiles of 16 rows (a layer of 2 and of 8 tokens on 16 experts of
+        # 3,072 x 2,048 78 and 98 us, on tiles of 32 89 and 111); few pairs an expert on average: tiles of 32.  The products of a layer that the
+        # tcgen05 kernel does not take, tiles of 32 and of 128 rows: 16 experts of 3,072 x 2,048 with 64 pairs each 240 and 270 us, with 80
+        # 282 and 274; 64 of 768 x 2,048 271 and 292, 323 and 301.
         tile_rows = self.grouped_tile_rows(tc, 2 if T <= 16 else int(P <= 64 * E))
         if by_table:             # the product reads the tokens' rows where they are
             pair_weight, row_map, tiles, a_rows = self.moe_table(router, T, top, E, tile_rows)
